@@ -94,6 +94,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return true;
 }
 
+// The same by a whole warp, with one outcome for all of it
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long max_cycles = kMaxWaitCycles)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, max_cycles));
+}
+
+// true in one lane of a converged warp, and the compiler knows that it is one
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
+}
+
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialization attribute may
 // start while its predecessor in the stream is still running; pdl_wait() returns once that predecessor
 // has completed and its writes are visible (a no-op for a normal launch).  Everything before it may
@@ -169,6 +189,28 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs                                          = attr;
     cfg.numAttrs                                       = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// The same in clusters of `cluster` CTAs along x
+template<typename... KArgs, typename... Args>
+inline cudaError_t launch_cluster_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st, bool pdl,
+                                         Args&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = grid;
+    cfg.blockDim         = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream           = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id                                         = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x                           = cluster;
+    attr[0].val.clusterDim.y                           = 1;
+    attr[0].val.clusterDim.z                           = 1;
+    attr[1].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs                                          = attr;
+    cfg.numAttrs                                       = pdl ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -1,6 +1,7 @@
 // Dense GEMM of the config-driven decoder (gemm_dense.h): bf16 on the tcgen05 tensor core, fp32 on the CUDA cores.
 //
-// dense_tc_kernel: 128 output columns (UMMA M) x up to 256 tokens (UMMA N) per tile, persistent, one CTA per SM.
+// dense_tc_kernel: 128 output columns (UMMA M) x up to 256 tokens (UMMA N) per tile, persistent, one CTA per SM; or 256
+// columns and a pair of CTAs (cta_group::2).
 //   warp 0    one lane feeds a ring of stages with TMA: a [128 weight rows x 64 k] box and a [tokens x 64 k] box,
 //             128-byte swizzle (every CTA loads for itself); weight boxes start before the kernel ahead is complete
 //   warp 1    allocates TMEM (two accumulators, so that one tile's epilogue overlaps the next tile's products); one lane
@@ -18,6 +19,7 @@
 #include "tm_b200.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace tmb {
 namespace {
@@ -27,6 +29,12 @@ constexpr int kThreads   = 6 * 32;
 constexpr int kMaxStages = 12;
 constexpr int kMaxTokens = 256;  // tokens of one tile
 constexpr int kEpiBar    = 1;    // named barrier of the epilogue warps
+constexpr int kPairMinTokens = 64;
+// Pairs of CTAs: token tiles of a band.  74 pairs then work on 8 token tiles x 9 column tiles, which the L2 serves; measured at
+// 22016 x 4096 with 4096 / 16384 tokens: 4 tiles 530 / 2330 us, 8 tiles 509 / 2204, 16 tiles 546 / 2316.
+constexpr int kBand = 8;
+
+constexpr int kRowPitch  = 80;   // bytes between the staged rows of 64: aligned, and two rows' halves fall into other banks
 
 struct DenseShared {
     uint64_t full[kMaxStages], empty[kMaxStages];
@@ -37,12 +45,17 @@ struct DenseShared {
     int      stop;
     float    scale[kMaxTokens];
     float    red[4][kMaxTokens];
+    alignas(16) unsigned char rows[4][16 * kRowPitch];  // per epilogue warp: 16 tokens x 32 columns on their way out
 };
 // behind DenseShared, groups only: first tile of every group, [groups + 1]
 
 template<bool FAST>
 __device__ __forceinline__ float activate(const DenseEpilogue& ep, float gate, float up)
 {
+    if (ep.activation == DenseActivation::kSiluHalf) {
+        const float g = __half2float(__float2half_rn(gate));
+        return g / (1.f + __expf(-g)) * __half2float(__float2half_rn(up));
+    }
     return ep.activation == DenseActivation::kGeluTanh ? gelu_tanh_f32<FAST>(gate) * up : clamped_swish_f32<FAST>(gate, up, ep.limit, ep.slope);
 }
 
@@ -54,6 +67,8 @@ struct DenseTcParams {
     int           stages, tmem_columns;
     int           x2_tile;     // weight tiles from here on multiply the second operand
     int           column_tiles, half_box;
+    int           wide_out, wide_act;  // columns below / from which on a warp's rows leave in 16-byte pieces (epilogue16_wide)
+    int           band;        // pairs of CTAs: token tiles of a band, which all column tiles pass before the next band's turn
     DenseGroups   groups;
     float*        scratch;
     int*          tickets;
@@ -96,9 +111,9 @@ __device__ __forceinline__ void residual_add(const DenseEpilogue& ep, const floa
 }
 
 // What happens to 16 consecutive tokens of one output column (lane = column); `live` = tokens of the 16 that exist
+template<typename E>
 __device__ __forceinline__ void epilogue16(const DenseEpilogue& ep, const float (&y)[16], int t0, int live, int n, int n_out)
 {
-    using E        = __nv_bfloat16;
     const bool col = n < n_out;
     if (ep.kind == DenseKind::kF32) {
 #pragma unroll
@@ -127,14 +142,70 @@ __device__ __forceinline__ void epilogue16(const DenseEpilogue& ep, const float 
         }
         return;
     }
-    const bool th = ep.kind == DenseKind::kInput && n >= ep.tanh_lo && n < ep.tanh_hi;
+    if (ep.kind == DenseKind::kInput && __any_sync(0xffffffffu, n >= ep.tanh_lo && n < ep.tanh_hi)) {
+        const bool th = n >= ep.tanh_lo && n < ep.tanh_hi;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (i < live && col) static_cast<E*>(ep.out)[(size_t)(t0 + i) * ep.out_ld + n] = from_f32<E>(th ? tanhf(y[i]) : y[i]);
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        if (i < live && col) static_cast<E*>(ep.out)[(size_t)(t0 + i) * ep.out_ld + n] = from_f32<E>(th ? tanhf(y[i]) : y[i]);
+        if (i < live && col) static_cast<E*>(ep.out)[(size_t)(t0 + i) * ep.out_ld + n] = from_f32<E>(y[i]);
     }
 }
 
-template<bool GROUPS>
+// The same for a warp whose 32 columns all exist and go to one place in the element type, 16-byte aligned: the rows pass
+// through shared memory, so that a lane stores 16 bytes (lane = column stores 2 bytes a lane, 16 instructions where these are
+// two).  n0: first column of the warp; `buf`: its own staging rows.
+template<typename E>
+__device__ __forceinline__ void epilogue16_wide(const DenseEpilogue& ep, const float (&y)[16], int t0, int live, int n0, int lane, unsigned char* buf)
+{
+    const int  n   = n0 + lane;
+    const bool act = ep.kind == DenseKind::kInput && n0 >= ep.split;
+    if (act) {
+        const bool odd = lane & 1;
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+            const float other = __shfl_xor_sync(0xffffffffu, odd ? y[i] : y[i + 1], 1);
+            const float gate = odd ? other : y[i], up = odd ? y[i + 1] : other;
+            reinterpret_cast<E*>(buf + (i + (odd ? 1 : 0)) * kRowPitch)[lane >> 1] = from_f32<E>(activate<true>(ep, gate, up));
+        }
+        __syncwarp();
+        const int r = lane >> 1, c = lane & 1;
+        if (r < live) {
+            *reinterpret_cast<uint4*>(static_cast<E*>(ep.act) + (size_t)(t0 + r) * ep.act_ld + ((n0 - ep.split) >> 1) + c * 8) =
+                *reinterpret_cast<const uint4*>(buf + r * kRowPitch + c * 16);
+        }
+    }
+    else {
+        // a branch of the whole warp: as a select per value, tanhf took four fifths of the epilogue's time in launches without it
+        if (ep.kind == DenseKind::kInput && n0 + 32 > ep.tanh_lo && n0 < ep.tanh_hi) {
+            const bool th = n >= ep.tanh_lo && n < ep.tanh_hi;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) reinterpret_cast<E*>(buf + i * kRowPitch)[lane] = from_f32<E>(th ? tanhf(y[i]) : y[i]);
+        }
+        else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) reinterpret_cast<E*>(buf + i * kRowPitch)[lane] = from_f32<E>(y[i]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = h * 8 + (lane >> 2), c = lane & 3;
+            if (r < live) {
+                *reinterpret_cast<uint4*>(static_cast<E*>(ep.out) + (size_t)(t0 + r) * ep.out_ld + n0 + c * 8) =
+                    *reinterpret_cast<const uint4*>(buf + r * kRowPitch + c * 16);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// E: element type of operands and outputs.  PAIR: two CTAs (a cluster) on a tile of 256 output columns; either one loads its
+// 128 weight rows and half of the tile's tokens, and runs the epilogue of its own columns, which lie in its own TMEM.
+template<typename E, bool GROUPS, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
                 const __grid_constant__ CUtensorMap x2_map)
@@ -144,8 +215,10 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
     const uint32_t base = (raw + 1023u) & ~1023u;  // operand tiles on 1024-byte boundaries (the swizzle is a function of the address)
     const int      NT      = p.token_tile;
     const uint32_t w_bytes = kDenseTile * 128;
-    const uint32_t stage_b = w_bytes + (uint32_t)NT * 128;
+    const uint32_t stage_b = w_bytes + (uint32_t)(PAIR ? NT / 2 : NT) * 128;
     const int      ST      = p.stages;
+    const int      rank    = PAIR ? (int)cluster_rank() : 0;
+    const int      unit = PAIR ? blockIdx.x / 2 : blockIdx.x, units = PAIR ? gridDim.x / 2 : gridDim.x;  // who walks through the tiles
     DenseShared*   sh      = reinterpret_cast<DenseShared*>(smem_dyn + (base - raw) + (size_t)ST * stage_b);
     const int      tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -156,12 +229,19 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(&sh->acc_full[a], 1);
-            mbar_init(&sh->acc_empty[a], 4);
+            mbar_init(&sh->acc_empty[a], PAIR ? 8 : 4);
         }
         sh->dead = 0;
         fence_mbar_init();
     }
-    if (warp == 1) tmem_alloc(&sh->tmem_base, p.tmem_columns);
+    if (warp == 1) {
+        if (PAIR) {
+            tmem_pair_alloc(&sh->tmem_base, p.tmem_columns);
+        }
+        else {
+            tmem_alloc(&sh->tmem_base, p.tmem_columns);
+        }
+    }
     int* const first_tile = reinterpret_cast<int*>(sh + 1);
     if (GROUPS) {
         pdl_wait();  // the offsets come from a kernel ahead
@@ -184,7 +264,12 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
         }
     }
     tcgen05_before_sync();
-    __syncthreads();
+    if (PAIR) {
+        cluster_sync_all();
+    }
+    else {
+        __syncthreads();
+    }
     tcgen05_after_sync();
     const uint32_t tmem = sh->tmem_base;
     const int      tiles = GROUPS ? first_tile[p.groups.count] : p.tiles;
@@ -207,6 +292,12 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
             q.height = ((n + tts - 1) / tts + 15) / 16 * 16;  // the group's tiles are equally high
             q.t0 = begin + q.tt * q.height, q.rows = min(q.height, n - q.tt * q.height), q.w_row = lo * p.n_out + q.ct * kDenseTile;
         }
+        else if (PAIR) {
+            const int cols = (p.column_tiles + 1) / 2, band = tile / (p.band * cols), in = tile - band * p.band * cols;
+            const int tts = min(p.band, p.token_tiles - band * p.band), cp = in / tts;
+            q.ct = 2 * cp + rank, q.tt = band * p.band + in - cp * tts;
+            q.t0 = q.tt * NT, q.rows = min(NT, p.tokens - q.t0), q.w_row = q.ct * kDenseTile, q.height = NT;
+        }
         else {
             q.ct = tile / p.token_tiles, q.tt = tile - q.ct * p.token_tiles;
             q.t0 = q.tt * NT, q.rows = min(NT, p.tokens - q.t0), q.w_row = q.ct * kDenseTile, q.height = NT;
@@ -220,7 +311,7 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
     auto            cut       = [&](int c) { return (long long)c * cut_total / cut_ctas; };
     auto            segment   = [&](int i, int& tile, int& kb0, int& kb1) {
         if (p.cut_ctas == 0) {
-            tile = i * (int)gridDim.x + (int)blockIdx.x, kb0 = 0, kb1 = p.k_blocks;
+            tile = i * units + unit, kb0 = 0, kb1 = p.k_blocks;
             return tile < (GROUPS ? tiles : p.grid_tiles);
         }
         if (GROUPS && (int)blockIdx.x >= cut_ctas) return false;
@@ -230,94 +321,146 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
         return true;
     };
 
+    // The two single-thread roles run as whole warps with one elected lane (elect.sync): inside `if (lane == 0)` the compiler
+    // cannot know that one thread is left, and hands every operand of a copy or product over lane by lane.
     if (warp == 0) {
         // ===================================================================================== loader
-        if (lane == 0) {
-            int  issued = 0;
-            bool ok = true, waited = false;
-            // groups: a low tile's rows come in a box of half the height (one copy either way: their issue rate counts)
-            auto low    = [&](const Place& q) { return GROUPS && q.height <= p.half_box; };
-            auto load_w = [&](int kb, const Place& q, int s) {
-                mbar_arrive_expect_tx(&sh->full[s], low(q) ? w_bytes + (uint32_t)p.half_box * 128 : stage_b);
-                tma_load_2d(base + s * stage_b, &w_map, kb * kKBlock, q.w_row, &sh->full[s]);
-            };
-            auto load_x = [&](int kb, const Place& q, int s) {
-                tma_load_2d(base + s * stage_b + w_bytes, low(q) || q.ct >= p.x2_tile ? &x2_map : &x_map, kb * kKBlock, q.t0, &sh->full[s]);
-            };
-            int tile, kb0, kb1;
-            for (int seg = 0; ok && segment(seg, tile, kb0, kb1); ++seg) {
-                const Place q = place(tile);
-                int       kb = kb0;
-                if (!waited) {
-                    // weights are written by no kernel: the first boxes go out before the kernel ahead is complete
-                    const int pre = min(ST, kb1 - kb0);
+        int      issued = 0, s = 0;
+        uint32_t phase = 0;  // parity of the ring's pass
+        bool     ok = true, waited = false;
+        // groups: a low tile's rows come in a box of half the height (one copy either way: their issue rate counts)
+        auto low    = [&](const Place& q) { return GROUPS && q.height <= p.half_box; };
+        auto full_of = [&](int s) { return PAIR ? cluster_address(smem_u32(&sh->full[s]), 0) : smem_u32(&sh->full[s]); };
+        auto load_w = [&](int kb, const Place& q, int s) {
+            if (PAIR) {
+                if (rank == 0) mbar_arrive_expect_tx(&sh->full[s], 2 * stage_b);  // what both CTAs bring
+                tma_pair_load_2d(base + s * stage_b, &w_map, kb * kKBlock, q.w_row, full_of(s));
+                return;
+            }
+            mbar_arrive_expect_tx(&sh->full[s], low(q) ? w_bytes + (uint32_t)p.half_box * 128 : stage_b);
+            tma_load_2d(base + s * stage_b, &w_map, kb * kKBlock, q.w_row, &sh->full[s]);
+        };
+        auto load_x = [&](int kb, const Place& q, int s) {
+            if (PAIR) {
+                tma_pair_load_2d(base + s * stage_b + w_bytes, q.ct >= p.x2_tile ? &x2_map : &x_map, kb * kKBlock, q.t0 + rank * (NT / 2), full_of(s));
+                return;
+            }
+            tma_load_2d(base + s * stage_b + w_bytes, &(low(q) || q.ct >= p.x2_tile ? x2_map : x_map), kb * kKBlock, q.t0, &sh->full[s]);
+        };
+        int tile, kb0, kb1;
+        for (int seg = 0; ok && segment(seg, tile, kb0, kb1); ++seg) {
+            const Place q = place(tile);
+            int       kb = kb0;
+            if (!waited) {
+                // weights are written by no kernel: the first boxes go out before the kernel ahead is complete
+                const int pre = min(ST, kb1 - kb0);
+                if (elect_one()) {
                     for (int i = 0; i < pre; ++i) load_w(kb0 + i, q, i);
-                    pdl_wait();
-                    pdl_launch_dependents();
-                    waited = true;
-                    for (int i = 0; i < pre; ++i) load_x(kb0 + i, q, i);
-                    issued = pre;
-                    kb += pre;
                 }
-                for (; kb < kb1; ++kb, ++issued) {
-                    const int s = issued % ST;
-                    if (issued >= ST && !mbar_wait(&sh->empty[s], ((issued / ST) - 1) & 1, p.max_wait)) {
+                __syncwarp();
+                pdl_wait();
+                pdl_launch_dependents();
+                waited = true;
+                if (elect_one()) {
+                    for (int i = 0; i < pre; ++i) load_x(kb0 + i, q, i);
+                }
+                __syncwarp();
+                issued = pre;
+                kb += pre;
+                s = pre;
+                if (s == ST) s = 0, phase ^= 1;
+            }
+            for (; kb < kb1; ++kb, ++issued) {
+                if (issued >= ST && !mbar_wait_warp(&sh->empty[s], phase ^ 1, p.max_wait)) {
+                    if (lane == 0) {
                         atomicOr(p.status, kStatusGemmPipeWait);
                         *(volatile int*)&sh->dead = 1;
-                        ok = false;
-                        break;
                     }
+                    ok = false;
+                    break;
+                }
+                if (elect_one()) {
                     load_w(kb, q, s);
                     load_x(kb, q, s);
                 }
-            }
-            if (!waited) {
-                pdl_wait();
-                pdl_launch_dependents();
-            }
-            if (!ok) {
-                // the CTA leaves early: not before its own copies have landed
-                for (int i = max(0, issued - ST); i < issued; ++i) mbar_wait(&sh->full[i % ST], (i / ST) & 1, p.max_wait);
+                __syncwarp();
+                if (++s == ST) s = 0, phase ^= 1;
             }
         }
-        else {
+        if (!waited) {
             pdl_wait();
             pdl_launch_dependents();
+        }
+        if (PAIR && ok) {
+            // the products that free the last stages also arrive at the other CTA's barriers: nobody leaves before
+            for (int i = max(0, issued - ST); i < issued; ++i) mbar_wait_warp(&sh->empty[i % ST], (i / ST) & 1, p.max_wait);
+        }
+        if (!ok) {
+            // the CTA leaves early: not before its own copies have landed
+            for (int i = max(0, issued - ST); i < issued; ++i) mbar_wait_warp(&sh->full[i % ST], (i / ST) & 1, p.max_wait);
         }
     }
     else if (warp == 1) {
         // ===================================================================================== MMA issuer
         pdl_wait();
         pdl_launch_dependents();
-        if (lane == 0) {
-            uint32_t       idesc = umma_idesc_bf16(kDenseTile, NT);
-            int            it = 0, local = 0;
+        if (rank == 0) {
+            constexpr int  kM    = PAIR ? 2 * kDenseTile : kDenseTile;
+            uint32_t       idesc = std::is_same<E, __half>::value ? umma_idesc_f16(kM, NT) : umma_idesc_bf16(kM, NT);
+            const uint64_t desc0 = umma_desc_k(base);  // the address field never carries out: shared memory has 18 bits of address
+            int            s = 0, local = 0;
+            uint32_t       phase = 0;
             bool           ok = true;
             int            tile, kb0, kb1;
             for (; ok && segment(local, tile, kb0, kb1); ++local) {
                 const int a = local & 1;
                 if (GROUPS) idesc = umma_idesc_bf16(kDenseTile, place(tile).height);
-                if (local >= 2 && !mbar_wait(&sh->acc_empty[a], ((local >> 1) - 1) & 1, p.max_wait)) ok = false;
+                if (local >= 2 && !mbar_wait_warp(&sh->acc_empty[a], ((local >> 1) - 1) & 1, p.max_wait)) ok = false;
                 tcgen05_after_sync();
-                for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-                    const int s = it % ST;
-                    if (!mbar_wait(&sh->full[s], (it / ST) & 1, p.max_wait)) {
+                const uint32_t acc = tmem + a * NT;
+                for (int kb = kb0; kb < kb1 && ok; ++kb) {
+                    if (!mbar_wait_warp(&sh->full[s], phase, p.max_wait)) {
                         ok = false;
                         break;
                     }
                     tcgen05_after_sync();
-                    const uint64_t da = umma_desc_k(base + s * stage_b), db = umma_desc_k(base + s * stage_b + w_bytes);
+                    const uint64_t da = desc0 + (uint64_t)((s * stage_b) >> 4), db = da + (uint64_t)(w_bytes >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        umma_f16_ss(tmem + a * NT, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, (kb > kb0 || j) ? 1u : 0u);
+                        for (int j = 0; j < 4; ++j) {
+                            if (PAIR) {
+                                umma_pair_f16_ss(acc, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, (kb > kb0 || j) ? 1u : 0u);
+                            }
+                            else {
+                                umma_f16_ss(acc, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, (kb > kb0 || j) ? 1u : 0u);
+                            }
+                        }
+                        if (PAIR) {
+                            umma_pair_commit(&sh->empty[s]);
+                        }
+                        else {
+                            umma_commit(&sh->empty[s]);
+                        }
                     }
-                    umma_commit(&sh->empty[s]);
+                    __syncwarp();
+                    if (++s == ST) s = 0, phase ^= 1;
                 }
-                if (!ok) {
+                if (!ok && lane == 0) {
                     atomicOr(p.status, kStatusGemmPipeWait);
                     *(volatile int*)&sh->dead = 1;
+                    if (PAIR) asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(cluster_address(smem_u32(&sh->dead), 1)), "r"(1) : "memory");
                 }
-                umma_commit(&sh->acc_full[a]);  // arrives when everything issued so far is complete (also on the give-up path)
+                __syncwarp();
+                // arrives when everything issued so far is complete (also on the give-up path)
+                if (elect_one()) {
+                    if (PAIR) {
+                        umma_pair_commit(&sh->acc_full[a]);
+                    }
+                    else {
+                        umma_commit(&sh->acc_full[a]);
+                    }
+                }
+                __syncwarp();
             }
         }
     }
@@ -346,7 +489,7 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
                 named_bar_sync(kEpiBar, 128);
                 scaled_tile = tt;
             }
-            const bool  adds = p.ep.kind == DenseKind::kResidual;
+            const bool  adds = !std::is_same<E, __half>::value && p.ep.kind == DenseKind::kResidual;
             const float bias = adds && p.ep.gate && n < p.n_out ? p.ep.gate_bias[n] : 0.f;
             ResidualIn  in;
             if (adds && kb1 - kb0 == p.k_blocks) residual_load(p.ep, t0, min(16, rows), n, p.n_out, in);
@@ -403,6 +546,8 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
                 if (finish) __threadfence();
             }
             if (finish) {
+                const int  n0   = ct * kDenseTile + q * 32;
+                const bool wide = n0 + 32 <= p.n_out && (n0 >= p.wide_act || n0 + 32 <= p.wide_out);
                 const bool sums = adds && p.ep.ssq_out;
                 if (adds && kb1 - kb0 < p.k_blocks) residual_load(p.ep, t0, min(16, rows), n, p.n_out, in);
                 for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -441,8 +586,11 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
                         residual_add(p.ep, v, in, bias, t0 + c0, live, n, p.n_out, sq);
                         in = next;
                     }
+                    else if (wide) {
+                        epilogue16_wide<E>(p.ep, v, t0 + c0, live, n0, lane, sh->rows[q]);
+                    }
                     else {
-                        epilogue16(p.ep, v, t0 + c0, live, n, p.n_out);
+                        epilogue16<E>(p.ep, v, t0 + c0, live, n, p.n_out);
                     }
                     if (sums) {
 #pragma unroll
@@ -462,13 +610,26 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
             }
             tcgen05_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sh->acc_empty[a]);
+            if (lane == 0) {
+                if (PAIR) {
+                    mbar_arrive_cluster(cluster_address(smem_u32(&sh->acc_empty[a]), 0));
+                }
+                else {
+                    mbar_arrive(&sh->acc_empty[a]);
+                }
+            }
         }
     }
 
     tcgen05_before_sync();
-    __syncthreads();
-    if (warp == 1) tmem_free(tmem, p.tmem_columns);
+    if (PAIR) {
+        cluster_sync_all();
+        if (warp == 1) tmem_pair_free(tmem, p.tmem_columns);
+    }
+    else {
+        __syncthreads();
+        if (warp == 1) tmem_free(tmem, p.tmem_columns);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ fp32
@@ -558,44 +719,67 @@ EncodeTiled lookup_encode_tiled()
     return reinterpret_cast<EncodeTiled>(fn);
 }
 
-bool encode_rows(EncodeTiled encode, CUtensorMap* map, const void* ptr, int rows, int k, int ld, int box_rows)
+bool encode_rows(EncodeTiled encode, CUtensorMap* map, const void* ptr, int rows, int k, int ld, int box_rows, bool half = false)
 {
     const cuuint64_t dims[2]    = {(cuuint64_t)k, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2]     = {(cuuint32_t)kKBlock, (cuuint32_t)box_rows};
     const cuuint32_t estr[2]    = {1u, 1u};
-    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    return encode(map, half ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
            == CUDA_SUCCESS;
 }
 
 cudaError_t dense_prepare(int max_smem)
 {
-    const cudaError_t e = cudaFuncSetAttribute(dense_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
-    return e == cudaSuccess ? cudaFuncSetAttribute(dense_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem) : e;
+    cudaError_t e = cudaSuccess;
+    auto        raise = [&](auto kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    };
+    raise(dense_tc_kernel<__nv_bfloat16, false, false>);
+    raise(dense_tc_kernel<__nv_bfloat16, true, false>);
+    raise(dense_tc_kernel<__nv_bfloat16, false, true>);
+    raise(dense_tc_kernel<__half, false, true>);
+    return e;
 }
 const KernelPreparation g_prepare(dense_prepare);
 
 struct Plan {
     int  token_tile;
-    bool cut;
+    bool cut, pair = false;
 };
-// Tile height and whether the tiles are cut, by a model of the launch's time in microseconds: a k block takes what its
-// bytes or its products need, cutting costs the exchange of the parts.
-Plan choose_plan(int tokens, int n_out, int k_blocks, int sms)
+// Tile height, whether the tiles are cut, and whether pairs of CTAs take them, by a model of the launch's time in microseconds
+// (of what differs between the choices): a k block takes what its copies and the issue of its products need (the constant) or
+// the tensor pipe and the L2 (per token of the tile); cutting costs the exchange of the parts.  Fitted to 640 launches over
+// 22016x4096, 10240x4096, 4096x4096 and 4096x11008 with 32 to 4096 tokens (mean error 5 %, 8 % of the cut ones).  The
+// choice is within 5 % of the best measured one in nearly all of them; pairs win from about 100 tokens on, as a CTA
+// loads half as many tokens (4096 x 4096, 300 tokens: 37 us, single CTAs cut 53; 22016 x 4096, 1024 tokens: 141 against 149).
+Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool pairs, double* cost_us = nullptr)
 {
-    Plan   best{0, false};
-    double best_cost = 1e30;
-    const int first = tokens >= kMaxTokens ? kMaxTokens : (tokens + 15) / 16 * 16;
-    const int last  = tokens >= kMaxTokens ? 128 : first;
-    for (int nt = first; nt >= last; nt -= 16) {
-        const long long tiles = (long long)((n_out + kDenseTile - 1) / kDenseTile) * ((tokens + nt - 1) / nt);
-        const double    block = std::max(0.4, 0.45 * nt / 256);
-        const double    whole = (double)((tiles + sms - 1) / sms) * (k_blocks * block + 1.0);
-        const double    cut   = (double)tiles * k_blocks / sms * block + 3.0 + 0.06 * nt;
-        if (whole < best_cost - 1e-9) best_cost = whole, best = {nt, false};
-        if (tiles < 2 * sms && cut < best_cost - 1e-9) best_cost = cut, best = {nt, true};
+    Plan      best{0, false};
+    double    best_cost = 1e30;
+    const int columns   = (n_out + kDenseTile - 1) / kDenseTile;
+    auto consider = [&](double cost, Plan plan) {
+        if (cost < best_cost - 1e-9) best_cost = cost, best = plan;
+    };
+    if (single) {
+        const int first = tokens >= kMaxTokens ? kMaxTokens : (tokens + 15) / 16 * 16;
+        const int last  = std::min(first, 64);
+        for (int nt = first; nt >= last; nt -= 16) {
+            const long long tiles = (long long)columns * ((tokens + nt - 1) / nt);
+            if (tiles < 2 * sms) consider((double)tiles * k_blocks / sms * std::max(0.36, 0.073 + 0.00182 * nt) + 0.15 * nt, {nt, true, false});
+            consider((double)((tiles + sms - 1) / sms) * (k_blocks * std::max(0.2, 0.112 + 0.00108 * nt) - 0.35) + 1.8, {nt, false, false});
+        }
     }
+    if (pairs) {
+        const int first = tokens >= kMaxTokens ? kMaxTokens : (tokens + 31) / 32 * 32;
+        const int last  = std::min(first, 96);
+        for (int nt = first; nt >= last; nt -= 32) {
+            const long long tiles = (long long)((columns + 1) / 2) * ((tokens + nt - 1) / nt);
+            consider((double)((tiles + sms / 2 - 1) / (sms / 2)) * (k_blocks * std::max(0.183, 0.066 + 0.00108 * nt) + 1.0) + 1.0, {nt, false, true});
+        }
+    }
+    if (cost_us) *cost_us = best_cost;
     return best;
 }
 
@@ -609,7 +793,8 @@ Plan choose_group_plan(int rows, int groups, int n_out, int sms)
     return {nt, tiles < 4 * sms};
 }
 
-int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl)
+// `half`: fp16 operands, pairs of CTAs only
+int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool half = false)
 {
     static const EncodeTiled encode = lookup_encode_tiled();
     if (!encode) return TM_ERR_CUDA;
@@ -622,22 +807,27 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl)
     p.n_out        = g.n_out;
     p.k_blocks     = (g.k + kKBlock - 1) / kKBlock;
     const bool grouped = g.groups.count > 0;
-    const Plan plan    = grouped ? choose_group_plan(g.tokens, g.groups.count, g.n_out, h->sm_count) : choose_plan(g.tokens, g.n_out, p.k_blocks, h->sm_count);
+    const int  sms     = h->sm_count;
+    // the tile of a pair has one operand; with few tokens the k blocks of a tile are rather cut than shared
+    const bool pairs = sms >= 2 && (half || g.tokens > kPairMinTokens) && (!g.x2 || g.x2_from % (2 * kDenseTile) == 0);
+    const Plan plan  = grouped ? choose_group_plan(g.tokens, g.groups.count, g.n_out, sms) : choose_plan(g.tokens, g.n_out, p.k_blocks, sms, !half, pairs);
+    if (plan.token_tile == 0) return TM_ERR_UNSUPPORTED;
     p.groups           = g.groups;
     p.x2_tile          = g.x2 ? g.x2_from / kDenseTile : 1 << 30;
     p.column_tiles     = (g.n_out + kDenseTile - 1) / kDenseTile;
     p.half_box         = plan.token_tile / 2 / 16 * 16;
+    p.band             = kBand;
     p.token_tile    = plan.token_tile;
     p.token_tiles   = (g.tokens + p.token_tile - 1) / p.token_tile;
-    p.tiles         = (g.n_out + kDenseTile - 1) / kDenseTile * p.token_tiles;
+    p.tiles         = (plan.pair ? (p.column_tiles + 1) / 2 : p.column_tiles) * p.token_tiles;
     p.tmem_columns = 32;
     while (p.tmem_columns < 2 * p.token_tile) p.tmem_columns *= 2;
-    const size_t stage_b = (size_t)kDenseTile * 128 + (size_t)p.token_tile * 128;
+    const int    box     = plan.pair ? p.token_tile / 2 : p.token_tile;  // token rows that a CTA loads
+    const size_t stage_b = (size_t)kDenseTile * 128 + (size_t)box * 128;
     const size_t shared  = sizeof(DenseShared) + (grouped ? (size_t)(g.groups.count + 1) * sizeof(int) : 0);
     p.stages             = (int)(((size_t)h->max_smem - 1024 - shared) / stage_b);
     if (p.stages > kMaxStages) p.stages = kMaxStages;
     if (p.stages < 2) return TM_ERR_UNSUPPORTED;
-    const int sms = h->sm_count;
     // tiles that tickets have to be there for
     const long long most = grouped ? (long long)p.column_tiles * std::min(g.tokens, g.groups.count + g.tokens / p.token_tile) : p.tiles;
     if (plan.cut && most <= (long long)h->counter_ints && (size_t)2 * sms * p.token_tile * kDenseTile * 4 <= h->scratch_bytes) {
@@ -645,21 +835,33 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl)
         p.cut_ctas = grouped ? sms : (int)std::min<long long>(sms, std::max<long long>(1, (long long)p.tiles * p.k_blocks / 4));
     }
     p.grid_tiles        = p.cut_ctas > 0 ? 0 : p.tiles;
-    const int grid_ctas = p.cut_ctas > 0 ? p.cut_ctas : (int)std::min<long long>(sms, most);
+    const int grid_ctas = plan.pair       ? 2 * (int)std::min<long long>(sms / 2, most) :
+                          p.cut_ctas > 0 ? p.cut_ctas :
+                                           (int)std::min<long long>(sms, most);
     p.scratch  = static_cast<float*>(h->scratch);
     p.tickets  = h->counters;
     p.status   = h->status;
     p.max_wait = h->gemm_wait_cycles > 0 ? h->gemm_wait_cycles : kMaxWaitCycles;
     p.ep       = g.ep;
+    // rows of `out` and `act` that 16-byte stores reach
+    auto aligned = [](const void* ptr, int ld) { return ptr && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
+    const bool input = g.ep.kind == DenseKind::kInput;
+    p.wide_act = input && aligned(g.ep.act, g.ep.act_ld) ? g.ep.split : 1 << 30;
+    p.wide_out = (input || g.ep.kind == DenseKind::kStore) && aligned(g.ep.out, g.ep.out_ld) ? g.n_out : 0;
+    if (input) p.wide_out = std::min(p.wide_out, g.ep.split);
+    if (g.ep.f32_out) p.wide_out = std::min(p.wide_out, g.ep.f32_from);
     CUtensorMap w_map, x_map, x2_map;
-    if (!encode_rows(encode, &w_map, g.w, g.n_out * std::max(1, g.groups.count), g.k, g.ldw, kDenseTile)) return TM_ERR_CUDA;
-    if (!encode_rows(encode, &x_map, g.x, g.tokens, g.k, g.ldx, p.token_tile)) return TM_ERR_CUDA;
+    if (!encode_rows(encode, &w_map, g.w, g.n_out * std::max(1, g.groups.count), g.k, g.ldw, kDenseTile, half)) return TM_ERR_CUDA;
+    if (!encode_rows(encode, &x_map, g.x, g.tokens, g.k, g.ldx, box, half)) return TM_ERR_CUDA;
     // the second operand, or the half-height boxes of the groups
-    if (!encode_rows(encode, &x2_map, g.x2 ? g.x2 : g.x, g.tokens, g.k, g.ldx, grouped ? std::max(16, p.half_box) : p.token_tile)) return TM_ERR_CUDA;
+    if (!encode_rows(encode, &x2_map, g.x2 ? g.x2 : g.x, g.tokens, g.k, g.ldx, grouped ? std::max(16, p.half_box) : box, half)) return TM_ERR_CUDA;
     const size_t smem = 1024 + (size_t)p.stages * stage_b + shared;
-    const dim3   grid(grid_ctas);
-    const cudaError_t e = grouped ? launch_kernel(dense_tc_kernel<true>, grid, dim3(kThreads), smem, st, pdl, p, w_map, x_map, x2_map) :
-                                    launch_kernel(dense_tc_kernel<false>, grid, dim3(kThreads), smem, st, pdl, p, w_map, x_map, x2_map);
+    const dim3   grid(grid_ctas), block(kThreads);
+    using B = __nv_bfloat16;
+    const cudaError_t e = half      ? launch_cluster_kernel(dense_tc_kernel<__half, false, true>, grid, block, 2, smem, st, pdl, p, w_map, x_map, x2_map) :
+                          plan.pair ? launch_cluster_kernel(dense_tc_kernel<B, false, true>, grid, block, 2, smem, st, pdl, p, w_map, x_map, x2_map) :
+                          grouped   ? launch_kernel(dense_tc_kernel<B, true, false>, grid, block, smem, st, pdl, p, w_map, x_map, x2_map) :
+                                      launch_kernel(dense_tc_kernel<B, false, false>, grid, block, smem, st, pdl, p, w_map, x_map, x2_map);
     if (e != cudaSuccess) {
         h->last_cuda_error = (int)e;
         return TM_ERR_CUDA;
@@ -684,6 +886,20 @@ int dense_gemm(tm_handle* h, const DenseGemm& g, bool f32, cudaStream_t st, bool
     }
     ++h->launches;
     return TM_OK;
+}
+
+double dense_pair_us(int tokens, int n_out, int k_blocks, int sms)
+{
+    double us = 0.;
+    choose_plan(tokens, n_out, k_blocks, sms, false, true, &us);
+    return us;
+}
+
+int dense_gemm_f16(tm_handle* h, const DenseGemm& g, cudaStream_t st)
+{
+    if (!g.w || !g.x || g.tokens <= 0 || g.n_out <= 0 || g.k <= 0 || g.ldw < g.k || g.ldx < g.k) return TM_ERR_INVALID_ARG;
+    if (g.groups.count > 0 || g.ep.kind == DenseKind::kResidual || g.ep.ssq) return TM_ERR_UNSUPPORTED;
+    return dense_tc(h, g, st, false, true);
 }
 
 }  // namespace tmb

@@ -2,6 +2,7 @@
 // activations, weights and cached rows: __nv_bfloat16 or float; all arithmetic is fp32.
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -14,6 +15,7 @@ template<> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 
 template<typename E> __device__ __forceinline__ E from_f32(float x);
 template<> __device__ __forceinline__ float from_f32<float>(float x) { return x; }
 template<> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
+template<> __device__ __forceinline__ __half from_f32<__half>(float x) { return __float2half_rn(x); }
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
