@@ -197,21 +197,24 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_scores_kernel(const ChunkTc
             }
         }
     }
-    else if ((tid & 31) == 0) {
-        const uint32_t idesc = umma_idesc_bf16(kBM, kBN);
+    else {
+        const uint32_t idesc = umma_idesc_bf16(kBM, kBN);  // the products: one elected lane of the warp
         for (int t = 0; t < ti.n_tiles; ++t) {
-            if (!mbar_wait(&bars->kv_full[t & 1], (t >> 1) & 1, p.max_wait)) {
-                atomicOr(p.status, kStatusGemmPipeWait);
+            if (!mbar_wait_warp(&bars->kv_full[t & 1], (t >> 1) & 1, p.max_wait)) {
+                if ((tid & 31) == 0) atomicOr(p.status, kStatusGemmPipeWait);
                 break;
             }
             tcgen05_after_sync();
+            if (elect_one()) {
 #pragma unroll
-            for (int blk = 0; blk < DK / 64; ++blk) {
-                const uint64_t dq = umma_desc_k(base + blk * kQBlock), dk = umma_desc_k(k_s + (t & 1) * L::kK + blk * kTBlock);
+                for (int blk = 0; blk < DK / 64; ++blk) {
+                    const uint64_t dq = umma_desc_k(base + blk * kQBlock), dk = umma_desc_k(k_s + (t & 1) * L::kK + blk * kTBlock);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_f16_ss(tmem + (t & 1) * kBN, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc, (blk | j) ? 1u : 0u);
+                    for (int j = 0; j < 4; ++j) umma_f16_ss(tmem + (t & 1) * kBN, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc, (blk | j) ? 1u : 0u);
+                }
+                umma_commit(&bars->s_full[t & 1]);
             }
-            umma_commit(&bars->s_full[t & 1]);
+            __syncwarp();
         }
     }
     tcgen05_before_sync();
@@ -384,21 +387,24 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_values_kernel(const ChunkTc
             for (int d = a.heads * a.vdim; d < p.c.out_pad; ++d) out[d] = from_f32<E>(0.f);
         }
     }
-    else if ((tid & 31) == 0) {
+    else {
         const uint32_t idesc = umma_idesc_bf16(kBM, DV, true);
         for (int t = 0; t < ti.n_tiles; ++t) {
-            if (!mbar_wait(&bars->full[t % kStages], (t / kStages) & 1, p.max_wait)) {
-                atomicOr(p.status, kStatusGemmPipeWait);
+            if (!mbar_wait_warp(&bars->full[t % kStages], (t / kStages) & 1, p.max_wait)) {
+                if ((tid & 31) == 0) atomicOr(p.status, kStatusGemmPipeWait);
                 break;
             }
             tcgen05_after_sync();
             const uint32_t p_addr = base + (t % kStages) * L::kStage;
             const uint64_t dp = umma_desc_k(p_addr), dv = umma_desc_mn(p_addr + L::kP, kTBlock);
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) umma_f16_ss(tmem, dp + (uint64_t)(2 * j), dv + (uint64_t)(128 * j), idesc, (t | j) ? 1u : 0u);
-            umma_commit(&bars->done[t % kStages]);
+                for (int j = 0; j < 4; ++j) umma_f16_ss(tmem, dp + (uint64_t)(2 * j), dv + (uint64_t)(128 * j), idesc, (t | j) ? 1u : 0u);
+                umma_commit(&bars->done[t % kStages]);
+            }
+            __syncwarp();
         }
-        umma_commit(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
+        if (elect_one()) umma_commit(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
     }
     tcgen05_before_sync();
     __syncthreads();

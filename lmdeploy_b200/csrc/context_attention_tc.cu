@@ -384,40 +384,47 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
             }
         }
     }
-    else if ((tid & 31) == 0) {
-        // ============================================================ MMA issuer
+    else {
+        // ============================================================ MMA issuer: one elected lane of the warp
         const uint32_t idesc_qk = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
         const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(kD >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // B is MN-major
         bool           ok       = true;
         for (int t = 0; t < n_tiles && ok; ++t) {
             const int buf = t & 1;
-            if (!mbar_wait(&bars->kv_full[buf], (t >> 1) & 1, p.max_wait_cycles)) {
+            if (!mbar_wait_warp(&bars->kv_full[buf], (t >> 1) & 1, p.max_wait_cycles)) {
                 ok = false;
                 break;
             }
             tc_after();
             const uint32_t k_addr = kv_s + buf * 2 * kTileBytes, v_addr = k_addr + kTileBytes;
+            if (elect_one()) {
 #pragma unroll
-            for (int blk = 0; blk < 2; ++blk) {
-                const uint64_t dq = desc_kmajor(q_s + blk * kQBlock), dk = desc_kmajor(k_addr + blk * kTBlock);
+                for (int blk = 0; blk < 2; ++blk) {
+                    const uint64_t dq = desc_kmajor(q_s + blk * kQBlock), dk = desc_kmajor(k_addr + blk * kTBlock);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_ss(tmem + kColS, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
+                    for (int j = 0; j < 4; ++j) umma_ss(tmem + kColS, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
+                }
+                umma_commit_to(&bars->s_full);
             }
-            umma_commit_to(&bars->s_full);
-            if (!mbar_wait(&bars->p_full, t & 1, p.max_wait_cycles)) {
+            __syncwarp();
+            if (!mbar_wait_warp(&bars->p_full, t & 1, p.max_wait_cycles)) {
                 ok = false;
                 break;
             }
             tc_after();
             const uint64_t dv = desc_mnmajor(v_addr, kTBlock);
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) umma_ts(tmem + kColO, tmem + kColP + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+                for (int j = 0; j < 4; ++j) umma_ts(tmem + kColO, tmem + kColP + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+            }
+            __syncwarp();
         }
-        if (!ok) {
+        if (!ok && (tid & 31) == 0) {
             atomicOr(p.status, kStatusGemmPipeWait);
             *(volatile int*)&bars->dead = 1;
         }
-        umma_commit_to(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
+        __syncwarp();
+        if (elect_one()) umma_commit_to(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
     }
 
     tc_before();

@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             const int sx = it % kXST;
             TC_TRACE(trow, 10, it);
             if (it >= kXST) warp_wait(&bars->x_empty[sx], ((it / kXST) - 1) & 1, dead, p.status, kStatusGemmPipeWait);
-            if (!dead && lane == 0) {
+            if (!dead && elect_one()) {
                 const uint32_t xb = base + (uint32_t)(x_ring - sm) + sx * x_bytes;
                 mbar_arrive_expect_tx(&bars->x_full[sx], (uint32_t)x_bytes);
                 tma_load_2d(xb, &x_map, g * kGroup, t0, &bars->x_full[sx]);
@@ -390,13 +390,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     }
     else if (warp <= kIssuers) {
         // ================================================================== MMA issuers
-        // One lane per (team, K half) runs the whole loop: waits, four (or eight) MMAs, commits.  The issue rate
-        // of one thread among busy warps (about 100 cycles per MMA), not the tensor pipe (about 35 at 64 tokens),
-        // bounds the MMA throughput of small token tiles: four issuers on four different schedulers share the
-        // work there, each half of K with an accumulator of its own (summed by the epilogue).
+        // One warp per (team, K half) runs the whole loop: waits, four (or eight) MMAs by an elected lane, commits.  At
+        // small token tiles four issuers on four different schedulers share the work, each half of K with an
+        // accumulator of its own (summed by the epilogue).
         const int m = (warp - 1) & 1;
         const int h = (warp - 1) >> 1;
-        if (lane == 0 && h < KS) {
+        if (h < KS) {
             const uint32_t idesc   = (1u << 4) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
             const uint32_t d_tmem  = tmem + (m * KS + h) * accS;
             const uint32_t kb_step = (uint32_t)(TT * 128) >> 4;  // descriptor units (16 B) between the two K blocks
@@ -417,22 +416,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     ok = mbar_wait(&bars->acc_empty[m], (seg_idx - 1) & 1);
                 }
                 ok = ok && mbar_wait(&bars->x_full[sx], px) && mbar_wait(&bars->a_full[m][sa], pa);
-                if (!ok) {
-                    atomicOr(p.status, kStatusGemmPipeWait);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) atomicOr(p.status, kStatusGemmPipeWait);
                     break;
                 }
                 tc_fence_after();
                 TC_TRACE(trow, 20, it);
                 const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + (uint32_t)h * 32;
                 const uint32_t lo     = d_lo + (uint32_t)sx * x_step;
-                umma_f16_ts_x4(d_tmem, a_tmem, lo, d_hi, idesc, first ? 1u : 0u);
-                if (KS == 1) umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
-                umma_commit(&bars->a_empty[m][sa]);
-                umma_commit(&bars->x_empty[sx]);
+                const bool last = (it == n_units - 1) || (g == G - 1);
+                if (elect_one()) {
+                    umma_f16_ts_x4(d_tmem, a_tmem, lo, d_hi, idesc, first ? 1u : 0u);
+                    if (KS == 1) umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
+                    umma_commit(&bars->a_empty[m][sa]);
+                    umma_commit(&bars->x_empty[sx]);
+                    if (last) umma_commit(&bars->acc_full[m]);
+                }
+                __syncwarp();
                 TC_TRACE(trow, 21, it);
                 first = false;
-                if ((it == n_units - 1) || (g == G - 1)) {
-                    umma_commit(&bars->acc_full[m]);
+                if (last) {
                     ++seg_idx;
                     first = true;
                 }

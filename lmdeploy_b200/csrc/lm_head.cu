@@ -137,57 +137,68 @@ lm_head_kernel(LmHeadParams p, const __grid_constant__ CUtensorMap w_map, const 
 
     if (warp == 0) {
         // ===================================================================================== loader
-        if (lane == 0) {
-            // the weight is written by no kernel: its first boxes start before the kernel ahead of this one is known to
-            // be complete; the activations follow after that wait, on the same barriers
-            const int pre = min(ST, nkb);
+        // one elected lane issues; the weight is written by no kernel: its first boxes start before the kernel ahead of this
+        // one is known to be complete; the activations follow after that wait, on the same barriers
+        const int pre = min(ST, nkb);
+        if (elect_one()) {
             for (int kb = 0; kb < pre; ++kb) {
                 mbar_arrive_expect_tx(&bars->full[kb], stage_b);
                 lm_tma_2d(base + kb * stage_b, &w_map, kb * kLmKBlock, v0, &bars->full[kb]);
             }
-            pdl_wait();
-            pdl_launch_dependents();
+        }
+        __syncwarp();
+        pdl_wait();
+        pdl_launch_dependents();
+        if (elect_one()) {
             for (int kb = 0; kb < pre; ++kb) lm_tma_2d(base + kb * stage_b + w_bytes, &x_map, kb * kLmKBlock, 0, &bars->full[kb]);
-            for (int kb = pre; kb < nkb; ++kb) {
-                const int s = kb % ST;
-                if (!mbar_wait(&bars->empty[s], ((kb / ST) - 1) & 1, p.max_wait_cycles)) {
+        }
+        __syncwarp();
+        int      s     = pre == ST ? 0 : pre;
+        uint32_t phase = 0;
+        for (int kb = pre; kb < nkb; ++kb) {
+            if (!mbar_wait_warp(&bars->empty[s], phase, p.max_wait_cycles)) {
+                if (lane == 0) {
                     atomicOr(p.status, kStatusGemmPipeWait);
                     *(volatile int*)&bars->dead = 1;
-                    break;
                 }
+                break;
+            }
+            if (elect_one()) {
                 mbar_arrive_expect_tx(&bars->full[s], stage_b);
                 lm_tma_2d(base + s * stage_b, &w_map, kb * kLmKBlock, v0, &bars->full[s]);
                 lm_tma_2d(base + s * stage_b + w_bytes, &x_map, kb * kLmKBlock, 0, &bars->full[s]);
             }
-        }
-        else {
-            pdl_wait();
-            pdl_launch_dependents();
+            __syncwarp();
+            if (++s == ST) s = 0, phase ^= 1;
         }
     }
     else if (warp == 1) {
         // ===================================================================================== MMA issuer
         pdl_wait();
         pdl_launch_dependents();
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kLmTileV >> 4) << 24);
-            bool           ok    = true;
-            for (int kb = 0; kb < nkb && ok; ++kb) {
-                const int s = kb % ST;
-                if (!mbar_wait(&bars->full[s], (kb / ST) & 1, p.max_wait_cycles)) {
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(kLmTileV >> 4) << 24);
+        int            s     = 0;
+        uint32_t       phase = 0;
+        for (int kb = 0; kb < nkb; ++kb) {
+            if (!mbar_wait_warp(&bars->full[s], phase, p.max_wait_cycles)) {
+                if (lane == 0) {
                     atomicOr(p.status, kStatusGemmPipeWait);
                     *(volatile int*)&bars->dead = 1;
-                    ok = false;
-                    break;
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t da = lm_desc(base + s * stage_b), db = lm_desc(base + s * stage_b + w_bytes);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t da = lm_desc(base + s * stage_b), db = lm_desc(base + s * stage_b + w_bytes);
+            if (elect_one()) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) lm_umma_ss(tmem, da + (uint64_t)(2 * j), db + (uint64_t)(2 * j), idesc, (kb | j) ? 1u : 0u);
                 lm_commit(&bars->empty[s]);  // the stage is free once these MMAs have read it
             }
-            lm_commit(&bars->acc_full);  // arrives when everything issued so far is complete (also on the give-up path)
+            __syncwarp();
+            if (++s == ST) s = 0, phase ^= 1;
         }
+        __syncwarp();
+        if (elect_one()) lm_commit(&bars->acc_full);  // arrives when everything issued so far is complete (also on the give-up path)
     }
     else {
         // ===================================================================================== logits out

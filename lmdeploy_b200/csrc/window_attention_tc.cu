@@ -293,39 +293,46 @@ __global__ void __launch_bounds__(kThreads, 2) window_attention_tc_kernel(const 
             }
         }
     }
-    else if ((tid & 31) == 0) {
-        // ============================================================ MMA issuer
+    else {
+        // ============================================================ MMA issuer: one elected lane of the warp
         const uint32_t idesc_qk = umma_idesc_bf16(kBM, kBN), idesc_pv = umma_idesc_bf16(kBM, DV, true);
         bool           ok       = true;
         for (int t = 0; t < n_tiles && ok; ++t) {
             const int buf = t & 1;
-            if (!mbar_wait(&bars->kv_full[buf], (t >> 1) & 1, p.max_wait)) {
+            if (!mbar_wait_warp(&bars->kv_full[buf], (t >> 1) & 1, p.max_wait)) {
                 ok = false;
                 break;
             }
             tcgen05_after_sync();
             const uint32_t k_addr = kv_s + buf * (L::kKBytes + L::kVBytes), v_addr = k_addr + L::kKBytes;
+            if (elect_one()) {
 #pragma unroll
-            for (int blk = 0; blk < DK / 64; ++blk) {
-                const uint64_t dq = umma_desc_k(base + blk * kQBlock), dk = umma_desc_k(k_addr + blk * kTBlock);
+                for (int blk = 0; blk < DK / 64; ++blk) {
+                    const uint64_t dq = umma_desc_k(base + blk * kQBlock), dk = umma_desc_k(k_addr + blk * kTBlock);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_f16_ss(tmem + kColS, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
+                    for (int j = 0; j < 4; ++j) umma_f16_ss(tmem + kColS, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
+                }
+                umma_commit(&bars->s_full);
             }
-            umma_commit(&bars->s_full);
-            if (!mbar_wait(&bars->p_full, t & 1, p.max_wait)) {
+            __syncwarp();
+            if (!mbar_wait_warp(&bars->p_full, t & 1, p.max_wait)) {
                 ok = false;
                 break;
             }
             tcgen05_after_sync();
             const uint64_t dv = umma_desc_mn(v_addr, kTBlock);
+            if (elect_one()) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) umma_f16_ts(tmem + kColO, tmem + kColP + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+                for (int j = 0; j < 4; ++j) umma_f16_ts(tmem + kColO, tmem + kColP + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+            }
+            __syncwarp();
         }
-        if (!ok) {
+        if (!ok && (tid & 31) == 0) {
             atomicOr(p.status, kStatusGemmPipeWait);
             *(volatile int*)&bars->dead = 1;
         }
-        umma_commit(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
+        __syncwarp();
+        if (elect_one()) umma_commit(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
     }
 
     tcgen05_before_sync();
