@@ -55,6 +55,15 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
     if (type != TM_GEMM_PLAIN && type != TM_GEMM_FUSED_SILU_FFN) return TM_ERR_UNSUPPORTED;
     if (type == TM_GEMM_FUSED_SILU_FFN && m % 64) return TM_ERR_UNSUPPORTED;
 
+    if (!workspace && !g_gemm_fusion && n >= h->gemm_tc_min_n) {
+        const int columns = gemm_expanded_columns(h, m, n, k);
+        if (columns > 0) {
+            GemmTcParams p{};
+            p.C = (__half*)C, p.A = (const unsigned char*)A, p.X = (const unsigned char*)B, p.Q = (const unsigned char*)Q;
+            p.N = m, p.T = n, p.K = k, p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
+            return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream);
+        }
+    }
     if (n >= h->gemm_tc_min_n) {
         // tensor-core tiles; token ranges that would overflow the scratch go in several launches
         const size_t n_out_tc = type == TM_GEMM_FUSED_SILU_FFN ? (size_t)m / 2 : (size_t)m;

@@ -6,6 +6,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+struct tm_handle;
+
 namespace tmb {
 
 // ---- small-token (HBM-bound) kernel -----------------------------------------------------
@@ -96,5 +98,11 @@ GemmTcPlan  gemm_tc_plan(int N, int T, int K, int sm_count);
 bool        gemm_tc_all_tiles_split(const GemmTcPlan& plan, int K);
 cudaError_t gemm_tc_prepare(int max_smem);
 cudaError_t gemm_tc_launch(const GemmTcPlan& plan, GemmTcParams p, cudaStream_t st, bool pdl = false);
+
+// ---- many tokens: the weight expanded to fp16 rows in the handle's scratch, then a dense product (gemm_s4_f16_expand.cu) ----
+// output columns that are expanded and multiplied at a time (all, or pieces that fit the scratch); 0: the other kernel is faster
+int gemm_expanded_columns(const tm_handle* h, int N, int T, int K);
+// C, A, X, Q, N, T, K and fused_silu of `p` are read
+int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaStream_t st);
 
 }  // namespace tmb

@@ -1,0 +1,71 @@
+"""Products with many tokens: the dense kernel's pairs of CTAs and the W4A16 GEMM that expands its weight first, at the edges of
+their tiles, against 64-bit sums of the same operands."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _stream():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _check(got, want, scale, k, digits, what):
+    # one rounding of the result to `digits` binary digits, and fp32 sums of k products whose absolute values add up to `scale`
+    bound = want.abs() * 2.0 ** -digits + scale * (k * 2.0 ** -24) + 1e-7
+    over = ((got.double() - want).abs() / bound).max().item()
+    assert over <= 1.0, f"{what}: {over:.2f} of the bound"
+
+
+@pytest.mark.parametrize("tokens", [65, 128, 255, 256, 257, 2049])
+@pytest.mark.parametrize("n_out,k,ld", [(128, 64, 128), (384, 200, 392), (1000, 136, 1000), (2080, 512, 2083)])
+def test_dense_pairs(tokens, n_out, k, ld):
+    """Odd column tiles (the second CTA of a pair has none or a part), k that ends inside a block, tokens around a tile's and a
+    band's end, rows that 16-byte stores cannot reach; both output types.  Nothing beyond a row's n_out columns is written."""
+    from lmdeploy_b200 import lib as l
+    g = torch.Generator(device="cuda").manual_seed(tokens + n_out)
+    x = torch.randn(tokens, k, device="cuda", generator=g).bfloat16()
+    w = torch.randn(n_out, k, device="cuda", generator=g).bfloat16()
+    want, scale = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    h = l.default_handle(0)
+    for f32 in (0, 1):
+        out = torch.full((tokens, ld), 7.0, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+        l.check(l.lib.tm_gemm_dense(h.ptr, out.data_ptr(), ld, f32, x.data_ptr(), k, w.data_ptr(), k, tokens, n_out, k, l.TM_DTYPE_BF16,
+                                    _stream()), "tm_gemm_dense")
+        h.check_device_status(torch.cuda.current_stream().cuda_stream)
+        _check(out[:, :n_out], want, scale, k, 24 if f32 else 8, (tokens, n_out, k, f32))
+        assert bool((out[:, n_out:] == 7.0).all())
+
+
+@pytest.mark.parametrize("n,k,silu,tokens", [(4128, 2048, False, 1300), (4128, 2048, False, 2049), (7168, 8192, True, 1300), (4160, 4096, True, 1300),
+                                             (4160, 4096, True, 2049), (20512, 4096, False, 3001)])
+def test_expanded_weight(n, k, silu, tokens, monkeypatch):
+    """Sizes that the launch rule sends through expanded rows (the scratch of a handle of its own: one piece, or several where the
+    weight does not fit), feature counts that fill no tile of a pair."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    monkeypatch.setenv("TM_B200_GEMM_SCRATCH_MB", "64")
+    h = l.Handle(0)
+    w = cases._linear(cases._gen(3, n), n, k)
+    exact = cases._exact_weight(cases._gen(3, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    out = torch.empty(tokens, n // 2 if silu else n, dtype=torch.float16, device="cuda")
+    launches = h.launch_count()
+    l.check(l.lib.tm_gemm_s4_f16(h.ptr, out.data_ptr(), w.kernel.data_ptr(), x.data_ptr(), w.scales_and_zeros.data_ptr(), n, tokens, k, 128,
+                                 int(silu), None, 0, _stream()), "tm_gemm_s4_f16")
+    h.check_device_status(torch.cuda.current_stream().cuda_stream)
+    pieces = -(-n * k * 2 // (64 << 20))
+    assert h.launch_count() - launches == 2 * pieces
+    y, scale = x.double() @ exact, x.double().abs() @ exact.abs()
+    if not silu:
+        _check(out, y, scale, k, 11, (n, k, tokens))
+        return
+    # gate and up are rounded to fp16 first; |silu'| <= 1.1
+    slack = y.abs() * 2.0 ** -11 + scale * (k * 2.0 ** -24)
+    gate, up = y[:, 0::2], y[:, 1::2]
+    want = torch.nn.functional.silu(gate) * up
+    bound = want.abs() * 2.0 ** -10 + 1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2] + 1e-5
+    over = ((out.double() - want).abs() / bound).max().item()
+    assert over <= 1.0, f"{over:.2f} of the bound"
