@@ -63,7 +63,7 @@ TM_API int tm_check_device_status(tm_handle* h, void* stream, unsigned* word);
 /* Number of kernel launches issued through this handle since creation. */
 TM_API unsigned long long tm_launch_count(const tm_handle* h);
 /* Tuning knobs of this handle (no reference counterpart; the same knobs are read from the environment
- * at tm_create).  `name`: "gemm_tc_min_n" (token count from which the tcgen05 GEMM is used),
+ * at tm_create).  `name`: "gemm_tc_min_n" (token count from which the tcgen05 GEMM is used; by the product's size unless set),
  * "pdl_direct" (1: GEMM / attention calls made directly through the handle launch with programmatic stream
  * serialization, as the decode driver's do; only where no kernel ahead in the stream writes weights or cached rows),
  * "gemm_wait_cycles" (bound of the tcgen05 GEMM's wait for the partners of a split tile, 0 = default; tests),

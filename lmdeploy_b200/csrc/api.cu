@@ -12,9 +12,22 @@ using namespace tmb;
 namespace tmb {
 thread_local const GemmNormFusion* g_gemm_fusion = nullptr;
 
+// The tcgen05 kernel, or the small-token ones?  Unless the caller drew the line: from 17 tokens on, and with 9 to 16 except
+//  - products that the column-owner kernel does in one go of short rows, where the other's set-up and exchange weigh more than
+//    its own re-reading of the activations (us, column owner / tcgen05: 4096 x 4096 with 12 tokens 9.0 / 10.0, 8192 x 1024 with
+//    16 tokens 6.2 / 8.2; 4096 x 11008 with 9 tokens 16.1 / 15.3, 8192 x 3584 with 16 13.8 / 12.3);
+//  - weights so large that the expansion is all of the time (57344 x 8192: stream-K 87, tcgen05 110; 8192 x 28672: 52 / 49).
+static bool gemm_uses_tc(const tm_handle* h, int m, int n, int k)
+{
+    if (h->gemm_tc_min_n >= 0) return n >= h->gemm_tc_min_n;
+    if (n >= 17 || n <= 8) return n >= 17;
+    if ((long long)m * k > 64ll * 256 * 128 * h->sm_count) return false;
+    return (long long)n * k > 52 * 1024 || h->gemv_cols != 1 || gemm_small_plan(m, n, k, h->sm_count, h->max_smem, h->gemv_cols).cols_tiles == 0;
+}
+
 bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k)
 {
-    if (!h || n < h->gemm_tc_min_n || n > 128 || k % 128 || m % 32) return false;
+    if (!h || !gemm_uses_tc(h, m, n, k) || n > 128 || k % 128 || m % 32) return false;
     const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count);
     return gemm_tc_all_tiles_split(pl, k) && pl.workspace_floats * sizeof(float) <= h->scratch_bytes && pl.counter_ints <= h->counter_ints;
 }
@@ -55,7 +68,9 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
     if (type != TM_GEMM_PLAIN && type != TM_GEMM_FUSED_SILU_FFN) return TM_ERR_UNSUPPORTED;
     if (type == TM_GEMM_FUSED_SILU_FFN && m % 64) return TM_ERR_UNSUPPORTED;
 
-    if (!workspace && !g_gemm_fusion && n >= h->gemm_tc_min_n) {
+    // a caller's workspace has the size that tm_gemm_s4_f16_workspace_bytes gave: the small-token kernels' up to 16 tokens
+    const bool tc = workspace ? n >= (h->gemm_tc_min_n >= 0 ? h->gemm_tc_min_n : 17) : gemm_uses_tc(h, m, n, k);
+    if (!workspace && !g_gemm_fusion && tc) {
         const int columns = gemm_expanded_columns(h, m, n, k);
         if (columns > 0) {
             GemmTcParams p{};
@@ -64,7 +79,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream);
         }
     }
-    if (n >= h->gemm_tc_min_n) {
+    if (tc) {
         // tensor-core tiles; token ranges that would overflow the scratch go in several launches
         const size_t n_out_tc = type == TM_GEMM_FUSED_SILU_FFN ? (size_t)m / 2 : (size_t)m;
         int          per      = n;

@@ -22,7 +22,7 @@ struct GemmSmallParams {
     int                  N, T, K;
     int                  fused_silu;
     // filled in by gemm_small_launch from the plan
-    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, stages;
+    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, stages, cluster;
 };
 
 struct GemmSmallPlan {
@@ -35,7 +35,8 @@ struct GemmSmallPlan {
     int    slots_per_chunk;  // split-K scratch slots per token chunk (= ctas + n_col_tiles)
     int    stages;
     int    cols_tiles;     // 1 or 2: the column-owner kernel runs instead, on strips of that many 32-column tiles (up to 8 tokens,
-                           // at least one strip per SM); 0: the split-K kernel
+                           // or 16 tokens); 0: the split-K kernel
+    int    cols_cluster;   // CTAs that share a strip
     size_t smem_bytes;
     size_t workspace_floats;
     size_t counter_ints;

@@ -27,6 +27,7 @@
 #include "gemm_s4_f16.h"
 #include "tm_b200.h"
 
+#include <algorithm>
 #include <mutex>
 
 #ifdef TM_B200_GEMM_TRACE
@@ -66,6 +67,7 @@ constexpr int kUnitRows     = 64;   // input rows per unit: two 32-row slabs
 constexpr int kWarps        = 8;
 constexpr int kTilesPerWarp = kTilesPerUnit / kWarps;        // 2
 constexpr int kThreads      = kWarps * 32;
+constexpr int kMaxCluster   = 8;    // CTAs that share a strip of the column-owner kernel
 constexpr int kSlabBytes    = kTilesPerWarp * kTileBytes;    // a warp's part of one slab: 1 KB
 constexpr int kWarpStage    = 2 * kSlabBytes + 256;          // two slabs + {zero, scale} of the 64 columns
 
@@ -497,9 +499,9 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
 #endif
 }
 
-// ---- column-owner variant for up to 8 tokens --------------------------------------------------------------------
-// Where the weight has at least as many column strips as the device has SMs (the qkv and gate/up projections),
-// nothing needs to be split between CTAs: a CTA owns one strip of TILES packed tiles (32 or 64 columns: 512 B or 1 KB
+// ---- column-owner variant for up to 16 tokens -------------------------------------------------------------------
+// Where the weight's column strips are resident at once (the qkv, output and down projections), nothing needs to go through
+// scratch: a CTA, or a cluster of them, owns one strip of TILES packed tiles (32 or 64 columns: 512 B or 1 KB
 // contiguous per 32-row slab) over the whole K range, its eight warps take the 128-row quantisation groups round
 // robin (warp w: groups w, w + 8, ...), each through a private cp.async ring of whole groups (2 KB of weight per tile
 // + its {zero, scale}), and the eight partial sums meet once in shared memory, in a fixed order.  No scratch, no
@@ -525,8 +527,22 @@ __device__ __forceinline__ void cp_async_wait_pending(int n)
 
 __host__ __device__ constexpr int co_stage_bytes(int tiles) { return tiles * (4 * kTileBytes + 128); }  // four slabs + {zero, scale} per tile
 
-template<int TILES, bool kOne>
-__global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols_kernel(GemmSmallParams p)
+// kSplit: too few strips for the device's slots.  A cluster of p.cluster CTAs shares a strip, its warps take the groups round
+// robin across all of them, and the CTAs' sums meet in the shared memory of the first, added in the order of the ranks.  No
+// scratch, tickets or fences here either.  Against the split through scratch (stream-K), us with 1 / 8 tokens: 4096 x 4096
+// 8.5 / 15.0 -> 6.8 / 8.5, 4096 x 11008 13.4 / 19.1 -> 10.7 / 14.2, 1280 x 8192 9.2 / 19.3 -> 4.8 / 6.2.
+// NT: eight-token tiles (kOne: NT = 1).
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template<int TILES, bool kOne, bool kSplit, int NT>
+__global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16_cols_kernel(GemmSmallParams p)
 {
     constexpr int kStage = co_stage_bytes(TILES);
     constexpr int kSlab  = TILES * kTileBytes;  // one 32-row slab of the strip
@@ -541,14 +557,18 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
 
     const int    n_tiles32   = p.N / kColsPerTile;
     const int    G           = p.K / 128;
-    const int    tile0       = blockIdx.x * TILES;
+    const int    parts       = kSplit ? p.cluster : 1;                   // CTAs that share the strip
+    const int    rank        = kSplit ? (int)blockIdx.x % parts : 0;
+    const int    tile0       = (kSplit ? (int)blockIdx.x / parts : (int)blockIdx.x) * TILES;
+    const int    warps       = kWarps * parts, gw = rank * kWarps + warp;  // warps of the strip, and this one among them
     const int    step        = (TILES == 2 && tile0 + 1 < n_tiles32) ? kTileBytes : 0;  // a strip at the edge of N: one tile, read twice
     const size_t slab_stride = (size_t)n_tiles32 * kTileBytes;
-    const int    n_groups    = warp < G ? (G - 1 - warp) / kWarps + 1 : 0;
+    const int    n_groups    = gw < G ? (G - 1 - gw) / warps + 1 : 0;
+    if (kSplit) cluster_arrive();  // that every CTA of the strip runs: waited for ahead of the first access to another's memory
 
     const uint32_t       ring_s = smem_s + warp * (ST * kStage);
-    const unsigned char* i_w    = p.A + ((size_t)(4 * warp) * n_tiles32 + tile0) * kTileBytes + lane * 16;
-    const unsigned char* i_q    = p.Q + ((size_t)warp * p.N + (size_t)tile0 * kColsPerTile) * 4 + lane * 16;
+    const unsigned char* i_w    = p.A + ((size_t)(4 * gw) * n_tiles32 + tile0) * kTileBytes + lane * 16;
+    const unsigned char* i_q    = p.Q + ((size_t)gw * p.N + (size_t)tile0 * kColsPerTile) * 4 + lane * 16;
     const bool           i_qok  = lane < 8 * TILES && tile0 * kColsPerTile + lane * 4 < p.N;
     auto issue_group = [&](int slot) {
         const uint32_t dst = ring_s + slot * kStage;
@@ -559,8 +579,8 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
         }
         if (i_qok) cp_async16(dst + 4 * kSlab + lane * 16, i_q);
         cp_async_commit();
-        i_w += (size_t)(4 * kWarps) * slab_stride;  // this warp's next group: eight groups further down
-        i_q += (size_t)kWarps * p.N * 4;
+        i_w += (size_t)(4 * warps) * slab_stride;  // this warp's next group: eight groups (of a strip's CTA) further down
+        i_q += (size_t)warps * p.N * 4;
     };
     // the packed weight is written by no kernel: its first copies start ahead of the wait for the kernel before
     int issued = 0;
@@ -569,26 +589,32 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
     pdl_launch_dependents();
 
     // B fragments: token = fragment row (tokens beyond T repeat the last one: their columns are never stored)
-    const uint32_t* x_row = reinterpret_cast<const uint32_t*>(p.X + (size_t)min(r, p.T - 1) * p.K * 2) + c;
+    const uint32_t* x_row[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) x_row[j] = reinterpret_cast<const uint32_t*>(p.X + (size_t)min(8 * j + r, p.T - 1) * p.K * 2) + c;
 
-    float tot[TILES][2][4];
+    float tot[TILES][2][NT][4];
 #pragma unroll
     for (int w = 0; w < TILES; ++w)
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) tot[w][a][i] = 0.f;
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) tot[w][a][j][i] = 0.f;
     const uint32_t ones[4] = {0x3c003c00u, 0x3c003c00u, 0x3c003c00u, 0x3c003c00u};
 
     int slot = 0;  // ring slot of group `it`
     for (int it = 0; it < n_groups; ++it) {
-        const int g = warp + it * kWarps;
+        const int g = gw + it * warps;
         // the group's activations: k = 128 g + 32 h + 8 i + 2 c, + 1
-        uint32_t bf[4][4];
+        uint32_t bf[NT][4][4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h)
+        for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) bf[h][i] = __ldg(x_row + g * 64 + h * 16 + i * 4);
+            for (int h = 0; h < 4; ++h)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) bf[j][h][i] = __ldg(x_row[j] + g * 64 + h * 16 + i * 4);
         uint2 xs = make_uint2(0u, 0u);
         if (kOne) xs = __ldg(reinterpret_cast<const uint2*>(p.X) + g * 32 + lane);  // this lane's four values of the group
         // copies complete in the order they were committed: group `it` has landed once at most issued - it - 1 are pending
@@ -614,26 +640,29 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
                 sh[w][a] = q_hi.y * 0.0625f;
             }
         }
-        float acc[TILES][2][4];
-        float sx[4];
+        float acc[TILES][2][NT][4];
+        float sx[NT][4];
         if (kOne) {
             float part = (__half2float(__ushort_as_half((unsigned short)(xs.x & 0xffffu))) + __half2float(__ushort_as_half((unsigned short)(xs.x >> 16))))
                          + (__half2float(__ushort_as_half((unsigned short)(xs.y & 0xffffu))) + __half2float(__ushort_as_half((unsigned short)(xs.y >> 16))));
 #pragma unroll
             for (int o = 16; o >= 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-            sx[0] = sx[1] = sx[2] = sx[3] = part;  // every column is the one token
+            sx[0][0] = sx[0][1] = sx[0][2] = sx[0][3] = part;  // every column is the one token
         }
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             if (!kOne) {
                 // group sum of the activations, in the accumulator layout (every row alike)
-                if (h == 0) {
-                    mma_m16n8k16_init(sx, ones, bf[h][0], bf[h][1]);
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    if (h == 0) {
+                        mma_m16n8k16_init(sx[j], ones, bf[j][h][0], bf[j][h][1]);
+                    }
+                    else {
+                        mma_m16n8k16(sx[j], ones, bf[j][h][0], bf[j][h][1]);
+                    }
+                    mma_m16n8k16(sx[j], ones, bf[j][h][2], bf[j][h][3]);
                 }
-                else {
-                    mma_m16n8k16(sx, ones, bf[h][0], bf[h][1]);
-                }
-                mma_m16n8k16(sx, ones, bf[h][2], bf[h][3]);
             }
             uint32_t af[TILES][4][4];
 #pragma unroll
@@ -649,11 +678,14 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
                 for (int w = 0; w < TILES; ++w) {
 #pragma unroll
                     for (int a = 0; a < 2; ++a) {
-                        if (h == 0 && k16 == 0) {
-                            mma_m16n8k16_init(acc[w][a], af[w][2 * k16 + a], bf[h][0], bf[h][1]);
-                        }
-                        else {
-                            mma_m16n8k16(acc[w][a], af[w][2 * k16 + a], bf[h][2 * k16], bf[h][2 * k16 + 1]);
+#pragma unroll
+                        for (int j = 0; j < NT; ++j) {
+                            if (h == 0 && k16 == 0) {
+                                mma_m16n8k16_init(acc[w][a][j], af[w][2 * k16 + a], bf[j][h][0], bf[j][h][1]);
+                            }
+                            else {
+                                mma_m16n8k16(acc[w][a][j], af[w][2 * k16 + a], bf[j][h][2 * k16], bf[j][h][2 * k16 + 1]);
+                            }
                         }
                     }
                 }
@@ -663,33 +695,63 @@ __global__ void __launch_bounds__(kThreads, TILES == 1 ? 3 : 2) gemm_s4_f16_cols
 #pragma unroll
         for (int w = 0; w < TILES; ++w)
 #pragma unroll
-            for (int a = 0; a < 2; ++a) {
-                tot[w][a][0] = fmaf(sl[w][a], fmaf(-zl[w][a], sx[0], acc[w][a][0]), tot[w][a][0]);
-                tot[w][a][1] = fmaf(sl[w][a], fmaf(-zl[w][a], sx[1], acc[w][a][1]), tot[w][a][1]);
-                tot[w][a][2] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[0], acc[w][a][2]), tot[w][a][2]);
-                tot[w][a][3] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[1], acc[w][a][3]), tot[w][a][3]);
-            }
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    tot[w][a][j][0] = fmaf(sl[w][a], fmaf(-zl[w][a], sx[j][0], acc[w][a][j][0]), tot[w][a][j][0]);
+                    tot[w][a][j][1] = fmaf(sl[w][a], fmaf(-zl[w][a], sx[j][1], acc[w][a][j][1]), tot[w][a][j][1]);
+                    tot[w][a][j][2] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[j][0], acc[w][a][j][2]), tot[w][a][j][2]);
+                    tot[w][a][j][3] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[j][1], acc[w][a][j][3]), tot[w][a][j][3]);
+                }
         slot = (slot == ST - 1) ? 0 : slot + 1;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // the rings are free: they now hold the eight warps' partial sums, [warp][TILES x 8 values][lane]
-    constexpr int kVals = TILES * 8;
+    constexpr int kVals = TILES * 8 * NT;
     float*        red   = reinterpret_cast<float*>(smem_raw);
 #pragma unroll
     for (int w = 0; w < TILES; ++w)
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) red[(warp * kVals + (w * 2 + a) * 4 + i) * 32 + lane] = tot[w][a][i];
-    __syncthreads();
-    for (int e = warp; e < kVals; e += kWarps) {
-        float v = 0.f;
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int wp = 0; wp < kWarps; ++wp) v += red[(wp * kVals + e) * 32 + lane];  // fixed order
-        const int  w     = e >> 3, a = (e >> 2) & 1, i = e & 3;
-        const int  n     = (tile0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8;
-        const int  t     = 2 * c + (i & 1);
-        const bool valid = tile0 + w < n_tiles32 && t < p.T;
+                for (int i = 0; i < 4; ++i) red[(warp * kVals + ((w * 2 + a) * NT + j) * 4 + i) * 32 + lane] = tot[w][a][j][i];
+    __syncthreads();
+    float sums[kVals / kWarps];  // values warp, warp + 8, ...
+#pragma unroll
+    for (int q = 0; q < kVals / kWarps; ++q) {
+        sums[q] = 0.f;
+#pragma unroll
+        for (int wp = 0; wp < kWarps; ++wp) sums[q] += red[(wp * kVals + warp + q * kWarps) * 32 + lane];  // fixed order
+    }
+    if (kSplit) {
+        // [rank][value][lane] behind the rings of the first CTA
+        const uint32_t inbox = smem_s + (uint32_t)(kWarps * ST * kStage);
+        cluster_wait();
+#pragma unroll
+        for (int q = 0; q < kVals / kWarps; ++q) {
+            uint32_t at;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(inbox + (uint32_t)((rank * kVals + warp + q * kWarps) * 32 + lane) * 4), "r"(0));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(sums[q]) : "memory");
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (rank != 0) return;
+        const float* in = reinterpret_cast<const float*>(smem_raw + kWarps * ST * kStage);
+#pragma unroll
+        for (int q = 0; q < kVals / kWarps; ++q) {
+            sums[q] = 0.f;
+            for (int k = 0; k < parts; ++k) sums[q] += in[(k * kVals + warp + q * kWarps) * 32 + lane];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kVals / kWarps; ++q) {
+        const float v     = sums[q];
+        const int   e     = warp + q * kWarps, w = e / (8 * NT), a = e / (4 * NT) & 1, j = e / 4 % NT, i = e & 3;
+        const int   n     = (tile0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8;
+        const int   t     = 8 * j + 2 * c + (i & 1);
+        const bool  valid = tile0 + w < n_tiles32 && t < p.T;
         if (p.fused_silu) {
             // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair; the partner column n ^ 1 lives in lane ^ 4
             const float mine  = __half2float(__float2half_rn(v));
@@ -742,14 +804,18 @@ GemmSmallPlan gemm_small_plan(int N, int T, int K, int sm_count, int max_smem, i
     // Measured on the 7B shapes: with all strips resident at once (qkv: 384 strips for 444 slots) it wins at every
     // token count up to 8; with more strips than slots (gate/up: 688) it wins at one token, ties up to four and loses at
     // eight, where every CTA re-reads 64 KB of activations.
-    const int  co_slots   = sm_count * (tiles == 2 ? 2 : 3);
-    const bool worthwhile = strips >= sm_count && (strips <= co_slots || T == 1);
-    pl.cols_tiles         = (cols_variant != 0 && T <= 8 && worthwhile) ? tiles : 0;
+    const int  wide       = T > 8 ? 2 : 1;  // eight-token tiles
+    const int  co_slots   = sm_count * (tiles * wide == 1 ? 3 : 2);
+    const bool worthwhile = strips <= co_slots || T == 1;
+    pl.cols_tiles         = (cols_variant != 0 && T <= 8 * (tiles == 1 ? 2 : 1) && worthwhile) ? tiles : 0;
     if (pl.cols_tiles) {
-        const int per_warp = (K / 128 + kWarps - 1) / kWarps;  // groups of the busiest warp
-        pl.ctas       = strips;
+        // few strips: clusters of up to eight CTAs share one, as many as have a slot at once and a group for each warp
+        const int warps_full = (K / 128 + kWarps - 1) / kWarps;
+        pl.cols_cluster      = std::max(1, std::min({kMaxCluster, co_slots / strips, warps_full}));
+        const int per_warp   = (K / 128 + kWarps * pl.cols_cluster - 1) / (kWarps * pl.cols_cluster);  // groups of the busiest warp
+        pl.ctas       = strips * pl.cols_cluster;
         pl.stages     = tiles == 2 ? 3 : (per_warp < 2 ? 2 : (per_warp > 4 ? 4 : per_warp));
-        pl.smem_bytes = (size_t)kWarps * pl.stages * co_stage_bytes(tiles);
+        pl.smem_bytes = (size_t)kWarps * pl.stages * co_stage_bytes(tiles) + (pl.cols_cluster > 1 ? (size_t)pl.cols_cluster * tiles * wide * 1024 : 0);
     }
     return pl;
 }
@@ -761,14 +827,20 @@ cudaError_t gemm_small_prepare(int max_smem)
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(gemm_s4_f16_small_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     if (e != cudaSuccess) return e;
-    constexpr int kCoSmemMax = kWarps * 4 * co_stage_bytes(2);
-    e = cudaFuncSetAttribute(gemm_s4_f16_cols_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoSmemMax);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_s4_f16_cols_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoSmemMax);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_s4_f16_cols_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoSmemMax);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(gemm_s4_f16_cols_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoSmemMax);
+    constexpr int kCoSmemMax = kWarps * 4 * co_stage_bytes(2) + kMaxCluster * 2 * 1024;
+    auto raise = [&](auto kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoSmemMax);
+    };
+    raise(gemm_s4_f16_cols_kernel<1, true, false, 1>);
+    raise(gemm_s4_f16_cols_kernel<1, true, true, 1>);
+    raise(gemm_s4_f16_cols_kernel<1, false, false, 1>);
+    raise(gemm_s4_f16_cols_kernel<1, false, true, 1>);
+    raise(gemm_s4_f16_cols_kernel<1, false, false, 2>);
+    raise(gemm_s4_f16_cols_kernel<1, false, true, 2>);
+    raise(gemm_s4_f16_cols_kernel<2, true, false, 1>);
+    raise(gemm_s4_f16_cols_kernel<2, true, true, 1>);
+    raise(gemm_s4_f16_cols_kernel<2, false, false, 1>);
+    raise(gemm_s4_f16_cols_kernel<2, false, true, 1>);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(gemm_s4_f16_small_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
 }
@@ -783,13 +855,19 @@ cudaError_t gemm_small_launch(const GemmSmallPlan& pl, GemmSmallParams p, cudaSt
     p.stages          = pl.stages;
     dim3 grid(pl.ctas, pl.t_chunks);
     dim3 block(kThreads);
+    p.cluster = pl.cols_cluster;
+    auto columns = [&](auto whole, auto split) {
+        return pl.cols_cluster > 1 ? launch_cluster_kernel(split, grid, block, pl.cols_cluster, pl.smem_bytes, st, pdl, p) :
+                                     launch_kernel(whole, grid, block, pl.smem_bytes, st, pdl, p);
+    };
     if (pl.cols_tiles == 1) {
-        return p.T == 1 ? launch_kernel(gemm_s4_f16_cols_kernel<1, true>, grid, block, pl.smem_bytes, st, pdl, p) :
-                          launch_kernel(gemm_s4_f16_cols_kernel<1, false>, grid, block, pl.smem_bytes, st, pdl, p);
+        return p.T == 1 ? columns(gemm_s4_f16_cols_kernel<1, true, false, 1>, gemm_s4_f16_cols_kernel<1, true, true, 1>) :
+               p.T <= 8 ? columns(gemm_s4_f16_cols_kernel<1, false, false, 1>, gemm_s4_f16_cols_kernel<1, false, true, 1>) :
+                          columns(gemm_s4_f16_cols_kernel<1, false, false, 2>, gemm_s4_f16_cols_kernel<1, false, true, 2>);
     }
     if (pl.cols_tiles == 2) {
-        return p.T == 1 ? launch_kernel(gemm_s4_f16_cols_kernel<2, true>, grid, block, pl.smem_bytes, st, pdl, p) :
-                          launch_kernel(gemm_s4_f16_cols_kernel<2, false>, grid, block, pl.smem_bytes, st, pdl, p);
+        return p.T == 1 ? columns(gemm_s4_f16_cols_kernel<2, true, false, 1>, gemm_s4_f16_cols_kernel<2, true, true, 1>) :
+                          columns(gemm_s4_f16_cols_kernel<2, false, false, 1>, gemm_s4_f16_cols_kernel<2, false, true, 1>);
     }
     switch (pl.nt) {
         case 1: return launch_kernel(gemm_s4_f16_small_kernel<1>, grid, block, pl.smem_bytes, st, pdl, p);

@@ -95,7 +95,7 @@ extern "C" int tm_create(tm_handle** out, int device)
     h->lm_head_cublas = env_int("TM_B200_LM_HEAD_CUBLAS", 0);
     h->fold_norm      = env_int("TM_B200_FOLD_NORM", 1);
     h->gemv_cols      = env_int("TM_B200_GEMV_COLS", 1);
-    h->gemm_tc_min_n = env_int("TM_B200_GEMM_TC_MIN", 17);
+    h->gemm_tc_min_n = env_int("TM_B200_GEMM_TC_MIN", -1);
     h->mmha_chunk  = env_int("TM_B200_MMHA_CHUNK", 0);
     h->mmha_warps  = env_int("TM_B200_MMHA_WARPS", 0);
     cudaSetDevice(prev);

@@ -25,7 +25,7 @@ struct tm_handle {
     unsigned long long launches        = 0;
     int                mmha_chunk      = 0;  // 0 = automatic; TM_B200_MMHA_CHUNK overrides
     int                mmha_warps      = 0;  // 0 = automatic; TM_B200_MMHA_WARPS (1, 2 or 4) overrides
-    int                gemm_tc_min_n   = 17; // token count from which the tcgen05 kernel is used; TM_B200_GEMM_TC_MIN overrides
+    int                gemm_tc_min_n   = -1; // token count from which the tcgen05 kernel is used (-1: by the product's size); TM_B200_GEMM_TC_MIN overrides
     int                gemm_wait_cycles = 0; // 0 = default bound of the split-tile wait of the tcgen05 GEMM (option "gemm_wait_cycles")
     int                pdl_direct      = 0;  // option "pdl_direct": direct GEMM / attention calls launch with programmatic serialization too
     int                p2p_allreduce   = 1;  // TM_B200_P2P_ALLREDUCE / option "p2p_allreduce": peer-memory all-reduce + norm in the decode step

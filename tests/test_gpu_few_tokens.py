@@ -1,0 +1,40 @@
+"""W4A16 products with up to 17 tokens at the sizes where the launch rules change: strips shared by clusters of every size, groups
+that leave warps without work, both sides of the line to the tensor-core kernel, against 64-bit sums."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# (output features, input features): clusters of 1, 2, 3, 4, 7 and 8 CTAs on a strip, and a strip count that fills no cluster evenly
+SHAPES = [(8192, 1024), (7104, 4096), (4096, 4096), (4096, 11008), (3520, 8192), (2048, 8192), (1280, 8192), (32, 8192), (64, 128)]
+
+
+@pytest.mark.parametrize("n,k", SHAPES)
+@pytest.mark.parametrize("silu", [False, True])
+def test_strips_shared_by_clusters(n, k, silu):
+    from lmdeploy_b200 import turbomind as tm
+    from perf import cases
+    if silu and n % 64:
+        pytest.skip("pairs of columns come in blocks of 64")
+    w = cases._linear(cases._gen(5, n), n, k)
+    exact = cases._exact_weight(cases._gen(5, n), n, k)
+    op = tm.LlamaLinear(0)
+    for tokens in (1, 2, 8, 9, 12, 16, 17):
+        x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).half()
+        n_out = n // 2 if silu else n
+        buf = torch.full((tokens + 1, n_out), 777.0, dtype=torch.float16, device="cuda")
+        op.forward(buf[:tokens], x, tokens, w, op.kFusedSiluFfn if silu else op.kGemm)
+        op.gemm_s4_f16_.handle.check_device_status(torch.cuda.current_stream().cuda_stream)
+        assert bool((buf[tokens] == 777.0).all())
+        y, size = x.double() @ exact, x.double().abs() @ exact.abs()
+        # one rounding of the result, and weights that are not rounded to fp16 where the products are summed per group
+        slack = y.abs() * 2.0 ** -11 + size * (2.0 ** -11 + k * 2.0 ** -24) + 1e-7
+        if silu:
+            gate, up = y[:, 0::2], y[:, 1::2]
+            y = torch.nn.functional.silu(gate) * up
+            # gate and up are rounded to fp16 first (again 2^-11); |silu'| <= 1.1
+            slack = 2 * (1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2]) + y.abs() * 2.0 ** -11 + 1e-6
+        over = ((buf[:tokens].double() - y).abs() / slack).max().item()
+        assert over <= 1.0, f"{n} x {k}, {tokens} tokens: {over:.2f} of the bound"
