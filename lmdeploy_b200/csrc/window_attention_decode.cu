@@ -100,9 +100,26 @@ __global__ void __launch_bounds__(kThreads) window_step_kernel(const StepParams 
     const int              slot0 = vis.first % a.ring;  // the visible tokens span less than a ring
     const uint32_t         sm_b = smem_u32(sm), ring = sm_b + L::kQ + warp * L::kRing;
 
+    const bool             full_rows = a.dim == D && a.vdim == D;
+
     auto fetch = [&](int b, int stage) {
         const uint32_t dst = ring + stage * 2 * L::kTile;
-        if (b < blk1) {
+        const int      key0 = b * kKeys, ring0 = slot0 + key0 - vis.blocks, slot = ring0 >= a.ring ? ring0 - a.ring : ring0;
+        const bool     pooled = key0 + kKeys <= vis.blocks;
+        if (b < blk1 && full_rows && key0 + kKeys <= total && (pooled || (key0 >= vis.blocks && slot + kKeys <= a.ring))) {
+            // sixteen whole rows that lie one after the other: all but the blocks at an edge
+            const int      first = pooled ? key0 : slot, chunk = lane % (D / 8), row = lane / (D / 8);
+            const E* const k_src = (pooled ? k_blk : k_tok) + (size_t)(first + row) * D + chunk * 8;
+            const E* const v_src = (pooled ? v_blk : v_tok) + (size_t)(first + row) * D + chunk * 8;
+#pragma unroll
+            for (int r = 0; r < kKeys * D / 8 / 32; ++r) {
+                constexpr int  kStep = 32 / (D / 8);  // rows that the warp's lanes cover at a time
+                const uint32_t at    = sw<D>(row + r * kStep, chunk);
+                cp_async16z(dst + at, k_src + r * kStep * D, 16);
+                cp_async16z(dst + L::kTile + at, v_src + r * kStep * D, 16);
+            }
+        }
+        else if (b < blk1) {
 #pragma unroll
             for (int r = 0; r < kKeys * D / 8 / 32; ++r) {
                 const int  c = lane + r * 32, row = c / (D / 8), chunk = c % (D / 8), idx = b * kKeys + row;
@@ -239,12 +256,18 @@ __global__ void __launch_bounds__(kThreads) window_step_kernel(const StepParams 
             }
         }
         const uint32_t pf[4] = {pack_bf16(s[0][0], s[0][1]), pack_bf16(s[0][2], s[0][3]), pack_bf16(s[1][0], s[1][1]), pack_bf16(s[1][2], s[1][3])};
+        // the maximum moves a few times in a row's life
+        if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[n][e] *= alpha[e >> 1];
+            }
+        }
 #pragma unroll
         for (int n = 0; n < D / 8; n += 2) {
             uint32_t f[4];  // keys 0-7 / d low, keys 8-15 / d low, keys 0-7 / d high, keys 8-15 / d high
             ldsm4t(vt + sw<D>(lane & 15, n + (lane >> 4)), f);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[n][e] *= alpha[e >> 1], o[n + 1][e] *= alpha[e >> 1];
             mma_bf16(o[n], pf, f[0], f[1]);
             mma_bf16(o[n + 1], pf, f[2], f[3]);
         }
@@ -292,9 +315,17 @@ __global__ void __launch_bounds__(kThreads) window_step_kernel(const StepParams 
         __syncthreads();
     };
     auto combine = [&](const float* src, int parts, int hh, int d) {
+        // eight parts on their way at a time, also the last ones (a loop's remainder would wait for them one by one)
         float y = 0.f;
-#pragma unroll 8
-        for (int w = 0; w < parts; ++w) y = fmaf(s_m[hh][w], __ldcg(src + ((size_t)w * kHeads + hh) * (D + 2) + 2 + d), y);
+        for (int w0 = 0; w0 < parts; w0 += 8) {
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = __ldcg(src + ((size_t)min(w0 + j, parts - 1) * kHeads + hh) * (D + 2) + 2 + d);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (w0 + j < parts) y = fmaf(s_m[hh][w0 + j], x[j], y);
+            }
+        }
         return y;
     };
     auto store = [&](int hh, int d, float y) {
@@ -401,13 +432,22 @@ int window_attention_step(tm_handle* h, const WindowAttention& a, const MixerCal
     const int D   = a.dim <= 64 && a.vdim <= 64 ? 64 : 128;
     // the bound on the visible keys is the host's
     const long long items = (long long)c.batch * a.kv_heads * p.head_blocks;
-    const long long keys  = a.window > 0 ? (long long)a.window + (a.pool > 0 ? c.max_context / a.pool : 0) : c.max_context;
-    // two CTAs fit an SM; a CTA's set-up and the merge cost as much as hundreds of keys, so sequences are split only to
-    // occupy SMs that would idle, each warp with at least two blocks of keys
-    const long long most = std::min<long long>(kMaxSplits, std::max(1ll, keys / (kKeys * kWarps * 2)));
-    long long splits     = std::min((2ll * h->sm_count + items - 1) / items, most);
-    if (items >= h->sm_count) splits = 1;
-    splits = std::min(splits, (long long)(h->attn_scratch_bytes / (items * kHeads * (D + 2) * 4)));
+    const long long seen  = a.window > 0 ? std::min<long long>(a.window, c.max_context) : c.max_context;
+    const long long keys  = seen + (a.window > 0 && a.pool > 0 ? (c.max_context - seen) / a.pool : 0);
+    const int       blocks = (int)((keys + kKeys - 1) / kKeys);
+    // Two CTAs fit an SM: no more splits than have a slot at once (16 sequences x 8 kv heads, 2177 keys, us with 1 / 2 / 3 / 4
+    // splits: 47 / 49 / 59 / 55), and of these the number that leaves the busiest warp the fewest blocks for what a split
+    // costs in the merge (one sequence with 1 / 2 / 4 / 8 / 16 / 32 splits: 43 / 33 / 27 / 25 / 25 / 29; a block takes a warp
+    // 0.62 us, the merge 2 and 0.12 a split; 200 keys: 16 unsplit, 18 with two or four).
+    const long long most = std::min<long long>(kMaxSplits, std::max(1ll, 2ll * h->sm_count / items));
+    long long splits = 1;
+    double    best   = 1e30;
+    for (long long n = 1; n <= most; ++n) {
+        const long long per_warp = ((blocks + n - 1) / n + kWarps - 1) / kWarps;
+        const double    us       = 0.62 * per_warp + (n > 1 ? 2.0 + 0.12 * n : 0.0);
+        if (us < best - 1e-9) best = us, splits = n;
+    }
+    splits = std::min<long long>(splits, (long long)(h->attn_scratch_bytes / (items * kHeads * (D + 2) * 4)));
     if (splits < 1 || items > (long long)h->attn_counter_ints) splits = 1;
     p.splits  = (int)splits;
     p.scratch = static_cast<float*>(h->attn_scratch);
