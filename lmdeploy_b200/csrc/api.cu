@@ -12,23 +12,22 @@ using namespace tmb;
 namespace tmb {
 thread_local const GemmNormFusion* g_gemm_fusion = nullptr;
 
-// The tcgen05 kernel, or the small-token ones?  Unless the caller drew the line: from 17 tokens on, and with 9 to 16 except
-//  - products that the column-owner kernel does in one go of short rows, where the other's set-up and exchange weigh more than
-//    its own re-reading of the activations (us, column owner / tcgen05: 4096 x 4096 with 12 tokens 9.0 / 10.0, 8192 x 1024 with
-//    16 tokens 6.2 / 8.2; 4096 x 11008 with 9 tokens 16.1 / 15.3, 8192 x 3584 with 16 13.8 / 12.3);
-//  - weights so large that the expansion is all of the time (57344 x 8192: stream-K 87, tcgen05 110; 8192 x 28672: 52 / 49).
+// The tcgen05 kernel, or the small-token ones?  Unless the caller drew the line: from 17 tokens on, and with 9 to 16 except for
+// products that the column-owner kernel does in one go of short rows, where the other's set-up and exchange weigh more than
+// its own re-reading of the activations (us, column owner / tcgen05: 4096 x 4096 with 12 tokens 9.0 / 9.9, 8192 x 1024 with
+// 16 tokens 6.2 / 8.4; 4096 x 11008 with 9 tokens 16.1 / 14.1, 8192 x 3584 with 16 13.8 / 11.6; stream-K for 57344 x 8192 with
+// 16 tokens 87 / 75).
 static bool gemm_uses_tc(const tm_handle* h, int m, int n, int k)
 {
     if (h->gemm_tc_min_n >= 0) return n >= h->gemm_tc_min_n;
     if (n >= 17 || n <= 8) return n >= 17;
-    if ((long long)m * k > 64ll * 256 * 128 * h->sm_count) return false;
     return (long long)n * k > 52 * 1024 || h->gemv_cols != 1 || gemm_small_plan(m, n, k, h->sm_count, h->max_smem, h->gemv_cols).cols_tiles == 0;
 }
 
 bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k)
 {
     if (!h || !gemm_uses_tc(h, m, n, k) || n > 128 || k % 128 || m % 32) return false;
-    const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count);
+    const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count, true);
     return gemm_tc_all_tiles_split(pl, k) && pl.workspace_floats * sizeof(float) <= h->scratch_bytes && pl.counter_ints <= h->counter_ints;
 }
 }
@@ -40,7 +39,7 @@ extern "C" size_t tm_gemm_s4_f16_workspace_bytes(int m, int n, int k)
     GemmSmallPlan pl = gemm_small_plan(m, n, k, 256, 227 * 1024);
     size_t        b  = pl.workspace_floats * sizeof(float) + pl.counter_ints * sizeof(int) + 256;
     if (n > 16) {
-        GemmTcPlan   tc = gemm_tc_plan(m, n, k, 256);
+        GemmTcPlan   tc = gemm_tc_plan(m, n, k, 256, false);
         const size_t t  = tc.workspace_floats * sizeof(float) + tc.counter_ints * sizeof(int) + 256;
         if (t > b) b = t;
     }
@@ -83,19 +82,24 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
         // tensor-core tiles; token ranges that would overflow the scratch go in several launches
         const size_t n_out_tc = type == TM_GEMM_FUSED_SILU_FFN ? (size_t)m / 2 : (size_t)m;
         int          per      = n;
+        bool         balance  = workspace == nullptr;
         for (;;) {
-            GemmTcPlan   pl   = gemm_tc_plan(m, per, k, h->sm_count);
+            GemmTcPlan   pl   = gemm_tc_plan(m, per, k, h->sm_count, balance);
             const size_t c_b  = ((pl.counter_ints * sizeof(int) + 255) / 256) * 256;
             const bool   fits = workspace ? workspace_bytes >= pl.workspace_floats * sizeof(float) + c_b :
                                             (pl.workspace_floats * sizeof(float) <= h->scratch_bytes
                                              && pl.counter_ints <= h->counter_ints);
             if (fits) break;
+            if (balance) {
+                balance = false;
+                continue;
+            }
             if (per <= 128) return TM_ERR_WORKSPACE;
             per = ((per / 2 + 127) / 128) * 128;
         }
         for (int t0 = 0; t0 < n; t0 += per) {
             const int    nt = n - t0 < per ? n - t0 : per;
-            GemmTcPlan   pl = gemm_tc_plan(m, nt, k, h->sm_count);
+            GemmTcPlan   pl = gemm_tc_plan(m, nt, k, h->sm_count, balance);
             GemmTcParams p{};
             p.C          = (__half*)C + (size_t)t0 * n_out_tc;
             p.A          = (const unsigned char*)A;

@@ -94,6 +94,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return true;
 }
 
+// The same for a warp that waits beside warps that compute: it sleeps between its tests (a suspended try_wait comes back after
+// some hundred cycles, and a loop around it takes up to half of a scheduler's issue slots)
+__device__ __forceinline__ bool mbar_wait_asleep(uint64_t* bar, uint32_t parity, unsigned ns, long long max_cycles = kMaxWaitCycles)
+{
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    do {
+        __nanosleep(ns);
+        if (mbar_try_wait(bar, parity)) return true;
+    } while (clock64() - t0 <= max_cycles);
+    return false;
+}
+
 // The same by a whole warp, with one outcome for all of it
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long max_cycles = kMaxWaitCycles)
 {

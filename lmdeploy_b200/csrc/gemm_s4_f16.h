@@ -74,7 +74,7 @@ struct GemmTcParams {
     int                  N, T, K;
     int                  fused_silu;
     // filled in by gemm_tc_launch from the plan
-    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, x_stages, a_stages, acc_stride, k_split, parts_per_tile;
+    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, x_stages, a_stages, acc_stride, parts_per_tile;
     long long max_wait_cycles;  // bound of the wait for the partners of a split tile; 0 = the default
     GemmNormFusion norm;        // all null: a plain GEMM
 };
@@ -91,10 +91,12 @@ struct GemmTcPlan {
     size_t smem_bytes;
     size_t workspace_floats;
     size_t counter_ints;
+    double us;             // the launch's time by the plan's model
 };
 
 size_t      gemm_tc_smem_bytes(int token_tile);
-GemmTcPlan  gemm_tc_plan(int N, int T, int K, int sm_count);
+// `balance` = false: never cuts tiles where there are at least as many as SMs (what tm_gemm_s4_f16_workspace_bytes counts on)
+GemmTcPlan  gemm_tc_plan(int N, int T, int K, int sm_count, bool balance);
 // true when every output tile of the plan is reduced by reduce_share (the only place that applies GemmNormFusion)
 bool        gemm_tc_all_tiles_split(const GemmTcPlan& plan, int K);
 cudaError_t gemm_tc_prepare(int max_smem);

@@ -91,12 +91,11 @@ __global__ void __launch_bounds__(kWarps * 32) expand_s4_kernel(__half* w, const
 
 }  // namespace
 
-// Which way is faster, by a model of both in microseconds (what they share left out).  Expanding while multiplying: units of
-// 128 k x 256 features x 128 tokens, in waves of tiles, or split evenly and exchanged.  Expanding first: 2.5 bytes per weight
-// beside the dense product.  Fitted to 144 launches of twelve projections with 200 to 3000 tokens; where the model picks the
-// slower way (17 of them) the two are within 10 us or 20 % of each other.  The line lies between 400 (8192 x 3584) and 1024
-// tokens (8192 x 1024).  Both sides, us: 22016 x 4096 with 512 / 1024 / 2048 tokens 142 / 186 / 323 expanding first and
-// 121 / 199 / 410 while multiplying; 4096 x 11008: 79 / 101 / 149 and 64 / 110 / 162.
+// Which way is faster, by models of both in microseconds: the plan's of expanding while multiplying; expanding first, 2.5 bytes
+// per weight beside the dense product.  Fitted to 144 launches of twelve projections with 200 to 3000 tokens (mean error 9 %):
+// in 20 of them another way than the model's is more than 6 % faster, by a quarter at most.  Both sides, us: 22016 x 4096
+// with 1024 / 2048 / 3000 tokens 186 / 317 / 440 expanding first and 182 / 341 / 484 while multiplying; 8192 x 28672: 456 / 775 /
+// 1137 and 357 / 816 / 1096.
 int gemm_expanded_columns(const tm_handle* h, int N, int T, int K)
 {
     if (T <= 128 || K % 128 || N % 32 || h->sm_count < 2) return 0;
@@ -104,15 +103,12 @@ int gemm_expanded_columns(const tm_handle* h, int N, int T, int K)
     if (room < 256) return 0;
     const int pieces  = (N + room - 1) / room;
     const int columns = std::min(room, ((N + pieces - 1) / pieces + 255) / 256 * 256);
-    double first = -11.9;
+    double first = -24.7;
     for (int n0 = 0; n0 < N; n0 += columns) {
         const int n = std::min(columns, N - n0);
-        first += 28.9 + 0.505e-6 * n * K + 0.95 * dense_pair_us(T, n, (K + 63) / 64, h->sm_count);
+        first += 48.2 + 0.42e-6 * n * K + 0.98 * dense_pair_us(T, n, (K + 63) / 64, h->sm_count);
     }
-    const GemmTcPlan pl    = gemm_tc_plan(N, T, K, h->sm_count);
-    const bool       split = pl.units_per_cta % (K / 128) != 0 || pl.parts_per_tile > 1;
-    const int        waves = (pl.t_chunks * pl.ctas + h->sm_count - 1) / h->sm_count;
-    const double     along = split ? 27.1 + 0.88 * pl.units_per_cta : waves * (0.88 * pl.units_per_cta + 11.4) - 4.0;
+    const double along = gemm_tc_plan(N, T, K, h->sm_count, true).us;
     return first < along ? columns : 0;
 }
 

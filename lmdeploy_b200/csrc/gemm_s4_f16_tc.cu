@@ -27,6 +27,7 @@
 #include "handle.h"
 #include "gemm_s4_f16.h"
 
+#include <algorithm>
 #include <cuda.h>  // CUtensorMap (types only: the encoder is looked up through the runtime)
 
 #ifdef TM_B200_GEMM_TRACE
@@ -89,16 +90,18 @@ constexpr int kSuperN    = kTileN * kTeams;
 constexpr int kGroup     = 128;  // K extent of a unit
 constexpr int kTileBytes = 512;
 constexpr int kACols     = kGroup / 2;           // TMEM columns of one expanded weight stage (128 k as fp16 pairs)
-constexpr int kWarpStage = 2 * kTileBytes + 128; // per expanding warp and unit: 2 x 512 B of weight + 32 {zero, scale}
-constexpr int kWST       = 5;                    // stages of those private rings (cp.async groups in flight <= 4)
-constexpr int kASTMax    = 2;                    // expanded-weight stages per team (in TMEM)
+constexpr int kSlabs     = kGroup / 32;
+constexpr int kWarpStage = kSlabs * kTileBytes + 128; // per expanding warp and unit: 4 x 512 B of weight + 32 {zero, scale}
+constexpr int kWST       = 3;                    // stages of those private rings (cp.async groups in flight <= 2, every other unit)
+constexpr int kASTMax    = 3;                    // expanded-weight stages per team (in TMEM)
 constexpr int kXSTMax    = 6;                    // activation stages
 constexpr int kTeamWarps = 8;
 constexpr int kDqWarps   = kTeams * kTeamWarps;
 constexpr int kDqThreads = kDqWarps * 32;
-constexpr int kIssuers   = 2 * kTeams;           // issuer warps: (team, K half); the second halves idle at token tiles > 64
+constexpr int kIssuers   = kTeams;
 constexpr int kDqWarp0   = 1 + kIssuers;         // first expanding warp
 constexpr int kThreads   = (kDqWarp0 + kDqWarps) * 32;
+constexpr unsigned kNap = 20, kLongNap = 200;  // nanoseconds between a waiting warp's tests; the loader is several units ahead
 constexpr int kTmemCols  = 512;                  // accumulators + expanded-weight stages, power of two
 
 struct Bars {
@@ -145,11 +148,13 @@ __device__ __forceinline__ void umma_f16_ts_x4(uint32_t tmem_d, uint32_t tmem_a,
         : "memory");
 }
 
-// 16 TMEM lanes x 8 columns from an mma A-fragment: regs = {rows r | k pair c, rows r+8 | k pair c,
-// rows r | k pair c+4, rows r+8 | k pair c+4} with r = lane / 4, c = lane % 4
-__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
+// 16 TMEM lanes x 32 columns from eight halves of mma A-fragments, 4 columns each: regs[2 i], regs[2 i + 1] = {row r, row r + 8 |
+// k pair c} of columns 4 i .. 4 i + 3 with r = lane / 4, c = lane % 4
+__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&f)[16])
 {
-    asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(f[0]),
+                 "r"(f[1]), "r"(f[2]), "r"(f[3]), "r"(f[4]), "r"(f[5]), "r"(f[6]), "r"(f[7]), "r"(f[8]), "r"(f[9]), "r"(f[10]), "r"(f[11]),
+                 "r"(f[12]), "r"(f[13]), "r"(f[14]), "r"(f[15])
                  : "memory");
 }
 
@@ -176,17 +181,6 @@ __device__ __forceinline__ void tc_fence_before()
 __device__ __forceinline__ void tc_fence_after()
 {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
-{
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 // sixteen fp32 columns of this thread's TMEM lane
@@ -216,7 +210,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
 }
 
 // Bounded wait of a whole warp; on a time-out the warp records `bit` and plays dead from then on.
-__device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, bool& dead, unsigned* status, unsigned bit)
+__device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, bool& dead, unsigned* status, unsigned bit, unsigned ns = kNap)
 {
     if (dead) return;
     // Usually the phase is complete already: every lane tests it (same answer in every lane, no divergence).
@@ -224,7 +218,7 @@ __device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, bool& 
     // Otherwise one lane sleeps in the barrier; the shuffle hands the outcome (and, as a warp-level sync, the
     // ordering) to the rest.
     int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity) ? 1 : 0;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait_asleep(bar, parity, ns) ? 1 : 0;
     ok = __shfl_sync(0xffffffffu, ok, 0);
     if (!ok) {
         if ((threadIdx.x & 31) == 0) atomicOr(status, bit);
@@ -237,7 +231,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     const int kXST = p.x_stages;
     const int kAST = p.a_stages;    // per team
     const int accS = p.acc_stride;  // TMEM columns of one accumulator
-    const int KS   = p.k_split;     // issuers (and accumulators) per team: 2 at token tiles <= 64, else 1
     extern __shared__ unsigned char smem_dyn[];
     // tiles the tensor core reads must sit on 1024-byte boundaries (the swizzle is a function of
     // the address bits)
@@ -292,13 +285,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     const int  dw   = warp - kDqWarp0; // 0..15 for the expanding warps
     const int  m_dq = (dw >> 3) & 1;   // team = 128-feature tile of the unit
     const int  q    = warp & 3;        // TMEM lane quarter this warp may access = its 32-feature tile
-    const int  kh   = (dw >> 2) & 1;   // which pair of 32-row slabs of the group it expands,
-                                       // and which half of the token columns it drains
-    // private ring of this warp: per unit its own 2 x 512 B of packed weight (32-feature tile,
-    // 32-row slabs 2 kh, 2 kh + 1 of the group) + the 128 B of {zero, scale} of its 32 features
+    const int  kh   = (dw >> 2) & 1;   // which of two units it expands (what a unit costs beside the words is shared by
+                                       // twice as many), and which half of the token columns it drains
+    // private ring of this warp: per unit of its own 4 x 512 B of packed weight (32-feature tile, the group's
+    // 32-row slabs) + the 128 B of {zero, scale} of its 32 features
     const uint32_t       my_ring   = base + (uint32_t)(w_ring - sm) + (uint32_t)(dw < 0 ? 0 : dw) * kWST * kWarpStage + lane * 16;
     const unsigned char* my_ring_g = w_ring + (dw < 0 ? 0 : dw) * kWST * kWarpStage;
-    // the copy front runs kWST - 1 units ahead of the expansion: this lane's 16 bytes of the warp's
+    // the copy front runs kWST - 1 of its units ahead of the expansion: this lane's 16 bytes of the warp's
     // first slab and of the {zero, scale} row.  A warp whose tile lies beyond N re-reads the last
     // tile; what it produces is never stored.
     int                  i_js = u_begin / G, i_g = u_begin - i_js * G;
@@ -308,16 +301,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     const size_t         q_row_b = (size_t)p.N * 4;                 // bytes between {zero, scale} rows
     auto i_seek = [&]() {
         const int tile = min((i_js * kTeams + m_dq) * 4 + q, n_tiles32 - 1);
-        i_w = p.A + (((size_t)i_g * 4 + kh * 2) * n_tiles32 + tile) * kTileBytes + lane * 16;
+        i_w = p.A + ((size_t)i_g * kSlabs * n_tiles32 + tile) * kTileBytes + lane * 16;
         i_q = p.Q + ((size_t)i_g * p.N + (size_t)tile * 32) * 4 + (lane & 7) * 16;
     };
-    int to_issue = n_units;
-    auto issue_unit = [&](int stage) {
-        const uint32_t dst = my_ring + stage * kWarpStage;
-        cp_async16(dst, i_w);
-        cp_async16(dst + kTileBytes, i_w + slab_b);
-        if (lane < 8) cp_async16(dst + 2 * kTileBytes, i_q);
-        i_w += 4 * slab_b;
+    int  to_issue = (n_units + 1 - kh) / 2;  // units of this warp: kh, kh + 2, ...
+    auto i_next   = [&]() {
+        i_w += kSlabs * slab_b;
         i_q += q_row_b;
         if (++i_g == G) {
             i_g = 0;
@@ -325,10 +314,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             i_seek();
         }
     };
+    auto issue_unit = [&](int stage) {
+        const uint32_t dst = my_ring + stage * kWarpStage;
+#pragma unroll
+        for (int i = 0; i < kSlabs; ++i) cp_async16(dst + i * kTileBytes, i_w + i * slab_b);
+        if (lane < 8) cp_async16(dst + kSlabs * kTileBytes, i_q);
+        i_next();
+        i_next();
+    };
     if (dw >= 0) {
         // The packed weights are written by no kernel: their first copies start at once, ahead of the
         // barrier and TMEM set-up and of the wait for the kernel before this one.
         i_seek();
+        if (kh) i_next();
 #pragma unroll
         for (int sidx = 0; sidx < kWST - 1; ++sidx) {
             if (to_issue > 0) issue_unit(sidx);
@@ -340,15 +338,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     if (tid == 0) {
         for (int m = 0; m < kTeams; ++m) {
             for (int s = 0; s < kASTMax; ++s) {
-                mbar_init(&bars->a_full[m][s], kTeamWarps);
-                mbar_init(&bars->a_empty[m][s], KS);
+                mbar_init(&bars->a_full[m][s], kTeamWarps / 2);
+                mbar_init(&bars->a_empty[m][s], 1);
             }
-            mbar_init(&bars->acc_full[m], KS);
+            mbar_init(&bars->acc_full[m], 1);
             mbar_init(&bars->acc_empty[m], kTeamWarps);
         }
         for (int s = 0; s < kXSTMax; ++s) {
             mbar_init(&bars->x_full[s], 1);
-            mbar_init(&bars->x_empty[s], kTeams * KS);
+            mbar_init(&bars->x_empty[s], kTeams);
         }
         fence_mbar_init();
     }
@@ -363,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     tc_fence_after();
     const uint32_t tmem   = bars->tmem_base;
     TC_TRACE(trow, 2, 0);
-    const uint32_t a_base = tmem + kTeams * KS * accS;  // first expanded-weight stage
+    const uint32_t a_base = tmem + kTeams * accS;  // first expanded-weight stage
 
     if (warp == 0) {
         // ================================================================== activation loader
@@ -377,7 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         for (int it = 0; it < n_units; ++it) {
             const int sx = it % kXST;
             TC_TRACE(trow, 10, it);
-            if (it >= kXST) warp_wait(&bars->x_empty[sx], ((it / kXST) - 1) & 1, dead, p.status, kStatusGemmPipeWait);
+            if (it >= kXST) warp_wait(&bars->x_empty[sx], ((it / kXST) - 1) & 1, dead, p.status, kStatusGemmPipeWait, kLongNap);
             if (!dead && elect_one()) {
                 const uint32_t xb = base + (uint32_t)(x_ring - sm) + sx * x_bytes;
                 mbar_arrive_expect_tx(&bars->x_full[sx], (uint32_t)x_bytes);
@@ -390,19 +388,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     }
     else if (warp <= kIssuers) {
         // ================================================================== MMA issuers
-        // One warp per (team, K half) runs the whole loop: waits, four (or eight) MMAs by an elected lane, commits.  At
-        // small token tiles four issuers on four different schedulers share the work, each half of K with an
-        // accumulator of its own (summed by the epilogue).
-        const int m = (warp - 1) & 1;
-        const int h = (warp - 1) >> 1;
-        if (h < KS) {
+        // One warp per team runs the whole loop: waits, eight MMAs by an elected lane, commits.
+        const int m = warp - 1;
+        {
             const uint32_t idesc   = (1u << 4) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
-            const uint32_t d_tmem  = tmem + (m * KS + h) * accS;
+            const uint32_t d_tmem  = tmem + m * accS;
             const uint32_t kb_step = (uint32_t)(TT * 128) >> 4;  // descriptor units (16 B) between the two K blocks
             const uint64_t d_ring  = make_desc(base + (uint32_t)(x_ring - sm));
             const uint32_t d_hi    = (uint32_t)(d_ring >> 32);
             // (the low word of the descriptor carries the address: 14 bits of 16-byte units, never a carry out)
-            const uint32_t d_lo    = (uint32_t)d_ring + (uint32_t)h * kb_step;
+            const uint32_t d_lo    = (uint32_t)d_ring;
             const uint32_t x_step  = (uint32_t)x_bytes >> 4;
             int  seg_idx = 0;
             bool first   = true;  // first MMA of the current segment overwrites the accumulator
@@ -413,21 +408,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 bool ok = true;
                 if (first && seg_idx > 0) {
                     // the epilogue of the previous segment must have drained the accumulators
-                    ok = mbar_wait(&bars->acc_empty[m], (seg_idx - 1) & 1);
+                    ok = mbar_wait_asleep(&bars->acc_empty[m], (seg_idx - 1) & 1, kNap);
                 }
-                ok = ok && mbar_wait(&bars->x_full[sx], px) && mbar_wait(&bars->a_full[m][sa], pa);
+                ok = ok && mbar_wait_asleep(&bars->x_full[sx], px, kNap) && mbar_wait_asleep(&bars->a_full[m][sa], pa, kNap);
                 if (!__all_sync(0xffffffffu, ok)) {
                     if (lane == 0) atomicOr(p.status, kStatusGemmPipeWait);
                     break;
                 }
                 tc_fence_after();
                 TC_TRACE(trow, 20, it);
-                const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + (uint32_t)h * 32;
+                const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols;
                 const uint32_t lo     = d_lo + (uint32_t)sx * x_step;
                 const bool last = (it == n_units - 1) || (g == G - 1);
                 if (elect_one()) {
                     umma_f16_ts_x4(d_tmem, a_tmem, lo, d_hi, idesc, first ? 1u : 0u);
-                    if (KS == 1) umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
+                    umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
                     umma_commit(&bars->a_empty[m][sa]);
                     umma_commit(&bars->x_empty[sx]);
                     if (last) umma_commit(&bars->acc_full[m]);
@@ -574,24 +569,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
 
         const int      ccount = TT / 2;                      // token columns per warp: [kh * ccount, +ccount)
         const int      n_row  = m * kTileN + q * 32 + lane;  // feature row of the CTA tile held by this thread
-        const uint32_t a_lane = ((uint32_t)(q * 32) << 16) + (uint32_t)(kh * 32);  // TMEM lanes and first column of this warp's share of a stage
+        const uint32_t a_lane = (uint32_t)(q * 32) << 16;    // TMEM lanes of this warp
 
         int      js = u_begin / G, g = u_begin - js * G;
-        int      sw = 0, sw_fill = kWST - 1;  // ring slot read now / refilled now (the one read one unit ago)
+        int      sw = 0, sw_fill = kWST - 1;  // ring slot read now / refilled now (the one read one unit of its own ago)
         int      sa = 0;
         uint32_t pa = 0;                      // phase parity of the team's expanded-weight ring
         for (int it = 0; it < n_units; ++it) {
             TC_TRACE(trow, 30, it);
-            asm volatile("cp.async.wait_group %0;" ::"n"(kWST - 2) : "memory");
-            __syncwarp();
-            // the tensor core must be done with what this TMEM stage held kAST units ago (the first
-            // round passes at once: a fresh barrier counts as having completed the phase before)
-            warp_wait(&bars->a_empty[m][sa], pa ^ 1u, dead, p.status, kStatusGemmPipeWait);
-            tc_fence_after();
-            TC_TRACE(trow, 32, it);
-            {
+            if ((it & 1) == kh) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kWST - 2) : "memory");
+                __syncwarp();
                 const unsigned char* sb = my_ring_g + sw * kWarpStage;
-                const __half2*       qs = reinterpret_cast<const __half2*>(sb + 2 * kTileBytes);
+                const __half2*       qs = reinterpret_cast<const __half2*>(sb + kSlabs * kTileBytes);
                 uint32_t z1024[2], nz64[2], s_lo[2], s_hi[2];
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
@@ -607,47 +597,51 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     s_hi[a]  = reinterpret_cast<const uint32_t&>(sh2);
                 }
                 const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + a_lane;
-                // all fragments first (independent chains the scheduler can interleave), then the stores
-                uint32_t f[8][4];
+                bool           room   = false;
 #pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    const uint4    w     = reinterpret_cast<const uint4*>(sb)[kk * 32 + lane];
-                    const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+                for (int half = 0; half < 2; ++half) {
+                    // two slabs: all fragments first (independent chains the scheduler can interleave), then the stores
+                    uint32_t f[2][16];  // [16-row half][pieces of 4 columns]
 #pragma unroll
-                    for (int wi = 0; wi < 4; ++wi) {
-                        const int a = wi & 1;
-                        uint32_t (&fr)[4] = f[kk * 4 + wi];
-                        unpack_s4_minus_zero(wv[wi], z1024[a], nz64[a], fr);
-                        fr[0] = hmul2_ftz(fr[0], s_lo[a]);
-                        fr[1] = hmul2_ftz(fr[1], s_hi[a]);
-                        fr[2] = hmul2_ftz(fr[2], s_lo[a]);
-                        fr[3] = hmul2_ftz(fr[3], s_hi[a]);
+                    for (int kk = 0; kk < 2; ++kk) {
+                        const uint4    w     = reinterpret_cast<const uint4*>(sb)[(2 * half + kk) * 32 + lane];
+                        const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                        for (int wi = 0; wi < 4; ++wi) {
+                            const int a = wi & 1, at = kk * 8 + (wi >> 1) * 4;
+                            uint32_t  fr[4];
+                            unpack_s4_minus_zero(wv[wi], z1024[a], nz64[a], fr);
+                            f[a][at]     = hmul2_ftz(fr[0], s_lo[a]);
+                            f[a][at + 1] = hmul2_ftz(fr[1], s_hi[a]);
+                            f[a][at + 2] = hmul2_ftz(fr[2], s_lo[a]);
+                            f[a][at + 3] = hmul2_ftz(fr[3], s_hi[a]);
+                        }
                     }
-                }
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-#pragma unroll
-                    for (int wi = 0; wi < 4; ++wi) {
-                        const int k16 = wi >> 1;
-                        const int a   = wi & 1;
-                        const uint32_t (&fr)[4] = f[kk * 4 + wi];
-                        // rows q*32 + a*16 .. +15 (TMEM lanes), k = 32 (2 kh + kk) + 16 k16 .. +15 (8 columns)
-                        tmem_st_16x128b_x2(a_tmem + ((uint32_t)(a * 16) << 16) + (uint32_t)(kk * 16 + k16 * 8), fr[0], fr[1], fr[2], fr[3]);
+                    if (!room) {
+                        // the tensor core must be done with what this TMEM stage held kAST units ago (the first round passes at
+                        // once: a fresh barrier counts as having completed the phase before)
+                        warp_wait(&bars->a_empty[m][sa], pa ^ 1u, dead, p.status, kStatusGemmPipeWait);
+                        tc_fence_after();
+                        TC_TRACE(trow, 32, it);
+                        room = true;
                     }
+                    // rows q*32 + a*16 .. +15 (TMEM lanes), k = 64 half .. +63 (32 columns)
+                    tmem_st_16x128b_x8(a_tmem + (uint32_t)(half * 32), f[0]);
+                    tmem_st_16x128b_x8(a_tmem + (16u << 16) + (uint32_t)(half * 32), f[1]);
                 }
+                // expanded tile visible to the tensor core; packed stage free again
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->a_full[m][sa]);
+                TC_TRACE(trow, 33, it);
+                // refill the slot that was read one unit of this warp ago (everyone in the warp is past its reads)
+                if (to_issue > 0) issue_unit(sw_fill);
+                --to_issue;
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                sw      = (sw == kWST - 1) ? 0 : sw + 1;
+                sw_fill = (sw_fill == kWST - 1) ? 0 : sw_fill + 1;
             }
-            // expanded tile visible to the tensor core; packed stage free again
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->a_full[m][sa]);
-            TC_TRACE(trow, 33, it);
-            // refill the slot that was read one unit ago (everyone in the warp is past its reads)
-            if (to_issue > 0) issue_unit(sw_fill);
-            --to_issue;
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            sw      = (sw == kWST - 1) ? 0 : sw + 1;
-            sw_fill = (sw_fill == kWST - 1) ? 0 : sw_fill + 1;
             if (++sa == kAST) {
                 sa = 0;
                 pa ^= 1u;
@@ -670,7 +664,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             tc_fence_after();
             TC_TRACE(trow, 35, it);
             const int n_glob = col0 + n_row;
-            const uint32_t my_acc = tmem + m * KS * accS + ((uint32_t)(q * 32) << 16);
+            const uint32_t my_acc = tmem + m * accS + ((uint32_t)(q * 32) << 16);
             if (!dead) {
                 float* mine = slots + (size_t)(blockIdx.x + this_js) * slot_floats + n_row;
                 for (int cb = 0; cb < ccount; cb += 16) {
@@ -679,12 +673,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     const int col = kh * ccount + cb;
                     float     v[16];
                     tmem_ld16(my_acc + (uint32_t)col, v);
-                    if (KS == 2) {
-                        float v2[16];
-                        tmem_ld16(my_acc + (uint32_t)(accS + col), v2);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] += v2[i];
-                    }
                     const int valid = min(16, ccount - cb);  // 8 or 16
                     if (n_split > 1) {
 #pragma unroll
@@ -790,8 +778,7 @@ PFN_encodeTiled lookup_encode_tiled()
 }
 
 int x_stages_for(int token_tile) { return token_tile > 64 ? 3 : kXSTMax; }
-int a_stages_for(int token_tile) { (void)token_tile; return 2; }
-int k_split_for(int token_tile) { return token_tile > 64 ? 1 : 2; }
+int a_stages_for(int token_tile) { return token_tile > 64 ? 2 : kASTMax; }  // beside the accumulators, all of TMEM
 int acc_stride_for(int token_tile) { return token_tile > 64 ? 128 : 64; }
 
 }  // namespace
@@ -801,7 +788,7 @@ size_t gemm_tc_smem_bytes(int token_tile)
     return 1024 + (size_t)x_stages_for(token_tile) * 2 * token_tile * 128 + (size_t)kWST * kDqWarps * kWarpStage + sizeof(Bars) + 64;
 }
 
-GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count)
+GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
 {
     GemmTcPlan pl{};
     pl.token_tile  = T >= 128 ? 128 : ((T + 15) / 16) * 16;
@@ -810,8 +797,22 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count)
     const int G    = K / kGroup;
     pl.total_units = pl.n_col_tiles * G;
     pl.parts_per_tile = 0;
-    if ((long long)pl.t_chunks * pl.n_col_tiles >= sm_count) {
-        // enough whole column tiles to fill the device: one per CTA, nothing is split, nobody waits
+    // With at least as many whole column tiles as SMs: one per CTA, nothing is split, nobody waits.  `balance`: unless their last
+    // wave is so empty that cutting the units evenly is faster, by a model fitted to 270 launches of twelve projections with 32
+    // to 3000 tokens (microseconds; mean error 10 %).  57344 x 8192, 224 tiles: two waves of 64 units, or 97 units for every SM:
+    // 88 / 76 us with 32 tokens, 4096 x 11008 with 1600 tokens 178 / 125.
+    const long long tiles = (long long)pl.t_chunks * pl.n_col_tiles;
+    const double    fill  = std::max(0, pl.token_tile - 32) / 96.0;  // what a unit costs beyond its expansion
+    auto cut_us = [&](int units) { return 8.5 + units * (0.711 + 0.083 * fill) + 10.2 * units / G + 13.8 * pl.token_tile / 128; };
+    bool whole = tiles >= sm_count;
+    if (whole) {
+        pl.us = 4.2 + (double)((tiles + sm_count - 1) / sm_count) * (G * (0.56 + 0.14 * fill) + 12.7);
+        if (balance && pl.t_chunks <= sm_count / 2) {
+            const int per_chunk = sm_count / pl.t_chunks;
+            whole = pl.us <= cut_us((pl.total_units + per_chunk - 1) / per_chunk);
+        }
+    }
+    if (whole) {
         pl.units_per_cta = G;
         pl.ctas          = pl.n_col_tiles;
     }
@@ -834,6 +835,7 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count)
             pl.units_per_cta = flat;
             pl.ctas          = (pl.total_units + flat - 1) / flat;
         }
+        pl.us = cut_us(pl.units_per_cta);
     }
     pl.slots_per_chunk = pl.ctas + pl.n_col_tiles;
     pl.smem_bytes      = gemm_tc_smem_bytes(pl.token_tile);
@@ -865,7 +867,6 @@ cudaError_t gemm_tc_launch(const GemmTcPlan& pl, GemmTcParams p, cudaStream_t st
     p.token_tile      = pl.token_tile;
     p.x_stages        = x_stages_for(pl.token_tile);
     p.a_stages        = a_stages_for(pl.token_tile);
-    p.k_split         = k_split_for(pl.token_tile);
     if (p.max_wait_cycles <= 0) p.max_wait_cycles = kMaxWaitCycles;
     p.acc_stride      = acc_stride_for(pl.token_tile);
 

@@ -39,8 +39,7 @@ def test_dense_pairs(tokens, n_out, k, ld):
         assert bool((out[:, n_out:] == 7.0).all())
 
 
-@pytest.mark.parametrize("n,k,silu,tokens", [(4128, 2048, False, 1300), (4128, 2048, False, 2049), (7168, 8192, True, 1300), (4160, 4096, True, 1300),
-                                             (4160, 4096, True, 2049), (20512, 4096, False, 3001)])
+@pytest.mark.parametrize("n,k,silu,tokens", [(4128, 2048, False, 6000), (4160, 4096, True, 6001), (4160, 4096, True, 8193), (20512, 4096, False, 8192)])
 def test_expanded_weight(n, k, silu, tokens, monkeypatch):
     """Sizes that the launch rule sends through expanded rows (the scratch of a handle of its own: one piece, or several where the
     weight does not fit), feature counts that fill no tile of a pair."""
@@ -69,3 +68,20 @@ def test_expanded_weight(n, k, silu, tokens, monkeypatch):
     bound = want.abs() * 2.0 ** -10 + 1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2] + 1e-5
     over = ((out.double() - want).abs() / bound).max().item()
     assert over <= 1.0, f"{over:.2f} of the bound"
+
+
+@pytest.mark.parametrize("n,k,tokens", [(57344, 1024, 17), (57344, 1024, 128), (40960, 2048, 100), (22016, 4096, 200)])
+def test_units_cut_evenly(n, k, tokens):
+    """At least as many column tiles as SMs, cut all the same: runs over several tiles, of which the first and the last are shared."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    h = l.default_handle(0)
+    w = cases._linear(cases._gen(4, n), n, k)
+    exact = cases._exact_weight(cases._gen(4, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    out = torch.empty(tokens, n, dtype=torch.float16, device="cuda")
+    for _ in range(2):
+        l.check(l.lib.tm_gemm_s4_f16(h.ptr, out.data_ptr(), w.kernel.data_ptr(), x.data_ptr(), w.scales_and_zeros.data_ptr(), n, tokens, k, 128,
+                                     0, None, 0, _stream()), "tm_gemm_s4_f16")
+    h.check_device_status(torch.cuda.current_stream().cuda_stream)
+    _check(out, x.double() @ exact, x.double().abs() @ exact.abs(), k, 11, (n, k, tokens))
