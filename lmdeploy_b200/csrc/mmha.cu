@@ -809,7 +809,7 @@ cudaError_t mmha_prepare()
 }
 static const KernelPreparation g_prepare([](int) { return mmha_prepare(); });
 
-MmhaPlan mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_chunk, int want_warps)
+MmhaPlan mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_chunk, int want_warps, bool int8)
 {
     MmhaPlan  pl{};
     const int rep = H / Hkv;
@@ -823,7 +823,15 @@ MmhaPlan mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_ch
         // two SMs.  So: no split up to 2048 tokens when there are that many items; 2048-token splits
         // beyond (they even out the tail of long sequences); with fewer items, just enough splits of at
         // least 256 tokens to put two CTAs on every SM.
-        if (items * 2 >= sm_count) {
+        // An int8 cache is expanded in registers, which takes a CTA's four warps longer than its bytes: there, splits of at
+        // least 192 tokens up to what four CTAs per SM can take of lengths of four fifths of the longest (7B layers, 128 items of
+        // 300 to 900 tokens: 8 layers 638 us unsplit, 565 with 192; 384 items: 741, 704 with 512; the same with an fp16 cache and
+        // 168 items: 1721 and 1769).
+        if (int8 && items < 3ll * sm_count) {
+            const long long even = (long long)max_len * 4 * items / (5 * 4ll * sm_count);
+            chunk = (int)(even < 192 ? 192 : even);
+        }
+        else if (items * 2 >= sm_count) {
             chunk = max_len < 2048 ? max_len : 2048;
         }
         else {

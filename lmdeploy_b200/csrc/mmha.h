@@ -50,7 +50,7 @@ struct MmhaPlan {
 };
 
 cudaError_t mmha_prepare();
-MmhaPlan    mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_chunk, int want_warps = 0);
+MmhaPlan    mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_chunk, int want_warps, bool int8);
 cudaError_t mmha_launch(const MmhaPlan& plan, MmhaParams p, bool int8, cudaStream_t st, bool pdl = false);
 
 // RMSNorm kernels (norm.cu)
