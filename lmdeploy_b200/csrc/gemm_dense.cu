@@ -30,6 +30,7 @@ constexpr int kMaxStages = 12;
 constexpr int kMaxTokens = 256;  // tokens of one tile
 constexpr int kEpiBar    = 1;    // named barrier of the epilogue warps
 constexpr int kPairMinTokens = 64;
+constexpr int kPairMinBlocks = 8;  // k blocks: below, a tile is its epilogue, and the pair's barriers come on top (4096 x 96, 4096 tokens: 40 us, single CTAs 32)
 // Pairs of CTAs: token tiles of a band.  74 pairs then work on 8 token tiles x 9 column tiles, which the L2 serves; measured at
 // 22016 x 4096 with 4096 / 16384 tokens: 4 tiles 530 / 2330 us, 8 tiles 509 / 2204, 16 tiles 546 / 2316.
 constexpr int kBand = 8;
@@ -759,6 +760,7 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
     Plan      best{0, false};
     double    best_cost = 1e30;
     const int columns   = (n_out + kDenseTile - 1) / kDenseTile;
+    constexpr double kOut = 0.023;  // a token of a tile on its way out: beside the next tile's products, alone after the last
     auto consider = [&](double cost, Plan plan) {
         if (cost < best_cost - 1e-9) best_cost = cost, best = plan;
     };
@@ -768,7 +770,8 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
         for (int nt = first; nt >= last; nt -= 16) {
             const long long tiles = (long long)columns * ((tokens + nt - 1) / nt);
             if (tiles < 2 * sms) consider((double)tiles * k_blocks / sms * std::max(0.36, 0.073 + 0.00182 * nt) + 0.15 * nt, {nt, true, false});
-            consider((double)((tiles + sms - 1) / sms) * (k_blocks * std::max(0.2, 0.112 + 0.00108 * nt) - 0.35) + 1.8, {nt, false, false});
+            const double tile = std::max(k_blocks * std::max(0.2, 0.112 + 0.00108 * nt) - 0.35, kOut * nt);
+            consider((double)((tiles + sms - 1) / sms) * tile + kOut * nt + 1.8, {nt, false, false});
         }
     }
     if (pairs) {
@@ -776,7 +779,8 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
         const int last  = std::min(first, 96);
         for (int nt = first; nt >= last; nt -= 32) {
             const long long tiles = (long long)((columns + 1) / 2) * ((tokens + nt - 1) / nt);
-            consider((double)((tiles + sms / 2 - 1) / (sms / 2)) * (k_blocks * std::max(0.183, 0.066 + 0.00108 * nt) + 1.0) + 1.0, {nt, false, true});
+            const double tile = std::max(k_blocks * std::max(0.183, 0.066 + 0.00108 * nt) + 1.0, kOut * nt);
+            consider((double)((tiles + sms / 2 - 1) / (sms / 2)) * tile + kOut * nt + 1.0, {nt, false, true});
         }
     }
     if (cost_us) *cost_us = best_cost;
@@ -809,7 +813,7 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     const bool grouped = g.groups.count > 0;
     const int  sms     = h->sm_count;
     // the tile of a pair has one operand; with few tokens the k blocks of a tile are rather cut than shared
-    const bool pairs = sms >= 2 && (half || g.tokens > kPairMinTokens) && (!g.x2 || g.x2_from % (2 * kDenseTile) == 0);
+    const bool pairs = sms >= 2 && (half || (g.tokens > kPairMinTokens && p.k_blocks >= kPairMinBlocks)) && (!g.x2 || g.x2_from % (2 * kDenseTile) == 0);
     const Plan plan  = grouped ? choose_group_plan(g.tokens, g.groups.count, g.n_out, sms) : choose_plan(g.tokens, g.n_out, p.k_blocks, sms, !half, pairs);
     if (plan.token_tile == 0) return TM_ERR_UNSUPPORTED;
     p.groups           = g.groups;

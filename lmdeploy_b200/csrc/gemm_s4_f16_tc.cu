@@ -1,23 +1,25 @@
-// W4A16 GEMM for more than 16 tokens: tcgen05 tensor-core tiles with the accumulators in TMEM.
+// W4A16 GEMM from 9 to 17 tokens on (api.cu): tcgen05 tensor-core tiles with the accumulators in TMEM.
 //
 // A CTA computes C^T tiles of 256 output features (two 128-feature UMMA tiles that share one
-// activation slice) x up to 128 tokens.  It is persistent and stream-K balanced over
-// (256-feature tile, 128-row quantisation group) units, like the small-token kernel.  Warp roles:
-//   warp 0       one lane streams the activation slices: two tensor-map copies (TMA, 128-byte
+// activation slice) x up to 128 tokens.  Work units are (256-feature tile, 128-row quantisation
+// group); a CTA has a whole tile, or the units of all tiles are cut evenly (gemm_tc_plan).  Warp roles:
+//   warp 0       an elected lane streams the activation slices: two tensor-map copies (TMA, 128-byte
 //                swizzle, tokens beyond T read as zero) per unit, completion on an mbarrier
 //   warps 1, 2   one issuer per 128-feature tile (warp 1 also allocates TMEM): an elected lane issues
 //                tcgen05.mma (M = 128, N = token tile, K = 16 per instruction, fp16 x fp16 -> fp32, A
 //                from TMEM, B from shared memory) and commits completions to mbarriers
-//   warps 3..18  two teams of eight, one per 128-feature tile.  Every warp streams its own share of
-//                the packed weight through a private cp.async ring and expands it: lop3 nibble
+//   warps 3..18  two teams of eight, one per 128-feature tile; four warps of a team (32 features each)
+//                take the even units, four the odd ones.  Bound by their issue slots (74 % used, ALU
+//                pipe 55 %): what a unit costs beside its words is paid by half as many warps as
+//                when all eight shared it (57344 x 8192, 17 tokens: 1.15 us a unit before, 0.91
+//                now).  Every warp streams its own share of the packed weight through a private cp.async ring and expands it: lop3 nibble
 //                unpack, exact (q - z) in fp16, one fp16 multiply by the scale (bit-identical to the
 //                reference's dequantised weight, kernels/gemm_s_f16/common.h:115-156, 218-235),
 //                tcgen05.st of the fragments straight into TMEM, from where the tensor core takes
 //                its A operand (no shared-memory round trip); at the end of a column tile the
 //                warps read the accumulators with tcgen05.ld and store C (optionally through the
 //                SiLU(gate) * up epilogue) or the split-K partial
-// A waiting thread sleeps in the mbarrier (try_wait with a time hint): the three single-lane roles
-// would otherwise take a quarter of the issue slots from the expanding warps.
+// A waiting warp sleeps between its tests: it would otherwise take issue slots from the expanding ones.
 // Partial tiles of CTAs that share a column tile meet in scratch memory; every CTA of the tile then
 // sums its own share of the feature rows in a fixed order.  Every wait is bounded.
 //
