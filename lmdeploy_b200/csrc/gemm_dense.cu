@@ -760,7 +760,7 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
     Plan      best{0, false};
     double    best_cost = 1e30;
     const int columns   = (n_out + kDenseTile - 1) / kDenseTile;
-    constexpr double kOut = 0.023;  // a token of a tile on its way out: beside the next tile's products, alone after the last
+    constexpr double kOut = 0.023;  // a token of a tile on its way out (1.6 us a tile on top): beside the next tile's products, alone after the last
     auto consider = [&](double cost, Plan plan) {
         if (cost < best_cost - 1e-9) best_cost = cost, best = plan;
     };
@@ -770,7 +770,7 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
         for (int nt = first; nt >= last; nt -= 16) {
             const long long tiles = (long long)columns * ((tokens + nt - 1) / nt);
             if (tiles < 2 * sms) consider((double)tiles * k_blocks / sms * std::max(0.36, 0.073 + 0.00182 * nt) + 0.15 * nt, {nt, true, false});
-            const double tile = std::max(k_blocks * std::max(0.2, 0.112 + 0.00108 * nt) - 0.35, kOut * nt);
+            const double tile = std::max(k_blocks * std::max(0.2, 0.112 + 0.00108 * nt) - 0.35, 1.6 + kOut * nt);
             consider((double)((tiles + sms - 1) / sms) * tile + kOut * nt + 1.8, {nt, false, false});
         }
     }
@@ -779,7 +779,7 @@ Plan choose_plan(int tokens, int n_out, int k_blocks, int sms, bool single, bool
         const int last  = std::min(first, 96);
         for (int nt = first; nt >= last; nt -= 32) {
             const long long tiles = (long long)((columns + 1) / 2) * ((tokens + nt - 1) / nt);
-            const double tile = std::max(k_blocks * std::max(0.183, 0.066 + 0.00108 * nt) + 1.0, kOut * nt);
+            const double tile = std::max(k_blocks * std::max(0.183, 0.066 + 0.00108 * nt) + 1.0, 1.6 + kOut * nt);
             consider((double)((tiles + sms / 2 - 1) / (sms / 2)) * tile + kOut * nt + 1.0, {nt, false, true});
         }
     }
