@@ -117,9 +117,16 @@ __device__ __forceinline__ void epilogue16(const DenseEpilogue& ep, const float 
 {
     const bool col = n < n_out;
     if (ep.kind == DenseKind::kF32) {
+        float* const dst = static_cast<float*>(ep.out) + (size_t)t0 * ep.out_ld + n;
+        if (live == 16 && col) {  // all but a tile's last rows: no test per row
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            if (i < live && col) static_cast<float*>(ep.out)[(size_t)(t0 + i) * ep.out_ld + n] = y[i];
+            for (int i = 0; i < 16; ++i) dst[(size_t)i * ep.out_ld] = y[i];
+        }
+        else if (col) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                if (i < live) dst[(size_t)i * ep.out_ld] = y[i];
+            }
         }
         return;
     }
