@@ -556,7 +556,7 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
             if (finish) {
                 const int  n0   = ct * kDenseTile + q * 32;
                 const bool wide = n0 + 32 <= p.n_out && (n0 >= p.wide_act || n0 + 32 <= p.wide_out);
-                const bool sums = adds && p.ep.ssq_out;
+                const bool sums = adds && p.ep.ssq_out && ct < p.column_tiles;  // an odd column tile's pair has a CTA without one
                 if (adds && kb1 - kb0 < p.k_blocks) residual_load(p.ep, t0, min(16, rows), n, p.n_out, in);
                 for (int c0 = 0; c0 < rows; c0 += 16) {
                     float     v[16], sq[16];
@@ -804,6 +804,15 @@ Plan choose_group_plan(int rows, int groups, int n_out, int sms)
     return {nt, tiles < 4 * sms};
 }
 
+Plan plan_of(const DenseGemm& g, int sms, bool half)
+{
+    if (g.groups.count > 0) return choose_group_plan(g.tokens, g.groups.count, g.n_out, sms);
+    // the tile of a pair has one operand; with few tokens the k blocks of a tile are rather cut than shared
+    const int  k_blocks = (g.k + kKBlock - 1) / kKBlock;
+    const bool pairs = sms >= 2 && (half || (g.tokens > kPairMinTokens && k_blocks >= kPairMinBlocks)) && (!g.x2 || g.x2_from % (2 * kDenseTile) == 0);
+    return choose_plan(g.tokens, g.n_out, k_blocks, sms, !half, pairs);
+}
+
 // `half`: fp16 operands, pairs of CTAs only
 int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool half = false)
 {
@@ -819,9 +828,7 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     p.k_blocks     = (g.k + kKBlock - 1) / kKBlock;
     const bool grouped = g.groups.count > 0;
     const int  sms     = h->sm_count;
-    // the tile of a pair has one operand; with few tokens the k blocks of a tile are rather cut than shared
-    const bool pairs = sms >= 2 && (half || (g.tokens > kPairMinTokens && p.k_blocks >= kPairMinBlocks)) && (!g.x2 || g.x2_from % (2 * kDenseTile) == 0);
-    const Plan plan  = grouped ? choose_group_plan(g.tokens, g.groups.count, g.n_out, sms) : choose_plan(g.tokens, g.n_out, p.k_blocks, sms, !half, pairs);
+    const Plan plan    = plan_of(g, sms, half);
     if (plan.token_tile == 0) return TM_ERR_UNSUPPORTED;
     p.groups           = g.groups;
     p.x2_tile          = g.x2 ? g.x2_from / kDenseTile : 1 << 30;

@@ -1,0 +1,102 @@
+"""The bf16 dense product where pairs of CTAs take its tiles, with the epilogues of the config-driven decoders, against 64-bit
+sums of the same operands.  Every size is one that the plan gives to pairs, and the test says so."""
+import ctypes as C
+import os
+import shutil
+import subprocess
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+ULP = 2.0 ** -24
+GUARD = 7.0
+
+
+@pytest.fixture(scope="module")
+def dense(tmp_path_factory):
+    from lmdeploy_b200 import build
+    so = str(tmp_path_factory.mktemp("dense") / "libdense.so")
+    flags = [f for f in build.NVCC_FLAGS if f not in ("-lineinfo",)]
+    r = subprocess.run([NVCC] + flags + ["-Xcompiler", "-fvisibility=default", "-w", "-shared", os.path.join(ROOT, "tests", "native", "dense_epilogues.cu"),
+                                         "-o", so], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    lib = C.CDLL(so)
+    lib.call_new.restype = C.c_void_p
+    h = C.c_void_p()
+    assert lib.tm_create(C.byref(h), 0) == 0
+    yield lib, h
+    lib.tm_destroy(h)
+
+
+def _p(t):
+    return C.c_void_p(0 if t is None else t.data_ptr())
+
+
+class _Product:
+    """x [tokens, k] (and x2 from column x2_from on) times w [n, k], its exact value and the bound of fp32 sums of it"""
+
+    def __init__(self, dense, tokens, n, k, x2_from=0):
+        self.lib, self.h = dense
+        g = torch.Generator(device="cuda").manual_seed(tokens + n + k)
+        draw = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+        self.draw, self.tokens, self.n = draw, tokens, n
+        self.x, self.w = draw(tokens, k).bfloat16(), (draw(n, k) / k ** 0.5).bfloat16()
+        self.x2 = draw(tokens, k).bfloat16() if x2_from else None
+        wd = self.w.double()
+        self.y, size = self.x.double() @ wd.T, self.x.double().abs() @ wd.abs().T
+        if x2_from:
+            self.y[:, x2_from:] = self.x2.double() @ wd[x2_from:].T
+            size[:, x2_from:] = self.x2.double().abs() @ wd[x2_from:].abs().T
+        self.err = size * (k * ULP)
+        self.c = C.c_void_p(self.lib.call_new())
+        self.lib.set_operands(self.c, _p(self.x), _p(self.x2), x2_from, k, _p(self.w), k, tokens, n, k)
+
+    def run(self):
+        assert self.lib.route(self.c, self.lib.sm_count(self.h)) == 3, "the plan gives this size to pairs no more: choose another"
+        st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert self.lib.run(self.h, self.c, st) == 0
+        word = C.c_uint(0)
+        assert self.lib.tm_check_device_status(self.h, st, C.byref(word)) == 0, hex(word.value)
+        self.lib.call_free(self.c)
+
+
+def _within(got, want, bound, what):
+    over = ((got.double() - want).abs() / (bound + 1e-30)).max().item()
+    assert over <= 1.0, f"{what}: {over:.2f} of the bound"
+
+
+# columns: 19, 17 and 39 tiles (the last one of 72 columns), 40 tiles (the last one of 8); tokens of one tile, of several, ragged ones
+@pytest.mark.parametrize("tokens,n,k", [(160, 2432, 4864), (600, 2176, 512), (257, 4936, 1000), (300, 5000, 512)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_residual_and_row_sums(dense, tokens, n, k, gated):
+    """Residual, its cast and its sums of squares per tile of columns; nothing is written behind the last tile's sums (a pair's
+    second CTA has no tile where their number is odd)."""
+    q = _Product(dense, tokens, n, k)
+    before = q.draw(tokens, n)
+    tiles, stride = -(-n // 128), (tokens + 7) // 8 * 8
+    residual, cast = before.clone(), torch.full((tokens, n + 8), GUARD, device="cuda", dtype=torch.bfloat16)
+    sums = torch.full((tiles + 2, stride), GUARD, device="cuda")
+    gate = q.draw(tokens, n).bfloat16() if gated else None
+    bias = q.draw(n) if gated else None
+    mult = 0.5 if gated else 1.0
+    q.lib.set_residual(q.c, _p(residual), n, _p(cast), n + 8, _p(sums), stride, _p(gate), n, _p(bias), C.c_float(mult))
+    q.run()
+    y, err = q.y, q.err
+    if gated:
+        a = gate.double() + bias.double()
+        f = mult * torch.sigmoid(a)
+        # __expf: 2 + 1.2 |a| ulps; the sum, the quotient and its product a few more
+        err, y = f * err + (f * y).abs() * ((8 + 1.2 * a.abs()) * 2 * ULP), f * y
+    want = before.double() + y
+    err = err + want.abs() * ULP
+    _within(residual, want, err, "residual")
+    _within(cast[:, :n], want, err + want.abs() * 2.0 ** -8, "cast")
+    assert bool((cast[:, n:] == GUARD).all())
+    pad = lambda v: torch.nn.functional.pad(v, (0, tiles * 128 - n)).view(tokens, tiles, 128).sum(-1).T  # noqa: E731
+    _within(sums[:tiles, :tokens], pad(want ** 2), pad(2 * want.abs() * err + err ** 2) + pad(want ** 2) * (32 * ULP), "sums of squares")
+    assert bool((sums[tiles:] == GUARD).all()), "written behind the last tile's sums"
+    assert bool((sums[:tiles, tokens:] == GUARD).all())
