@@ -826,8 +826,8 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
         const int flat = (pl.total_units + ctas - 1) / ctas;  // units per CTA when the flat unit list is cut evenly
         // Prefer a whole number of CTAs per column tile when that costs at most one unit more per CTA: a CTA whose
         // run of units crosses from one tile into the next publishes and reduces two partial tiles instead of one.
-        const int per_tile = ctas / pl.n_col_tiles;            // >= 1 here
-        const int part     = (G + per_tile - 1) / per_tile;    // units per CTA with per_tile CTAs on every tile
+        const int per_tile = ctas / pl.n_col_tiles;  // 0 where more tiles than CTAs are cut
+        const int part     = per_tile >= 2 ? (G + per_tile - 1) / per_tile : G;  // units per CTA with per_tile CTAs on every tile
         if (per_tile >= 2 && part <= flat + 1) {
             pl.parts_per_tile = (G + part - 1) / part;
             pl.units_per_cta  = part;
