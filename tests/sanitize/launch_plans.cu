@@ -1,5 +1,6 @@
 // The launch plans of the W4A16 tensor-core GEMM over a range of products and devices: every plan covers the product, and CTAs
 // that wait for one another are resident together.  Built with the undefined-behaviour checks of the host compiler; no CUDA call is made.
+#include "handle.cu"
 #include "gemm_s4_f16_tc.cu"
 
 #include <cstdio>
