@@ -20,6 +20,7 @@
 #include "handle.h"
 #include "mmha.h"
 
+#include <algorithm>
 #include <cfloat>
 
 #ifdef TM_B200_GEMM_TRACE
@@ -823,15 +824,7 @@ MmhaPlan mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_ch
         // two SMs.  So: no split up to 2048 tokens when there are that many items; 2048-token splits
         // beyond (they even out the tail of long sequences); with fewer items, just enough splits of at
         // least 256 tokens to put two CTAs on every SM.
-        // An int8 cache is expanded in registers, which takes a CTA's four warps longer than its bytes: there, splits of at
-        // least 192 tokens up to what four CTAs per SM can take of lengths of four fifths of the longest (7B layers, 128 items of
-        // 300 to 900 tokens: 8 layers 638 us unsplit, 565 with 192; 384 items: 741, 704 with 512; the same with an fp16 cache and
-        // 168 items: 1721 and 1769).
-        if (int8 && items < 3ll * sm_count) {
-            const long long even = (long long)max_len * 4 * items / (5 * 4ll * sm_count);
-            chunk = (int)(even < 192 ? 192 : even);
-        }
-        else if (items * 2 >= sm_count) {
+        if (items * 2 >= sm_count) {
             chunk = max_len < 2048 ? max_len : 2048;
         }
         else {
@@ -841,6 +834,15 @@ MmhaPlan mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want_ch
             if (splits < 1) splits = 1;
             chunk = (int)((max_len + splits - 1) / splits);
             if (chunk < 256) chunk = 256;
+        }
+        // An int8 cache is expanded in registers, which takes a CTA's four warps longer than its bytes: there, splits of at
+        // least 192 tokens up to what four CTAs per SM can take of lengths of four fifths of the longest (7B layers, 128 items of
+        // 300 to 900 tokens: 8 layers 638 us unsplit, 565 with 192; 384 items: 741, 704 with 512; the same with an fp16 cache and
+        // 168 items: 1721 and 1769).  `max_len` is the room of a sequence, its length may be far below: never longer splits than
+        // the rule above has, so that a long session among short ones is not the tail of the launch.
+        if (int8 && items < 3ll * sm_count) {
+            const long long even = std::max(192ll, (long long)max_len * 4 * items / (5 * 4ll * sm_count));
+            chunk                = (int)std::min<long long>(chunk, even);
         }
         if (chunk < 64) chunk = 64;
     }

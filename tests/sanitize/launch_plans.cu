@@ -46,6 +46,6 @@ int main()
             }
         }
     }
-    if (!failures) std::puts("launch plans ok");
+    if (!failures) std::puts("plans ok");
     return failures ? 1 : 0;
 }
