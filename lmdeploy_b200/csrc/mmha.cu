@@ -129,7 +129,68 @@ __device__ __forceinline__ int qk_d0(int c, int j)
     return INT8 ? 32 * c + 4 * j : 16 * c + 64 * (j >> 2) + 4 * (j & 3);
 }
 
-template<bool INT8, int W>
+constexpr int kRec = 2 + kD;  // split record: m | l | o[128]
+
+// Sums the splits' records of the query heads of a kv head.  A function of its own: inlined, it takes registers from the loop over
+// the cached rows (64 sequences of 64 / 8 heads, 512 to 3000 tokens, fp16: 88.2 us inlined, 84.3 so).
+template<int kWarps>
+__device__ __noinline__ void merge_splits(const float* ws, __half* out, int nheads, int n_split, int max_splits)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // A warp takes two heads at a time, a lane four dimensions; the loads of four splits of both are on their way together
+    // (one head after the other, split by split, the merge of eight heads took 9 us).
+    for (int h0 = warp; h0 < nheads; h0 += 2 * kWarps) {
+        const int    h1   = min(h0 + kWarps, nheads - 1);
+        const float* rec[2] = {ws + (size_t)h0 * max_splits * kRec, ws + (size_t)h1 * max_splits * kRec};
+        float        top[2] = {-INFINITY, -INFINITY}, ll[2] = {0.f, 0.f}, oo[2][4] = {};
+        for (int s = lane; s < n_split; s += 32) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) top[j] = fmaxf(top[j], __ldcg(rec[j] + (size_t)s * kRec));
+        }
+#pragma unroll
+        for (int m = 16; m >= 1; m /= 2) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) top[j] = fmaxf(top[j], __shfl_xor_sync(0xffffffffu, top[j], m));
+        }
+        for (int s0 = 0; s0 < n_split; s0 += 4) {
+            float2 ml[2][4], o[2][4][2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float* r = rec[j] + (size_t)min(s0 + e, n_split - 1) * kRec;  // records are 8-byte aligned
+                    ml[j][e]       = __ldcg(reinterpret_cast<const float2*>(r));
+                    o[j][e][0]     = __ldcg(reinterpret_cast<const float2*>(r + 2 + 2 * lane));
+                    o[j][e][1]     = __ldcg(reinterpret_cast<const float2*>(r + 2 + kD / 2 + 2 * lane));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (s0 + e >= n_split) break;
+                    const float f = exp2f(ml[j][e].x - top[j]);
+                    ll[j] += ml[j][e].y * f;
+                    oo[j][0] += o[j][e][0].x * f, oo[j][1] += o[j][e][0].y * f;
+                    oo[j][2] += o[j][e][1].x * f, oo[j][3] += o[j][e][1].y * f;
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j == 1 && h0 + kWarps >= nheads) break;
+            __half2*    dst = reinterpret_cast<__half2*>(out + (size_t)(j ? h1 : h0) * kD);
+            const float div = ll[j] + 1.e-6f;
+            dst[lane]          = __floats2half2_rn(oo[j][0] / div, oo[j][1] / div);
+            dst[kD / 4 + lane] = __floats2half2_rn(oo[j][2] / div, oo[j][3] / div);
+        }
+    }
+}
+
+// MANY: several query heads share a kv head.  With one there is little to merge, and that warps share the work would leave all but
+// one of them idle: the loop below stays there, and with it the code ahead of it that the compiler makes (64 sequences of 32 heads, 180
+// to 1180 tokens, int8, no splits: 67.5 us, and 70.0 with the other merge; 128 to 4096 tokens 182 and 187).
+template<bool INT8, int W, bool MANY>
 __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kernel(MmhaParams p)
 {
     constexpr int kWarps   = W;
@@ -629,7 +690,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
     __syncthreads();
 
     // thread = head-dim index (a CTA of fewer than 128 threads takes several); loop over heads
-    constexpr int kRec = 2 + kD;  // split record: m | l | o[128]
     for (int d = tid; d < kD; d += kThreads) {
 #pragma unroll
         for (int h = 0; h < kHeadsPerCta; ++h) {
@@ -726,52 +786,23 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
         return;
     }
     __threadfence();
-    // A warp takes two heads at a time, a lane four dimensions; the loads of four splits of both are on their way together
-    // (one head after the other, split by split, the merge of eight heads took 9 us).
-    for (int h0 = warp; h0 < nheads; h0 += 2 * kWarps) {
-        const int    h1   = min(h0 + kWarps, nheads - 1);
-        const float* rec[2] = {p.ws + (((size_t)bi * p.H + head0 + h0) * p.max_splits) * kRec, p.ws + (((size_t)bi * p.H + head0 + h1) * p.max_splits) * kRec};
-        float        top[2] = {-INFINITY, -INFINITY}, ll[2] = {0.f, 0.f}, oo[2][4] = {};
-        for (int s = lane; s < n_split; s += 32) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) top[j] = fmaxf(top[j], __ldcg(rec[j] + (size_t)s * kRec));
-        }
-#pragma unroll
-        for (int m = 16; m >= 1; m /= 2) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) top[j] = fmaxf(top[j], __shfl_xor_sync(0xffffffffu, top[j], m));
-        }
-        for (int s0 = 0; s0 < n_split; s0 += 4) {
-            float2 ml[2][4], o[2][4][2];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float* r = rec[j] + (size_t)min(s0 + e, n_split - 1) * kRec;  // records are 8-byte aligned
-                    ml[j][e]       = __ldcg(reinterpret_cast<const float2*>(r));
-                    o[j][e][0]     = __ldcg(reinterpret_cast<const float2*>(r + 2 + 2 * lane));
-                    o[j][e][1]     = __ldcg(reinterpret_cast<const float2*>(r + 2 + kD / 2 + 2 * lane));
-                }
+    if (MANY) {
+        merge_splits<kWarps>(p.ws + ((size_t)bi * p.H + head0) * p.max_splits * kRec, p.out + ((size_t)bi * p.H + head0) * kD, nheads, n_split, p.max_splits);
+        return;
+    }
+    for (int d = tid; d < kD; d += kThreads) {
+        for (int h = 0; h < nheads; ++h) {
+            const float* rec0 = p.ws + (((size_t)bi * p.H + head0 + h) * p.max_splits) * kRec;
+            float        mm   = -INFINITY;
+            for (int s = 0; s < n_split; ++s) mm = fmaxf(mm, __ldcg(rec0 + (size_t)s * kRec));
+            float ll = 0.f, oo = 0.f;
+            for (int s = 0; s < n_split; ++s) {
+                const float* rec = rec0 + (size_t)s * kRec;
+                const float  f   = exp2f(__ldcg(rec) - mm);
+                ll += __ldcg(rec + 1) * f;
+                oo += __ldcg(rec + 2 + d) * f;
             }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    if (s0 + e >= n_split) break;
-                    const float f = exp2f(ml[j][e].x - top[j]);
-                    ll[j] += ml[j][e].y * f;
-                    oo[j][0] += o[j][e][0].x * f, oo[j][1] += o[j][e][0].y * f;
-                    oo[j][2] += o[j][e][1].x * f, oo[j][3] += o[j][e][1].y * f;
-                }
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (j == 1 && h0 + kWarps >= nheads) break;
-            __half2*    dst = reinterpret_cast<__half2*>(p.out + ((size_t)bi * p.H + head0 + (j ? h1 : h0)) * kD);
-            const float div = ll[j] + 1.e-6f;
-            dst[lane]          = __floats2half2_rn(oo[j][0] / div, oo[j][1] / div);
-            dst[kD / 4 + lane] = __floats2half2_rn(oo[j][2] / div, oo[j][3] / div);
+            p.out[((size_t)bi * p.H + head0 + h) * kD + d] = __float2half_rn(oo / (ll + 1.e-6f));
         }
     }
 }
@@ -787,13 +818,15 @@ constexpr size_t mmha_smem_bytes()
 template<bool INT8, int W>
 cudaError_t mmha_prepare_one()
 {
-    return cudaFuncSetAttribute(mmha_decode_kernel<INT8, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mmha_smem_bytes<INT8, W>());
+    const cudaError_t e = cudaFuncSetAttribute(mmha_decode_kernel<INT8, W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mmha_smem_bytes<INT8, W>());
+    return e == cudaSuccess ? cudaFuncSetAttribute(mmha_decode_kernel<INT8, W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mmha_smem_bytes<INT8, W>()) : e;
 }
 
 template<bool INT8, int W>
 cudaError_t mmha_launch_one(dim3 grid, const MmhaParams& p, cudaStream_t st, bool pdl)
 {
-    return launch_kernel(mmha_decode_kernel<INT8, W>, grid, dim3(W * 32), mmha_smem_bytes<INT8, W>(), st, pdl, p);
+    return p.H > p.Hkv ? launch_kernel(mmha_decode_kernel<INT8, W, true>, grid, dim3(W * 32), mmha_smem_bytes<INT8, W>(), st, pdl, p) :
+                         launch_kernel(mmha_decode_kernel<INT8, W, false>, grid, dim3(W * 32), mmha_smem_bytes<INT8, W>(), st, pdl, p);
 }
 
 }  // namespace
