@@ -150,7 +150,8 @@ __device__ __forceinline__ void epilogue16(const DenseEpilogue& ep, const float 
         }
         return;
     }
-    if (ep.kind == DenseKind::kInput && __any_sync(0xffffffffu, n >= ep.tanh_lo && n < ep.tanh_hi)) {
+    const int n0 = n & ~31;  // the warp's first column: one answer for its lanes, of which some may have left above
+    if (ep.kind == DenseKind::kInput && n0 + 32 > ep.tanh_lo && n0 < ep.tanh_hi) {
         const bool th = n >= ep.tanh_lo && n < ep.tanh_hi;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {

@@ -55,8 +55,8 @@ class _Product:
         self.c = C.c_void_p(self.lib.call_new())
         self.lib.set_operands(self.c, _p(self.x), _p(self.x2), x2_from, k, _p(self.w), k, tokens, n, k)
 
-    def run(self):
-        assert self.lib.route(self.c, self.lib.sm_count(self.h)) == 3, "the plan gives this size to pairs no more: choose another"
+    def run(self, route=3):
+        assert self.lib.route(self.c, self.lib.sm_count(self.h)) == route, "the plan gives this size to pairs no more: choose another"
         st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
         assert self.lib.run(self.h, self.c, st) == 0
         word = C.c_uint(0)
@@ -100,3 +100,41 @@ def test_residual_and_row_sums(dense, tokens, n, k, gated):
     _within(sums[:tiles, :tokens], pad(want ** 2), pad(2 * want.abs() * err + err ** 2) + pad(want ** 2) * (32 * ULP), "sums of squares")
     assert bool((sums[tiles:] == GUARD).all()), "written behind the last tile's sums"
     assert bool((sums[:tiles, tokens:] == GUARD).all())
+
+
+def _input(q, split, tanh, f32_from=0):
+    """kInput: columns below `split` (some through tanh, some in fp32), gated ones behind; checks all of them"""
+    n, tokens = q.n, q.tokens
+    out, act = (torch.full((tokens, w + 8), GUARD, device="cuda", dtype=torch.bfloat16) for w in (split, (n - split) // 2))
+    q.lib.set_input(q.c, _p(out), split + 8, tanh[0], tanh[1], split, _p(act), act.shape[1])
+    f32 = torch.full((tokens, split - f32_from + 3), GUARD, device="cuda")
+    if f32_from:
+        q.lib.set_f32_columns(q.c, _p(f32), f32_from, f32.shape[1])
+
+    def check():
+        y, err = q.y, q.err
+        want = y[:, :split].clone()
+        want[:, tanh[0]:tanh[1]] = torch.tanh(want[:, tanh[0]:tanh[1]])
+        stored = f32_from or split
+        # |tanh'| <= 1, tanhf is within two ulps
+        _within(out[:, :stored], want[:, :stored], err[:, :stored] + want[:, :stored].abs() * (2.0 ** -8 + 4 * ULP), "stored columns")
+        assert bool((out[:, stored:] == GUARD).all())
+        if f32_from:
+            _within(f32[:, :split - f32_from], y[:, f32_from:split], err[:, f32_from:split] + y[:, f32_from:split].abs() * ULP, "fp32 columns")
+            assert bool((f32[:, split - f32_from:] == GUARD).all())
+        gate, up, eg, eu = y[:, split::2], y[:, split + 1::2], err[:, split::2], err[:, split + 1::2]
+        gelu = torch.nn.functional.gelu(gate, approximate="tanh")
+        # |gelu'| <= 1.13; __expf's argument u is off by a few ulps and it by 2 + 1.2 |u| more: |gelu| (8 + 4 |u|) ulps
+        u = 1.5957691216057308 * (gate + 0.044715 * gate ** 3)
+        bound = 1.13 * eg * up.abs() + gelu.abs() * eu + 1.13 * eg * eu + (gelu * up).abs() * (2.0 ** -8 + (8 + 4 * u.abs()) * 2 * ULP)
+        _within(act[:, :(n - split) // 2], gelu * up, bound + 1e-30, "gated columns")
+        assert bool((act[:, (n - split) // 2:] == GUARD).all())
+    return check
+
+
+@pytest.mark.parametrize("tokens,n,split,tanh,f32_from,route", [(200, 9216, 1024, (100, 300), 500, 3), (40, 1024, 512, (70, 400), 300, 2)])
+def test_fp32_columns_that_begin_inside_a_warps(dense, tokens, n, split, tanh, f32_from, route):
+    q = _Product(dense, tokens, n, 4096)
+    check = _input(q, split, tanh, f32_from)
+    q.run(route)
+    check()
