@@ -138,3 +138,46 @@ def test_fp32_columns_that_begin_inside_a_warps(dense, tokens, n, split, tanh, f
     check = _input(q, split, tanh, f32_from)
     q.run(route)
     check()
+
+
+# 79 tiles with the gated columns ending inside the last one, a tile's k that ends inside a block, ragged tokens
+@pytest.mark.parametrize("tokens,n,k,split,tanh", [(300, 9344, 4096, 5120, (1000, 1100)), (257, 10056, 1000, 256, (0, 0)), (129, 9216, 512, 9088, (0, 9088))])
+def test_input_projection(dense, tokens, n, k, split, tanh):
+    """Columns through tanh, gated columns, and rows that are scaled by their norm (sums of squares in several parts)."""
+    q = _Product(dense, tokens, n, k)
+    parts, stride = 3, tokens + 5
+    ssq, gain = q.draw(parts, stride).abs() * k / parts, q.draw(1).abs() + 0.5
+    q.lib.set_scale(q.c, _p(ssq), parts, stride, C.c_float(1.0 / k), C.c_float(1e-5), _p(gain))
+    s = gain.double() / torch.sqrt(ssq.double()[:, :tokens].sum(0) / k + 1e-5)
+    q.y *= s[:, None]
+    q.err = q.err * s[:, None] + q.y.abs() * (8 * ULP)  # sums, quotient and root in fp32
+    check = _input(q, split, tanh)
+    q.run()
+    check()
+
+
+@pytest.mark.parametrize("tokens,n,k,x2_from,f32_from", [(300, 9377, 1024, 5120, 9344), (600, 2210, 512, 1024, 2177)])
+@pytest.mark.parametrize("ld", [0, 3])
+def test_second_operand_and_fp32_columns(dense, tokens, n, k, x2_from, f32_from, ld):
+    """Columns that multiply a second operand, the last of them in fp32; rows that 16-byte stores reach, and not."""
+    q = _Product(dense, tokens, n, k, x2_from)
+    width = (f32_from + 7) // 8 * 8 + ld
+    out, f32 = torch.full((tokens, width), GUARD, device="cuda", dtype=torch.bfloat16), torch.full((tokens, n - f32_from + 1), GUARD, device="cuda")
+    q.lib.set_store(q.c, _p(out), width)
+    q.lib.set_f32_columns(q.c, _p(f32), f32_from, f32.shape[1])
+    q.run()
+    _within(out[:, :f32_from], q.y[:, :f32_from], q.err[:, :f32_from] + q.y[:, :f32_from].abs() * 2.0 ** -8, "stored columns")
+    assert bool((out[:, f32_from:] == GUARD).all())
+    _within(f32[:, :-1], q.y[:, f32_from:], q.err[:, f32_from:] + q.y[:, f32_from:].abs() * ULP, "fp32 columns")
+    assert bool((f32[:, -1] == GUARD).all())
+
+
+# one tile of columns and a last one of 8, tokens of several bands of tiles and a last tile of one token
+@pytest.mark.parametrize("tokens,n,k,ld", [(257, 5000, 512, 5000), (2049, 5000, 1000, 5003), (513, 9608, 4096, 9608), (97, 9600, 584, 9600)])
+def test_stored_rows(dense, tokens, n, k, ld):
+    q = _Product(dense, tokens, n, k)
+    out = torch.full((tokens + 1, ld), GUARD, device="cuda", dtype=torch.bfloat16)
+    q.lib.set_store(q.c, _p(out), ld)
+    q.run()
+    _within(out[:tokens, :n], q.y, q.err + q.y.abs() * 2.0 ** -8, "rows")
+    assert bool((out[:, n:] == GUARD).all()) and bool((out[tokens] == GUARD).all())

@@ -1,5 +1,5 @@
-"""Products with many tokens: the dense kernel's pairs of CTAs and the W4A16 GEMM that expands its weight first, at the edges of
-their tiles, against 64-bit sums of the same operands."""
+"""Products with many tokens: the dense kernel and the W4A16 GEMM that expands its weight first (both with few columns and many
+tokens; the bf16 pairs of CTAs are in test_gpu_dense_pairs.py), at the edges of their tiles, against 64-bit sums of the same operands."""
 import ctypes as C
 
 import pytest
@@ -22,8 +22,8 @@ def _check(got, want, scale, k, digits, what):
 @pytest.mark.parametrize("tokens", [65, 128, 255, 256, 257, 2049])
 @pytest.mark.parametrize("n_out,k,ld", [(128, 64, 128), (384, 200, 392), (1000, 136, 1000), (2080, 512, 2083)])
 def test_dense_pairs(tokens, n_out, k, ld):
-    """Odd column tiles (the second CTA of a pair has none or a part), k that ends inside a block, tokens around a tile's and a
-    band's end, rows that 16-byte stores cannot reach; both output types.  Nothing beyond a row's n_out columns is written."""
+    """Odd column tiles, k that ends inside a block, tokens around a tile's end, rows that 16-byte stores cannot reach; both output
+    types (weights this small stay with single CTAs).  Nothing beyond a row's n_out columns is written."""
     from lmdeploy_b200 import lib as l
     g = torch.Generator(device="cuda").manual_seed(tokens + n_out)
     x = torch.randn(tokens, k, device="cuda", generator=g).bfloat16()
