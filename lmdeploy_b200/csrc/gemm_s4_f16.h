@@ -34,9 +34,9 @@ struct GemmSmallPlan {
     int    ctas;
     int    slots_per_chunk;  // split-K scratch slots per token chunk (= ctas + n_col_tiles)
     int    stages;
-    int    cols_tiles;     // 1 or 2: the column-owner kernel runs instead, on strips of that many 32-column tiles (up to 8 tokens,
-                           // or 16 tokens); 0: the split-K kernel
-    int    cols_cluster;   // CTAs that share a strip
+    int    cols_tiles;     // 1 or 2: the column-owner kernel runs instead, on strips of that many 32-column tiles (up to 16 tokens
+                           // with one, 8 with two); 0: the split-K kernel
+    int    cols_cluster;   // CTAs that share a strip, all strips' at once on the device (or 1)
     size_t smem_bytes;
     size_t workspace_floats;
     size_t counter_ints;

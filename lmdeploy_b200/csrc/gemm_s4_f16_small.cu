@@ -777,7 +777,6 @@ size_t gemm_small_smem_bytes(int nt)
 
 GemmSmallPlan gemm_small_plan(int N, int T, int K, int sm_count, int max_smem, int cols_variant)
 {
-    (void)max_smem;
     GemmSmallPlan pl{};
     pl.nt = T <= 8 ? 1 : (T <= 16 ? 2 : 4);
     const int tp   = pl.nt * 8;
@@ -795,10 +794,11 @@ GemmSmallPlan gemm_small_plan(int N, int T, int K, int sm_count, int max_smem, i
     pl.smem_bytes       = gemm_small_smem_bytes(pl.nt);
     pl.workspace_floats = (size_t)pl.t_chunks * pl.slots_per_chunk * tp * kUnitCols;
     pl.counter_ints     = (size_t)pl.t_chunks * pl.n_col_tiles;
-    // Enough column strips to give every SM one: the column-owner kernel, which splits nothing between CTAs.  The
-    // scratch sizes above stay (unused) so that a caller's workspace is sized the same way for both kernels.
-    // Variant 1: 32-column strips, three CTAs per SM, a ring of up to four groups per warp (the whole K range of a
-    // 4096-row weight is requested at once); variant 2: 64-column strips, two CTAs per SM, three groups.
+    // All column strips resident at once, or one token: the column-owner kernel, which sends nothing through scratch (up to 16 tokens
+    // with 32-column strips, 8 with 64-column ones).  The scratch sizes above stay (unused) so that a caller's workspace is sized
+    // the same way for both kernels.
+    // Variant 1: 32-column strips, three CTAs per SM (two above 8 tokens), a ring of up to four groups per warp (the whole K range
+    // of a 4096-row weight is requested at once); variant 2: 64-column strips, two CTAs per SM, three groups.
     const int tiles  = cols_variant == 2 ? 2 : 1;
     const int strips = (N / kColsPerTile + tiles - 1) / tiles;
     // Measured on the 7B shapes: with all strips resident at once (qkv: 384 strips for 444 slots) it wins at every
@@ -809,13 +809,27 @@ GemmSmallPlan gemm_small_plan(int N, int T, int K, int sm_count, int max_smem, i
     const bool worthwhile = strips <= co_slots || T == 1;
     pl.cols_tiles         = (cols_variant != 0 && T <= 8 * (tiles == 1 ? 2 : 1) && worthwhile) ? tiles : 0;
     if (pl.cols_tiles) {
-        // few strips: clusters of up to eight CTAs share one, as many as have a slot at once and a group for each warp
-        const int warps_full = (K / 128 + kWarps - 1) / kWarps;
-        pl.cols_cluster      = std::max(1, std::min({kMaxCluster, co_slots / strips, warps_full}));
-        const int per_warp   = (K / 128 + kWarps * pl.cols_cluster - 1) / (kWarps * pl.cols_cluster);  // groups of the busiest warp
-        pl.ctas       = strips * pl.cols_cluster;
-        pl.stages     = tiles == 2 ? 3 : (per_warp < 2 ? 2 : (per_warp > 4 ? 4 : per_warp));
-        pl.smem_bytes = (size_t)kWarps * pl.stages * co_stage_bytes(tiles) + (pl.cols_cluster > 1 ? (size_t)pl.cols_cluster * tiles * wide * 1024 : 0);
+        // Few strips: clusters of up to eight CTAs share one, as many as have a slot at once and a group for each warp.  The slots of
+        // an SM follow from the shared memory, of which the sums that a strip's first CTA takes in are a part; a cluster lies in
+        // one GPC, so not all slots can be used (of 444 / 296: 426 / 279 by clusters of three, 384 / 264 by clusters of eight).  A
+        // ring of three groups costs less than a smaller cluster, and either less than a second wave (us, 1 / 8 tokens, 1312 x 32768:
+        // 11.9 / 17.0 in two waves, 10.2 / 14.6 with clusters of seven, 9.0 / 12.5 with eight and three groups).
+        const int  warps_full = (K / 128 + kWarps - 1) / kWarps, per_sm = co_slots / sm_count;
+        const auto resident   = [&](int cluster, size_t smem) {
+            const long long slots = (long long)sm_count * std::min<size_t>(per_sm, ((size_t)max_smem + 1024) / (smem + 1024));
+            return strips * cluster * 100ll <= slots * (cluster <= 2 ? 100 : cluster <= 6 ? 91 : 86);
+        };
+        for (int cluster = std::max(1, std::min({kMaxCluster, co_slots / strips, warps_full}));; --cluster) {
+            const int    per_warp = (K / 128 + kWarps * cluster - 1) / (kWarps * cluster);  // groups of the busiest warp
+            const size_t inbox    = cluster > 1 ? (size_t)cluster * tiles * wide * 1024 : 0;
+            auto         bytes    = [&](int stages) { return (size_t)kWarps * stages * co_stage_bytes(tiles) + inbox; };
+            pl.cols_cluster = cluster;
+            pl.ctas         = strips * cluster;
+            pl.stages       = tiles == 2 ? 3 : std::min(4, std::max(2, per_warp));
+            if (cluster > 1 && pl.stages == 4 && !resident(cluster, bytes(4))) pl.stages = 3;
+            pl.smem_bytes = bytes(pl.stages);
+            if (cluster == 1 || resident(cluster, pl.smem_bytes)) break;
+        }
     }
     return pl;
 }

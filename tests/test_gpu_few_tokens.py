@@ -38,3 +38,21 @@ def test_strips_shared_by_clusters(n, k, silu):
             slack = 2 * (1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2]) + y.abs() * 2.0 ** -11 + 1e-6
         over = ((buf[:tokens].double() - y).abs() / slack).max().item()
         assert over <= 1.0, f"{n} x {k}, {tokens} tokens: {over:.2f} of the bound"
+
+
+# rings of three groups beside the sums of a large cluster, strips for which clusters of eight or seven do not all find room
+@pytest.mark.parametrize("n,k", [(1280, 28672), (1312, 32768), (1760, 8192), (1760, 28672), (2016, 4096)])
+@pytest.mark.parametrize("tokens", [1, 8, 12])
+def test_long_strips_shared_by_clusters(n, k, tokens):
+    from lmdeploy_b200 import turbomind as tm
+    from perf import cases
+    w = cases._linear(cases._gen(5, n), n, k)
+    exact = cases._exact_weight(cases._gen(5, n), n, k)
+    op = tm.LlamaLinear(0)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).half()
+    out = torch.empty(tokens, n, dtype=torch.float16, device="cuda")
+    op.forward(out, x, tokens, w, op.kGemm)
+    op.gemm_s4_f16_.handle.check_device_status(torch.cuda.current_stream().cuda_stream)
+    y, size = x.double() @ exact, x.double().abs() @ exact.abs()
+    over = ((out.double() - y).abs() / (y.abs() * 2.0 ** -11 + size * (2.0 ** -11 + k * 2.0 ** -24) + 1e-7)).max().item()
+    assert over <= 1.0, f"{over:.2f} of the bound"

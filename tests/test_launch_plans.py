@@ -9,7 +9,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("what", ["launch", "attention"])
+@pytest.mark.parametrize("what", ["launch", "attention", "strip"])
 def test_plans_under_ubsan(what, tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc) or shutil.which("g++") is None:
