@@ -63,7 +63,7 @@ TM_API int tm_check_device_status(tm_handle* h, void* stream, unsigned* word);
 /* Number of kernel launches issued through this handle since creation. */
 TM_API unsigned long long tm_launch_count(const tm_handle* h);
 /* Tuning knobs of this handle (no reference counterpart; the same knobs are read from the environment
- * at tm_create).  `name`: "gemm_tc_min_n" (token count from which the tcgen05 GEMM is used; by the product's size unless set),
+ * at tm_create).  `name`: "gemm_tc_min_n" (token count from which the tcgen05 GEMM is used; -1, the default: by the product's size),
  * "pdl_direct" (1: GEMM / attention calls made directly through the handle launch with programmatic stream
  * serialization, as the decode driver's do; only where no kernel ahead in the stream writes weights or cached rows),
  * "gemm_wait_cycles" (bound of the tcgen05 GEMM's wait for the partners of a split tile, 0 = default; tests),
@@ -71,8 +71,8 @@ TM_API unsigned long long tm_launch_count(const tm_handle* h);
  * them into the tensor-core GEMMs on either side),
  * "lm_head_cublas" (1: the decode driver computes the lm-head with cuBLAS, as the reference does, instead of this
  * library's kernel; for comparison),
- * "gemv_cols" (the GEMM for 1..8 tokens: 0 = always the stream-K kernel, 1 = the column-owner kernel on 32-column strips
- * where the weight has a strip for every SM, 2 = on 64-column strips),
+ * "gemv_cols" (the GEMM for few tokens: 0 = always the stream-K kernel, 1 = the column-owner kernel on 32-column strips where
+ * all of them are resident at once, up to 16 tokens, 2 = on 64-column strips, up to 8 tokens),
  * "mmha_chunk" (cached tokens per KV split, 0 = automatic), "mmha_warps" (warps per attention CTA: 1, 2,
  * 4 or 0 = automatic), "pdl" (1 = tm_llama_decode launches with programmatic dependent launch).
  * Returns TM_ERR_INVALID_ARG for an unknown name or value. */
@@ -90,6 +90,10 @@ TM_API int tm_set_option(tm_handle* h, const char* name, int value);
  * Requirements: group_size == 128, k % 128 == 0, m % 32 == 0 (type 1: m % 64 == 0), n >= 1.
  * `workspace` may be NULL (the handle's own scratch is used); otherwise it must hold
  * tm_gemm_s4_f16_workspace_bytes(m, n, k) bytes, zero-filled once before first use.
+ * The two are not the same launches: a caller's workspace has room for the small-token kernels up to 16 tokens and for whole
+ * tiles of the tcgen05 kernel above, so that with 9 to 16 tokens the result is rounded as with 8 (the weight is not rounded to
+ * fp16 before the product), and from 17 tokens on neither are tiles cut that fill the device nor is the weight expanded
+ * ahead of the product: some products take up to 1.4 times as long.  Prefer NULL.
  */
 enum { TM_GEMM_PLAIN = 0, TM_GEMM_FUSED_SILU_FFN = 1 };
 TM_API size_t tm_gemm_s4_f16_workspace_bytes(int m, int n, int k);

@@ -147,8 +147,8 @@ extern "C" int tm_set_option(tm_handle* h, const char* name, int value)
 {
     if (!h || !name) return TM_ERR_INVALID_ARG;
     const std::string n(name);
-    if (n == "gemm_tc_min_n" && value >= 1) {
-        h->gemm_tc_min_n = value;
+    if (n == "gemm_tc_min_n" && (value >= 1 || value == -1)) {
+        h->gemm_tc_min_n = value;  // -1: by the product's size again
     }
     else if (n == "mmha_chunk" && value >= 0) {
         h->mmha_chunk = value;

@@ -56,3 +56,29 @@ def test_long_strips_shared_by_clusters(n, k, tokens):
     y, size = x.double() @ exact, x.double().abs() @ exact.abs()
     over = ((out.double() - y).abs() / (y.abs() * 2.0 ** -11 + size * (2.0 ** -11 + k * 2.0 ** -24) + 1e-7)).max().item()
     assert over <= 1.0, f"{over:.2f} of the bound"
+
+
+def test_the_line_between_the_kernels_can_be_drawn_and_taken_back():
+    """gemm_tc_min_n: the two kernels round differently, so a product's bits tell which one ran."""
+    from lmdeploy_b200 import lib as l, turbomind as tm
+    from perf import cases
+    n, k, tokens = 11008, 4096, 16
+    w = cases._linear(cases._gen(5, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).half()
+    op = tm.LlamaLinear(0)
+    op.gemm_s4_f16_.handle = h = l.Handle(0)
+
+    def product():
+        out = torch.empty(tokens, n, dtype=torch.float16, device="cuda")
+        op.forward(out, x, tokens, w, op.kGemm)
+        h.check_device_status(torch.cuda.current_stream().cuda_stream)
+        return out
+
+    by_size = product()
+    h.set_option("gemm_tc_min_n", 17)
+    drawn = product()
+    h.set_option("gemm_tc_min_n", -1)
+    assert not torch.equal(by_size, drawn) and torch.equal(by_size, product())
+    with pytest.raises(l.TmError):
+        h.set_option("gemm_tc_min_n", 0)
+    h.close()
