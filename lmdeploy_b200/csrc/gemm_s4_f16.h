@@ -75,6 +75,7 @@ struct GemmTcParams {
     int                  fused_silu;
     // filled in by gemm_tc_launch from the plan
     int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, x_stages, a_stages, acc_stride, parts_per_tile;
+    int       last_sums;        // 1: a split tile is reduced by the CTA that is done last, without a wait (no GemmNormFusion)
     long long max_wait_cycles;  // bound of the wait for the partners of a split tile; 0 = the default
     GemmNormFusion norm;        // all null: a plain GEMM
 };
@@ -88,6 +89,7 @@ struct GemmTcPlan {
     int    parts_per_tile;  // CTAs per column tile (each with up to units_per_cta groups of it); 0 = the flat unit list cut evenly
     int    ctas;
     int    slots_per_chunk;
+    int    last_sums;      // see GemmTcParams
     size_t smem_bytes;
     size_t workspace_floats;
     size_t counter_ints;

@@ -467,11 +467,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         int           n_pend = 0;
         // Every CTA of a split tile reduces its own share of the feature rows, once all partials of the
         // tile are in scratch: nobody reads more than one tile's worth, and the sum runs in CTA order.
+        // p.last_sums: the CTA whose partial is the last one reduces all rows, and nobody waits.
         auto reduce_share = [&](int tjs) {
             int       c_first;
             const int n_split = tile_ctas(tjs, c_first);
             const int col0    = tjs * kSuperN;
-            if (dtid == 0) {
+            if (dtid == 0 && !p.last_sums) {
                 // Bounded wait for the other CTAs of the tile.  The plan splits tiles between CTAs only
                 // when the whole grid is one wave of at most one CTA per SM (gemm_tc_plan), so the
                 // partners are running or waiting for an SM that a kernel ahead in the stream still
@@ -492,12 +493,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             if (p.norm.ssq_out && dtid < t_rows) s_ssq[dtid] = 0ull;
             named_bar_sync(1, kDqThreads);
             TC_TRACE(trow, 42, tjs);
-            const bool tile_ok = bars->flag != 0;  // read between the barriers: the next call may rewrite the flag
+            const bool tile_ok = p.last_sums || bars->flag != 0;  // read between the barriers: the next call may rewrite the flag
             if (tile_ok) {
                 const int j      = blockIdx.x - c_first;
                 const int n_cols = min(kSuperN, p.N - col0);  // N % 32 == 0
-                const int f0     = (n_cols * j / n_split) & ~3;
-                const int f1     = j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
+                const int f0     = p.last_sums ? 0 : (n_cols * j / n_split) & ~3;
+                const int f1     = p.last_sums || j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
                 const int quads  = (f1 - f0) / 4;
                 const int items  = t_rows * quads;
                 const float* tile_slots = slots + (size_t)(c_first + tjs) * slot_floats;
@@ -559,7 +560,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             }
             named_bar_sync(1, kDqThreads);  // everyone is done reading; the flag may be reused
             if (p.norm.ssq_out && tile_ok && dtid < t_rows && s_ssq[dtid]) atomicAdd(p.norm.ssq_out + t0 + dtid, s_ssq[dtid]);
-            if (dtid == 0) {
+            if (dtid == 0 && p.last_sums) arrive[tjs] = 0;
+            if (dtid == 0 && !p.last_sums) {
                 // the last reader of the tile resets both counts for the next launch; a CTA that gave up
                 // on the wait counts as a reader too, so the counts recover after a time-out
                 if (atomicAdd(done + tjs, 1) == n_split - 1) {
@@ -715,7 +717,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 named_bar_sync(1, kDqThreads);
                 if (dtid == 0) {
                     __threadfence();
-                    atomicAdd(arrive + this_js, 1);
+                    const int before = atomicAdd(arrive + this_js, 1);
+                    if (p.last_sums) {
+                        __threadfence();
+                        bars->flag = before == n_split - 1;
+                    }
+                }
+                if (p.last_sums) {
+                    named_bar_sync(1, kDqThreads);
+                    if (bars->flag == 0) continue;  // rewritten behind the next barrier of these threads at the earliest
                 }
                 if (n_pend == kMaxPending) {
                     reduce_share(pend[0]);
@@ -807,6 +817,7 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
     const double    fill  = std::max(0, pl.token_tile - 32) / 96.0;  // what a unit costs beyond its expansion
     auto cut_us = [&](int units) { return 8.5 + units * (0.711 + 0.083 * fill) + 10.2 * units / G + 13.8 * pl.token_tile / 128; };
     bool whole = tiles >= sm_count;
+    const bool could = whole;
     if (whole) {
         pl.us = 4.2 + (double)((tiles + sm_count - 1) / sm_count) * (G * (0.56 + 0.14 * fill) + 12.7);
         if (balance && pl.t_chunks <= sm_count / 2) {
@@ -839,6 +850,10 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
         }
         pl.us = cut_us(pl.units_per_cta);
     }
+    // Tiles that are cut only because it is faster are summed by the CTA that is done last: a product of that size never depended on
+    // its CTAs running together (4096 x 11008 with 1200 tokens 104.0 us, 105.0 with the wait; 57344 x 8192 with 32 tokens 79.9 / 81.8).
+    // With fewer tiles than SMs every CTA sums a share (4096 x 11008 with 16 / 64 tokens: 13.7 / 15.7 us, by the last one 15.0 / 25.2).
+    pl.last_sums       = could && !whole;
     pl.slots_per_chunk = pl.ctas + pl.n_col_tiles;
     pl.smem_bytes      = gemm_tc_smem_bytes(pl.token_tile);
     pl.workspace_floats = pl.units_per_cta % G == 0 ? 0 : (size_t)pl.t_chunks * pl.slots_per_chunk * pl.token_tile * kSuperN;
@@ -867,6 +882,7 @@ cudaError_t gemm_tc_launch(const GemmTcPlan& pl, GemmTcParams p, cudaStream_t st
     p.slots_per_chunk = pl.slots_per_chunk;
     p.n_col_tiles     = pl.n_col_tiles;
     p.token_tile      = pl.token_tile;
+    p.last_sums       = pl.last_sums;
     p.x_stages        = x_stages_for(pl.token_tile);
     p.a_stages        = a_stages_for(pl.token_tile);
     if (p.max_wait_cycles <= 0) p.max_wait_cycles = kMaxWaitCycles;

@@ -31,6 +31,7 @@ static void check_tc(int N, int T, int K, int sms, bool balance)
         check((long long)pl.ctas * pl.t_chunks <= sms, "CTAs that wait for one another do not fit", N, T, K, sms, balance);
         check(pl.workspace_floats > 0, "no workspace", N, T, K, sms, balance);
     }
+    check(pl.last_sums == (tiles >= sms && pl.units_per_cta != G), "who sums", N, T, K, sms, balance);
     if (!balance && tiles >= sms) check(pl.units_per_cta == G && pl.workspace_floats == 0, "cut without balance", N, T, K, sms, balance);
 }
 
@@ -45,6 +46,12 @@ int main()
                 check_tc(s[0], T, s[1], sms, true);
             }
         }
+    }
+    // the sizes that tests/test_gpu_many_tokens.py runs as products cut evenly although there is a tile for every SM
+    const int even[][3] = {{57344, 1024, 17}, {40960, 2048, 100}, {22016, 4096, 200}};
+    for (auto& s : even) {
+        const tmb::GemmTcPlan pl = tmb::gemm_tc_plan(s[0], s[2], s[1], 148, true);
+        check(pl.last_sums && pl.units_per_cta % (s[1] / 128) && pl.t_chunks * pl.n_col_tiles >= 148, "not cut evenly", s[0], s[2], s[1], 148, true);
     }
     if (!failures) std::puts("plans ok");
     return failures ? 1 : 0;

@@ -85,3 +85,24 @@ def test_units_cut_evenly(n, k, tokens):
                                      0, None, 0, _stream()), "tm_gemm_s4_f16")
     h.check_device_status(torch.cuda.current_stream().cuda_stream)
     _check(out, x.double() @ exact, x.double().abs() @ exact.abs(), k, 11, (n, k, tokens))
+
+
+@pytest.mark.parametrize("n,k,tokens", [(57344, 1024, 17), (22016, 4096, 200)])
+def test_units_cut_evenly_wait_for_nobody(n, k, tokens):
+    """A product that has a tile for every SM does not need its CTAs to run together: a bound of one cycle on the wait for a split
+    tile's other CTAs changes nothing."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    h = l.Handle(0)
+    w = cases._linear(cases._gen(4, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    out = []
+    for bound in (0, 1, 1, 1):
+        h.set_option("gemm_wait_cycles", bound)
+        launches = h.launch_count()
+        out.append(torch.empty(tokens, n, dtype=torch.float16, device="cuda"))
+        l.check(l.lib.tm_gemm_s4_f16(h.ptr, out[-1].data_ptr(), w.kernel.data_ptr(), x.data_ptr(), w.scales_and_zeros.data_ptr(), n, tokens, k, 128,
+                                     0, None, 0, _stream()), "tm_gemm_s4_f16")
+        h.check_device_status(torch.cuda.current_stream().cuda_stream)
+        assert h.launch_count() - launches == 1 and torch.equal(out[-1], out[0])
+    h.close()
