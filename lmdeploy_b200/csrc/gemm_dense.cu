@@ -404,9 +404,12 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
             // the products that free the last stages also arrive at the other CTA's barriers: nobody leaves before
             for (int i = max(0, issued - ST); i < issued; ++i) mbar_wait_warp(&sh->empty[i % ST], (i / ST) & 1, p.max_wait);
         }
-        if (!ok) {
-            // the CTA leaves early: not before its own copies have landed
-            for (int i = max(0, issued - ST); i < issued; ++i) mbar_wait_warp(&sh->full[i % ST], (i / ST) & 1, p.max_wait);
+        if (!ok && rank == 0) {
+            // the CTA leaves early: not before its own copies have landed (a pair's are all counted here, and both leave together;
+            // what has not landed by the end of a wait was never issued)
+            for (int i = max(0, issued - ST); i < issued; ++i) {
+                if (!mbar_wait_warp(&sh->full[i % ST], (i / ST) & 1, p.max_wait)) break;
+            }
         }
     }
     else if (warp == 1) {
@@ -860,7 +863,7 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     p.scratch  = static_cast<float*>(h->scratch);
     p.tickets  = h->counters;
     p.status   = h->status;
-    p.max_wait = h->gemm_wait_cycles > 0 ? h->gemm_wait_cycles : kMaxWaitCycles;
+    p.max_wait = kMaxWaitCycles;  // of the pipeline's waits: no CTA of this kernel waits for another one's part of a tile
     p.ep       = g.ep;
     // rows of `out` and `act` that 16-byte stores reach
     auto aligned = [](const void* ptr, int ld) { return ptr && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };

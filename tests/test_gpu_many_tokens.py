@@ -106,3 +106,24 @@ def test_units_cut_evenly_wait_for_nobody(n, k, tokens):
         h.check_device_status(torch.cuda.current_stream().cuda_stream)
         assert h.launch_count() - launches == 1 and torch.equal(out[-1], out[0])
     h.close()
+
+
+def test_the_bound_on_split_tiles_is_not_the_dense_pipelines():
+    """gemm_wait_cycles bounds the wait for a split tile's other CTAs: an expanded weight's product has none."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    n, k, tokens = 4128, 2048, 6000
+    h = l.Handle(0)
+    w = cases._linear(cases._gen(4, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    out = []
+    for bound in (0, 1):
+        h.set_option("gemm_wait_cycles", bound)
+        out.append(torch.empty(tokens, n, dtype=torch.float16, device="cuda"))
+        launches = h.launch_count()
+        l.check(l.lib.tm_gemm_s4_f16(h.ptr, out[-1].data_ptr(), w.kernel.data_ptr(), x.data_ptr(), w.scales_and_zeros.data_ptr(), n, tokens, k, 128,
+                                     0, None, 0, _stream()), "tm_gemm_s4_f16")
+        h.check_device_status(torch.cuda.current_stream().cuda_stream)
+        assert h.launch_count() - launches == 2
+    assert torch.equal(out[0], out[1])
+    h.close()
