@@ -75,7 +75,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             GemmTcParams p{};
             p.C = (__half*)C, p.A = (const unsigned char*)A, p.X = (const unsigned char*)B, p.Q = (const unsigned char*)Q;
             p.N = m, p.T = n, p.K = k, p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
-            return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream);
+            return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
         }
     }
     if (tc) {

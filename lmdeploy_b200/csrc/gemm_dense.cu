@@ -69,6 +69,7 @@ struct DenseTcParams {
     int           x2_tile;     // weight tiles from here on multiply the second operand
     int           column_tiles, half_box;
     int           wide_out, wide_act;  // columns below / from which on a warp's rows leave in 16-byte pieces (epilogue16_wide)
+    int           late_weight; // 1: the kernel ahead writes the weight
     int           band;        // pairs of CTAs: token tiles of a band, which all column tiles pass before the next band's turn
     DenseGroups   groups;
     float*        scratch;
@@ -361,7 +362,8 @@ dense_tc_kernel(const DenseTcParams p, const __grid_constant__ CUtensorMap w_map
             const Place q = place(tile);
             int       kb = kb0;
             if (!waited) {
-                // weights are written by no kernel: the first boxes go out before the kernel ahead is complete
+                // weights are written by no kernel (but an expanded one): the first boxes go out before the kernel ahead is complete
+                if (p.late_weight) pdl_wait();
                 const int pre = min(ST, kb1 - kb0);
                 if (elect_one()) {
                     for (int i = 0; i < pre; ++i) load_w(kb0 + i, q, i);
@@ -839,6 +841,7 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     p.column_tiles     = (g.n_out + kDenseTile - 1) / kDenseTile;
     p.half_box         = plan.token_tile / 2 / 16 * 16;
     p.band             = kBand;
+    p.late_weight      = half;
     p.token_tile    = plan.token_tile;
     p.token_tiles   = (g.tokens + p.token_tile - 1) / p.token_tile;
     p.tiles         = (plan.pair ? (p.column_tiles + 1) / 2 : p.column_tiles) * p.token_tiles;
@@ -917,11 +920,11 @@ double dense_pair_us(int tokens, int n_out, int k_blocks, int sms)
     return us;
 }
 
-int dense_gemm_f16(tm_handle* h, const DenseGemm& g, cudaStream_t st)
+int dense_gemm_f16(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl)
 {
     if (!g.w || !g.x || g.tokens <= 0 || g.n_out <= 0 || g.k <= 0 || g.ldw < g.k || g.ldx < g.k) return TM_ERR_INVALID_ARG;
     if (g.groups.count > 0 || g.ep.kind == DenseKind::kResidual || g.ep.ssq) return TM_ERR_UNSUPPORTED;
-    return dense_tc(h, g, st, false, true);
+    return dense_tc(h, g, st, pdl, true);
 }
 
 }  // namespace tmb

@@ -82,9 +82,9 @@ constexpr int kDenseTile = 128;  // output columns of one tile: the granularity 
 
 // bf16: ldw and ldx multiples of 8, 16-byte aligned bases.  Scratch and tickets come from the handle.
 int dense_gemm(tm_handle* h, const DenseGemm& g, bool f32, cudaStream_t st, bool pdl);
-// fp16 operands and outputs: more than 128 tokens, plain or (gate, up) epilogue, no groups.  A plain launch: the weight may
-// come from the kernel ahead.
-int dense_gemm_f16(tm_handle* h, const DenseGemm& g, cudaStream_t st);
+// fp16 operands and outputs: more than 128 tokens, plain or (gate, up) epilogue, no groups.  The weight may come from the kernel
+// ahead.
+int dense_gemm_f16(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl);
 // its time by the model that chooses its tiles, microseconds without what every launch costs
 double dense_pair_us(int tokens, int n_out, int k_blocks, int sms);
 

@@ -108,6 +108,6 @@ cudaError_t gemm_tc_launch(const GemmTcPlan& plan, GemmTcParams p, cudaStream_t 
 // output columns that are expanded and multiplied at a time (all, or pieces that fit the scratch); 0: the other kernel is faster
 int gemm_expanded_columns(const tm_handle* h, int N, int T, int K);
 // C, A, X, Q, N, T, K and fused_silu of `p` are read
-int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaStream_t st);
+int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaStream_t st, bool pdl);
 
 }  // namespace tmb

@@ -29,7 +29,7 @@ __device__ __forceinline__ uint32_t scaled(uint32_t x, uint32_t s)
 __global__ void __launch_bounds__(kWarps * 32) expand_s4_kernel(__half* w, const unsigned char* packed, const __half2* zs, int n_tiles, int N, int K, int tile0,
                                                               int tiles)
 {
-    pdl_wait();
+    pdl_wait();  // the rows of the product before lie in the same scratch
     pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const int i = blockIdx.x * kWarps + warp, groups = K / 128;
@@ -112,12 +112,12 @@ int gemm_expanded_columns(const tm_handle* h, int N, int T, int K)
     return first < along ? columns : 0;
 }
 
-int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaStream_t st)
+int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaStream_t st, bool pdl)
 {
     __half* const w = static_cast<__half*>(h->scratch);
     for (int n0 = 0; n0 < p.N; n0 += columns) {
         const int n = std::min(columns, p.N - n0), units = n / 32 * (p.K / 128);
-        const cudaError_t e = launch_kernel(expand_s4_kernel, dim3((units + kWarps - 1) / kWarps), dim3(kWarps * 32), 0, st, false, w, p.A,
+        const cudaError_t e = launch_kernel(expand_s4_kernel, dim3((units + kWarps - 1) / kWarps), dim3(kWarps * 32), 0, st, pdl, w, p.A,
                                             reinterpret_cast<const __half2*>(p.Q), p.N / 32, p.N, p.K, n0 / 32, n / 32);
         if (e != cudaSuccess) {
             h->last_cuda_error = (int)e;
@@ -132,7 +132,7 @@ int gemm_expanded_launch(tm_handle* h, const GemmTcParams& p, int columns, cudaS
         else {
             g.ep.kind = DenseKind::kStore, g.ep.out = p.C + n0, g.ep.out_ld = p.N;
         }
-        const int rc = dense_gemm_f16(h, g, st);
+        const int rc = dense_gemm_f16(h, g, st, pdl);
         if (rc != TM_OK) return rc;
     }
     return TM_OK;

@@ -127,3 +127,33 @@ def test_the_bound_on_split_tiles_is_not_the_dense_pipelines():
         assert h.launch_count() - launches == 2
     assert torch.equal(out[0], out[1])
     h.close()
+
+
+def _enqueue(h, out, w, x, stream):
+    from lmdeploy_b200 import lib as l
+    n, k = w.output_dims, w.input_dims
+    l.check(l.lib.tm_gemm_s4_f16(h.ptr, out.data_ptr(), w.kernel.data_ptr(), x.data_ptr(), w.scales_and_zeros.data_ptr(), n, x.shape[0], k, 128,
+                                 0, None, 0, C.c_void_p(stream.cuda_stream)), "tm_gemm_s4_f16")
+
+
+def test_expanded_weights_as_dependent_launches():
+    """A chain of products, each with a weight of its own in the same scratch, launched with and without programmatic serialisation."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    n, tokens = 4096, 6001
+    h, st = l.Handle(0), torch.cuda.current_stream()
+    ws = [cases._linear(cases._gen(4, i), n, n) for i in range(4)]
+    x = torch.randn(tokens, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    ends = []
+    for pdl in (0, 1, 1):
+        h.set_option("pdl_direct", pdl)
+        y, launches = [x] + [torch.empty(tokens, n, dtype=torch.float16, device="cuda") for _ in range(len(ws))], h.launch_count()
+        for _ in range(3):
+            for w, a, b in zip(ws, y, y[1:]):
+                _enqueue(h, b, w, a, st)
+        assert h.launch_count() - launches == 3 * 2 * len(ws)
+        h.check_device_status(st.cuda_stream)
+        ends.append(y)
+    assert all(torch.equal(a, b) for e in ends[1:] for a, b in zip(e, ends[0]))
+    assert bool(torch.isfinite(ends[0][1]).all())
+    h.close()
