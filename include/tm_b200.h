@@ -44,7 +44,11 @@ typedef struct tm_handle tm_handle;
 /* Per-device state: SM count, split-K scratch, split-KV scratch, device status word.
  * One handle is used by one host thread at a time (the reference runs one engine thread per
  * GPU: src/turbomind/models/llama/LlamaV2.cc:435-438); handles of different devices may be
- * used concurrently.  No process-global mutable state, with three exceptions: the per-device table behind
+ * used concurrently.  Its scratch is one for all streams: calls on several streams may be mixed, and those that use the
+ * scratch wait for one another on the device (the operators on spans of a slab, tm_window_attention and its like, pass
+ * their arguments through a buffer of the handle and keep to one stream).  Work that the caller captures into a graph of its own is not ordered that
+ * way: do not run such a graph beside other work of the handle (products that fill the device without scratch make do
+ * without it while they are captured).  No process-global mutable state, with three exceptions: the per-device table behind
  * tm_gemm_s4_f16_noalloc (guarded by a mutex), the shared handles of tm_handle_of_current_device and a thread-local switch the decode driver sets around its
  * own launches. */
 TM_API int tm_create(tm_handle** out, int device);

@@ -68,10 +68,14 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
     if (type == TM_GEMM_FUSED_SILU_FFN && m % 64) return TM_ERR_UNSUPPORTED;
 
     // a caller's workspace has the size that tm_gemm_s4_f16_workspace_bytes gave: the small-token kernels' up to 16 tokens
+    ScratchUse use(h, (cudaStream_t)stream);
     const bool tc = workspace ? n >= (h->gemm_tc_min_n >= 0 ? h->gemm_tc_min_n : 17) : gemm_uses_tc(h, m, n, k);
-    if (!workspace && !g_gemm_fusion && tc) {
+    // Products of whole tiles need no scratch.  That a weight is expanded into it, or tiles are cut only for balance, is for calls that
+    // are in order with all others that use the handle's.
+    if (!workspace && !g_gemm_fusion && tc && use.in_order()) {
         const int columns = gemm_expanded_columns(h, m, n, k);
         if (columns > 0) {
+            if (!use.begin(kGemmScratch)) return TM_ERR_CUDA;
             GemmTcParams p{};
             p.C = (__half*)C, p.A = (const unsigned char*)A, p.X = (const unsigned char*)B, p.Q = (const unsigned char*)Q;
             p.N = m, p.T = n, p.K = k, p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
@@ -82,7 +86,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
         // tensor-core tiles; token ranges that would overflow the scratch go in several launches
         const size_t n_out_tc = type == TM_GEMM_FUSED_SILU_FFN ? (size_t)m / 2 : (size_t)m;
         int          per      = n;
-        bool         balance  = workspace == nullptr;
+        bool         balance  = workspace == nullptr && use.in_order();
         for (;;) {
             GemmTcPlan   pl   = gemm_tc_plan(m, per, k, h->sm_count, balance);
             const size_t c_b  = ((pl.counter_ints * sizeof(int) + 255) / 256) * 256;
@@ -100,6 +104,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
         for (int t0 = 0; t0 < n; t0 += per) {
             const int    nt = n - t0 < per ? n - t0 : per;
             GemmTcPlan   pl = gemm_tc_plan(m, nt, k, h->sm_count, balance);
+            if (!workspace && pl.workspace_floats > 0 && !use.begin(kGemmScratch)) return TM_ERR_CUDA;
             GemmTcParams p{};
             p.C          = (__half*)C + (size_t)t0 * n_out_tc;
             p.A          = (const unsigned char*)A;
@@ -156,6 +161,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             ws_f = (float*)((char*)workspace + ((pl.counter_ints * sizeof(int) + 255) / 256) * 256);
         }
         else {
+            if (pl.cols_tiles == 0 && !use.begin(kGemmScratch)) return TM_ERR_CUDA;
             ws_f = (float*)h->scratch;
             ws_c = h->counters;
         }
@@ -242,6 +248,8 @@ int tm_mmha_decode_impl(tm_handle* h, const tm_mmha_params* a, void* stream, int
         return TM_ERR_WORKSPACE;
     }
 
+    ScratchUse use(h, (cudaStream_t)stream);
+    if (pl.max_splits > 1 && !use.begin(kAttentionScratch)) return TM_ERR_CUDA;
     MmhaParams p{};
     p.out             = (__half*)a->out;
     p.qkv             = q;

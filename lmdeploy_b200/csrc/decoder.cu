@@ -685,6 +685,8 @@ int tm_decoder::prefill(const tm_model_prefill_state& st, cudaStream_t s)
 {
     const int B = st.batch_size, total = st.cu_seqlens[B];
     if (total == 0) return TM_OK;
+    ScratchUse use(h, s);
+    if (!use.hold()) return TM_ERR_CUDA;
     const size_t V = (size_t)cfg.vocab, W = (size_t)cfg.width;
     std::vector<int> done(B, 0);
     for (int left = total; left > 0;) {

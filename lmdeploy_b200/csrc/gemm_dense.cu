@@ -863,6 +863,8 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     const int grid_ctas = plan.pair       ? 2 * (int)std::min<long long>(sms / 2, most) :
                           p.cut_ctas > 0 ? p.cut_ctas :
                                            (int)std::min<long long>(sms, most);
+    ScratchUse use(h, st);
+    if (p.cut_ctas > 0 && !use.begin(kGemmScratch)) return TM_ERR_CUDA;
     p.scratch  = static_cast<float*>(h->scratch);
     p.tickets  = h->counters;
     p.status   = h->status;

@@ -15,6 +15,63 @@ namespace tmb {
 thread_local int g_pdl = 0;
 
 namespace {
+thread_local const tm_handle* t_scratch_holder = nullptr;
+}
+
+ScratchUse::ScratchUse(tm_handle* h, cudaStream_t st): h_(h), st_(st), nested_(t_scratch_holder == h) {}
+
+bool ScratchUse::captured()
+{
+    if (captured_ < 0) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st_, &status) != cudaSuccess) {
+            cudaGetLastError();  // the legacy stream while another one is captured
+            status = cudaStreamCaptureStatusActive;
+        }
+        captured_ = status != cudaStreamCaptureStatusNone;
+    }
+    return captured_ != 0;
+}
+
+bool ScratchUse::begin(ScratchArea area)
+{
+    if (nested_ || captured() || begun_[area]) return true;
+    ScratchOrder&      order = h_->scratch_order[area];
+    unsigned long long id    = 0;
+    cudaError_t        e     = cudaStreamGetId(st_, &id);
+    if (e == cudaSuccess && order.used && order.stream != id) e = cudaStreamWaitEvent(st_, order.done, 0);
+    if (e != cudaSuccess) {
+        h_->last_cuda_error = (int)e;
+        return false;
+    }
+    order.stream = id;
+    begun_[area] = true;
+    return true;
+}
+
+bool ScratchUse::hold()
+{
+    for (int a = 0; a < kScratchAreas; ++a) {
+        if (!begin((ScratchArea)a)) return false;
+    }
+    outer_           = t_scratch_holder;
+    t_scratch_holder = h_;
+    holds_           = true;
+    return true;
+}
+
+ScratchUse::~ScratchUse()
+{
+    if (holds_) t_scratch_holder = outer_;
+    for (int a = 0; a < kScratchAreas; ++a) {
+        if (!begun_[a]) continue;
+        const cudaError_t e = cudaEventRecord(h_->scratch_order[a].done, st_);
+        if (e == cudaSuccess) h_->scratch_order[a].used = true;
+        else h_->last_cuda_error = (int)e;
+    }
+}
+
+namespace {
 std::vector<cudaError_t (*)(int)>& prepare_hooks()
 {
     static std::vector<cudaError_t (*)(int)> hooks;
@@ -86,6 +143,9 @@ extern "C" int tm_create(tm_handle** out, int device)
     if (e == cudaSuccess) e = cudaMemset(h->attn_counters, 0, h->attn_counter_ints * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&h->status, 256);
     if (e == cudaSuccess) e = cudaMemset(h->status, 0, 256);
+    for (ScratchOrder& order : h->scratch_order) {
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&order.done, cudaEventDisableTiming);
+    }
     for (auto prepare : prepare_hooks()) {
         if (e == cudaSuccess) e = prepare(h->max_smem);
     }
@@ -133,6 +193,9 @@ extern "C" int tm_destroy(tm_handle* h)
     if (h->attn_counters) cudaFree(h->attn_counters);
     if (h->status) cudaFree(h->status);
     if (h->op_buffer) cudaFree(h->op_buffer);
+    for (ScratchOrder& order : h->scratch_order) {
+        if (order.done) cudaEventDestroy(order.done);
+    }
     cudaSetDevice(prev);
     delete h;
     return TM_OK;

@@ -5,6 +5,16 @@
 #include "gemm_s4_f16.h"
 #include "mmha.h"
 
+namespace tmb {
+// The last call that used one of a handle's scratch areas
+struct ScratchOrder {
+    cudaEvent_t        done   = nullptr;
+    unsigned long long stream = 0;  // cudaStreamGetId
+    bool               used   = false;
+};
+enum ScratchArea { kGemmScratch = 0, kAttentionScratch = 1, kScratchAreas = 2 };
+}  // namespace tmb
+
 struct tm_handle {
     int                device          = 0;
     int                sm_count        = 0;
@@ -20,6 +30,7 @@ struct tm_handle {
     size_t             attn_counter_ints = 0;
     void*              op_buffer       = nullptr;  // device copies and scratch of single operator calls, grown on demand
     size_t             op_buffer_bytes = 0;
+    tmb::ScratchOrder  scratch_order[tmb::kScratchAreas];
     unsigned*          status          = nullptr;  // device status word (bounded waits)
     int                last_cuda_error = 0;
     unsigned long long launches        = 0;
@@ -49,6 +60,30 @@ struct KernelPreparation {
 // the C ABI on this thread carry the programmatic-dependent-launch attribute.  Off for direct callers,
 // who may put any kernel in front of ours.
 extern thread_local int g_pdl;
+
+// Held by a call around the launches that use the handle's scratch and tickets.  Calls of one stream are in order by themselves; a
+// call on another stream than the last one waits for it on the device.  A captured call is not ordered against others (its graph runs
+// later, on any stream): whoever can do without scratch should ask in_order().
+class ScratchUse {
+public:
+    ScratchUse(tm_handle* h, cudaStream_t st);
+    ~ScratchUse();
+    ScratchUse(const ScratchUse&)            = delete;
+    ScratchUse& operator=(const ScratchUse&) = delete;
+    bool in_order() { return nested_ || !captured(); }
+    bool begin(ScratchArea area);  // ahead of the first launch; false: a CUDA call failed
+    bool hold();                   // all areas, for every call of this host thread on the handle until this object ends
+
+private:
+    bool captured();
+
+    tm_handle*   h_;
+    cudaStream_t st_;
+    bool         nested_, holds_ = false;
+    int          captured_ = -1;  // not asked yet: calls without scratch need not
+    bool         begun_[kScratchAreas] = {};
+    const tm_handle* outer_ = nullptr;
+};
 // Set by the decode driver around ONE tm_gemm_s4_f16 call whose launch should carry a GemmNormFusion (gemm_s4_f16.h);
 // the driver has checked with gemm_can_fuse_norm that the call is a single tensor-core launch with every tile split.
 struct GemmNormFusion;

@@ -67,6 +67,8 @@ int tmb::StepGraph::run(tm_handle* h, const tm_llama_decode_state& st, int n_ste
                         unsigned long long* total, Step step)
 {
     *total = 0;
+    ScratchUse use(h, s);
+    if (!use.hold()) return TM_ERR_CUDA;
     if (!use_graph) {
         for (int i = 0; i < n_steps; ++i) {
             unsigned long long n  = 0;

@@ -69,6 +69,8 @@ extern "C" int tm_llama_prefill(tm_llama* m, const tm_llama_prefill_state* st, v
     const int    H = m->local_heads, Hkv = m->local_kv_heads;
     const size_t hid = (size_t)m->hidden;
     cudaStream_t s   = (cudaStream_t)stream;
+    ScratchUse   use(m->h, s);
+    if (!use.hold()) return TM_ERR_CUDA;
     int          prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(m->h->device);

@@ -157,3 +157,59 @@ def test_expanded_weights_as_dependent_launches():
     assert all(torch.equal(a, b) for e in ends[1:] for a, b in zip(e, ends[0]))
     assert bool(torch.isfinite(ends[0][1]).all())
     h.close()
+
+
+def test_streams_that_share_a_handle():
+    """Products that keep an expanded weight or parts of tiles in the handle's scratch, on two streams at once: the same bits as one
+    after the other."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    h = l.Handle(0)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    jobs = []  # (weight, activations): expanded, cut evenly, cut, split by the small-token kernel
+    for i, (n, k, tokens) in enumerate([(4096, 4096, 6001), (57344, 1024, 17), (4096, 4096, 40), (22016, 4096, 4), (8192, 4096, 2048)]):
+        jobs.append((cases._linear(cases._gen(6, i), n, k), torch.randn(tokens, k, device="cuda", generator=g).half()))
+    new = lambda: [torch.empty(x.shape[0], w.output_dims, dtype=torch.float16, device="cuda") for w, x in jobs]  # noqa: E731
+    one = torch.cuda.current_stream()
+    want = new()
+    for out, (w, x) in zip(want, jobs):
+        _enqueue(h, out, w, x, one)
+    h.check_device_status(one.cuda_stream)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[new() for _ in range(6)] for _ in streams]
+    torch.cuda.synchronize()
+    for r in range(6):
+        for i in range(len(jobs)):
+            for s, st in enumerate(streams):
+                j = (i + 2 * s) % len(jobs)
+                _enqueue(h, got[s][r][j], *jobs[j], st)
+    for st in streams:
+        h.check_device_status(st.cuda_stream)
+    for s in range(2):
+        for r in range(6):
+            for j, out in enumerate(got[s][r]):
+                assert torch.equal(out, want[j]), (s, r, j)
+    h.close()
+
+
+@pytest.mark.parametrize("n,k,tokens", [(4096, 4096, 6001), (57344, 1024, 17)])
+def test_captured_products_make_do_without_scratch(n, k, tokens):
+    """A caller's graph may run beside other work of the handle: products that fill the device are captured as whole tiles."""
+    from lmdeploy_b200 import lib as l
+    from perf import cases
+    h, st = l.Handle(0), torch.cuda.Stream()
+    w, exact = cases._linear(cases._gen(4, n), n, k), cases._exact_weight(cases._gen(4, n), n, k)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n)).half()
+    out = torch.empty(tokens, n, dtype=torch.float16, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        launches, graph = h.launch_count(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            _enqueue(h, out, w, x, st)
+        assert h.launch_count() - launches == 1
+        for _ in range(2):
+            out.zero_()
+            graph.replay()
+        h.check_device_status(st.cuda_stream)
+    _check(out, x.double() @ exact, x.double().abs() @ exact.abs(), k, 11, (n, k, tokens))
+    h.close()
