@@ -322,7 +322,7 @@ def run_gemm_workload(args, rank, world, device):
                    "l2": "inputs larger than L2: weights replicated beyond 2x L2, next replica each launch",
                    "parallelism": "replicas only" if world > 1 else "single GPU"},
         "roofline": {"bound": "hbm", "kernel": ("reference gemm_s4_f16_nn" if reflib is not None else
-                                                "gemm_s4_f16_tc_kernel" if T > 16 else "gemm_s4_f16_cols_kernel" if T == 1 else "gemm_s4_f16_small_kernel") + " (gate_up)",
+                                                "gemm_s4_f16_tc_kernel" if T > 8 else "gemm_s4_f16_cols_kernel" if T == 1 else "gemm_s4_f16_small_kernel") + " (gate_up)",
                      "achieved": dom["gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": round(dom["gbs"] / peaks["hbm_gbs"], 4), "peak_source": peaks["source"],
                      "algorithmic_bytes": dom["bytes"],
@@ -1303,10 +1303,9 @@ def run_decode_workload(args, rank, world, device, name):
                           "frac_of_hbm_peak": round(total_b / (ms_step * 1e-3) * 1e-9 / peaks["hbm_gbs"], 4)},
         "per_kernel_m1": {k: dict(v, frac=round(v["gbs"] / peaks["hbm_gbs"], 4), us_chained=m1c[k]["us"], gbs_chained=m1c[k]["gbs"],
                                   frac_chained=round(m1c[k]["gbs"] / peaks["hbm_gbs"], 4)) for k, v in m1.items()},
-        "per_kernel_m1_note": "the 1-token GEMM on this model's weights (per-rank shapes; gemm_s4_f16_cols_kernel where the weight has a "
-                              "64-column strip per SM: qkv and gate_up, gemm_s4_f16_small_kernel otherwise); us / gbs / frac: launches "
-                              "back to back, each waiting for the one before it; *_chained: with programmatic dependent launch, as "
-                              "inside the decode step",
+        "per_kernel_m1_note": "the 1-token GEMM on this model's weights (per-rank shapes; gemm_s4_f16_cols_kernel, strips of o and w2 "
+                              "shared by clusters of CTAs); us / gbs / frac: launches back to back, each waiting for the one before it; "
+                              "*_chained: with programmatic dependent launch, as inside the decode step",
         "per_kernel_m1_large": None if m1_large is None else {
             k: dict(v, frac=round(v["gbs"] / peaks["hbm_gbs"], 4)) for k, v in m1_large.items()},
         "per_kernel_m1_large_note": "same kernel at 1 token on the un-sharded Llama-2-70B projection shapes (seeded random nibbles and "
@@ -1442,7 +1441,8 @@ def time_decode_kernels(model, st, cfg, B, tp, stream, tm, session_len):
         gemm_us += us
         gemm_b += nb
         per[nm] = dict(us=round(us, 2), gbs=round(nb / us * 1e-3, 1), us_per_step=round(us * cfg.num_layer, 1), bytes=int(nb))
-    kname = "gemm_s4_f16_tc_kernel" if B > 16 else "gemm_s4_f16_small_kernel" if B > 8 else "gemm_s4_f16_cols_kernel + gemm_s4_f16_small_kernel"
+    kname = ("gemm_s4_f16_tc_kernel" if B > 13 else "gemm_s4_f16_tc_kernel + gemm_s4_f16_cols_kernel" if B > 8 else
+             "gemm_s4_f16_cols_kernel + gemm_s4_f16_small_kernel" if B > 1 else "gemm_s4_f16_cols_kernel")
     per[f"{kname} (4 projections of a layer)"] = dict(us=round(gemm_us / 4, 2), gbs=round(gemm_b / gemm_us * 1e-3, 1),
                                                       us_per_step=round(gemm_us * cfg.num_layer, 1), bytes=int(gemm_b / 4))
     # attention over the caches as they stand (layer l of every sequence)
