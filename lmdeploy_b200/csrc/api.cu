@@ -26,11 +26,16 @@ static bool gemm_uses_tc(const tm_handle* h, int m, int n, int k)
     return (long long)n * k > 52 * 1024 || h->gemv_cols != 1 || gemm_small_plan(m, n, k, h->sm_count, h->max_smem, h->gemv_cols).cols_tiles == 0;
 }
 
-bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k)
+bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k, bool producer)
 {
-    if (!h || !gemm_uses_tc(h, m, n, k) || n > 128 || k % 128 || m % 32) return false;
-    const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count, true);
-    return gemm_tc_all_tiles_split(pl, k) && pl.workspace_floats * sizeof(float) <= h->scratch_bytes && pl.counter_ints <= h->counter_ints;
+    if (!h || n > 128 || k % 128 || m % 32) return false;
+    const auto fits = [&](const auto& pl) { return pl.workspace_floats * sizeof(float) <= h->scratch_bytes && pl.counter_ints <= h->counter_ints; };
+    if (gemm_uses_tc(h, m, n, k)) {
+        const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count, true);
+        return fits(pl) && (!producer || gemm_tc_all_tiles_split(pl, k));
+    }
+    const GemmSmallPlan pl = gemm_small_plan(m, n, k, h->sm_count, h->max_smem, h->gemv_cols);
+    return fits(pl) && pl.t_chunks == 1 && (!producer || pl.cols_tiles > 0);
 }
 }
 
@@ -122,7 +127,8 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
             p.max_wait_cycles = h->gemm_wait_cycles;
             if (g_gemm_fusion) {
-                if (per != n || workspace || !gemm_tc_all_tiles_split(pl, k)) return TM_ERR_UNSUPPORTED;  // the driver checked
+                // the driver checked
+                if (per != n || workspace || (g_gemm_fusion->ssq_out && !gemm_tc_all_tiles_split(pl, k))) return TM_ERR_UNSUPPORTED;
                 p.norm = *g_gemm_fusion;
             }
             cudaError_t e = gemm_tc_launch(pl, p, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
@@ -135,7 +141,6 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
         return TM_OK;
     }
 
-    if (g_gemm_fusion) return TM_ERR_UNSUPPORTED;  // only the tensor-core kernel folds the norm in
     // One launch covers up to `n_launch` tokens; more tokens than the scratch can hold partial
     // tiles for are processed in several launches over consecutive token ranges.
     const size_t n_out = type == TM_GEMM_FUSED_SILU_FFN ? (size_t)m / 2 : (size_t)m;
@@ -179,6 +184,10 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
         p.T          = nt;
         p.K          = k;
         p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
+        if (g_gemm_fusion) {
+            if (n_launch != n || workspace || pl.t_chunks != 1 || (g_gemm_fusion->ssq_out && pl.cols_tiles == 0)) return TM_ERR_UNSUPPORTED;
+            p.norm = *g_gemm_fusion;
+        }
 
         cudaError_t e = gemm_small_launch(pl, p, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
         h->launches += 1;

@@ -10,6 +10,28 @@ struct tm_handle;
 
 namespace tmb {
 
+// Residual add + RMSNorm folded into the GEMMs on either side in the decode step (decode driver only).
+// Producer side (o_proj, w2): whoever has the whole sum of an output adds the residual, stores it, writes
+// half((residual + y) * norm_weight) as the output and adds up every token's sum of squares in 2^-20 fixed point
+// (integer atomics: the order of the additions cannot change the result).
+// Consumer side (qkv, w13): the rows of the accumulator are scaled by rsqrt(ssq[t] * 2^-20 * inv_n + eps) before the
+// output is rounded, which completes the normalisation of its input.
+struct GemmNormFusion {
+    __half*                   residual    = nullptr;  // [T][N], producer
+    const __half*             norm_weight = nullptr;  // [N], producer
+    unsigned long long*       ssq_out     = nullptr;  // [T], producer
+    const unsigned long long* ssq_in      = nullptr;  // [T], consumer
+    float                     inv_n       = 0.f;      // 1 / (length of the normalised row), consumer
+    float                     eps         = 0.f;
+};
+#ifdef __CUDACC__
+// consumer: 1 / rms of row t
+__device__ __forceinline__ float norm_row_scale(const GemmNormFusion& f, int t)
+{
+    return rsqrtf((float)__ldcg(f.ssq_in + t) * (1.f / 1048576.f) * f.inv_n + f.eps);
+}
+#endif
+
 // ---- small-token (HBM-bound) kernel -----------------------------------------------------
 struct GemmSmallParams {
     __half*              C;
@@ -23,6 +45,7 @@ struct GemmSmallParams {
     int                  fused_silu;
     // filled in by gemm_small_launch from the plan
     int units_per_cta, total_units, slots_per_chunk, n_col_tiles, stages, cluster;
+    GemmNormFusion norm;  // all null: a plain GEMM
 };
 
 struct GemmSmallPlan {
@@ -46,21 +69,6 @@ size_t        gemm_small_smem_bytes(int nt);
 GemmSmallPlan gemm_small_plan(int N, int T, int K, int sm_count, int max_smem, int cols_variant = 1);
 cudaError_t   gemm_small_prepare(int max_smem);
 cudaError_t   gemm_small_launch(const GemmSmallPlan& plan, GemmSmallParams p, cudaStream_t st, bool pdl = false);
-
-// Residual add + RMSNorm folded into two consecutive tensor-core GEMMs of the decode step (decode driver only).
-// Producer side (o_proj, w2): the reducers of the output tiles add the residual, store it, write
-// half((residual + y) * norm_weight) as the output and add up every token's sum of squares in 2^-20 fixed point
-// (integer atomics: the order of the additions cannot change the result).
-// Consumer side (qkv, w13): the rows of the accumulator are scaled by rsqrt(ssq[t] * 2^-20 * inv_n + eps) before the
-// output is rounded, which completes the normalisation of its input.
-struct GemmNormFusion {
-    __half*                   residual    = nullptr;  // [T][N], producer
-    const __half*             norm_weight = nullptr;  // [N], producer
-    unsigned long long*       ssq_out     = nullptr;  // [T], producer
-    const unsigned long long* ssq_in      = nullptr;  // [T], consumer
-    float                     inv_n       = 0.f;      // 1 / (length of the normalised row), consumer
-    float                     eps         = 0.f;
-};
 
 // ---- tensor-core (tcgen05) kernel for more than 16 tokens ---------------------------------
 struct GemmTcParams {

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                             for (int i = 0; i < 4; ++i) {
                                 const int   n = col0 + (my_t0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8;
                                 const int   t = t0 + j * 8 + 2 * c + (i & 1);
-                                const float v = tot[w][a][j][i];
+                                const float v = p.norm.ssq_in ? tot[w][a][j][i] * norm_row_scale(p.norm, min(t, p.T - 1)) : tot[w][a][j][i];
                                 if (p.fused_silu) {
                                     // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair;
                                     // the partner column n^1 lives in lane^4
@@ -465,6 +465,10 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                             v.z += part[e].z;
                             v.w += part[e].w;
                         }
+                    }
+                    if (p.norm.ssq_in) {
+                        const float inv = norm_row_scale(p.norm, t0 + t);
+                        v.x *= inv, v.y *= inv, v.z *= inv, v.w *= inv;
                     }
                     const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
                     if (p.fused_silu) {
@@ -588,6 +592,28 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     pdl_wait();
     pdl_launch_dependents();
 
+    // What this lane's outputs need beside their sums (value e = warp + 8 q of the strip's kVals) is on its way during the products:
+    // the row's 1 / rms (consumer of a folded norm), the residual and the norm weight (its producer).
+    constexpr int kVals = TILES * 8 * NT;
+    struct Place {
+        int n, t;
+    };
+    const auto place = [&](int q) {
+        const int e = warp + q * kWarps, w = e / (8 * NT), a = e / (4 * NT) & 1, j = e / 4 % NT, i = e & 3;
+        return Place{(tile0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8, 8 * j + 2 * c + (i & 1)};
+    };
+    float row_scale[kVals / kWarps], res[kVals / kWarps], gain[kVals / kWarps];
+#pragma unroll
+    for (int q = 0; q < kVals / kWarps; ++q) {
+        const Place at = place(q);
+        row_scale[q]   = p.norm.ssq_in ? norm_row_scale(p.norm, min(at.t, p.T - 1)) : 1.f;
+        res[q] = gain[q] = 0.f;
+        if (p.norm.ssq_out && rank == 0 && at.n < p.N && at.t < p.T) {
+            res[q]  = __half2float(p.norm.residual[(size_t)at.t * p.N + at.n]);
+            gain[q] = __half2float(__ldg(p.norm.norm_weight + at.n));
+        }
+    }
+
     // B fragments: token = fragment row (tokens beyond T repeat the last one: their columns are never stored)
     const uint32_t* x_row[NT];
 #pragma unroll
@@ -707,8 +733,10 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // the rings are free: they now hold the eight warps' partial sums, [warp][TILES x 8 values][lane]
-    constexpr int kVals = TILES * 8 * NT;
-    float*        red   = reinterpret_cast<float*>(smem_raw);
+    float* red = reinterpret_cast<float*>(smem_raw);
+    // sums of squares per token behind them (producer of a folded norm)
+    unsigned long long* s_ssq = reinterpret_cast<unsigned long long*>(red + kWarps * kVals * 32);
+    if (tid < 8 * NT) s_ssq[tid] = 0ull;
 #pragma unroll
     for (int w = 0; w < TILES; ++w)
 #pragma unroll
@@ -747,12 +775,25 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     }
 #pragma unroll
     for (int q = 0; q < kVals / kWarps; ++q) {
-        const float v     = sums[q];
-        const int   e     = warp + q * kWarps, w = e / (8 * NT), a = e / (4 * NT) & 1, j = e / 4 % NT, i = e & 3;
-        const int   n     = (tile0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8;
-        const int   t     = 8 * j + 2 * c + (i & 1);
-        const bool  valid = tile0 + w < n_tiles32 && t < p.T;
-        if (p.fused_silu) {
+        const float v     = p.norm.ssq_in ? sums[q] * row_scale[q] : sums[q];
+        const int   n     = place(q).n, t = place(q).t;
+        const bool  valid = n < p.N && t < p.T;
+        if (p.norm.ssq_out) {
+            // llama_decoder_kernels.cu:104-160 split in two: residual += y in fp32, stored as fp16; the sum of squares is taken
+            // before that rounding, the norm weight applied to the stored value
+            const float  s  = res[q] + __half2float(__float2half_rn(v));
+            const __half hs = __float2half_rn(s);
+            if (valid) {
+                p.norm.residual[(size_t)t * p.N + n] = hs;
+                p.C[(size_t)t * p.N + n]             = __float2half_rn(__half2float(hs) * gain[q]);
+            }
+            // whole numbers: the same sum in any order.  The eight rows of a token first, then the warps, then the strips.
+            unsigned long long ss = valid ? (unsigned long long)__float2ll_rn(s * s * 1048576.f) : 0ull;
+#pragma unroll
+            for (int m = 4; m < 32; m *= 2) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+            if (r == 0 && t < p.T) atomicAdd(s_ssq + t, ss);
+        }
+        else if (p.fused_silu) {
             // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair; the partner column n ^ 1 lives in lane ^ 4
             const float mine  = __half2float(__float2half_rn(v));
             const float other = __shfl_xor_sync(0xffffffffu, mine, 4);
@@ -764,6 +805,10 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
         else if (valid) {
             p.C[(size_t)t * p.N + n] = __float2half_rn(v);
         }
+    }
+    if (p.norm.ssq_out) {
+        __syncthreads();
+        if (tid < p.T) atomicAdd(p.norm.ssq_out + tid, s_ssq[tid]);
     }
 }
 

@@ -505,8 +505,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 auto finish = [&](int t, int n, float4 acc) {
                     if (p.norm.ssq_in) {
                         // consumer side: the row's 1 / rms completes the normalisation of this GEMM's input
-                        const float ssq = (float)__ldcg(p.norm.ssq_in + t0 + t) * (1.f / 1048576.f);
-                        const float inv = rsqrtf(ssq * p.norm.inv_n + p.norm.eps);
+                        const float inv = norm_row_scale(p.norm, t0 + t);
                         acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
                     }
                     const __half2 h0 = __floats2half2_rn(acc.x, acc.y), h1 = __floats2half2_rn(acc.z, acc.w);
@@ -723,6 +722,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                         for (int i = 0; i < 16; ++i) {
                             const int t = t0 + col + i;
                             const bool in = i < valid && t < p.T && n_glob < p.N;
+                            if (p.norm.ssq_in) v[i] *= norm_row_scale(p.norm, min(t, p.T - 1));
                             if (p.fused_silu) {
                                 // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair (gate, up) = rows (n, n + 1)
                                 const float mine_v = __half2float(__float2half_rn(v[i]));

@@ -85,9 +85,9 @@ private:
     const tm_handle* outer_ = nullptr;
 };
 // Set by the decode driver around ONE tm_gemm_s4_f16 call whose launch should carry a GemmNormFusion (gemm_s4_f16.h);
-// the driver has checked with gemm_can_fuse_norm that the call is a single tensor-core launch with every tile split.
+// the driver has checked with gemm_can_fuse_norm that the call is a single launch that can carry it.
 struct GemmNormFusion;
 extern thread_local const GemmNormFusion* g_gemm_fusion;
-bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k);
+bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k, bool producer);
 }  // namespace tmb
 

@@ -199,14 +199,16 @@ int run_step(StepCtx& c)
         return c.ok(tm_add_residual_rmsnorm(m.x, m.hbuf, nullptr, norm_w, cfg.norm_eps, B, m.hidden, s));
     };
 
-    // Residual add + RMSNorm folded into the GEMMs on either side (gemm_s4_f16.h, GemmNormFusion): single GPU, a batch
-    // the tensor-core kernel takes in one launch with every output tile split.  The first norm of the step and the
-    // last one (in front of the lm-head) stay kernels of their own.
+    // Residual add + RMSNorm folded into the GEMMs on either side (gemm_s4_f16.h, GemmNormFusion): single GPU, a batch that each
+    // projection takes in one launch, and the two producers by kernels that hold whole sums (the column-owner kernel, or the
+    // tensor-core kernel with every tile split).  The first norm of the step and the last one (in front of the lm-head) stay
+    // kernels of their own.
     const LlamaDecoderLayerWeight& w0 = m.layers[0];
-    const bool fold = !tp_on && m.h->fold_norm && gemm_can_fuse_norm(m.h, (int)w0.qkv.output_dims, B, (int)w0.qkv.input_dims)
-                      && gemm_can_fuse_norm(m.h, (int)w0.output.output_dims, B, (int)w0.output.input_dims)
-                      && gemm_can_fuse_norm(m.h, (int)w0.fused_gating_intermediate.output_dims, B, (int)w0.fused_gating_intermediate.input_dims)
-                      && gemm_can_fuse_norm(m.h, (int)w0.ffn_output.output_dims, B, (int)w0.ffn_output.input_dims);
+    auto foldable = [&](const LlamaDenseWeight& w, bool producer) {
+        return gemm_can_fuse_norm(m.h, (int)w.output_dims, B, (int)w.input_dims, producer);
+    };
+    const bool fold = !tp_on && m.h->fold_norm && foldable(w0.qkv, false) && foldable(w0.output, true)
+                      && foldable(w0.fused_gating_intermediate, false) && foldable(w0.ffn_output, true);
     if (fold) {
         if (!c.ok(cudaMemsetAsync(m.ssq, 0, (size_t)2 * cfg.num_layer * cfg.max_batch_size * sizeof(unsigned long long), s) == cudaSuccess ?
                       TM_OK :

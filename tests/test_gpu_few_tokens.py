@@ -82,3 +82,32 @@ def test_the_line_between_the_kernels_can_be_drawn_and_taken_back():
     with pytest.raises(l.TmError):
         h.set_option("gemm_tc_min_n", 0)
     h.close()
+
+
+@pytest.mark.parametrize("batch", [1, 2, 8, 9, 13])
+def test_folded_norm_with_few_sequences(batch):
+    """Residual add + RMSNorm folded into the GEMMs around it, by the column-owner kernel and by either kernel on either side, against
+    norm kernels of their own: the bounds of the driver's test with 24 sequences, and the same bits from run to run."""
+    import numpy as np
+    from tests.test_gpu_llama import CFG, build
+    model, _, _ = build(True, max_batch=16)
+    steps, rng = 4, np.random.default_rng(batch)
+    forced = np.full((steps, batch), -1, np.int32)
+    forced[0] = rng.integers(0, CFG["vocab_size"], batch)
+    runs, stream = [], torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for fold in (1, 0, 1):
+            model.handle.set_option("fold_norm", fold)
+            st, logits = model.new_state(batch, steps, np.zeros(batch, np.int32), forced, keep_logits=True), []
+            for _ in range(steps):
+                model.decode(st, 1, use_graph=True, stream=stream.cuda_stream)
+                stream.synchronize()
+                logits.append(st.logits.cpu().numpy().copy())
+            model.check_status(stream.cuda_stream)
+            runs.append((np.stack(logits), model.last_launches()))
+    model.close()
+    (a, launches), (b, separate), (again, _) = runs
+    assert separate - launches == 2 * CFG["num_layer"] - 1
+    err = np.abs(a - b)
+    assert err.max() <= 3e-2 and err.mean() / np.abs(b).mean() <= 5e-3, (err.max(), err.mean() / np.abs(b).mean())
+    assert np.array_equal(a, again)
