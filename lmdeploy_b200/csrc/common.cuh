@@ -94,19 +94,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, long l
     return true;
 }
 
-// The same with a sleep of `ns` between the tests, for a warp that waits beside warps that compute (the W4A16 tensor-core
-// kernel took the same time with 8 to 100 ns and with the suspended test)
-__device__ __forceinline__ bool mbar_wait_asleep(uint64_t* bar, uint32_t parity, unsigned ns, long long max_cycles = kMaxWaitCycles)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    do {
-        __nanosleep(ns);
-        if (mbar_try_wait(bar, parity)) return true;
-    } while (clock64() - t0 <= max_cycles);
-    return false;
-}
-
 // The same by a whole warp, with one outcome for all of it
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, long long max_cycles = kMaxWaitCycles)
 {

@@ -82,7 +82,7 @@ struct GemmTcParams {
     int                  N, T, K;
     int                  fused_silu;
     // filled in by gemm_tc_launch from the plan
-    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, x_stages, a_stages, acc_stride, parts_per_tile;
+    int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, parts_per_tile;
     int       last_sums;        // 1: a split tile is reduced by the CTA that is done last, without a wait (no GemmNormFusion)
     long long max_wait_cycles;  // bound of the wait for the partners of a split tile; 0 = the default
     GemmNormFusion norm;        // all null: a plain GEMM

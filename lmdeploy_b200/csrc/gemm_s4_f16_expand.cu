@@ -92,10 +92,9 @@ __global__ void __launch_bounds__(kWarps * 32) expand_s4_kernel(__half* w, const
 }  // namespace
 
 // Which way is faster, by models of both in microseconds: the plan's of expanding while multiplying; expanding first, 2.5 bytes
-// per weight beside the dense product.  Fitted to 144 launches of twelve projections with 200 to 3000 tokens (mean error 9 %):
-// in 20 of them another way than the model's is more than 6 % faster, by a quarter at most.  Both sides, us: 22016 x 4096
-// with 1024 / 2048 / 3000 tokens 186 / 317 / 440 expanding first and 182 / 341 / 484 while multiplying; 8192 x 28672: 456 / 775 /
-// 1137 and 357 / 816 / 1096.
+// per weight beside the dense product.  The line lies between 2000 and 4000 tokens on most shapes.  Both sides, us, expanding first and
+// while multiplying: 22016 x 4096 with 1536 / 2048 / 8192 / 16384 tokens 254 / 337 / 1216 / 2524 and 233 / 331 / 1318 / 2626;
+// 8192 x 28672 with 1024 / 2048 tokens 515 / 912 and 420 / 789; 57344 x 8192 with 8192 / 16384 tokens 7005 / 14353 and 7792 / 15555.
 int gemm_expanded_columns(const tm_handle* h, int N, int T, int K)
 {
     if (T <= 128 || K % 128 || N % 32 || h->sm_count < 2) return 0;
@@ -103,7 +102,7 @@ int gemm_expanded_columns(const tm_handle* h, int N, int T, int K)
     if (room < 256) return 0;
     const int pieces  = (N + room - 1) / room;
     const int columns = std::min(room, ((N + pieces - 1) / pieces + 255) / 256 * 256);
-    double first = -24.7;
+    double first = -36.7;
     for (int n0 = 0; n0 < N; n0 += columns) {
         const int n = std::min(columns, N - n0);
         first += 48.2 + 0.42e-6 * n * K + 0.98 * dense_pair_us(T, n, (K + 63) / 64, h->sm_count);

@@ -3,23 +3,24 @@
 // A CTA computes C^T tiles of 256 output features (two 128-feature UMMA tiles that share one
 // activation slice) x up to 128 tokens.  Work units are (256-feature tile, 128-row quantisation
 // group); a CTA has a whole tile, or the units of all tiles are cut evenly (gemm_tc_plan).  Warp roles:
-//   warp 0       an elected lane streams the activation slices: two tensor-map copies (TMA, 128-byte
+//   warp 0       an elected lane streams the activation slices: one tensor-map copy (TMA, 128-byte
 //                swizzle, tokens beyond T read as zero) per unit, completion on an mbarrier
 //   warps 1, 2   one issuer per 128-feature tile (warp 1 also allocates TMEM): an elected lane issues
 //                tcgen05.mma (M = 128, N = token tile, K = 16 per instruction, fp16 x fp16 -> fp32, A
 //                from TMEM, B from shared memory) and commits completions to mbarriers
 //   warps 3..18  two teams of eight, one per 128-feature tile; four warps of a team (32 features each)
-//                take the even units, four the odd ones.  Bound by their issue slots (74 % used, ALU
-//                pipe 55 %): what a unit costs beside its words is paid by half as many warps as
-//                when all eight shared it (57344 x 8192, 17 tokens: 1.15 us a unit before, 0.91
-//                now).  Every warp streams its own share of the packed weight through a private cp.async ring and expands it: lop3 nibble
+//                take the even units, four the odd ones.  A warp takes its words from shared memory and expands them: lop3 nibble
 //                unpack, exact (q - z) in fp16, one fp16 multiply by the scale (bit-identical to the
 //                reference's dequantised weight, kernels/gemm_s_f16/common.h:115-156, 218-235),
 //                tcgen05.st of the fragments straight into TMEM, from where the tensor core takes
 //                its A operand (no shared-memory round trip); at the end of a column tile the
 //                warps read the accumulators with tcgen05.ld and store C (optionally through the
 //                SiLU(gate) * up epilogue) or the split-K partial
-// A waiting warp sleeps between its tests: it would otherwise take issue slots from the expanding ones.
+//   warp 19      an elected lane streams the packed weight: a box of the weight and one of {zero, scale} per unit
+// What bounds it.  With few tokens the bytes of a unit take 0.4 us, its expansion 0.5-0.55 (65 % of the issue slots; 375 warp
+// instructions per warp and unit, of which 208 unpack and scale).  Copies by the expanding warps (cp.async, 64-bit addresses) and
+// issuers that voted between the steps of a unit cost 82 more instructions and left the issuing lane, a chain of 1100 cycles a unit,
+// as the bound.  57344 x 8192, 21 / 64 tokens: 74 / 84 -> 59 / 75 us in a row of dependent launches (4.1 TB/s).
 // Partial tiles of CTAs that share a column tile meet in scratch memory; every CTA of the tile then
 // sums its own share of the feature rows in a fixed order.  Every wait is bounded.
 //
@@ -30,6 +31,7 @@
 #include "gemm_s4_f16.h"
 
 #include <algorithm>
+#include <array>
 #include <cuda.h>  // CUtensorMap (types only: the encoder is looked up through the runtime)
 
 #ifdef TM_B200_GEMM_TRACE
@@ -86,32 +88,49 @@ extern "C" __attribute__((visibility("default"))) int tm_dev_gemm_trace(long lon
 namespace tmb {
 namespace {
 
+template<int V>
+struct Int {
+    static constexpr int value = V;
+};
 constexpr int kTileN     = 128;  // output features per UMMA tile (UMMA M)
 constexpr int kTeams     = 2;    // UMMA tiles per CTA tile
 constexpr int kSuperN    = kTileN * kTeams;
 constexpr int kGroup     = 128;  // K extent of a unit
 constexpr int kTileBytes = 512;
-constexpr int kACols     = kGroup / 2;           // TMEM columns of one expanded weight stage (128 k as fp16 pairs)
 constexpr int kSlabs     = kGroup / 32;
-constexpr int kWarpStage = kSlabs * kTileBytes + 128; // per expanding warp and unit: 4 x 512 B of weight + 32 {zero, scale}
-constexpr int kWST       = 3;                    // stages of those private rings (cp.async groups in flight <= 2, every other unit)
-constexpr int kASTMax    = 3;                    // expanded-weight stages per team (in TMEM)
-constexpr int kXSTMax    = 6;                    // activation stages
+constexpr int kSlabBytes = kSuperN / 32 * kTileBytes;  // the packed weight of a 32-row slab of a unit: eight tiles, contiguous
+constexpr int kWStage    = kSlabs * kSlabBytes + kSuperN * 4;  // a unit's packed weight and its row of {zero, scale}
+constexpr int kWST       = 6;                    // stages of packed weight: 104 KB on their way, 44 KB hide the memory's latency
+// Tokens of a tile decide how TMEM is shared out: two accumulators, and stages of expanded weight in the rest
+template<bool kWide>
+struct Shape {
+    static constexpr int kAcc   = kWide ? 128 : 64;   // TMEM columns of an accumulator: the largest token tile
+    // From 65 tokens on the products of a unit take as long as its expansion; stages of half a unit let the two overlap where there
+    // is no room for a third whole one (4096 x 4096, 735 tokens: 39 us with two whole ones, 34 with four halves).
+    static constexpr int kStageK = kWide ? 64 : 128;  // k values of a stage
+    static constexpr int kParts  = kGroup / kStageK;  // stages of a unit
+    static constexpr int kACols  = kStageK / 2;       // TMEM columns of a stage (fp16 pairs)
+    static constexpr int kAST    = kWide ? 4 : 3;     // stages per team
+    static constexpr int kXST    = kWide ? 3 : 6;     // activation stages in shared memory
+};
+constexpr int kASTMax = 4, kXSTMax = 6;
 constexpr int kTeamWarps = 8;
 constexpr int kDqWarps   = kTeams * kTeamWarps;
 constexpr int kDqThreads = kDqWarps * 32;
 constexpr int kIssuers   = kTeams;
 constexpr int kDqWarp0   = 1 + kIssuers;         // first expanding warp
-constexpr int kThreads   = (kDqWarp0 + kDqWarps) * 32;
-constexpr unsigned kNap = 20, kLongNap = 200;  // nanoseconds between a waiting warp's tests; the loader is several units ahead
+constexpr int kWLoadWarp = kDqWarp0 + kDqWarps;  // loader of the packed weight
+constexpr int kThreads   = (kWLoadWarp + 1) * 32;
 constexpr int kTmemCols  = 512;                  // accumulators + expanded-weight stages, power of two
 
 struct Bars {
     uint64_t a_full[kTeams][kASTMax], a_empty[kTeams][kASTMax];
     uint64_t x_full[kXSTMax], x_empty[kXSTMax];
+    uint64_t w_full[kWST], w_empty[kWST];
     uint64_t acc_full[kTeams], acc_empty[kTeams];  // per team
     uint32_t tmem_base;
     int      flag;
+    float    row_scale[128];  // 1 / rms per token (consumer of a folded norm)
 };
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
@@ -165,14 +184,17 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// One box of the activation tensor map -> shared memory, completion counted on an mbarrier
+// One box of a tensor map -> shared memory, completion counted on an mbarrier
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar)
+{
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
 {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(map)),
-                 "r"(x),
-                 "r"(y),
-                 "r"(smem_u32(bar))
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
 
@@ -206,33 +228,54 @@ __device__ __forceinline__ uint32_t hmul2_ftz(uint32_t a, uint32_t b)
     return r;
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src)
+// Bounded wait of a whole warp on a barrier at a shared-memory address; on a time-out the warp records `bit` and plays dead from then on.
+__device__ __noinline__ bool wait_on(uint32_t bar, uint32_t parity)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    return mbar_wait_warp(reinterpret_cast<uint64_t*>(__cvta_shared_to_generic(bar)), parity);
 }
-
-// Bounded wait of a whole warp; on a time-out the warp records `bit` and plays dead from then on.
-__device__ __forceinline__ void warp_wait(uint64_t* bar, uint32_t parity, bool& dead, unsigned* status, unsigned bit, unsigned ns = kNap)
+__device__ __forceinline__ void warp_wait(uint32_t bar, uint32_t parity, bool& dead, unsigned* status, unsigned bit)
 {
-    if (dead) return;
-    // Usually the phase is complete already: every lane tests it (same answer in every lane, no divergence).
-    if (mbar_try_wait(bar, parity)) return;
-    // Otherwise one lane sleeps in the barrier; the shuffle hands the outcome (and, as a warp-level sync, the
-    // ordering) to the rest.
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait_asleep(bar, parity, ns) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    // usually the phase is complete already
+    if (!__all_sync(0xffffffffu, ok | (dead ? 1u : 0u)) && !wait_on(bar, parity)) {
         if ((threadIdx.x & 31) == 0) atomicOr(status, bit);
         dead = true;
     }
 }
-
-__global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParams p, const __grid_constant__ CUtensorMap x_map)
+__device__ __forceinline__ void arrive_at(uint32_t bar)
 {
-    const int kXST = p.x_stages;
-    const int kAST = p.a_stages;    // per team
-    const int accS = p.acc_stride;  // TMEM columns of one accumulator
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+template<int kOffset>
+__device__ __forceinline__ uint4 shared_load16(uint32_t addr)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4+%5];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr), "n"(kOffset) : "memory");
+    return v;
+}
+template<int kOffset>
+__device__ __forceinline__ uint32_t shared_load4(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(addr), "n"(kOffset) : "memory");
+    return v;
+}
+
+template<bool kWide>
+__global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParams p, const __grid_constant__ CUtensorMap x_map,
+                                                                      const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap q_map)
+{
+    using S = Shape<kWide>;
+    constexpr int kXST = S::kXST, kAST = S::kAST, kACols = S::kACols, accS = S::kAcc;
     extern __shared__ unsigned char smem_dyn[];
     // tiles the tensor core reads must sit on 1024-byte boundaries (the swizzle is a function of
     // the address bits)
@@ -243,8 +286,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     const int TT      = p.token_tile;             // UMMA N, multiple of 16, <= 128
     const int x_bytes = 2 * TT * 128;             // two K blocks of TT rows x 128 B
     unsigned char* x_ring = sm;                                   // kXST x x_bytes (multiples of 1024)
-    unsigned char* w_ring = x_ring + kXST * x_bytes;              // kDqWarps x kWST x kWarpStage
-    Bars*          bars   = reinterpret_cast<Bars*>(w_ring + kWST * kDqWarps * kWarpStage);
+    unsigned char* w_ring = x_ring + kXST * x_bytes;              // kWST x kWStage
+    Bars*          bars   = reinterpret_cast<Bars*>(w_ring + kWST * kWStage);
 
     const int tid  = threadIdx.x;
     const int warp = tid >> 5;
@@ -283,58 +326,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     };
     const int n_tiles32 = p.N / 32;
 
-    // ---- expanding warps: identity and the state of their copy front ---------------------------
-    const int  dw   = warp - kDqWarp0; // 0..15 for the expanding warps
-    const int  m_dq = (dw >> 3) & 1;   // team = 128-feature tile of the unit
-    const int  q    = warp & 3;        // TMEM lane quarter this warp may access = its 32-feature tile
-    const int  kh   = (dw >> 2) & 1;   // which of two units it expands (what a unit costs beside the words is shared by
-                                       // twice as many), and which half of the token columns it drains
-    // private ring of this warp: per unit of its own 4 x 512 B of packed weight (32-feature tile, the group's
-    // 32-row slabs) + the 128 B of {zero, scale} of its 32 features
-    const uint32_t       my_ring   = base + (uint32_t)(w_ring - sm) + (uint32_t)(dw < 0 ? 0 : dw) * kWST * kWarpStage + lane * 16;
-    const unsigned char* my_ring_g = w_ring + (dw < 0 ? 0 : dw) * kWST * kWarpStage;
-    // the copy front runs kWST - 1 of its units ahead of the expansion: this lane's 16 bytes of the warp's
-    // first slab and of the {zero, scale} row.  A warp whose tile lies beyond N re-reads the last
-    // tile; what it produces is never stored.
-    int                  i_js = u_begin / G, i_g = u_begin - i_js * G;
-    const unsigned char* i_w  = nullptr;
-    const unsigned char* i_q  = nullptr;
-    const size_t         slab_b  = (size_t)n_tiles32 * kTileBytes;  // bytes between 32-row slabs
-    const size_t         q_row_b = (size_t)p.N * 4;                 // bytes between {zero, scale} rows
-    auto i_seek = [&]() {
-        const int tile = min((i_js * kTeams + m_dq) * 4 + q, n_tiles32 - 1);
-        i_w = p.A + ((size_t)i_g * kSlabs * n_tiles32 + tile) * kTileBytes + lane * 16;
-        i_q = p.Q + ((size_t)i_g * p.N + (size_t)tile * 32) * 4 + (lane & 7) * 16;
+    const int  dw = warp - kDqWarp0;  // 0..15 for the expanding warps
+    // A unit's packed weight, four slabs of eight adjacent tiles, and its row of {zero, scale}: a box each (zeros beyond N).  Copies of
+    // contiguous pieces, five a unit, kept the loader's lane busy for longer than the expansion takes.
+    auto w_load = [&](int js, int g, int stage) {
+        const uint32_t dst = base + (uint32_t)(w_ring - sm) + (uint32_t)stage * kWStage;
+        mbar_arrive_expect_tx(&bars->w_full[stage], (uint32_t)kWStage);
+        tma_load_3d(dst, &w_map, 0, js * (kSuperN / 32), g * kSlabs, &bars->w_full[stage]);
+        tma_load_2d(dst + kSlabs * kSlabBytes, &q_map, js * kSuperN, g, &bars->w_full[stage]);
     };
-    int  to_issue = (n_units + 1 - kh) / 2;  // units of this warp: kh, kh + 2, ...
-    auto i_next   = [&]() {
-        i_w += kSlabs * slab_b;
-        i_q += q_row_b;
-        if (++i_g == G) {
-            i_g = 0;
-            ++i_js;
-            i_seek();
+    int w_js = u_begin / G, w_g = u_begin - w_js * G;  // the weight loader's next unit
+    auto w_next = [&]() {
+        if (++w_g == G) w_g = 0, ++w_js;
+    };
+    if (warp == kWLoadWarp) {
+        // The packed weights are written by no kernel: the first copies start at once, ahead of the TMEM set-up (one stage: issuing
+        // them all takes longer than that) and of the wait for the kernel before this one.
+        if (elect_one()) {
+            for (int s = 0; s < kWST; ++s) {
+                mbar_init(&bars->w_full[s], 1);
+                mbar_init(&bars->w_empty[s], kDqWarps / 2);
+            }
+            fence_mbar_init();
+            w_load(w_js, w_g, 0);
         }
-    };
-    auto issue_unit = [&](int stage) {
-        const uint32_t dst = my_ring + stage * kWarpStage;
-#pragma unroll
-        for (int i = 0; i < kSlabs; ++i) cp_async16(dst + i * kTileBytes, i_w + i * slab_b);
-        if (lane < 8) cp_async16(dst + kSlabs * kTileBytes, i_q);
-        i_next();
-        i_next();
-    };
-    if (dw >= 0) {
-        // The packed weights are written by no kernel: their first copies start at once, ahead of the
-        // barrier and TMEM set-up and of the wait for the kernel before this one.
-        i_seek();
-        if (kh) i_next();
-#pragma unroll
-        for (int sidx = 0; sidx < kWST - 1; ++sidx) {
-            if (to_issue > 0) issue_unit(sidx);
-            --to_issue;
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
+        __syncwarp();
+        w_next();
     }
 
     if (tid == 0) {
@@ -370,29 +387,53 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         // slice [TT tokens][128 k] of a group -> two 64-wide K blocks, rows of 128 B with their 16-byte
         // chunks XOR-swizzled by (row & 7): the layout the tensor core expects and the one a tensor-map
         // copy with 128-byte swizzle writes.  One slice serves both feature tiles of the unit.
-        bool dead = false;
-        int  g    = u_begin % G;
+        if (elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&x_map)) : "memory");
+        __syncwarp();
         pdl_wait();  // the activations come from the kernel before this one
         pdl_launch_dependents();
-        for (int it = 0; it < n_units; ++it) {
-            const int sx = it % kXST;
-            TC_TRACE(trow, 10, it);
-            if (it >= kXST) warp_wait(&bars->x_empty[sx], ((it / kXST) - 1) & 1, dead, p.status, kStatusGemmPipeWait, kLongNap);
-            if (!dead && elect_one()) {
-                const uint32_t xb = base + (uint32_t)(x_ring - sm) + sx * x_bytes;
-                mbar_arrive_expect_tx(&bars->x_full[sx], (uint32_t)x_bytes);
-                tma_load_2d(xb, &x_map, g * kGroup, t0, &bars->x_full[sx]);
-                tma_load_2d(xb + TT * 128, &x_map, g * kGroup + 64, t0, &bars->x_full[sx]);
+        if (elect_one()) {
+            int g = u_begin % G, it = 0, st = 0;
+            for (uint32_t ph = 1; it < n_units; ++it) {  // (a fresh barrier counts as having completed the phase before)
+                TC_TRACE(trow, 10, it);
+                if (!mbar_wait(&bars->x_empty[st], ph)) {
+                    atomicOr(p.status, kStatusGemmPipeWait);
+                    break;
+                }
+                mbar_arrive_expect_tx(&bars->x_full[st], (uint32_t)x_bytes);
+                tma_load_3d(base + (uint32_t)(x_ring - sm) + st * x_bytes, &x_map, 0, t0, 2 * g, &bars->x_full[st]);
+                if (++g == G) g = 0;
+                if (++st == kXST) st = 0, ph ^= 1;
             }
-            __syncwarp();
-            if (++g == G) g = 0;
+            // this CTA's shared memory may not be left while copies are on their way into it
+            for (int i = max(0, it - kXST); i < it; ++i) mbar_wait(&bars->x_full[i % kXST], (i / kXST) & 1);
         }
+        __syncwarp();
+    }
+    else if (warp == kWLoadWarp) {
+        // ================================================================== loader of the packed weight
+        if (elect_one()) {
+            int it = 1, st = 1;
+            for (uint32_t ph = 1; it < n_units; ++it) {
+                if (!mbar_wait(&bars->w_empty[st], ph)) {
+                    atomicOr(p.status, kStatusGemmPipeWait);
+                    break;
+                }
+                w_load(w_js, w_g, st);
+                w_next();
+                if (++st == kWST) st = 0, ph ^= 1;
+            }
+            for (int i = max(0, it - kWST); i < it; ++i) mbar_wait(&bars->w_full[i % kWST], (i / kWST) & 1);
+        }
+        __syncwarp();
     }
     else if (warp <= kIssuers) {
         // ================================================================== MMA issuers
-        // One warp per team runs the whole loop: waits, eight MMAs by an elected lane, commits.
-        const int m = warp - 1;
-        {
+        // One elected lane per team runs the whole loop: waits, eight MMAs, commits.  What it does between two units is a chain that
+        // nothing hides, so the team is a constant (operands in uniform registers) and no vote stands in the loop: a unit took 1100
+        // cycles of this lane, whatever the tokens, where the tensor core needs 16 x (6 + tokens / 2).
+        auto issue = [&](auto team) {
+            constexpr int m = decltype(team)::value;
+            if (!elect_one()) return;
             const uint32_t idesc   = (1u << 4) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
             const uint32_t d_tmem  = tmem + m * accS;
             const uint32_t kb_step = (uint32_t)(TT * 128) >> 4;  // descriptor units (16 B) between the two K blocks
@@ -410,50 +451,56 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 bool ok = true;
                 if (first && seg_idx > 0) {
                     // the epilogue of the previous segment must have drained the accumulators
-                    ok = mbar_wait_asleep(&bars->acc_empty[m], (seg_idx - 1) & 1, kNap);
+                    ok = mbar_wait(&bars->acc_empty[m], (seg_idx - 1) & 1);
                 }
-                ok = ok && mbar_wait_asleep(&bars->x_full[sx], px, kNap) && mbar_wait_asleep(&bars->a_full[m][sa], pa, kNap);
-                if (!__all_sync(0xffffffffu, ok)) {
-                    if (lane == 0) atomicOr(p.status, kStatusGemmPipeWait);
+                ok = ok && mbar_wait(&bars->x_full[sx], px);
+                const bool     last = (it == n_units - 1) || (g == G - 1);
+                const uint32_t lo   = d_lo + (uint32_t)sx * x_step;
+#pragma unroll
+                for (int part = 0; part < S::kParts; ++part) {
+                    ok = ok && mbar_wait(&bars->a_full[m][sa], pa);
+                    if (!ok) break;
+                    tc_fence_after();
+                    TC_TRACE(trow, 20, it);
+                    const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols;
+                    umma_f16_ts_x4(d_tmem, a_tmem, lo + part * kb_step, d_hi, idesc, part == 0 && first ? 1u : 0u);
+                    if (S::kParts == 1) umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
+                    umma_commit(&bars->a_empty[m][sa]);
+                    if (++sa == kAST) sa = 0, pa ^= 1;
+                }
+                if (!ok) {
+                    atomicOr(p.status, kStatusGemmPipeWait);
                     break;
                 }
-                tc_fence_after();
-                TC_TRACE(trow, 20, it);
-                const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols;
-                const uint32_t lo     = d_lo + (uint32_t)sx * x_step;
-                const bool last = (it == n_units - 1) || (g == G - 1);
-                if (elect_one()) {
-                    umma_f16_ts_x4(d_tmem, a_tmem, lo, d_hi, idesc, first ? 1u : 0u);
-                    umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
-                    umma_commit(&bars->a_empty[m][sa]);
-                    umma_commit(&bars->x_empty[sx]);
-                    if (last) umma_commit(&bars->acc_full[m]);
-                }
-                __syncwarp();
+                umma_commit(&bars->x_empty[sx]);
                 TC_TRACE(trow, 21, it);
-                first = false;
+                first = last;
                 if (last) {
+                    umma_commit(&bars->acc_full[m]);
                     ++seg_idx;
-                    first = true;
                 }
                 if (++g == G) g = 0;
-                if (++sa == kAST) { sa = 0; pa ^= 1; }
-                if (++sx == kXST) { sx = 0; px ^= 1; }
+                if (++sx == kXST) sx = 0, px ^= 1;
             }
+        };
+        if (warp == 1) {
+            issue(Int<0>{});
+        }
+        else {
+            issue(Int<1>{});
         }
         __syncwarp();
     }
     else {
         // ================================================================== expand + epilogue
-        const int  m    = m_dq;
+        const int  m    = dw >> 3;        // team = 128-feature tile of the unit
+        const int  q    = warp & 3;       // TMEM lane quarter this warp may access = its 32-feature tile
+        const int  kh   = (dw >> 2) & 1;  // which of two units it expands (what a unit costs beside the words is shared by
+                                          // twice as many), and which half of the token columns it drains
         const int  r    = lane >> 2;
         bool       dead = false;
         int        seg_idx = 0;
         const int  dtid = tid - kDqWarp0 * 32;
-
-        // What follows reads and writes scratch, tickets and the output, which the kernel before this
-        // one may still be using.
-        pdl_wait();
 
         // split-K: [slot][TT tokens][256 feature rows] fp32 partial tiles (a warp touches 128 contiguous
         // bytes per token: whole sectors), per tile a count of CTAs whose partial is complete and a count of
@@ -465,6 +512,88 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         constexpr int kMaxPending = 4;
         int           pend[kMaxPending] = {0, 0, 0, 0};
         int           n_pend = 0;
+        // producer side of a folded norm: per-token sums of squares of this CTA's share, in fixed point, kept in the (by then idle)
+        // activation ring until they go out with one atomic per token
+        unsigned long long* s_ssq = reinterpret_cast<unsigned long long*>(x_ring);
+        // Outputs of four adjacent features of a token from their sum
+        auto finish = [&](int t, int col, float4 acc, uint2 res, uint2 gain, float inv) {
+            if (p.norm.ssq_in) acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
+            const __half2 h0 = __floats2half2_rn(acc.x, acc.y), h1 = __floats2half2_rn(acc.z, acc.w);
+            auto half2_of    = [](uint32_t v) { return __half22float2(reinterpret_cast<const __half2&>(v)); };
+            auto word_of     = [](__half2 v) { return reinterpret_cast<const uint32_t&>(v); };
+            if (p.norm.ssq_out) {
+                // producer side (llama_decoder_kernels.cu:104-160 split in two): residual += y in fp32, stored as
+                // fp16; the sum of squares is taken before that rounding, the norm weight applied to the stored value
+                const float2  r0 = half2_of(res.x), r1 = half2_of(res.y);
+                const float2  y0 = __half22float2(h0), y1 = __half22float2(h1);
+                const float2  s0 = make_float2(r0.x + y0.x, r0.y + y0.y), s1 = make_float2(r1.x + y1.x, r1.y + y1.y);
+                const float   ss = (s0.x * s0.x + s0.y * s0.y) + (s1.x * s1.x + s1.y * s1.y);
+                const __half2 n0 = __float22half2_rn(s0), n1 = __float22half2_rn(s1);
+                const size_t  at = (size_t)(t0 + t) * p.N + col;
+                *reinterpret_cast<uint2*>(p.norm.residual + at) = make_uint2(word_of(n0), word_of(n1));
+                const float2 a0 = __half22float2(n0), a1 = __half22float2(n1);
+                const float2 g0 = half2_of(gain.x), g1 = half2_of(gain.y);
+                *reinterpret_cast<uint2*>(p.C + at) =
+                    make_uint2(word_of(__floats2half2_rn(a0.x * g0.x, a0.y * g0.y)), word_of(__floats2half2_rn(a1.x * g1.x, a1.y * g1.y)));
+                atomicAdd(s_ssq + t, (unsigned long long)__float2ll_rn(ss * 1048576.f));
+            }
+            else if (p.fused_silu) {
+                // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pairs (gate, up)
+                const float2 u0 = __half22float2(h0), u1 = __half22float2(h1);
+                const float  s0 = u0.x / (1.f + __expf(-u0.x)), s1 = u1.x / (1.f + __expf(-u1.x));
+                *reinterpret_cast<__half2*>(p.C + (size_t)(t0 + t) * (p.N / 2) + col / 2) = __floats2half2_rn(s0 * u0.y, s1 * u1.y);
+            }
+            else {
+                *reinterpret_cast<uint2*>(p.C + (size_t)(t0 + t) * p.N + col) = make_uint2(word_of(h0), word_of(h1));
+            }
+        };
+        // Rows [f0, f1) of a tile, summed over its partials in CTA order.  A thread takes kPieces pieces of four features at a time and
+        // asks for kParts partials of each together: eight loads on their way, whatever the number of parts.
+        auto sum_rows = [&](auto pieces_of, auto parts_of, auto residual_of, const float* tile_slots, int n_split, int f0, int f1, int col0) {
+            constexpr int  kPieces = decltype(pieces_of)::value, kParts = decltype(parts_of)::value;
+            constexpr bool kResidual = decltype(residual_of)::value != 0;
+            const unsigned quads = (unsigned)(f1 - f0) / 4, items = (unsigned)t_rows * quads;
+            const unsigned magic = quads > 1 ? 0xffffffffu / quads + 1 : 0;  // i / quads for i < 2^16: the upper word of i * magic
+            for (unsigned i0 = dtid; i0 < items; i0 += kPieces * kDqThreads) {
+                float4 acc[kPieces];
+                uint2  res[kPieces], gain[kPieces];
+                int    tt[kPieces], nn[kPieces];
+#pragma unroll
+                for (int j = 0; j < kPieces; ++j) {
+                    const unsigned i = min(i0 + j * kDqThreads, items - 1);
+                    tt[j]  = quads > 1 ? (int)__umulhi(i, magic) : (int)i;
+                    nn[j]  = f0 + ((int)i - tt[j] * (int)quads) * 4;
+                    acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    res[j] = gain[j] = make_uint2(0u, 0u);
+                    if (kResidual && p.norm.ssq_out) {
+                        const uint32_t* g = reinterpret_cast<const uint32_t*>(p.norm.norm_weight + col0 + nn[j]);
+                        res[j]  = *reinterpret_cast<const uint2*>(p.norm.residual + (size_t)(t0 + tt[j]) * p.N + col0 + nn[j]);
+                        gain[j] = make_uint2(__ldg(g), __ldg(g + 1));
+                    }
+                }
+                for (int cc = 0; cc < n_split; cc += kParts) {
+                    float4 part[kPieces][kParts];
+#pragma unroll
+                    for (int j = 0; j < kPieces; ++j) {
+                        const float* src = tile_slots + (size_t)cc * slot_floats + tt[j] * kSuperN + nn[j];
+#pragma unroll
+                        for (int e = 0; e < kParts; ++e) {
+                            part[j][e] = make_float4(0.f, 0.f, 0.f, 0.f);  // an absent slot adds +0
+                            if (cc + e < n_split) part[j][e] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)e * slot_floats));
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < kPieces; ++j) {
+#pragma unroll
+                        for (int e = 0; e < kParts; ++e) acc[j].x += part[j][e].x, acc[j].y += part[j][e].y, acc[j].z += part[j][e].z, acc[j].w += part[j][e].w;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < kPieces; ++j) {
+                    if (i0 + j * kDqThreads < items) finish(tt[j], col0 + nn[j], acc[j], res[j], gain[j], p.norm.ssq_in ? bars->row_scale[tt[j]] : 1.f);
+                }
+            }
+        };
         // Every CTA of a split tile reduces its own share of the feature rows, once all partials of the
         // tile are in scratch: nobody reads more than one tile's worth, and the sum runs in CTA order.
         // p.last_sums: the CTA whose partial is the last one reduces all rows, and nobody waits.
@@ -472,6 +601,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             int       c_first;
             const int n_split = tile_ctas(tjs, c_first);
             const int col0    = tjs * kSuperN;
+            if (p.norm.ssq_in && dtid < t_rows) bars->row_scale[dtid] = norm_row_scale(p.norm, t0 + dtid);
+            if (p.norm.ssq_out && dtid < t_rows) s_ssq[dtid] = 0ull;
             if (dtid == 0 && !p.last_sums) {
                 // Bounded wait for the other CTAs of the tile.  The plan splits tiles between CTAs only
                 // when the whole grid is one wave of at most one CTA per SM (gemm_tc_plan), so the
@@ -481,126 +612,42 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 const long long t_begin = clock64();
                 for (;;) {
                     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(arrive + tjs) : "memory");
-                    if (seen >= n_split || clock64() - t_begin > p.max_wait_cycles) break;
-                    __nanosleep(64);
+                    if (seen >= n_split * kDqWarps || clock64() - t_begin > p.max_wait_cycles) break;
+                    __nanosleep(32);
                 }
-                if (seen < n_split) atomicOr(p.status, kStatusGemmTmemWait);
-                bars->flag = seen >= n_split;
+                if (seen < n_split * kDqWarps) atomicOr(p.status, kStatusGemmTmemWait);
+                bars->flag = seen >= n_split * kDqWarps;
             }
-            // producer side of a folded norm: per-token sums of squares of this CTA's share, in fixed point, kept in the
-            // (by now idle) activation ring until they go out with one atomic per token
-            unsigned long long* s_ssq = reinterpret_cast<unsigned long long*>(x_ring);
-            if (p.norm.ssq_out && dtid < t_rows) s_ssq[dtid] = 0ull;
             named_bar_sync(1, kDqThreads);
             TC_TRACE(trow, 42, tjs);
             const bool tile_ok = p.last_sums || bars->flag != 0;  // read between the barriers: the next call may rewrite the flag
+            int through = 0;
+            if (dtid == 0 && !p.last_sums) {
+                // looked at behind the sums; a CTA that gave up has seen no full count that says that its own warps' have arrived
+                if (!tile_ok) __threadfence();
+                through = atomicAdd(done + tjs, 1);
+                if (!tile_ok) __threadfence();
+            }
             if (tile_ok) {
-                const int j      = blockIdx.x - c_first;
-                const int n_cols = min(kSuperN, p.N - col0);  // N % 32 == 0
-                const int f0     = p.last_sums ? 0 : (n_cols * j / n_split) & ~3;
-                const int f1     = p.last_sums || j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
-                const int quads  = (f1 - f0) / 4;
-                const int items  = t_rows * quads;
+                const int    j      = blockIdx.x - c_first;
+                const int    n_cols = min(kSuperN, p.N - col0);  // N % 32 == 0
+                const int    f0     = p.last_sums ? 0 : (n_cols * j / n_split) & ~3;
+                const int    f1     = p.last_sums || j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
                 const float* tile_slots = slots + (size_t)(c_first + tjs) * slot_floats;
-                auto finish = [&](int t, int n, float4 acc) {
-                    if (p.norm.ssq_in) {
-                        // consumer side: the row's 1 / rms completes the normalisation of this GEMM's input
-                        const float inv = norm_row_scale(p.norm, t0 + t);
-                        acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
-                    }
-                    const __half2 h0 = __floats2half2_rn(acc.x, acc.y), h1 = __floats2half2_rn(acc.z, acc.w);
-                    if (p.norm.ssq_out) {
-                        // producer side (llama_decoder_kernels.cu:104-160 split in two): residual += y in fp32, stored as
-                        // fp16; the sum of squares is taken before that rounding, the norm weight applied to the stored value
-                        __half2*       rp = reinterpret_cast<__half2*>(p.norm.residual + (size_t)(t0 + t) * p.N + col0 + n);
-                        const __half2* gp = reinterpret_cast<const __half2*>(p.norm.norm_weight + col0 + n);
-                        const float2   r0 = __half22float2(rp[0]), r1 = __half22float2(rp[1]);
-                        const float2   y0 = __half22float2(h0), y1 = __half22float2(h1);
-                        const float2   s0 = make_float2(r0.x + y0.x, r0.y + y0.y), s1 = make_float2(r1.x + y1.x, r1.y + y1.y);
-                        const float    ss = (s0.x * s0.x + s0.y * s0.y) + (s1.x * s1.x + s1.y * s1.y);
-                        const __half2  n0 = __float22half2_rn(s0), n1 = __float22half2_rn(s1);
-                        rp[0] = n0, rp[1] = n1;
-                        const float2 a0 = __half22float2(n0), a1 = __half22float2(n1);
-                        const float2 g0 = __half22float2(gp[0]), g1 = __half22float2(gp[1]);
-                        __half2*     dst = reinterpret_cast<__half2*>(p.C + (size_t)(t0 + t) * p.N + col0 + n);
-                        dst[0]           = __floats2half2_rn(a0.x * g0.x, a0.y * g0.y);
-                        dst[1]           = __floats2half2_rn(a1.x * g1.x, a1.y * g1.y);
-                        atomicAdd(s_ssq + t, (unsigned long long)__float2ll_rn(ss * 1048576.f));
-                    }
-                    else if (p.fused_silu) {
-                        // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pairs (gate, up)
-                        const float2 u0 = __half22float2(h0), u1 = __half22float2(h1);
-                        const float  s0 = u0.x / (1.f + __expf(-u0.x)), s1 = u1.x / (1.f + __expf(-u1.x));
-                        *reinterpret_cast<__half2*>(p.C + (size_t)(t0 + t) * (p.N / 2) + (col0 + n) / 2) =
-                            __floats2half2_rn(s0 * u0.y, s1 * u1.y);
-                    }
-                    else {
-                        __half2* dst = reinterpret_cast<__half2*>(p.C + (size_t)(t0 + t) * p.N + col0 + n);
-                        dst[0]       = h0;
-                        dst[1]       = h1;
-                    }
-                };
-                // The last CTA of a tile has few parts and all rows: the loads of four pieces are on their way together (a step of the 70B
-                // model, 8 layers, 21 sequences: 1738 us piece by piece, 1702 so, 1709 when every CTA waited and summed a share; part of it
-                // is what the compiler makes of the loop over units beside either: 11008 x 4096, 16 tokens, 13.8 and 13.4 us).
-                constexpr int kPieces = 4;
-                for (int i0 = dtid; p.last_sums && i0 < items; i0 += kPieces * kDqThreads) {
-                    float4 acc[kPieces], part[kPieces][2];
-#pragma unroll
-                    for (int j = 0; j < kPieces; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int cc = 0; cc < n_split; cc += 2) {
-#pragma unroll
-                        for (int j = 0; j < kPieces; ++j) {
-                            const int    i = min(i0 + j * kDqThreads, items - 1), t = i / quads;
-                            const float* src = tile_slots + (size_t)t * kSuperN + f0 + (i - t * quads) * 4;
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                part[j][e] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                if (cc + e < n_split) part[j][e] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(cc + e) * slot_floats));
-                            }
-                        }
-#pragma unroll
-                        for (int j = 0; j < kPieces; ++j) {
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) acc[j].x += part[j][e].x, acc[j].y += part[j][e].y, acc[j].z += part[j][e].z, acc[j].w += part[j][e].w;
-                        }
-                    }
-#pragma unroll
-                    for (int j = 0; j < kPieces; ++j) {
-                        const int i = i0 + j * kDqThreads, t = i / quads;
-                        if (i < items) finish(t, f0 + (i - t * quads) * 4, acc[j]);
-                    }
-                }
-                for (int i = dtid; !p.last_sums && i < items; i += kDqThreads) {
-                    const int    t    = i / quads;
-                    const int    n    = f0 + (i - t * quads) * 4;
-                    const float* src  = tile_slots + (size_t)t * kSuperN + n;
-                    float4       acc  = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int cc = 0; cc < n_split; cc += 8) {
-                        float4 part[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            part[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (cc + e < n_split) part[e] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)(cc + e) * slot_floats));
-                        }
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {  // absent slots add +0
-                            acc.x += part[e].x, acc.y += part[e].y, acc.z += part[e].z, acc.w += part[e].w;
-                        }
-                    }
-                    finish(t, n, acc);
+                if (f1 > f0) {
+                    if (n_split <= 2 && !p.norm.ssq_out) sum_rows(Int<4>{}, Int<2>{}, Int<0>{}, tile_slots, n_split, f0, f1, col0);
+                    else if (n_split <= 4) sum_rows(Int<2>{}, Int<4>{}, Int<1>{}, tile_slots, n_split, f0, f1, col0);
+                    else sum_rows(Int<1>{}, Int<8>{}, Int<1>{}, tile_slots, n_split, f0, f1, col0);
                 }
             }
             named_bar_sync(1, kDqThreads);  // everyone is done reading; the flag may be reused
             if (p.norm.ssq_out && tile_ok && dtid < t_rows && s_ssq[dtid]) atomicAdd(p.norm.ssq_out + t0 + dtid, s_ssq[dtid]);
             if (dtid == 0 && p.last_sums) arrive[tjs] = 0;
-            if (dtid == 0 && !p.last_sums) {
-                // the last reader of the tile resets both counts for the next launch; a CTA that gave up
-                // on the wait counts as a reader too, so the counts recover after a time-out
-                if (atomicAdd(done + tjs, 1) == n_split - 1) {
-                    arrive[tjs] = 0;
-                    done[tjs]   = 0;
-                }
+            if (dtid == 0 && !p.last_sums && through == n_split - 1) {
+                // the last CTA through the wait resets both counts for the next launch; one that gave up counts too, so the counts
+                // recover after a time-out
+                arrive[tjs] = 0;
+                done[tjs]   = 0;
             }
         };
 
@@ -608,22 +655,31 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         const int      n_row  = m * kTileN + q * 32 + lane;  // feature row of the CTA tile held by this thread
         const uint32_t a_lane = (uint32_t)(q * 32) << 16;    // TMEM lanes of this warp
 
+        // shared-memory addresses: this warp's share of a stage of packed weight (a 32-feature tile of each slab) and of {zero, scale},
+        // and the barriers of its rings
+        const uint32_t my_w = base + (uint32_t)(w_ring - sm) + (uint32_t)((m * 4 + q) * kTileBytes + lane * 16);
+        const uint32_t my_q = base + (uint32_t)(w_ring - sm) + (uint32_t)(kSlabs * kSlabBytes + (m * 4 + q) * 128 + r * 4);
+        const uint32_t w_full = smem_u32(bars->w_full), w_empty = smem_u32(bars->w_empty);
+        const uint32_t a_full = smem_u32(bars->a_full[m]), a_empty = smem_u32(bars->a_empty[m]);
         int      js = u_begin / G, g = u_begin - js * G;
-        int      sw = 0, sw_fill = kWST - 1;  // ring slot read now / refilled now (the one read one unit of its own ago)
-        int      sa = 0;
-        uint32_t pa = 0;                      // phase parity of the team's expanded-weight ring
-        for (int it = 0; it < n_units; ++it) {
-            TC_TRACE(trow, 30, it);
-            if ((it & 1) == kh) {
-                asm volatile("cp.async.wait_group %0;" ::"n"(kWST - 2) : "memory");
-                __syncwarp();
-                const unsigned char* sb = my_ring_g + sw * kWarpStage;
-                const __half2*       qs = reinterpret_cast<const __half2*>(sb + kSlabs * kTileBytes);
+        int      u  = kh;           // this warp's next unit: every other one
+        int      sw = kh, sa = kh * S::kParts;  // its stages of packed and of expanded weight, and their phase parities
+        uint32_t pw = 0, pa = 0;
+        for (int it = 0; it < n_units;) {
+            const int this_js = js;
+            const int seg_end = it + min(G - g, n_units - it);
+            for (; u < seg_end; u += 2) {
+                TC_TRACE(trow, 30, u);
+                warp_wait(w_full + sw * 8, pw, dead, p.status, kStatusGemmPipeWait);
+                const uint32_t wa = my_w + sw * kWStage, qa = my_q + sw * kWStage;
+                const uint32_t qv[4]     = {shared_load4<0>(qa), shared_load4<32>(qa), shared_load4<64>(qa), shared_load4<96>(qa)};
+                const uint4    w[kSlabs] = {shared_load16<0>(wa), shared_load16<kSlabBytes>(wa), shared_load16<2 * kSlabBytes>(wa),
+                                            shared_load16<3 * kSlabBytes>(wa)};
                 uint32_t z1024[2], nz64[2], s_lo[2], s_hi[2];
 #pragma unroll
                 for (int a = 0; a < 2; ++a) {
-                    const __half2 q_lo = qs[a * 16 + r];
-                    const __half2 q_hi = qs[a * 16 + r + 8];
+                    const __half2 q_lo = reinterpret_cast<const __half2&>(qv[2 * a]);
+                    const __half2 q_hi = reinterpret_cast<const __half2&>(qv[2 * a + 1]);
                     const __half2 zl2  = __half2half2(__hadd(__low2half(q_lo), __float2half_rn(960.f)));
                     const __half2 zh2  = __half2half2(__hneg(__low2half(q_hi)));
                     const __half2 sl2  = __half2half2(__high2half(q_lo));
@@ -633,16 +689,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     s_lo[a]  = reinterpret_cast<const uint32_t&>(sl2);
                     s_hi[a]  = reinterpret_cast<const uint32_t&>(sh2);
                 }
-                const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + a_lane;
-                bool           room   = false;
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     // two slabs: all fragments first (independent chains the scheduler can interleave), then the stores
                     uint32_t f[2][16];  // [16-row half][pieces of 4 columns]
 #pragma unroll
                     for (int kk = 0; kk < 2; ++kk) {
-                        const uint4    w     = reinterpret_cast<const uint4*>(sb)[(2 * half + kk) * 32 + lane];
-                        const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+                        const uint4    v     = w[2 * half + kk];
+                        const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                         for (int wi = 0; wi < 4; ++wi) {
                             const int a = wi & 1, at = kk * 8 + (wi >> 1) * 4;
@@ -654,52 +708,58 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                             f[a][at + 3] = hmul2_ftz(fr[3], s_hi[a]);
                         }
                     }
-                    if (!room) {
-                        // the tensor core must be done with what this TMEM stage held kAST units ago (the first round passes at
+                    if (half == 0) {
+                        // everyone in the warp holds its words: the stage may be filled again
+                        __syncwarp();
+                        if (lane == 0) arrive_at(w_empty + sw * 8);
+                    }
+                    const bool begins = half == 0 || S::kParts == 2, ends = half == 1 || S::kParts == 2;  // of a TMEM stage
+                    if (begins) {
+                        // the tensor core must be done with what this TMEM stage held kAST stages ago (the first round passes at
                         // once: a fresh barrier counts as having completed the phase before)
-                        warp_wait(&bars->a_empty[m][sa], pa ^ 1u, dead, p.status, kStatusGemmPipeWait);
+                        warp_wait(a_empty + sa * 8, pa ^ 1u, dead, p.status, kStatusGemmPipeWait);
                         tc_fence_after();
-                        TC_TRACE(trow, 32, it);
-                        room = true;
+                        TC_TRACE(trow, 32, u);
                     }
                     // rows q*32 + a*16 .. +15 (TMEM lanes), k = 64 half .. +63 (32 columns)
-                    tmem_st_16x128b_x8(a_tmem + (uint32_t)(half * 32), f[0]);
-                    tmem_st_16x128b_x8(a_tmem + (16u << 16) + (uint32_t)(half * 32), f[1]);
+                    const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + a_lane + (begins ? 0u : 32u);
+                    tmem_st_16x128b_x8(a_tmem, f[0]);
+                    tmem_st_16x128b_x8(a_tmem + (16u << 16), f[1]);
+                    if (ends) {
+                        // expanded tile visible to the tensor core
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) arrive_at(a_full + sa * 8);
+                        TC_TRACE(trow, 33, u);
+                        if (half == 0) {
+                            ++sa;  // the unit's second stage; kAST is even then
+                        }
+                        else {
+                            sa += 1 + S::kParts;  // past the other warps' unit
+                            if (sa >= kAST) sa -= kAST, pa ^= 1u;
+                        }
+                    }
                 }
-                // expanded tile visible to the tensor core; packed stage free again
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->a_full[m][sa]);
-                TC_TRACE(trow, 33, it);
-                // refill the slot that was read one unit of this warp ago (everyone in the warp is past its reads)
-                if (to_issue > 0) issue_unit(sw_fill);
-                --to_issue;
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                sw      = (sw == kWST - 1) ? 0 : sw + 1;
-                sw_fill = (sw_fill == kWST - 1) ? 0 : sw_fill + 1;
+                sw += 2;
+                if (sw >= kWST) sw -= kWST, pw ^= 1u;
             }
-            if (++sa == kAST) {
-                sa = 0;
-                pa ^= 1u;
+            it = seg_end;
+            if (js == u_begin / G) {
+                // What follows reads and writes scratch, tickets and the output, which the kernel before this one may still be using.
+                pdl_wait();
             }
-
-            const int  this_js = js;
-            const bool seg_end = (it == n_units - 1) || (g == G - 1);
-            if (++g == G) {
-                g = 0;
-                ++js;
-            }
-            if (!seg_end) continue;
+            g = 0;
+            ++js;
 
             // ---- 256-feature tile this_js finished for this CTA: drain the accumulators -----------
             int       c_first;
             const int n_split = tile_ctas(this_js, c_first);
             const int col0    = this_js * kSuperN;
-            TC_TRACE(trow, 34, it);
-            warp_wait(&bars->acc_full[m], seg_idx & 1, dead, p.status, kStatusGemmTmemWait);
+            TC_TRACE(trow, 34, this_js);
+            warp_wait(smem_u32(&bars->acc_full[m]), seg_idx & 1, dead, p.status, kStatusGemmTmemWait);
             tc_fence_after();
-            TC_TRACE(trow, 35, it);
+            TC_TRACE(trow, 35, this_js);
             const int n_glob = col0 + n_row;
             const uint32_t my_acc = tmem + m * accS + ((uint32_t)(q * 32) << 16);
             if (!dead) {
@@ -718,23 +778,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                         }
                     }
                     else {
+                        if (p.norm.ssq_in) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int t = t0 + col + i;
-                            const bool in = i < valid && t < p.T && n_glob < p.N;
-                            if (p.norm.ssq_in) v[i] *= norm_row_scale(p.norm, min(t, p.T - 1));
-                            if (p.fused_silu) {
-                                // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair (gate, up) = rows (n, n + 1)
-                                const float mine_v = __half2float(__float2half_rn(v[i]));
-                                const float other  = __shfl_down_sync(0xffffffffu, mine_v, 1);
-                                if ((lane & 1) == 0 && in) {
-                                    const float silu = mine_v / (1.f + __expf(-mine_v));
-                                    p.C[(size_t)t * (p.N / 2) + n_glob / 2] = __float2half_rn(silu * other);
+                            for (int i = 0; i < 16; ++i) v[i] *= norm_row_scale(p.norm, min(t0 + col + i, p.T - 1));
+                        }
+                        // Neighbouring lanes trade a token each, so that a lane holds two adjacent features of one token of every two: whole
+                        // sectors, and (gate, up) side by side (22016 x 4096, 735 tokens: 129 us with a store of 2 bytes for every value, 114 so).
+                        const bool odd = lane & 1;
+                        const int  n0  = n_glob & ~1, tl = t0 + col + odd;
+                        const bool in  = n0 < p.N;
+                        __half*    out = p.fused_silu ? p.C + (size_t)tl * (p.N / 2) + n0 / 2 : p.C + (size_t)tl * p.N + n0;
+                        const int  ld  = p.fused_silu ? p.N : 2 * p.N;  // two tokens
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) {
+                            const float   got = __shfl_xor_sync(0xffffffffu, odd ? v[i] : v[i + 1], 1);
+                            const __half2 h   = odd ? __floats2half2_rn(got, v[i + 1]) : __floats2half2_rn(v[i], got);
+                            if (in && i < valid && tl + i < p.T) {
+                                if (p.fused_silu) {
+                                    // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair (gate, up)
+                                    const float2 u = __half22float2(h);
+                                    *out = __float2half_rn(u.x / (1.f + __expf(-u.x)) * u.y);
+                                }
+                                else {
+                                    *reinterpret_cast<__half2*>(out) = h;
                                 }
                             }
-                            else if (in) {
-                                p.C[(size_t)t * p.N + n_glob] = __float2half_rn(v[i]);
-                            }
+                            out += ld;
                         }
                     }
                 }
@@ -744,20 +813,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             tc_fence_before();
             __syncwarp();
             if (lane == 0 && !dead) mbar_arrive(&bars->acc_empty[m]);
-            TC_TRACE(trow, 37, it);
+            TC_TRACE(trow, 37, this_js);
             if (n_split > 1) {
-                // publish the partial (its reduction waits until this CTA has no units left): the barrier orders
-                // every thread's stores before the fence of the one thread that then counts the CTA in
-                named_bar_sync(1, kDqThreads);
-                if (dtid == 0) {
-                    __threadfence();
-                    const int before = atomicAdd(arrive + this_js, 1);
-                    if (p.last_sums) {
+                // Publish the partial (its reduction waits until this CTA has no units left).  Each warp counts itself in: the warp's
+                // barrier orders its lanes' stores before the release of the one that counts.
+                if (!p.last_sums && lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrive + this_js) : "memory");
+                if (p.last_sums) {
+                    // the barrier orders every thread's stores before the fence of the one thread that then counts the CTA in
+                    named_bar_sync(1, kDqThreads);
+                    if (dtid == 0) {
+                        __threadfence();
+                        const int before = atomicAdd(arrive + this_js, 1);
                         __threadfence();
                         bars->flag = before == n_split - 1;
                     }
-                }
-                if (p.last_sums) {
                     named_bar_sync(1, kDqThreads);
                     if (bars->flag == 0) continue;  // rewritten behind the next barrier of these threads at the earliest
                 }
@@ -768,14 +837,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 }
                 pend[n_pend++] = this_js;
             }
-            TC_TRACE(trow, 38, it);
+            TC_TRACE(trow, 38, this_js);
         }
         TC_TRACE(trow, 40, 0);
         for (int i = 0; i < n_pend; ++i) {
             reduce_share(pend[i]);
             TC_TRACE(trow, 41, i);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
     }
 
     tc_fence_before();
@@ -823,15 +891,11 @@ PFN_encodeTiled lookup_encode_tiled()
     return reinterpret_cast<PFN_encodeTiled>(fn);
 }
 
-int x_stages_for(int token_tile) { return token_tile > 64 ? 3 : kXSTMax; }
-int a_stages_for(int token_tile) { return token_tile > 64 ? 2 : kASTMax; }  // beside the accumulators, all of TMEM
-int acc_stride_for(int token_tile) { return token_tile > 64 ? 128 : 64; }
-
 }  // namespace
 
 size_t gemm_tc_smem_bytes(int token_tile)
 {
-    return 1024 + (size_t)x_stages_for(token_tile) * 2 * token_tile * 128 + (size_t)kWST * kDqWarps * kWarpStage + sizeof(Bars) + 64;
+    return 1024 + (size_t)(token_tile > 64 ? Shape<true>::kXST : Shape<false>::kXST) * 2 * token_tile * 128 + (size_t)kWST * kWStage + sizeof(Bars) + 64;
 }
 
 GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
@@ -844,16 +908,16 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
     pl.total_units = pl.n_col_tiles * G;
     pl.parts_per_tile = 0;
     // With at least as many whole column tiles as SMs: one per CTA, nothing is split, nobody waits.  `balance`: unless their last
-    // wave is so empty that cutting the units evenly is faster, by a model fitted to 270 launches of twelve projections with 32
-    // to 3000 tokens (microseconds; mean error 10 %).  57344 x 8192, 224 tiles: two waves of 64 units, or 97 units for every SM:
-    // 88 / 76 us with 32 tokens, 4096 x 11008 with 1600 tokens 178 / 125.
+    // wave is so empty that cutting the units evenly is faster, by a model fitted to 70 launches of seven projections with 17 to 1024
+    // tokens, both ways (microseconds; mean error 8 % and 4 %; the way it picks costs 1.8 % more than the better one, always whole
+    // tiles 5.5 %).  57344 x 8192, 224 tiles: two waves of 64 units, or 97 units for every SM: 71 / 62 us with 32 tokens.
     const long long tiles = (long long)pl.t_chunks * pl.n_col_tiles;
     const double    fill  = std::max(0, pl.token_tile - 32) / 96.0;  // what a unit costs beyond its expansion
-    auto cut_us = [&](int units) { return 8.5 + units * (0.711 + 0.083 * fill) + 10.2 * units / G + 13.8 * pl.token_tile / 128; };
+    auto cut_us = [&](int units) { return 1.0 + units * (0.547 + 0.409 * fill) + 2.5 * units / G + 3.4 * pl.token_tile / 128; };
     bool whole = tiles >= sm_count;
     const bool could = whole;
     if (whole) {
-        pl.us = 4.2 + (double)((tiles + sm_count - 1) / sm_count) * (G * (0.56 + 0.14 * fill) + 12.7);
+        pl.us = (double)((tiles + sm_count - 1) / sm_count) * (G * (0.489 + 0.317 * fill) + 3.5);
         if (balance && pl.t_chunks <= sm_count / 2) {
             const int per_chunk = sm_count / pl.t_chunks;
             whole = pl.us <= cut_us((pl.total_units + per_chunk - 1) / per_chunk);
@@ -904,7 +968,8 @@ bool gemm_tc_all_tiles_split(const GemmTcPlan& pl, int K)
 
 cudaError_t gemm_tc_prepare(int max_smem)
 {
-    return cudaFuncSetAttribute(gemm_s4_f16_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_s4_f16_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_s4_f16_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
 }
 static const KernelPreparation g_prepare(gemm_tc_prepare);
 
@@ -917,27 +982,30 @@ cudaError_t gemm_tc_launch(const GemmTcPlan& pl, GemmTcParams p, cudaStream_t st
     p.n_col_tiles     = pl.n_col_tiles;
     p.token_tile      = pl.token_tile;
     p.last_sums       = pl.last_sums;
-    p.x_stages        = x_stages_for(pl.token_tile);
-    p.a_stages        = a_stages_for(pl.token_tile);
     if (p.max_wait_cycles <= 0) p.max_wait_cycles = kMaxWaitCycles;
-    p.acc_stride      = acc_stride_for(pl.token_tile);
 
-    // Activations as a 2-D tensor [T][K] of fp16; one box = 64 k (128 bytes, the swizzle span) x token tile.
     static const PFN_encodeTiled encode = lookup_encode_tiled();
     if (encode == nullptr) return cudaErrorNotSupported;
-    CUtensorMap       x_map;
-    const cuuint64_t  dims[2]    = {(cuuint64_t)p.K, (cuuint64_t)p.T};
-    const cuuint64_t  strides[1] = {(cuuint64_t)p.K * 2};
-    const cuuint32_t  box[2]     = {64u, (cuuint32_t)pl.token_tile};
-    const cuuint32_t  estr[2]    = {1u, 1u};
-    if (encode(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<unsigned char*>(p.X), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
-        != CUDA_SUCCESS) {
+    auto map_of = [](CUtensorMap& map, CUtensorMapDataType type, int rank, const void* at, std::array<cuuint64_t, 3> dims,
+                     std::array<cuuint64_t, 2> strides, std::array<cuuint32_t, 3> box, CUtensorMapSwizzle swizzle) {
+        const cuuint32_t steps[3] = {1u, 1u, 1u};
+        return encode(&map, type, rank, const_cast<void*>(at), dims.data(), strides.data(), box.data(), steps, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+               == CUDA_SUCCESS;
+    };
+    CUtensorMap      x_map, w_map, q_map;
+    const cuuint64_t N = p.N, T = p.T, K = p.K;
+    // [K / 64][T][64] fp16: a unit's two 64-wide blocks (128 bytes, the swizzle span) of the token tile; [K / 32][N / 32][512 bytes]: four
+    // slabs of a column tile; [K / 128][N] {zero, scale}
+    if (!map_of(x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, p.X, {64, T, K / 64}, {K * 2, 128}, {64u, (cuuint32_t)pl.token_tile, 2u},
+                CU_TENSOR_MAP_SWIZZLE_128B)
+        || !map_of(w_map, CU_TENSOR_MAP_DATA_TYPE_INT64, 3, p.A, {kTileBytes / 8, N / 32, K / 32}, {kTileBytes, N / 32 * kTileBytes},
+                   {kTileBytes / 8, kSuperN / 32, kSlabs}, CU_TENSOR_MAP_SWIZZLE_NONE)
+        || !map_of(q_map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, p.Q, {N, K / kGroup, 1}, {N * 4, 0}, {kSuperN, 1u, 1u}, CU_TENSOR_MAP_SWIZZLE_NONE)) {
         return cudaErrorInvalidValue;
     }
     dim3 grid(pl.ctas, pl.t_chunks);
-    return launch_kernel(gemm_s4_f16_tc_kernel, grid, dim3(kThreads), pl.smem_bytes, st, pdl, p, x_map);
+    return launch_kernel(pl.token_tile > 64 ? gemm_s4_f16_tc_kernel<true> : gemm_s4_f16_tc_kernel<false>, grid, dim3(kThreads), pl.smem_bytes, st, pdl, p, x_map, w_map, q_map);
 }
 
 }  // namespace tmb

@@ -111,3 +111,30 @@ def test_folded_norm_with_few_sequences(batch):
     err = np.abs(a - b)
     assert err.max() <= 3e-2 and err.mean() / np.abs(b).mean() <= 5e-3, (err.max(), err.mean() / np.abs(b).mean())
     assert np.array_equal(a, again)
+
+
+# column tiles that end inside a box of the weight, one and many groups, both classes of token tiles and their edges
+@pytest.mark.parametrize("n,k", [(32, 128), (288, 384), (288, 4224), (4128, 1024), (38016, 256)])
+@pytest.mark.parametrize("tokens", [17, 63, 64, 65, 127, 129])
+@pytest.mark.parametrize("silu", [False, True])
+def test_tensor_core_tiles_at_their_edges(n, k, tokens, silu):
+    from lmdeploy_b200 import turbomind as tm
+    from perf import cases
+    if silu:
+        n = n // 64 * 64 or 64
+    w = cases._linear(cases._gen(5, n), n, k)
+    exact = cases._exact_weight(cases._gen(5, n), n, k)
+    op = tm.LlamaLinear(0)
+    x = torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(tokens)).half()
+    buf = torch.full((tokens + 1, n // 2 if silu else n), 777.0, dtype=torch.float16, device="cuda")
+    op.forward(buf[:tokens], x, tokens, w, op.kFusedSiluFfn if silu else op.kGemm)
+    op.gemm_s4_f16_.handle.check_device_status(torch.cuda.current_stream().cuda_stream)
+    assert bool((buf[tokens] == 777.0).all())
+    y, size = x.double() @ exact, x.double().abs() @ exact.abs()
+    slack = y.abs() * 2.0 ** -11 + size * k * 2.0 ** -24 + 1e-7  # one rounding of the result, fp32 sums
+    if silu:  # gate and up are rounded to fp16 first; |silu'| <= 1.1
+        gate, up = y[:, 0::2], y[:, 1::2]
+        y = torch.nn.functional.silu(gate) * up
+        slack = 2 * (1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2]) + y.abs() * 2.0 ** -11 + 1e-6
+    over = ((buf[:tokens].double() - y).abs() / slack).max().item()
+    assert over <= 1.0, f"{over:.2f} of the bound"
