@@ -4,8 +4,8 @@
 // The weights of all heads meet for every (query, key) pair, and neither the weights nor the outputs of all heads of a tile
 // fit an SM.  So the pass goes through memory, a block of query tiles (128 queries of one sequence) at a time, as many as
 // the scratch holds, [tile][head][query][key]:
-//   chunk_scores_kernel   CTA = (head, tile): S = Q K^T (tcgen05, accumulator in TMEM twice, so that the next product runs
-//                         under this one's epilogue), sigmoid, mask; fp16 weights
+//   chunk_scores_kernel   CTA = (head, tile): S = Q K^T (tcgen05, accumulator in TMEM twice, so that one product runs
+//                         under the other's epilogue), sigmoid, mask; fp16 weights
 //   chunk_mix_kernel      warp = 64 pairs of a query at a time: [heads x heads] times [heads x pairs] by mma.m16n8k16 with
 //                         fragments straight from and to memory, in place; the mixed weights are bf16
 //   chunk_values_kernel   CTA = (head, tile): O = P V (tcgen05)
@@ -43,6 +43,11 @@ struct TileInfo {
     SeqSpan sp;
     int     q0, rows, pos0, pos1, base, n_tiles;
 };
+// The last query tiles of a sequence, which see the most keys, begin first: the launch ends on short ones
+__device__ __forceinline__ int item_of_block()
+{
+    return gridDim.y - 1 - blockIdx.y;
+}
 __device__ __forceinline__ TileInfo tile_info(const ChunkTcParams& p, int item)
 {
     const QueryTile q = p.c.tiles[p.tile0 + item];
@@ -63,38 +68,51 @@ __device__ __forceinline__ void cp_async16z(uint32_t dst, const void* src, int b
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ float scaled_sigmoid_log2(float x)  // sigmoid of x / log2(e), times kWeightScale
+// sigmoids of x / log2(e) and y / log2(e), times kWeightScale.  One reciprocal serves both: with a = (1 + 2^-x) / scale and b for y,
+// 1 / a = b / (a b).  Beyond 2^60 the weight is zero in fp16 whatever the exponent; the bound keeps a b finite.
+__device__ __forceinline__ uint32_t scaled_sigmoids_log2(float x, float y)
 {
-    float e, y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaf(e, 1.f / kWeightScale, 1.f / kWeightScale)));
-    return y;
+    float a, b, r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(a) : "f"(-x), "f"(60.f));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(b) : "f"(-y), "f"(60.f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(a));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(b));
+    a = fmaf(a, 1.f / kWeightScale, 1.f / kWeightScale), b = fmaf(b, 1.f / kWeightScale, 1.f / kWeightScale);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
+    const __half2 v = __floats2half2_rn(r * b, r * a);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 // rows [0, count) of [row][width] at src into a swizzled tile of ROWS rows and D columns, zeros elsewhere
-template<int ROWS, int D>
-__device__ __forceinline__ void copy_rows(uint32_t dst, int block_bytes, const __nv_bfloat16* src, size_t ld, int count, int width)
+template<int ROWS, int D, int THREADS = kRowThreads>
+__device__ __forceinline__ void copy_rows(int thread, uint32_t dst, int block_bytes, const __nv_bfloat16* src, size_t ld, int count, int width)
 {
 #pragma unroll
-    for (int r = 0; r < ROWS * D / 8 / kRowThreads; ++r) {
-        const int  c = threadIdx.x + r * kRowThreads, row = c / (D / 8), chunk = c % (D / 8);
+    for (int r = 0; r < ROWS * D / 8 / THREADS; ++r) {
+        const int  c = thread + r * THREADS, row = c / (D / 8), chunk = c % (D / 8);
         const bool ok = row < count && chunk * 8 < width;
         cp_async16z(dst + sw_off(row, chunk, block_bytes), src + (ok ? (size_t)row * ld + chunk * 8 : 0), ok ? 16 : 0);
     }
 }
 
 // ------------------------------------------------------------------------------------------------ scores -> weights
+// 142 M weights of 4096 tokens in two chunks, 32 heads, take 120 us; 77 without the sigmoids and the stores (products of 64 keys and the
+// copies of their keys), 100 without the sigmoids, 105 without the stores.  Two groups of four warps take the key tiles in turn, each
+// with a buffer of keys and an accumulator of its own, so that one group's product runs under the other's epilogue (two of each a
+// group: no difference).  One reciprocal serves two weights; a thread has a query's 64 weights, whole sectors, and stores them as they
+// are.  With one group, a reciprocal per weight and the rows staged through shared memory 167 us.
+constexpr int kScoreThreads = 2 * kRowThreads + 32;
 struct ScoreBars {
-    uint64_t kv_full[2], s_full[2];
+    uint64_t q_full, kv_full[2], s_full[2];
     uint32_t tmem_base;
 };
 template<int DK>
 struct ScoreLayout {
-    static constexpr int kQ = kBM * DK * 2, kK = kBN * DK * 2, kOut = kBM * kBN * 2;
-    static constexpr int kSmem = 1024 + kQ + 2 * kK + kOut + 64;
+    static constexpr int kQ = kBM * DK * 2, kK = kBN * DK * 2;
+    static constexpr int kSmem = 1024 + kQ + 2 * kK + 64;
 };
 
 template<int DK>
-__global__ void __launch_bounds__(kThreads, 2) chunk_scores_kernel(const ChunkTcParams p)
+__global__ void __launch_bounds__(kScoreThreads, 2) chunk_scores_kernel(const ChunkTcParams p)
 {
     using L = ScoreLayout<DK>;
     using E = __nv_bfloat16;
@@ -103,104 +121,91 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_scores_kernel(const ChunkTc
     pdl_launch_dependents();
     const ChunkAttention& a = p.a;
     const int             tid = threadIdx.x, warp = tid >> 5, h = blockIdx.x, g = h / (a.heads / a.kv_heads);
-    const TileInfo        ti = tile_info(p, blockIdx.y);
+    const TileInfo        ti = tile_info(p, item_of_block());
     if (!ti.sp.live || ti.rows <= 0) return;
     const uint32_t raw = smem_u32(smem_dyn), base = (raw + 1023u) & ~1023u;
-    const uint32_t k_s = base + L::kQ, out_s = k_s + 2 * L::kK;
-    ScoreBars*     bars = reinterpret_cast<ScoreBars*>(smem_dyn + (base - raw) + L::kQ + 2 * L::kK + L::kOut);
+    const uint32_t k_s = base + L::kQ;
+    ScoreBars*     bars = reinterpret_cast<ScoreBars*>(smem_dyn + (base - raw) + L::kQ + 2 * L::kK);
     if (tid == 0) {
+        mbar_init(&bars->q_full, 2 * kRowThreads);
         for (int i = 0; i < 2; ++i) mbar_init(&bars->kv_full[i], kRowThreads), mbar_init(&bars->s_full[i], 1);
         fence_mbar_init();
     }
-    if (warp == 4) tmem_alloc(&bars->tmem_base, 2 * kBN);
+    if (warp == 8) tmem_alloc(&bars->tmem_base, 2 * kBN);
     tcgen05_before_sync();
     __syncthreads();
     tcgen05_after_sync();
     const uint32_t tmem = bars->tmem_base;
 
-    if (warp < 4) {
-        const E* keys = reinterpret_cast<const E*>(ti.sp.slab + a.k_off) + (size_t)g * a.ring * a.dim;
+    if (warp < 8) {
+        const int group = warp >> 2, row = tid % kRowThreads;
+        const E*  keys = reinterpret_cast<const E*>(ti.sp.slab + a.k_off) + (size_t)g * a.ring * a.dim;
         // a tile of keys starts on a multiple of 64 and the ring is one of 128 rows, so it never wraps inside
         auto load_keys = [&](int t) {
             const int key0 = ti.base + t * kBN;
-            copy_rows<kBN, DK>(k_s + (t & 1) * L::kK, kTBlock, keys + (size_t)(key0 % a.ring) * a.dim, a.dim, min(kBN, ti.pos1 + 1 - key0), a.dim);
+            copy_rows<kBN, DK>(row, k_s + group * L::kK, kTBlock, keys + (size_t)(key0 % a.ring) * a.dim, a.dim, min(kBN, ti.pos1 + 1 - key0), a.dim);
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        copy_rows<kBM, DK>(base, kQBlock, static_cast<const E*>(p.c.proj) + (size_t)(ti.sp.tok0 + ti.q0) * p.c.proj_ld + a.q_col + h * a.dim, p.c.proj_ld,
-                           ti.rows, a.dim);
-        load_keys(0);
-        if (ti.n_tiles > 1) {
-            load_keys(1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        }
-        else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        copy_rows<kBM, DK, 2 * kRowThreads>(tid, base, kQBlock,
+                                            static_cast<const E*>(p.c.proj) + (size_t)(ti.sp.tok0 + ti.q0) * p.c.proj_ld + a.q_col + h * a.dim,
+                                            p.c.proj_ld, ti.rows, a.dim);
+        if (group < ti.n_tiles) load_keys(group);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         fence_async_shared();  // this thread's copies become visible to the tensor core's reads
-        mbar_arrive(&bars->kv_full[0]);
+        mbar_arrive(&bars->q_full);
+        if (group < ti.n_tiles) mbar_arrive(&bars->kv_full[group]);
 
-        const bool     live  = tid < ti.rows;
-        const int      mine  = ti.pos0 + tid, lo = live ? chunk_first(mine, a.chunk) : 1 << 30;
-        const uint32_t lane  = tmem + ((uint32_t)(warp * 32) << 16);
+        const bool     live  = row < ti.rows;
+        const int      mine  = ti.pos0 + row, lo = live ? chunk_first(mine, a.chunk) : 1 << 30;
+        const uint32_t lane  = tmem + ((uint32_t)((warp & 3) * 32) << 16) + group * kBN;
         const float    scale = a.scale * kLog2e, bias = a.bias[h] * kLog2e;
-        __half*        out   = p.weights + ((size_t)blockIdx.y * a.heads + h) * kBM * p.ldk;
+        __half*        out   = p.weights + (((size_t)item_of_block() * a.heads + h) * kBM + row) * p.ldk;
         bool           dead  = false;
-        for (int t = 0; t < ti.n_tiles; ++t) {
-            if (t + 1 < ti.n_tiles) {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                fence_async_shared();
-                tcgen05_before_sync();  // the accumulator of tile t - 1, which tile t + 1 takes, has been read
-                mbar_arrive(&bars->kv_full[(t + 1) & 1]);
-            }
-            // uniform across the warp: the TMEM loads below are warp-wide instructions
-            // and, as the four warps share the barriers below, a wait that gave up is noted and not repeated
-            if (!dead && !__all_sync(0xffffffffu, mbar_wait(&bars->s_full[t & 1], (t >> 1) & 1, p.max_wait))) {
+        for (int t = group; t < ti.n_tiles; t += 2) {
+            // uniform across the warp: the TMEM loads below are warp-wide instructions; a wait that gave up is noted and not repeated
+            if (!dead && !__all_sync(0xffffffffu, mbar_wait(&bars->s_full[group], (t >> 1) & 1, p.max_wait))) {
                 atomicOr(p.status, kStatusGemmPipeWait);
                 dead = true;
             }
             tcgen05_after_sync();
             if (t + 2 < ti.n_tiles) load_keys(t + 2);
-            uint32_t s0[32], s1[32];
-            tmem_load32(lane + (t & 1) * kBN, s0);
-            tmem_load32(lane + (t & 1) * kBN + 32, s1);
-            const int key0 = ti.base + t * kBN;
-            uint32_t  w[32];
-            auto pair = [&](uint32_t x, uint32_t y) {
-                const __half2 v = __floats2half2_rn(scaled_sigmoid_log2(fmaf(__uint_as_float(x), scale, bias)),
-                                                    scaled_sigmoid_log2(fmaf(__uint_as_float(y), scale, bias)));
-                return *reinterpret_cast<const uint32_t*>(&v);
-            };
+            const int  key0   = ti.base + t * kBN;
+            const bool masked = !live || key0 < lo || key0 + kBN - 1 > mine;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) w[i] = pair(s0[2 * i], s0[2 * i + 1]), w[16 + i] = pair(s1[2 * i], s1[2 * i + 1]);
-            if (!live || key0 < lo || key0 + kBN - 1 > mine) {
+            for (int half = 0; half < 2; ++half) {
+                uint32_t s[32];
+                tmem_load32(lane + half * 32, s);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int  j  = key0 + 2 * i;
-                    const bool in0 = live && j >= lo && j <= mine, in1 = live && j + 1 >= lo && j + 1 <= mine;
-                    w[i] = (in0 ? w[i] & 0xffffu : 0u) | (in1 ? w[i] & 0xffff0000u : 0u);
+                for (int c = 0; c < 32; c += 16) {
+                    uint32_t w[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        float x = fmaf(__uint_as_float(s[c + 2 * i]), scale, bias), y = fmaf(__uint_as_float(s[c + 2 * i + 1]), scale, bias);
+                        if (masked) {  // ahead of the sigmoid, whose pairs share a reciprocal: nothing of a key that is not seen gets through
+                            const int j = key0 + half * 32 + c + 2 * i;
+                            x = live && j >= lo && j <= mine ? x : -INFINITY, y = live && j + 1 >= lo && j + 1 <= mine ? y : -INFINITY;
+                        }
+                        w[i] = scaled_sigmoids_log2(x, y);
+                    }
+                    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + t * kBN + half * 32 + c), "r"(w[0]), "r"(w[1]),
+                                 "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                                 : "memory");
                 }
             }
-            named_bar_sync(1, kRowThreads);  // the staging buffer has been read
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(out_s + sw_off(tid, c, 0)), "r"(w[4 * c]), "r"(w[4 * c + 1]),
-                             "r"(w[4 * c + 2]), "r"(w[4 * c + 3])
-                             : "memory");
-            }
-            named_bar_sync(1, kRowThreads);
-#pragma unroll
-            for (int r = 0; r < kBM * 8 / kRowThreads; ++r) {
-                const int c = tid + r * kRowThreads, row = c >> 3, chunk = c & 7;
-                uint4     v;
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(out_s + sw_off(row, chunk, 0)));
-                *reinterpret_cast<uint4*>(out + (size_t)row * p.ldk + t * kBN + chunk * 8) = v;
+            if (t + 2 < ti.n_tiles) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                fence_async_shared();
+                tcgen05_before_sync();  // the accumulator, which tile t + 2 takes, has been read
+                mbar_arrive(&bars->kv_full[group]);
             }
         }
     }
     else {
         const uint32_t idesc = umma_idesc_bf16(kBM, kBN);  // the products: one elected lane of the warp
+        bool           ok    = mbar_wait_warp(&bars->q_full, 0, p.max_wait);
         for (int t = 0; t < ti.n_tiles; ++t) {
-            if (!mbar_wait_warp(&bars->kv_full[t & 1], (t >> 1) & 1, p.max_wait)) {
+            ok = ok && mbar_wait_warp(&bars->kv_full[t & 1], (t >> 1) & 1, p.max_wait);
+            if (!ok) {
                 if ((tid & 31) == 0) atomicOr(p.status, kStatusGemmPipeWait);
                 break;
             }
@@ -219,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_scores_kernel(const ChunkTc
     }
     tcgen05_before_sync();
     __syncthreads();
-    if (warp == 4) tmem_free(tmem, 2 * kBN);
+    if (warp == 8) tmem_free(tmem, 2 * kBN);
 }
 
 // ------------------------------------------------------------------------------------------------ mixing across heads
@@ -241,12 +246,12 @@ __global__ void __launch_bounds__(256, HB <= 2 ? 2 : 1) chunk_mix_kernel(const C
     const ChunkAttention& a = p.a;
     const int             warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3, H = a.heads;
     const int             row = blockIdx.x * (8 / kMixSplit) + warp / kMixSplit;
-    const TileInfo        ti = tile_info(p, blockIdx.y);
+    const TileInfo        ti = tile_info(p, item_of_block());
     if (!ti.sp.live || row >= ti.rows) return;
     const int       pos = ti.pos0 + row, seg0 = (chunk_first(pos, a.chunk) - ti.base) / 64, seg1 = (pos - ti.base) / 64;  // beyond: zeros
     const __half*   talk = static_cast<const __half*>(a.talk_half);
     const size_t    head = (size_t)kBM * p.ldk;
-    __half*         w    = p.weights + (size_t)blockIdx.y * H * head + (size_t)row * p.ldk;
+    __half*         w    = p.weights + (size_t)item_of_block() * H * head + (size_t)row * p.ldk;
     uint32_t        tf[HB][HB][4];
 #pragma unroll
     for (int m = 0; m < HB; ++m) {
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_values_kernel(const ChunkTc
     pdl_launch_dependents();
     const ChunkAttention& a = p.a;
     const int             tid = threadIdx.x, warp = tid >> 5, h = blockIdx.x, g = h / (a.heads / a.kv_heads);
-    const TileInfo        ti = tile_info(p, blockIdx.y);
+    const TileInfo        ti = tile_info(p, item_of_block());
     if (!ti.sp.live || ti.rows <= 0) return;
     const uint32_t raw = smem_u32(smem_dyn), base = (raw + 1023u) & ~1023u;
     ValueBars*     bars = reinterpret_cast<ValueBars*>(smem_dyn + (base - raw) + kStages * L::kStage);
@@ -339,14 +344,14 @@ __global__ void __launch_bounds__(kThreads, 2) chunk_values_kernel(const ChunkTc
 
     if (warp < 4) {
         const E* vals    = reinterpret_cast<const E*>(ti.sp.slab + a.v_off) + (size_t)g * a.ring * a.vdim;
-        const E* weights = reinterpret_cast<const E*>(p.weights) + ((size_t)blockIdx.y * a.heads + h) * kBM * p.ldk;
+        const E* weights = reinterpret_cast<const E*>(p.weights) + ((size_t)item_of_block() * a.heads + h) * kBM * p.ldk;
         bool     ok      = true;
         auto load = [&](int t) {
             if (t < ti.n_tiles) {
                 const uint32_t dst  = base + (t % kStages) * L::kStage;
                 const int      key0 = ti.base + t * kBN;
-                copy_rows<kBM, kBN>(dst, 0, weights + t * kBN, p.ldk, kBM, kBN);
-                copy_rows<kBN, DV>(dst + L::kP, kTBlock, vals + (size_t)(key0 % a.ring) * a.vdim, a.vdim, min(kBN, ti.pos1 + 1 - key0), a.vdim);
+                copy_rows<kBM, kBN>(tid, dst, 0, weights + t * kBN, p.ldk, kBM, kBN);
+                copy_rows<kBN, DV>(tid, dst + L::kP, kTBlock, vals + (size_t)(key0 % a.ring) * a.vdim, a.vdim, min(kBN, ti.pos1 + 1 - key0), a.vdim);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -453,8 +458,8 @@ int chunk_attention_tc(tm_handle* h, const ChunkAttention& a, const MixerCall& c
     for (; p.tile0 < c.tile_count; p.tile0 += per) {
         const int  items = std::min(per, c.tile_count - p.tile0), hb = talk_pad(a.heads) / 16;
         const dim3 grid(a.heads, items), rows(kBM * kMixSplit / 8, items);
-        cudaError_t e = a.dim <= 64 ? launch_kernel(chunk_scores_kernel<64>, grid, dim3(kThreads), ScoreLayout<64>::kSmem, st, c.pdl, p) :
-                                      launch_kernel(chunk_scores_kernel<128>, grid, dim3(kThreads), ScoreLayout<128>::kSmem, st, c.pdl, p);
+        cudaError_t e = a.dim <= 64 ? launch_kernel(chunk_scores_kernel<64>, grid, dim3(kScoreThreads), ScoreLayout<64>::kSmem, st, c.pdl, p) :
+                                      launch_kernel(chunk_scores_kernel<128>, grid, dim3(kScoreThreads), ScoreLayout<128>::kSmem, st, c.pdl, p);
         if (e == cudaSuccess) {
             const auto mix = hb == 1 ? chunk_mix_kernel<1> : hb == 2 ? chunk_mix_kernel<2> : hb == 3 ? chunk_mix_kernel<3> : chunk_mix_kernel<4>;
             e              = launch_kernel(mix, rows, dim3(256), 0, st, c.pdl, p);
