@@ -76,6 +76,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
 
     // a caller's workspace has the size that tm_gemm_s4_f16_workspace_bytes gave: the small-token kernels' up to 16 tokens
     ScratchUse use(h, (cudaStream_t)stream);
+    const bool early = g_pdl != 0 || h->pdl_direct != 0, pdl = early || use.dependent();  // early: the weights are written by no kernel ahead
     const bool tc = workspace ? n >= (h->gemm_tc_min_n >= 0 ? h->gemm_tc_min_n : 17) : gemm_uses_tc(h, m, n, k);
     // Products of whole tiles need no scratch.  That a weight is expanded into it, or tiles are cut only for balance, is for calls that
     // are in order with all others that use the handle's.
@@ -86,7 +87,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             GemmTcParams p{};
             p.C = (__half*)C, p.A = (const unsigned char*)A, p.X = (const unsigned char*)B, p.Q = (const unsigned char*)Q;
             p.N = m, p.T = n, p.K = k, p.fused_silu = type == TM_GEMM_FUSED_SILU_FFN;
-            return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
+            return gemm_expanded_launch(h, p, columns, (cudaStream_t)stream, pdl);
         }
     }
     if (tc) {
@@ -131,7 +132,8 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
                 if (per != n || workspace || (g_gemm_fusion->ssq_out && !gemm_tc_all_tiles_split(pl, k))) return TM_ERR_UNSUPPORTED;
                 p.norm = *g_gemm_fusion;
             }
-            cudaError_t e = gemm_tc_launch(pl, p, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
+            p.late_weight = !early;
+            cudaError_t e = gemm_tc_launch(pl, p, (cudaStream_t)stream, pdl);
             h->launches += 1;
             if (e != cudaSuccess) {
                 h->last_cuda_error = (int)e;
@@ -189,7 +191,8 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             p.norm = *g_gemm_fusion;
         }
 
-        cudaError_t e = gemm_small_launch(pl, p, (cudaStream_t)stream, g_pdl != 0 || h->pdl_direct != 0);
+        p.late_weight = !early;
+        cudaError_t e = gemm_small_launch(pl, p, (cudaStream_t)stream, pdl);
         h->launches += 1;
         if (e != cudaSuccess) {
             h->last_cuda_error = (int)e;

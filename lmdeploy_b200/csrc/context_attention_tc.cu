@@ -18,6 +18,7 @@
 // Every barrier wait is bounded; on expiry a status bit is recorded and the CTA drains and leaves.
 #include "common.cuh"
 #include "context_attention.h"
+#include "handle.h"
 #include "tm_b200.h"
 
 namespace tmb {
@@ -443,7 +444,7 @@ cudaError_t context_attention_tc_launch(const CtxParams& p, bool int8, int batch
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     const dim3 grid((p.max_q_len + kBM - 1) / kBM, p.H, batch);
-    return launch_kernel(kernel, grid, dim3(kThreads), kSmemBytes, st, false, p);
+    return launch_kernel(kernel, grid, dim3(kThreads), kSmemBytes, st, g_pdl != 0, p);
 }
 
 }  // namespace tmb

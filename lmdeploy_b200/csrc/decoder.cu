@@ -954,21 +954,22 @@ extern "C" int tm_moe(tm_handle* h, const tm_moe_params* q, void* stream)
     m.ranks = (int*)(base + ranks), m.sorted = base + sorted, m.ld = q->input_ld;
     const MoeRouter r{q->experts, q->identity, q->top, q->groups, q->keep, q->correction};
     if (cudaMemsetAsync(m.counts, 0, (size_t)q->experts * 4, s) != cudaSuccess) return TM_ERR_CUDA;
-    int rc = moe_dispatch(h, r, m, q->logits, q->logits_ld, q->input, q->tokens, q->width, f32, s, false);
+    const bool pdl = ScratchUse(h, s).dependent();
+    int rc = moe_dispatch(h, r, m, q->logits, q->logits_ld, q->input, q->tokens, q->width, f32, s, pdl);
     if (rc != TM_OK) return rc;
     DenseGemm u;
     u.w = q->w_experts, u.ldw = q->input_ld, u.x = m.sorted, u.ldx = m.ld, u.tokens = (int)rows, u.n_out = 2 * q->ff, u.k = q->width;
     u.groups.count = q->experts, u.groups.offsets = m.offsets;
     u.ep.kind = DenseKind::kInput, u.ep.act = base + act, u.ep.act_ld = act_ld;
     u.ep.activation = DenseActivation::kClampedSwish, u.ep.limit = q->limit, u.ep.slope = q->slope;
-    if ((rc = dense_gemm(h, u, f32, s, false)) != TM_OK) return rc;
+    if ((rc = dense_gemm(h, u, f32, s, pdl)) != TM_OK) return rc;
     DenseGemm d;
     d.w = q->w_down, d.ldw = act_ld, d.x = base + act, d.ldx = act_ld, d.tokens = (int)rows, d.n_out = q->width, d.k = q->ff, d.groups = u.groups;
     d.ep.kind = DenseKind::kStore, d.ep.out = base + out, d.ep.out_ld = q->width;
-    if ((rc = dense_gemm(h, d, f32, s, false)) != TM_OK) return rc;
+    if ((rc = dense_gemm(h, d, f32, s, pdl)) != TM_OK) return rc;
     RowsCall c;
     c.x = q->x, c.tokens = q->tokens, c.width = q->width, c.expert_rows = base + out, c.input = q->input, c.input_ld = q->input_ld, c.slots = m.slots;
     c.weights = m.weights, c.top = q->top, c.gate = q->gate, c.gate_ld = q->gate_ld, c.gate_bias = q->gate_bias, c.mult = q->mult;
     c.weight_a = q->norm_weight, c.out_a = q->norm_weight ? q->norm_out : nullptr, c.out_ld = q->input_ld, c.eps = q->norm_eps;
-    return norm_rows(h, c, f32, s, false);
+    return norm_rows(h, c, f32, s, pdl);
 }

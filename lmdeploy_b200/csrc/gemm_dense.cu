@@ -841,7 +841,7 @@ int dense_tc(tm_handle* h, const DenseGemm& g, cudaStream_t st, bool pdl, bool h
     p.column_tiles     = (g.n_out + kDenseTile - 1) / kDenseTile;
     p.half_box         = plan.token_tile / 2 / 16 * 16;
     p.band             = kBand;
-    p.late_weight      = half;
+    p.late_weight      = half || g.late_weight;
     p.token_tile    = plan.token_tile;
     p.token_tiles   = (g.tokens + p.token_tile - 1) / p.token_tile;
     p.tiles         = (plan.pair ? (p.column_tiles + 1) / 2 : p.column_tiles) * p.token_tiles;
@@ -942,5 +942,6 @@ extern "C" int tm_gemm_dense(tm_handle* h, void* out, int out_ld, int out_f32, c
     g.w = w, g.x = x, g.ldw = w_ld, g.ldx = x_ld, g.tokens = tokens, g.n_out = n_out, g.k = k;
     g.ep.kind = out_f32 ? DenseKind::kF32 : DenseKind::kStore;
     g.ep.out = out, g.ep.out_ld = out_ld;
-    return dense_gemm(h, g, dtype == TM_DTYPE_F32, (cudaStream_t)stream, false);
+    g.late_weight = true;
+    return dense_gemm(h, g, dtype == TM_DTYPE_F32, (cudaStream_t)stream, ScratchUse(h, (cudaStream_t)stream).dependent());
 }

@@ -71,6 +71,7 @@ struct DenseGemm {
     const void* x = nullptr;  // [tokens][ldx]
     int         ldw = 0, ldx = 0;
     int         tokens = 0, n_out = 0, k = 0;
+    bool        late_weight = false;  // the kernel ahead may write the weight
     // output columns from x2_from on (a multiple of kDenseTile; 0: none) are products with x2 instead, rows as far apart as x's
     const void* x2      = nullptr;
     int         x2_from = 0;

@@ -587,6 +587,7 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
         i_q += (size_t)warps * p.N * 4;
     };
     // the packed weight is written by no kernel: its first copies start ahead of the wait for the kernel before
+    if (p.late_weight) pdl_wait();
     int issued = 0;
     for (; issued < ST && issued < n_groups; ++issued) issue_group(issued);
     pdl_wait();

@@ -348,6 +348,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 mbar_init(&bars->w_empty[s], kDqWarps / 2);
             }
             fence_mbar_init();
+            if (p.late_weight) pdl_wait();
             w_load(w_js, w_g, 0);
         }
         __syncwarp();

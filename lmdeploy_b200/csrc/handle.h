@@ -56,10 +56,14 @@ int lm_head_launch(float* logits, int ld, const __half* x, const __half* w, int 
 struct KernelPreparation {
     explicit KernelPreparation(cudaError_t (*fn)(int max_smem));
 };
-// Set by the decode driver around its launches (per host thread): the kernel launches made through
-// the C ABI on this thread carry the programmatic-dependent-launch attribute.  Off for direct callers,
-// who may put any kernel in front of ours.
+// Set by the drivers around their launches (per host thread): the kernel launches made through the C ABI on this thread carry the
+// programmatic-dependent-launch attribute, and read weights before the kernel ahead is complete.  Direct callers may put any kernel
+// in front of ours: ScratchUse::dependent.
 extern thread_local int g_pdl;
+struct PdlScope {
+    explicit PdlScope(int on) { g_pdl = on; }
+    ~PdlScope() { g_pdl = 0; }
+};
 
 // Held by a call around the launches that use the handle's scratch and tickets.  Calls of one stream are in order by themselves; a
 // call on another stream than the last one waits for it on the device.  A captured call is not ordered against others (its graph runs
@@ -72,6 +76,9 @@ public:
     ScratchUse& operator=(const ScratchUse&) = delete;
     bool in_order() { return nested_ || !captured(); }
     bool begin(ScratchArea area);  // ahead of the first launch; false: a CUDA call failed
+    // A direct call's kernels carry the attribute too, but wait for the kernel ahead before they read anything (late_weight): what
+    // they gain is its way out and their own launch (a plain launch of a 6 us kernel takes 8.2 us).  Not into a caller's capture.
+    bool dependent() { return h_->pdl != 0 && in_order(); }
     bool hold();                   // all areas, for every call of this host thread on the handle until this object ends
 
 private:

@@ -160,10 +160,7 @@ int run_step(StepCtx& c)
     LlamaLinear                  linear(m.h);
     const unsigned long long     l0 = m.h->launches;
     // kernels of this step overlap their prologues with the tail of the kernel before them
-    struct PdlScope {
-        explicit PdlScope(int on) { g_pdl = on; }
-        ~PdlScope() { g_pdl = 0; }
-    } pdl_scope(m.h->pdl);
+    PdlScope pdl_scope(m.h->pdl);
 
     prepare_step_kernel<<<B, 64, 0, s>>>(st.step, st.start_step, st.forced_ids, m.picked, m.ids_in, m.inactive, B, st.max_steps,
                                          cfg.vocab_size, st.sequence_lengths, m.order, m.seq_desc, st.k_cache_ptrs, st.v_cache_ptrs,

@@ -13,6 +13,7 @@
 // one CTA owns a token, computes its 64 (cos, sin) pairs once and applies them to all heads.
 // The transpose reads a cached row once and writes it to every query head of its group.
 #include "common.cuh"
+#include "handle.h"
 #include "mmha.h"
 
 namespace tmb {
@@ -285,7 +286,7 @@ extern "C" int tm_add_fused_qkv_bias_transpose(void* q_buf, void* k_buf, void* v
                 history_length, input_length, batch_size, seq_len, head_num, kv_head_num, rotary_embedding_dim, rotary_embedding_base,
                 max_position_embeddings, use_dynamic_ntk, use_logn_attn};
     const dim3 grid(token_num);
-    return status_of(launch_kernel(qkv_bias_rope_transpose_kernel, grid, dim3(kQkvThreads), 0, (cudaStream_t)stream, false, p));
+    return status_of(launch_kernel(qkv_bias_rope_transpose_kernel, grid, dim3(kQkvThreads), 0, (cudaStream_t)stream, g_pdl != 0, p));
 }
 
 extern "C" int tm_extend_kv_cache(void** k_dst, void** v_dst, size_t dst_offset, const void* k_src, const void* v_src,
@@ -308,8 +309,8 @@ extern "C" int tm_extend_kv_cache(void** k_dst, void** v_dst, size_t dst_offset,
     p.max_len = max_q_len, p.max_seq_len = max_seq_len, p.Hkv = local_head_num, p.n_rep = 1;
     if (int8) p.k_scale = kv_scale[0], p.k_zp = kv_scale[1], p.v_scale = kv_scale[2], p.v_zp = kv_scale[3];
     const dim3 grid((max_q_len * kVecPerHead + kCacheThreads - 1) / kCacheThreads, local_batch_size, 2 * local_head_num);
-    return status_of(int8 ? launch_kernel(extend_kv_cache_kernel<true>, grid, dim3(kCacheThreads), 0, (cudaStream_t)stream, false, p) :
-                            launch_kernel(extend_kv_cache_kernel<false>, grid, dim3(kCacheThreads), 0, (cudaStream_t)stream, false, p));
+    return status_of(int8 ? launch_kernel(extend_kv_cache_kernel<true>, grid, dim3(kCacheThreads), 0, (cudaStream_t)stream, g_pdl != 0, p) :
+                            launch_kernel(extend_kv_cache_kernel<false>, grid, dim3(kCacheThreads), 0, (cudaStream_t)stream, g_pdl != 0, p));
 }
 
 extern "C" int tm_transpose_kv_cache(void* key_cache_trans, void* val_cache_trans, const void** key_cache, const void** val_cache,

@@ -138,3 +138,42 @@ def test_tensor_core_tiles_at_their_edges(n, k, tokens, silu):
         slack = 2 * (1.1 * slack[:, 0::2] * up.abs() + torch.nn.functional.silu(gate).abs() * slack[:, 1::2]) + y.abs() * 2.0 ** -11 + 1e-6
     over = ((buf[:tokens].double() - y).abs() / slack).max().item()
     assert over <= 1.0, f"{over:.2f} of the bound"
+
+
+@pytest.mark.parametrize("n,k,tokens", [(4096, 4096, 1), (4096, 11008, 8), (22016, 4096, 4), (12288, 4096, 40), (22016, 4096, 300)])
+def test_a_weight_written_by_the_kernel_ahead(n, k, tokens):
+    """Direct calls are dependent launches: the packed weight, its scales and the tokens that the kernel just ahead of the call writes
+    are the ones it multiplies."""
+    from lmdeploy_b200 import turbomind as tm
+    from perf import cases
+    sides = [cases._linear(cases._gen(s, n), n, k) for s in (1, 2)]
+    xs = [torch.randn(tokens, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(s)).half() for s in (1, 2)]
+    op = tm.LlamaLinear(0)
+    want = []
+    for w, x in zip(sides, xs):
+        want.append(torch.empty(tokens, n, dtype=torch.float16, device="cuda"))
+        op.forward(want[-1], x, tokens, w, op.kGemm)
+    live = tm.LlamaDenseWeight(k, n, sides[0].kernel.clone(), tm.WeightType.kINT4, None, sides[0].scales_and_zeros.clone(), 128)
+    x, outs = xs[0].clone(), torch.zeros(16, tokens, n, dtype=torch.float16, device="cuda")
+    for i in range(16):
+        x.copy_(xs[i % 2])
+        live.scales_and_zeros.copy_(sides[i % 2].scales_and_zeros)
+        live.kernel.copy_(sides[i % 2].kernel)
+        op.forward(outs[i], x, tokens, live, op.kGemm)
+    for i in range(16):
+        assert torch.equal(outs[i], want[i % 2]), i
+
+
+@pytest.mark.parametrize("tokens", [1, 200])
+def test_a_dense_weight_written_by_the_kernel_ahead(tokens):
+    from lmdeploy_b200 import lib as l
+    n, k, h = 4096, 4096, l.default_handle(0)
+    ws, x = [torch.randn(n, k, device="cuda").bfloat16() for _ in range(2)], torch.randn(tokens, k, device="cuda").bfloat16()
+    live, outs = torch.empty_like(ws[0]), torch.zeros(8, tokens, n, dtype=torch.bfloat16, device="cuda")
+    for i in range(8):
+        live.copy_(ws[i % 2])
+        l.check(l.lib.tm_gemm_dense(h.ptr, outs[i].data_ptr(), n, 0, x.data_ptr(), k, live.data_ptr(), k, tokens, n, k, l.TM_DTYPE_BF16,
+                                    torch.cuda.current_stream().cuda_stream), "tm_gemm_dense")
+    for i in range(2, 8):
+        assert torch.equal(outs[i], outs[i % 2])
+    assert not torch.equal(outs[0], outs[1])
