@@ -51,6 +51,10 @@ namespace tmb {
 // lm_head.cu: logits[tokens][ld] (fp32) = x[tokens][hidden] . w[vocab][hidden]^T, fp16 operands, tcgen05
 int lm_head_launch(float* logits, int ld, const __half* x, const __half* w, int tokens, int vocab, int hidden, unsigned* status,
                    long long max_wait_cycles, int max_smem, cudaStream_t st, bool pdl, unsigned long long* launches);
+// prefill.cu: q (rotated) to [batch][heads][seq_len][128], k (rotated) and v to their cache rows, as the two public writers do one after the other
+int prefill_write_qkv(void* q_buf, const void* qkv, const void* bias, const int* padding_offset, const int* history, const int* length, int batch,
+                      int seq_len, int tokens, int heads, int kv_heads, float rope_base, void* const* k_cache, void* const* v_cache,
+                      size_t cache_offset, int max_seq_len, bool int8, const float* kv_scale, cudaStream_t st);
 // A kernel file's per-device attributes (shared-memory limits and the like), set whenever a handle is created: one static
 // object of this type per file, so that a handle knows no kernel by name.
 struct KernelPreparation {

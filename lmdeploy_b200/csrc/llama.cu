@@ -424,8 +424,8 @@ tm_llama::~tm_llama()
         if (p) cudaFree(p);
     }
     for (void* p : owned) cudaFree(p);
-    for (void* p : {(void*)prefill_buf.x, (void*)prefill_buf.h, (void*)prefill_buf.qkv, (void*)prefill_buf.q, (void*)prefill_buf.k,
-                    (void*)prefill_buf.v, (void*)prefill_buf.ctx, (void*)prefill_buf.ffn, (void*)prefill_buf.pad, (void*)prefill_buf.len,
+    for (void* p : {(void*)prefill_buf.x, (void*)prefill_buf.h, (void*)prefill_buf.qkv, (void*)prefill_buf.q,
+                    (void*)prefill_buf.ctx, (void*)prefill_buf.ffn, (void*)prefill_buf.pad, (void*)prefill_buf.len,
                     prefill_buf.staged}) {
         if (p) cudaFree(p);
     }

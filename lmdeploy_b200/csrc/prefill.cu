@@ -25,6 +25,21 @@ constexpr int kHeadsPerCta  = 16;
 constexpr int kQkvThreads   = kHeadsPerCta * kVecPerHead;  // 256
 constexpr int kCacheThreads = 256;
 
+// llama_kernels.cu:318-341: (x - zp) / scale, round to nearest even, saturate to int8
+__device__ __forceinline__ uint32_t quant4(__half2 a, __half2 b, float scale, float zp)
+{
+    const float2 fa = __half22float2(a), fb = __half22float2(b);
+    int          q[4];
+    q[0] = __float2int_rn(__fdiv_rn(fa.x - zp, scale));
+    q[1] = __float2int_rn(__fdiv_rn(fa.y - zp, scale));
+    q[2] = __float2int_rn(__fdiv_rn(fb.x - zp, scale));
+    q[3] = __float2int_rn(__fdiv_rn(fb.y - zp, scale));
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w |= (uint32_t)(uint8_t)(int8_t)max(-128, min(127, q[i])) << (8 * i);
+    return w;
+}
+
 struct QkvParams {
     __half*       q_buf;
     __half*       k_buf;
@@ -41,12 +56,22 @@ struct QkvParams {
     int           max_pos;
     int           use_dynamic_ntk;
     int           use_logn;
+    // keys and values straight to their cache rows instead of k_buf and v_buf
+    void* const*  k_cache;
+    void* const*  v_cache;
+    size_t        cache_offset;  // elements
+    int           max_seq_len;
+    float         k_scale, k_zp, v_scale, v_zp;
 };
+enum class KvTarget { kBuffers, kCache, kCacheInt8 };
 
 constexpr int kHeadBatch = 4;  // 16-byte loads a thread keeps in flight: 4 x 16 heads per pass
 
 // grid (token_num); thread = (head within a group of 16, 16-byte vector of the head); the CTA walks all
-// H + 2 Hkv heads of its token in passes of 64, so the token's angles are computed once
+// H + 2 Hkv heads of its token in passes of 64, so the token's angles are computed once.  The prefill driver has the keys and values
+// written where the attention reads them: through buffers and extend_kv_cache_kernel they cross memory three times (per layer, 8 x
+// 2048 tokens: 200 + 102 us, 3 sessions of 735 tokens 11.2 + 8.2).
+template<KvTarget TARGET>
 __global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(QkvParams p)
 {
     __shared__ float2 coef[kD / 2];  // (cos, sin) of pair i = elements 2i, 2i + 1
@@ -133,8 +158,22 @@ __global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(Qk
             else {
                 const bool is_k = head < p.H + p.Hkv;
                 const int  kvh  = head - p.H - (is_k ? 0 : p.Hkv);
-                __half*    dst  = is_k ? p.k_buf : p.v_buf;
-                *reinterpret_cast<uint4*>(dst + (((size_t)bi * p.Hkv + kvh) * p.seq_len + si) * kD + vec * 8) = x[j];
+                if (TARGET == KvTarget::kBuffers) {
+                    __half* dst = is_k ? p.k_buf : p.v_buf;
+                    *reinterpret_cast<uint4*>(dst + (((size_t)bi * p.Hkv + kvh) * p.seq_len + si) * kD + vec * 8) = x[j];
+                }
+                else if (si < p.input_length[bi] && step < p.max_seq_len) {  // never past the rows a cache head holds
+                    const size_t at   = p.cache_offset + ((size_t)kvh * p.max_seq_len + step) * kD + vec * 8;
+                    void*        base = (is_k ? p.k_cache : p.v_cache)[bi];
+                    if (TARGET == KvTarget::kCacheInt8) {
+                        const float scale = is_k ? p.k_scale : p.v_scale, zp = is_k ? p.k_zp : p.v_zp;
+                        *reinterpret_cast<uint2*>(static_cast<int8_t*>(base) + at) =
+                            make_uint2(quant4(xh[0], xh[1], scale, zp), quant4(xh[2], xh[3], scale, zp));
+                    }
+                    else {
+                        *reinterpret_cast<uint4*>(static_cast<__half*>(base) + at) = x[j];
+                    }
+                }
             }
         }
     }
@@ -142,21 +181,6 @@ __global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(Qk
 
 // ------------------------------------------------------------------------------------------------
 // cache writers / readers.  One thread = 8 consecutive elements of one cache row.
-
-// llama_kernels.cu:318-341: (x - zp) / scale, round to nearest even, saturate to int8
-__device__ __forceinline__ uint32_t quant4(__half2 a, __half2 b, float scale, float zp)
-{
-    const float2 fa = __half22float2(a), fb = __half22float2(b);
-    int          q[4];
-    q[0] = __float2int_rn(__fdiv_rn(fa.x - zp, scale));
-    q[1] = __float2int_rn(__fdiv_rn(fa.y - zp, scale));
-    q[2] = __float2int_rn(__fdiv_rn(fb.x - zp, scale));
-    q[3] = __float2int_rn(__fdiv_rn(fb.y - zp, scale));
-    uint32_t w = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w |= (uint32_t)(uint8_t)(int8_t)max(-128, min(127, q[i])) << (8 * i);
-    return w;
-}
 
 // llama_kernels.cu:309-316: q * scale + zp in fp32 (one fused multiply-add), rounded to fp16
 __device__ __forceinline__ uint2 dequant4(uint32_t w, float scale, float zp)
@@ -286,7 +310,23 @@ extern "C" int tm_add_fused_qkv_bias_transpose(void* q_buf, void* k_buf, void* v
                 history_length, input_length, batch_size, seq_len, head_num, kv_head_num, rotary_embedding_dim, rotary_embedding_base,
                 max_position_embeddings, use_dynamic_ntk, use_logn_attn};
     const dim3 grid(token_num);
-    return status_of(launch_kernel(qkv_bias_rope_transpose_kernel, grid, dim3(kQkvThreads), 0, (cudaStream_t)stream, g_pdl != 0, p));
+    return status_of(launch_kernel(qkv_bias_rope_transpose_kernel<KvTarget::kBuffers>, grid, dim3(kQkvThreads), 0, (cudaStream_t)stream, g_pdl != 0, p));
+}
+
+int tmb::prefill_write_qkv(void* q_buf, const void* qkv, const void* bias, const int* padding_offset, const int* history, const int* length,
+                           int batch, int seq_len, int tokens, int heads, int kv_heads, float rope_base, void* const* k_cache, void* const* v_cache,
+                           size_t cache_offset, int max_seq_len, bool int8, const float* kv_scale, cudaStream_t st)
+{
+    if (!aligned16({q_buf, qkv, bias}) || cache_offset % 16) return TM_ERR_INVALID_ARG;
+    if (batch > 65535 || 2 * kv_heads > 65535) return TM_ERR_UNSUPPORTED;  // as tm_extend_kv_cache
+    QkvParams p{};
+    p.q_buf = (__half*)q_buf, p.qkv = (const __half*)qkv, p.bias = (const __half*)bias;
+    p.padding_offset = padding_offset, p.history_length = history, p.input_length = length;
+    p.batch = batch, p.seq_len = seq_len, p.H = heads, p.Hkv = kv_heads, p.rot_dim = kD, p.rope_base = rope_base, p.max_pos = max_seq_len;
+    p.k_cache = k_cache, p.v_cache = v_cache, p.cache_offset = cache_offset, p.max_seq_len = max_seq_len;
+    p.k_scale = kv_scale[0], p.k_zp = kv_scale[1], p.v_scale = kv_scale[2], p.v_zp = kv_scale[3];
+    return status_of(launch_kernel(int8 ? qkv_bias_rope_transpose_kernel<KvTarget::kCacheInt8> : qkv_bias_rope_transpose_kernel<KvTarget::kCache>,
+                                   dim3(tokens), dim3(kQkvThreads), 0, st, g_pdl != 0, p));
 }
 
 extern "C" int tm_extend_kv_cache(void** k_dst, void** v_dst, size_t dst_offset, const void* k_src, const void* v_src,

@@ -84,8 +84,6 @@ extern "C" int tm_llama_prefill(tm_llama* m, const tm_llama_prefill_state* st, v
     bool ok = grow(m, (void**)&pb.x, &pb.x_bytes, T * hid * 2) && grow(m, (void**)&pb.h, &pb.h_bytes, T * hid * 2)
               && grow(m, (void**)&pb.qkv, &pb.qkv_bytes, T * qkv_cols * 2)
               && grow(m, (void**)&pb.q, &pb.q_bytes, (size_t)B * H * S * 128 * 2)
-              && grow(m, (void**)&pb.k, &pb.k_bytes, (size_t)B * Hkv * S * 128 * 2)
-              && grow(m, (void**)&pb.v, &pb.v_bytes, (size_t)B * Hkv * S * 128 * 2)
               && grow(m, (void**)&pb.ctx, &pb.ctx_bytes, (size_t)T * H * 128 * 2)
               && grow(m, (void**)&pb.ffn, &pb.ffn_bytes, (size_t)T * m->local_inter * 2)
               && grow(m, (void**)&pb.pad, &pb.pad_bytes, (size_t)T * 4) && grow(m, (void**)&pb.len, &pb.len_bytes, (size_t)B * 4);
@@ -114,13 +112,9 @@ extern "C" int tm_llama_prefill(tm_llama* m, const tm_llama_prefill_state* st, v
         const size_t layer_offset = (size_t)l * Hkv * cfg.session_len * 128;  // LlamaContextAttentionLayer.cc:185
         // ---- LlamaContextAttentionLayer.cc:155-238
         if (!step(linear.forward(pb.qkv, pb.h, T, w.qkv, LlamaLinear::kGemm, s))) break;
-        if (!step(tm_add_fused_qkv_bias_transpose(pb.q, pb.k, pb.v, pb.qkv, w.qkv.bias, pb.pad, st->history_lengths, pb.len, B, S, T,
-                                                  H, Hkv, cfg.size_per_head, cfg.size_per_head, cfg.rope_theta, cfg.session_len, 0, 0,
-                                                  s))) {
-            break;
-        }
-        if (!step(tm_extend_kv_cache(st->k_cache_ptrs, st->v_cache_ptrs, layer_offset, pb.k, pb.v, B, pb.len, S, st->history_lengths,
-                                     cfg.session_len, cfg.size_per_head, Hkv, s, cfg.quant_policy, w.past_kv_scale))) {
+        if (!step(prefill_write_qkv(pb.q, pb.qkv, w.qkv.bias, pb.pad, st->history_lengths, pb.len, B, S, T, H, Hkv, cfg.rope_theta,
+                                    st->k_cache_ptrs, st->v_cache_ptrs, layer_offset, cfg.session_len, (cfg.quant_policy & 0x04) != 0,
+                                    w.past_kv_scale, s))) {
             break;
         }
         tm_context_attention_params a{};
