@@ -52,10 +52,12 @@ namespace {
 __global__ void prepare_step_kernel(const int* step, const int* start_step, const int* forced_ids, const int* picked,
                                     int* ids_in, unsigned char* inactive, int B, int max_steps, int vocab, const int* lengths,
                                     int* order, MmhaSeqDesc* desc, void* const* k_ptrs, void* const* v_ptrs, float2* rope_table,
-                                    float rope_base, int rot_dim)
+                                    float rope_base, int rot_dim, unsigned long long* ssq, int ssq_count)
 {
     const int b    = blockIdx.x;
     const int mine = lengths[b];
+    // the step's sums of squares (GemmNormFusion); here, as no operation that is not a kernel stands between dependent launches then
+    for (int i = b * blockDim.x + threadIdx.x; i < ssq_count; i += gridDim.x * blockDim.x) ssq[i] = 0ull;
     // attention launch order: longest cached sequence first (rank by length, ties by index)
     __shared__ int s_rank;
     if (threadIdx.x == 0) {
@@ -162,9 +164,21 @@ int run_step(StepCtx& c)
     // kernels of this step overlap their prologues with the tail of the kernel before them
     PdlScope pdl_scope(m.h->pdl);
 
+    const bool tp_on = m.comm && m.comm->world > 1;
+    // Residual add + RMSNorm folded into the GEMMs on either side (gemm_s4_f16.h, GemmNormFusion): single GPU, a batch that each
+    // projection takes in one launch, and the two producers by kernels that hold whole sums (the column-owner kernel, or the
+    // tensor-core kernel with every tile split).  The first norm of the step and the last one (in front of the lm-head) stay
+    // kernels of their own.
+    const LlamaDecoderLayerWeight& w0 = m.layers[0];
+    auto foldable = [&](const LlamaDenseWeight& w, bool producer) {
+        return gemm_can_fuse_norm(m.h, (int)w.output_dims, B, (int)w.input_dims, producer);
+    };
+    const bool fold = !tp_on && m.h->fold_norm && foldable(w0.qkv, false) && foldable(w0.output, true)
+                      && foldable(w0.fused_gating_intermediate, false) && foldable(w0.ffn_output, true);
+
     prepare_step_kernel<<<B, 64, 0, s>>>(st.step, st.start_step, st.forced_ids, m.picked, m.ids_in, m.inactive, B, st.max_steps,
                                          cfg.vocab_size, st.sequence_lengths, m.order, m.seq_desc, st.k_cache_ptrs, st.v_cache_ptrs,
-                                         m.rope_table, cfg.rope_theta, cfg.size_per_head);
+                                         m.rope_table, cfg.rope_theta, cfg.size_per_head, m.ssq, fold ? 2 * cfg.num_layer * cfg.max_batch_size : 0);
     if (!c.ok_cuda()) return c.rc;
     embedding_lookup_kernel<<<B, 128, 0, s>>>(m.x, (const __half*)m.tok_embeddings, m.ids_in, m.hidden);
     if (!c.ok_cuda()) return c.rc;
@@ -175,7 +189,6 @@ int run_step(StepCtx& c)
 
     // Tensor parallel: the row-split GEMMs write their partial sums into a slot that the peers have mapped, and one
     // kernel sums the ranks, adds the residual and normalises (allreduce.cu); otherwise NCCL + the plain fused norm.
-    const bool tp_on  = m.comm && m.comm->world > 1;
     const bool p2p    = tp_on && m.comm->p2p_ready && m.h->p2p_allreduce && (size_t)B * m.hidden * 2 <= m.comm->p2p_slot_bytes;
     __half*    part_o = p2p ? (__half*)tm_comm_p2p_slot(m.comm, 0) : m.hbuf;
     __half*    part_f = p2p ? (__half*)tm_comm_p2p_slot(m.comm, 1) : m.hbuf;
@@ -196,23 +209,6 @@ int run_step(StepCtx& c)
         return c.ok(tm_add_residual_rmsnorm(m.x, m.hbuf, nullptr, norm_w, cfg.norm_eps, B, m.hidden, s));
     };
 
-    // Residual add + RMSNorm folded into the GEMMs on either side (gemm_s4_f16.h, GemmNormFusion): single GPU, a batch that each
-    // projection takes in one launch, and the two producers by kernels that hold whole sums (the column-owner kernel, or the
-    // tensor-core kernel with every tile split).  The first norm of the step and the last one (in front of the lm-head) stay
-    // kernels of their own.
-    const LlamaDecoderLayerWeight& w0 = m.layers[0];
-    auto foldable = [&](const LlamaDenseWeight& w, bool producer) {
-        return gemm_can_fuse_norm(m.h, (int)w.output_dims, B, (int)w.input_dims, producer);
-    };
-    const bool fold = !tp_on && m.h->fold_norm && foldable(w0.qkv, false) && foldable(w0.output, true)
-                      && foldable(w0.fused_gating_intermediate, false) && foldable(w0.ffn_output, true);
-    if (fold) {
-        if (!c.ok(cudaMemsetAsync(m.ssq, 0, (size_t)2 * cfg.num_layer * cfg.max_batch_size * sizeof(unsigned long long), s) == cudaSuccess ?
-                      TM_OK :
-                      TM_ERR_CUDA)) {
-            return c.rc;
-        }
-    }
     struct FusionScope {
         explicit FusionScope(const GemmNormFusion* f) { g_gemm_fusion = f; }
         ~FusionScope() { g_gemm_fusion = nullptr; }
