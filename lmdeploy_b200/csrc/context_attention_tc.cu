@@ -10,9 +10,12 @@
 //               softmax in the log2 domain with one thread per row (no shuffles), write the probabilities as fp16 into
 //               TMEM (tcgen05.st) where the second product takes them as its A operand, and rescale the output
 //               accumulator only when a row's running maximum moved by more than 2^8 (the accumulator is fp32).
-//   warp 4      allocates TMEM (256 columns: S 64, P 32, O 128); one lane issues S = Q K^T (both operands from shared
-//               memory, M128 x N64 x K16, 8 per tile) and O += P V (A from TMEM, B = the value tile as an MN-major
-//               operand, M128 x N128 x K16, 4 per tile) and commits to mbarriers.
+//   warp 4      allocates TMEM (256 columns: S of two tiles, O 128; a tile's P takes its S's place); one lane issues S = Q K^T (both
+//               operands from shared memory, M128 x N64 x K16, 8 per tile) and O += P V (A from TMEM, B = the value tile as an
+//               MN-major operand, M128 x N128 x K16, 4 per tile) and commits to mbarriers.  The next tile's S is issued ahead of
+//               this one's P V, so that it is computed under the softmax: with one S a tile's two products (576 and 280 cycles) and
+//               its softmax came one after the other (fp16 cache, 8 x 2048 tokens, 32 heads 426 us, 373 so; 64 tokens behind 3000
+//               68 and 57; int8, whose expansion by the same warps bounds it, 587 and 565).
 // Two CTAs are resident per SM (97 KB of shared memory, 256 TMEM columns each), so one CTA's softmax overlaps the
 // other's MMAs.  Tiles above the causal diagonal are never visited; the longest query tiles are scheduled first.
 // Every barrier wait is bounded; on expiry a status bit is recorded and the CTA drains and leaves.
@@ -34,12 +37,13 @@ constexpr int kQBlock   = kBM * 128;           // 16 KB
 constexpr int kTileBytes = kBN * kD * 2;       // 16 KB: two blocks of [64 rows][128 B]
 constexpr int kTBlock   = kBN * 128;           // 8 KB
 constexpr int kTmemCols = 256;
-constexpr int kColS = 0, kColP = 64, kColO = 128;
+constexpr int kColS = 0, kColO = 128;  // two tiles' scores, whose place their probabilities take; the accumulator
 
 struct Bars {
-    uint64_t kv_full[2];  // tile t's keys and values are in shared memory (128 arrivals)
-    uint64_t s_full;      // S of tile t is in TMEM
-    uint64_t p_full;      // P of tile t is in TMEM, O rescaled (128 arrivals)
+    uint64_t k_full[2];   // tile t's keys are in shared memory (128 arrivals)
+    uint64_t s_full[2];   // S of tile t is in TMEM
+    uint64_t p_full;      // P of tile t is in TMEM, its values in shared memory, O rescaled (128 arrivals)
+    uint64_t pv_done;     // P V of tile t is in O
     uint64_t o_full;      // every product is done
     uint32_t tmem_base;
     int      dead;
@@ -184,10 +188,9 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
     Bars*          bars = reinterpret_cast<Bars*>(sm + kQBytes + 4 * kTileBytes);
 
     if (tid == 0) {
-        mbar_init(&bars->kv_full[0], kRowThreads);
-        mbar_init(&bars->kv_full[1], kRowThreads);
-        mbar_init(&bars->s_full, 1);
+        for (int i = 0; i < 2; ++i) mbar_init(&bars->k_full[i], kRowThreads), mbar_init(&bars->s_full[i], 1);
         mbar_init(&bars->p_full, kRowThreads);
+        mbar_init(&bars->pv_done, 1);
         mbar_init(&bars->o_full, 1);
         bars->dead = 0;
         fence_mbar_init();
@@ -207,57 +210,48 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
         const size_t         head_off = p.offset + (size_t)kvh * p.max_seq_len * kD;  // elements
         const unsigned char* k_base   = static_cast<const unsigned char*>(p.k_cache[bi]) + head_off * (INT8 ? 1 : 2);
         const unsigned char* v_base   = static_cast<const unsigned char*>(p.v_cache[bi]) + head_off * (INT8 ? 1 : 2);
-        auto load_tile_f16 = [&](int t, int buf) {
+        // tile t of the keys (which = 0) or the values (1) sits in buffer t & 1; tiles beyond the last one are not there
+        auto load_f16 = [&](int t, int which) {
             const int key0 = t * kBN;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int      c = tid + r * kRowThreads, row = c >> 4, chunk = c & 15;
-                const bool     ok  = key0 + row < kv_end;
-                const size_t   src = ((size_t)(ok ? key0 + row : 0) * kD + chunk * 8) * 2;
-                const uint32_t dst = kv_s + buf * 2 * kTileBytes + sw_off(row, chunk, kTBlock);
-                cp_async16z(dst, k_base + src, ok ? 16 : 0);
-                cp_async16z(dst + kTileBytes, v_base + src, ok ? 16 : 0);
+            for (int r = 0; t < n_tiles && r < 8; ++r) {
+                const int    c = tid + r * kRowThreads, row = c >> 4, chunk = c & 15;
+                const bool   ok  = key0 + row < kv_end;
+                const size_t src = ((size_t)(ok ? key0 + row : 0) * kD + chunk * 8) * 2;
+                cp_async16z(kv_s + (t & 1) * 2 * kTileBytes + which * kTileBytes + sw_off(row, chunk, kTBlock), (which ? v_base : k_base) + src,
+                            ok ? 16 : 0);
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        uint4 stage_k[4], stage_v[4];  // int8 only: the next tile on its way from global to shared memory
-        auto fetch_tile_s8 = [&](int t) {
+        uint4 stage[2][4];  // int8 only: the next tiles on their way from global to shared memory
+        auto  fetch_s8 = [&](int t, int which) {
             const int key0 = t * kBN;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                const int  c = tid + r * kRowThreads, row = c >> 3, chunk = c & 7;
-                const bool ok = key0 + row < kv_end;
-                stage_k[r] = stage_v[r] = make_uint4(0, 0, 0, 0);
-                if (ok) {
-                    const size_t src = (size_t)(key0 + row) * kD + chunk * 16;
-                    stage_k[r]       = *reinterpret_cast<const uint4*>(k_base + src);
-                    stage_v[r]       = *reinterpret_cast<const uint4*>(v_base + src);
-                }
+                const int c = tid + r * kRowThreads, row = c >> 3, chunk = c & 7;
+                stage[which][r] = make_uint4(0, 0, 0, 0);
+                if (key0 + row < kv_end) stage[which][r] = *reinterpret_cast<const uint4*>((which ? v_base : k_base) + (size_t)(key0 + row) * kD + chunk * 16);
             }
         };
-        auto store_tile_s8 = [&](int t, int buf) {
-            const int key0 = t * kBN;
+        auto store_s8 = [&](int t, int which) {
+            const int      key0 = t * kBN;
+            const float    scale = which ? p.v_scale : p.k_scale, zp = which ? p.v_zp : p.k_zp;
+            unsigned char* dst = sm + kQBytes + (t & 1) * 2 * kTileBytes + which * kTileBytes;
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                const int  c = tid + r * kRowThreads, row = c >> 3, chunk = c & 7;
-                const bool ok = key0 + row < kv_end;  // rows past the end stay exact zeros (not the zero point)
-                unsigned char* dst = sm + kQBytes + buf * 2 * kTileBytes;
-                uint4 k0 = make_uint4(0, 0, 0, 0), k1 = k0, v0 = k0, v1 = k0;
-                if (ok) {
-                    const uint2 a = dequant4(stage_k[r].x, p.k_scale, p.k_zp), b = dequant4(stage_k[r].y, p.k_scale, p.k_zp);
-                    const uint2 c2 = dequant4(stage_k[r].z, p.k_scale, p.k_zp), d = dequant4(stage_k[r].w, p.k_scale, p.k_zp);
-                    k0 = make_uint4(a.x, a.y, b.x, b.y), k1 = make_uint4(c2.x, c2.y, d.x, d.y);
-                    const uint2 e = dequant4(stage_v[r].x, p.v_scale, p.v_zp), f = dequant4(stage_v[r].y, p.v_scale, p.v_zp);
-                    const uint2 g2 = dequant4(stage_v[r].z, p.v_scale, p.v_zp), hh = dequant4(stage_v[r].w, p.v_scale, p.v_zp);
-                    v0 = make_uint4(e.x, e.y, f.x, f.y), v1 = make_uint4(g2.x, g2.y, hh.x, hh.y);
+                const int c = tid + r * kRowThreads, row = c >> 3, chunk = c & 7;
+                uint4     lo = make_uint4(0, 0, 0, 0), hi = lo;
+                if (key0 + row < kv_end) {  // rows past the end stay exact zeros (not the zero point)
+                    const uint4 q = stage[which][r];
+                    const uint2 a = dequant4(q.x, scale, zp), b = dequant4(q.y, scale, zp), c2 = dequant4(q.z, scale, zp), d = dequant4(q.w, scale, zp);
+                    lo = make_uint4(a.x, a.y, b.x, b.y), hi = make_uint4(c2.x, c2.y, d.x, d.y);
                 }
-                *reinterpret_cast<uint4*>(dst + sw_off(row, 2 * chunk, kTBlock))                  = k0;
-                *reinterpret_cast<uint4*>(dst + sw_off(row, 2 * chunk + 1, kTBlock))              = k1;
-                *reinterpret_cast<uint4*>(dst + kTileBytes + sw_off(row, 2 * chunk, kTBlock))     = v0;
-                *reinterpret_cast<uint4*>(dst + kTileBytes + sw_off(row, 2 * chunk + 1, kTBlock)) = v1;
+                *reinterpret_cast<uint4*>(dst + sw_off(row, 2 * chunk, kTBlock))     = lo;
+                *reinterpret_cast<uint4*>(dst + sw_off(row, 2 * chunk + 1, kTBlock)) = hi;
             }
         };
 
-        // ---- prologue: the query tile and key / value tile 0
+        // ---- prologue: the query tile, two tiles of keys, one of values
         {
             const __half* qsrc = p.q + ((size_t)bi * p.H + h) * p.max_q_len * kD;
 #pragma unroll
@@ -268,13 +262,20 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
             }
         }
         if (INT8) {
-            fetch_tile_s8(0);
-            store_tile_s8(0, 0);
+            fetch_s8(0, 0);
+            fetch_s8(0, 1);
+            store_s8(0, 0);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            fetch_s8(1, 0);
         }
         else {
-            load_tile_f16(0, 0);
+            load_f16(0, 0);
+            load_f16(1, 0);
+            load_f16(0, 1);
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        fence_async_smem();  // copies and stores of this thread become visible to the tensor core's reads
+        mbar_arrive(&bars->k_full[0]);
 
         const int      qi        = q0 + tid;
         const bool     row_live  = qi < q_len;
@@ -284,32 +285,35 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
         bool           dead = false;
         for (int t = 0; t < n_tiles; ++t) {
             const int buf = t & 1;
-            if (INT8 && t > 0) store_tile_s8(t, buf);  // fetched to registers during the tile before
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            fence_async_smem();  // copies and stores of this thread become visible to the tensor core's reads
-            mbar_arrive(&bars->kv_full[buf]);
+            // int8 values are stored here already: the product on the tile before the last, which had their buffer, is complete
+            if (INT8) store_s8(t, 1);
+            if (t + 1 < n_tiles) {  // the next tile's scores are computed under this one's softmax
+                if (INT8) store_s8(t + 1, 0);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");  // its keys have landed, this one's values may be on their way
+                fence_async_smem();
+                mbar_arrive(&bars->k_full[buf ^ 1]);
+            }
             // the outcome is made uniform across the warp: the TMEM loads and stores below are warp-wide instructions
-            if (!__all_sync(0xffffffffu, mbar_wait(&bars->s_full, t & 1, p.max_wait_cycles))) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&bars->s_full[buf], (t >> 1) & 1, p.max_wait_cycles))) {
                 atomicOr(p.status, kStatusGemmPipeWait);
                 *(volatile int*)&bars->dead = 1;
                 dead = true;
                 break;
             }
             tc_after();
-            // S of this tile is complete, so every product on the tile before it is too: its buffers are free
-            if (t + 1 < n_tiles) {
-                if (INT8) {
-                    fetch_tile_s8(t + 1);
-                }
-                else {
-                    load_tile_f16(t + 1, buf ^ 1);
-                }
+            // S of this tile is complete: its keys' buffer is free
+            if (INT8) {
+                fetch_s8(t + 2, 0);
+                fetch_s8(t + 1, 1);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            else {
+                load_f16(t + 2, 0);
+            }
+            const uint32_t scores = lane_base + kColS + buf * kBN;  // and, once they are read, the probabilities
 
             uint32_t s0[32], s1[32];
-            tmem_ld32(lane_base + kColS, s0);
-            tmem_ld32(lane_base + kColS + 32, s1);
+            tmem_ld32(scores, s0);
+            tmem_ld32(scores + 32, s1);
             const int key0 = t * kBN;
             // raw scores stay as they are; the softmax scale goes into the exponent's multiply-add.  Only tiles that
             // touch the causal diagonal or the end of the keys mask anything (the same for every row of the CTA).
@@ -343,6 +347,14 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
                 pr[16 + i] = pack2(c, d);
             }
             l = l * alpha + sum;
+            // the accumulator and the buffer of the next values are free once the product on the tile before is complete
+            if (t > 0 && !__all_sync(0xffffffffu, mbar_wait(&bars->pv_done, (t - 1) & 1, p.max_wait_cycles))) {
+                atomicOr(p.status, kStatusGemmPipeWait);
+                *(volatile int*)&bars->dead = 1;
+                dead = true;
+                break;
+            }
+            tc_after();
             if (t > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll 1
                 for (int c = 0; c < 4; ++c) {
@@ -353,10 +365,13 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
                     tmem_st32(lane_base + kColO + 32 * c, o);
                 }
             }
-            tmem_st32(lane_base + kColP, pr);
+            tmem_st32(scores, pr);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");  // this tile's values have landed, keys may be on their way
+            fence_async_smem();
             tmem_wait_st();
             tc_before();
             mbar_arrive(&bars->p_full);
+            if (!INT8) load_f16(t + 1, 1);
         }
         // ---- normalise and store: out[token, h * 128 + d]
         if (!dead && !__all_sync(0xffffffffu, mbar_wait(&bars->o_full, 0, p.max_wait_cycles))) {
@@ -390,33 +405,33 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
         const uint32_t idesc_qk = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
         const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(kD >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // B is MN-major
         bool           ok       = true;
-        for (int t = 0; t < n_tiles && ok; ++t) {
+        auto           issue_scores = [&](int t) {
             const int buf = t & 1;
-            if (!mbar_wait_warp(&bars->kv_full[buf], (t >> 1) & 1, p.max_wait_cycles)) {
-                ok = false;
-                break;
-            }
+            if (!mbar_wait_warp(&bars->k_full[buf], (t >> 1) & 1, p.max_wait_cycles)) return false;
             tc_after();
-            const uint32_t k_addr = kv_s + buf * 2 * kTileBytes, v_addr = k_addr + kTileBytes;
             if (elect_one()) {
 #pragma unroll
                 for (int blk = 0; blk < 2; ++blk) {
-                    const uint64_t dq = desc_kmajor(q_s + blk * kQBlock), dk = desc_kmajor(k_addr + blk * kTBlock);
+                    const uint64_t dq = desc_kmajor(q_s + blk * kQBlock), dk = desc_kmajor(kv_s + buf * 2 * kTileBytes + blk * kTBlock);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) umma_ss(tmem + kColS, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
+                    for (int j = 0; j < 4; ++j) umma_ss(tmem + kColS + buf * kBN, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
                 }
-                umma_commit_to(&bars->s_full);
+                umma_commit_to(&bars->s_full[buf]);
             }
             __syncwarp();
-            if (!mbar_wait_warp(&bars->p_full, t & 1, p.max_wait_cycles)) {
-                ok = false;
-                break;
-            }
+            return true;
+        };
+        ok = issue_scores(0);
+        for (int t = 0; t < n_tiles && ok; ++t) {
+            // (the columns that tile t + 1's scores take held tile t - 1's probabilities, whose product was issued before)
+            ok = (t + 1 >= n_tiles || issue_scores(t + 1)) && mbar_wait_warp(&bars->p_full, t & 1, p.max_wait_cycles);
+            if (!ok) break;
             tc_after();
-            const uint64_t dv = desc_mnmajor(v_addr, kTBlock);
+            const uint64_t dv = desc_mnmajor(kv_s + (t & 1) * 2 * kTileBytes + kTileBytes, kTBlock);
             if (elect_one()) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) umma_ts(tmem + kColO, tmem + kColP + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+                for (int j = 0; j < 4; ++j) umma_ts(tmem + kColO, tmem + kColS + (t & 1) * kBN + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
+                umma_commit_to(&bars->pv_done);
             }
             __syncwarp();
         }
