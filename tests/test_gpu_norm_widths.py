@@ -17,8 +17,8 @@ def test_norms(n, m):
     l.check(l.lib.tm_rmsnorm(out.data_ptr(), x.data_ptr(), w.data_ptr(), 1e-6, m, n, s), "norm")
     want = norm(x.double(), x.double())
     assert ((out.double() - want).abs() <= want.abs() * 2.0 ** -10.5 + 2.0 ** -24).all()  # one rounding, and the fp32 factor's
-    sums, res = r.double() + x.double(), r.clone()
+    sums, added, res = r.double() + x.double(), (r.float() + x.float()).half(), r.clone()
     l.check(l.lib.tm_add_residual_rmsnorm(res.data_ptr(), x.data_ptr(), None, w.data_ptr(), 1e-6, m, n, s), "add and norm")
-    assert torch.equal(res, (r.float() + x.float()).half())
+    assert torch.equal(res, added)
     want = norm(res.double(), sums)
     assert ((x.double() - want).abs() <= want.abs() * 2.0 ** -10.5 + 2.0 ** -24).all()
