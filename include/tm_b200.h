@@ -72,7 +72,7 @@ TM_API unsigned long long tm_launch_count(const tm_handle* h);
  * serialization, as the decode driver's do; only where no kernel ahead in the stream writes weights or cached rows),
  * "gemm_wait_cycles" (bound of the tcgen05 GEMM's wait for the partners of a split tile, 0 = default; tests),
  * "fold_norm" (0: the single-GPU decode step keeps residual add + RMSNorm as kernels of their own instead of folding
- * them into the tensor-core GEMMs on either side),
+ * them into the GEMMs on either side),
  * "lm_head_cublas" (1: the decode driver computes the lm-head with cuBLAS, as the reference does, instead of this
  * library's kernel; for comparison),
  * "gemv_cols" (the GEMM for few tokens: 0 = always the stream-K kernel, 1 = the column-owner kernel on 32-column strips where
