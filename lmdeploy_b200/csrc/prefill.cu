@@ -62,75 +62,95 @@ struct QkvParams {
     size_t        cache_offset;  // elements
     int           max_seq_len;
     float         k_scale, k_zp, v_scale, v_zp;
+    int           tokens;
 };
 enum class KvTarget { kBuffers, kCache, kCacheInt8 };
 
 constexpr int kHeadBatch = 4;  // 16-byte loads a thread keeps in flight: 4 x 16 heads per pass
 
-// grid (token_num); thread = (head within a group of 16, 16-byte vector of the head); the CTA walks all
-// H + 2 Hkv heads of its token in passes of 64, so the token's angles are computed once.  The prefill driver has the keys and values
-// written where the attention reads them: through buffers and extend_kv_cache_kernel they cross memory three times (per layer, 8 x
-// 2048 tokens: 200 + 102 us, 3 sessions of 735 tokens 11.2 + 8.2).
-template<KvTarget TARGET>
-__global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(QkvParams p)
+// grid (token_num / TOKENS); thread = (one of 16 rows of a (head, token), 16-byte vector of the head); the CTA walks all H + 2 Hkv heads
+// of its tokens in passes of 64 rows, so a token's angles are computed once.  The prefill driver has the keys and values written where
+// the attention reads them: through buffers and extend_kv_cache_kernel they cross memory three times (per layer, 8 x 2048 tokens:
+// 200 + 102 us, 3 sessions of 735 tokens 11.2 + 8.2).  Bound by the loads that its CTAs keep in flight: four CTAs to an SM, the bias read
+// where it is added and a sequence's cache rows found once (8 x 2048 tokens into fp16 / int8 rows: 139 / 213 us without, 136 / 184).
+template<KvTarget TARGET, int TOKENS>
+__global__ void __launch_bounds__(kQkvThreads, 4) qkv_bias_rope_transpose_kernel(QkvParams p)
 {
-    __shared__ float2 coef[kD / 2];  // (cos, sin) of pair i = elements 2i, 2i + 1
+    constexpr int kHeads = kHeadsPerCta / TOKENS;  // heads of the CTA's 16 rows
+    __shared__ float2 coef[TOKENS][kD / 2];        // (cos, sin) of pair i = elements 2i, 2i + 1
     pdl_wait();
     pdl_launch_dependents();
-    const int token = blockIdx.x;
+    const int slot  = threadIdx.x / kVecPerHead % TOKENS;  // this thread's token among the CTA's
+    const int token = blockIdx.x * TOKENS + slot;
     const int total = p.H + 2 * p.Hkv;
-    const int hsub  = threadIdx.x / kVecPerHead;
+    const int hsub  = threadIdx.x / kVecPerHead / TOKENS;
     const int vec   = threadIdx.x % kVecPerHead;
     const __half* row = p.qkv + (size_t)token * total * kD + vec * 8;
-    uint4 x[kHeadBatch], b[kHeadBatch];
+    const bool    there = TOKENS == 1 || token < p.tokens;
+    uint4 x[kHeadBatch];
     auto  load_pass = [&](int h0) {
 #pragma unroll
         for (int j = 0; j < kHeadBatch; ++j) {
-            const int head = h0 + j * kHeadsPerCta + hsub;
-            x[j] = b[j] = make_uint4(0, 0, 0, 0);
-            if (head < total) {
-                x[j] = *reinterpret_cast<const uint4*>(row + (size_t)head * kD);
-                if (p.bias) b[j] = *reinterpret_cast<const uint4*>(p.bias + (size_t)head * kD + vec * 8);
-            }
+            const int head = h0 + j * kHeads + hsub;
+            x[j] = make_uint4(0, 0, 0, 0);
+            if (there && head < total) x[j] = *reinterpret_cast<const uint4*>(row + (size_t)head * kD);
         }
     };
     load_pass(0);  // requested first: the angle arithmetic below runs while the rows are in flight
-    const int tgt  = token + (p.padding_offset ? p.padding_offset[token] : 0);  // :877-878
-    const int bi   = tgt / p.seq_len;
-    const int si   = tgt % p.seq_len;
-    if (tgt < 0 || bi >= p.batch) return;  // a padding offset that points outside [batch, seq_len]: nothing is written
-    const int hist = p.history_length[bi];
-    const int step = hist + si;  // :929
-    if (threadIdx.x < kD / 2) {
+    struct Place {
+        int  bi, si, hist;
+        bool ok;  // a padding offset that points outside [batch, seq_len]: nothing is written
+    };
+    auto place = [&](int t) {
+        Place at{0, 0, 0, false};
+        if (TOKENS == 1 || t < p.tokens) {
+            const int tgt = t + (p.padding_offset ? p.padding_offset[t] : 0);  // :877-878
+            at.bi = tgt / p.seq_len, at.si = tgt % p.seq_len;
+            at.ok = tgt >= 0 && at.bi < p.batch;
+            if (at.ok) at.hist = p.history_length[at.bi];
+        }
+        return at;
+    };
+    if (threadIdx.x < TOKENS * (kD / 2)) {
+        const int   pr = threadIdx.x % (kD / 2);
+        const Place at = place(blockIdx.x * TOKENS + threadIdx.x / (kD / 2));
         float2 c = make_float2(1.f, 0.f);
-        if (2 * (int)threadIdx.x < p.rot_dim) {
+        if (at.ok && 2 * pr < p.rot_dim) {
             float base = p.rope_base;
             if (p.use_dynamic_ntk) {
                 // decoder_masked_multihead_attention_utils.h:862-871 with the context length (:928,931-934)
-                const float len = (float)(hist + p.input_length[bi]);
+                const float len = (float)(at.hist + p.input_length[at.bi]);
                 if (!(len < (float)p.max_pos)) {
                     const float alpha = fmaxf(exp2f(ceilf(log2f(len / (float)p.max_pos) + 1.f)) - 1.f, 1.f);
                     base *= powf(alpha, (float)p.rot_dim / ((float)p.rot_dim - 2.f));
                 }
             }
-            const float ang = (float)step / powf(base, (float)(2 * threadIdx.x) / (float)p.rot_dim);  // utils.h:885-889
+            const float ang = (float)(at.hist + at.si) / powf(base, (float)(2 * pr) / (float)p.rot_dim);  // utils.h:885-889
             c = make_float2(cosf(ang), sinf(ang));  // two separate calls, as utils.h:888 makes them: the pair call rounds differently
         }
-        coef[threadIdx.x] = c;
+        coef[threadIdx.x / (kD / 2)][pr] = c;
     }
+    const Place at = place(token);
+    const int   bi = at.bi, si = at.si, step = at.hist + at.si;  // :929
     __syncthreads();
+    if (!at.ok) return;
     // :940-950: scaling of the length at this step, rounded to fp16, multiplied in fp16
     const float   len1 = (float)(step + 1);
     const __half2 logn = __half2half2(__float2half(len1 <= (float)p.max_pos ? 1.f : log2f(len1) / log2f((float)p.max_pos)));
-    for (int h0 = 0; h0 < total; h0 += kHeadBatch * kHeadsPerCta) {
+    char *k_base = nullptr, *v_base = nullptr;  // the sequence's rows of the cache
+    if (TARGET != KvTarget::kBuffers && si < p.input_length[bi] && step < p.max_seq_len) {  // never past the rows a cache head holds
+        k_base = static_cast<char*>(p.k_cache[bi]), v_base = static_cast<char*>(p.v_cache[bi]);
+    }
+    for (int h0 = 0; h0 < total; h0 += kHeadBatch * kHeads) {
         if (h0) load_pass(h0);
 #pragma unroll
         for (int j = 0; j < kHeadBatch; ++j) {
-            const int head = h0 + j * kHeadsPerCta + hsub;
+            const int head = h0 + j * kHeads + hsub;
             if (head >= total) continue;
             __half2* xh = reinterpret_cast<__half2*>(&x[j]);
             if (p.bias) {
-                const __half2* bh = reinterpret_cast<const __half2*>(&b[j]);
+                const uint4    b  = *reinterpret_cast<const uint4*>(p.bias + (size_t)head * kD + vec * 8);
+                const __half2* bh = reinterpret_cast<const __half2*>(&b);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) xh[e] = __hadd2(xh[e], bh[e]);  // fp16 add, :903-904
             }
@@ -140,7 +160,7 @@ __global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(Qk
                 for (int e = 0; e < 4; ++e) {
                     const int pr = vec * 4 + e;
                     if (2 * pr < p.rot_dim) {
-                        const float2 c = coef[pr];
+                        const float2 c = coef[slot][pr];
                         const float2 v = __half22float2(xh[e]);
                         // utils.h:891-904; the contraction the reference build ends up with: second product rounded, first fused
                         xh[e] = __floats2half2_rn(__fmaf_rn(c.x, v.x, -__fmul_rn(c.y, v.y)), __fmaf_rn(c.x, v.y, __fmul_rn(c.y, v.x)));
@@ -162,16 +182,15 @@ __global__ void __launch_bounds__(kQkvThreads) qkv_bias_rope_transpose_kernel(Qk
                     __half* dst = is_k ? p.k_buf : p.v_buf;
                     *reinterpret_cast<uint4*>(dst + (((size_t)bi * p.Hkv + kvh) * p.seq_len + si) * kD + vec * 8) = x[j];
                 }
-                else if (si < p.input_length[bi] && step < p.max_seq_len) {  // never past the rows a cache head holds
-                    const size_t at   = p.cache_offset + ((size_t)kvh * p.max_seq_len + step) * kD + vec * 8;
-                    void*        base = (is_k ? p.k_cache : p.v_cache)[bi];
+                else if (char* base = is_k ? k_base : v_base) {
+                    const size_t at = p.cache_offset + ((size_t)kvh * p.max_seq_len + step) * kD + vec * 8;
                     if (TARGET == KvTarget::kCacheInt8) {
                         const float scale = is_k ? p.k_scale : p.v_scale, zp = is_k ? p.k_zp : p.v_zp;
-                        *reinterpret_cast<uint2*>(static_cast<int8_t*>(base) + at) =
+                        *reinterpret_cast<uint2*>(base + at) =
                             make_uint2(quant4(xh[0], xh[1], scale, zp), quant4(xh[2], xh[3], scale, zp));
                     }
                     else {
-                        *reinterpret_cast<uint4*>(static_cast<__half*>(base) + at) = x[j];
+                        *reinterpret_cast<uint4*>(base + 2 * at) = x[j];
                     }
                 }
             }
@@ -274,6 +293,19 @@ __global__ void __launch_bounds__(kCacheThreads) transpose_kv_cache_kernel(Cache
     }
 }
 
+// A CTA takes one token, or four from 2048 tokens on: their angles are then one pass of all its threads instead of one of a quarter of
+// them ahead of each token, and a head's rows of four neighbouring tokens are written together.  Fewer tokens need the CTAs more (us,
+// one / four: 32 + 2 x 32 heads 735 tokens 12.5 / 14.6, 1024 14.5 / 15.9, 2048 26.8 / 22.6, 16384 161 / 136, 5.0 / 5.9 TB/s; 64 + 2 x 8
+// heads 1024 tokens 14.5 / 14.5, 2048 24.7 / 20.6, 16384 153 / 120).
+constexpr int kTokensInFours = 2048;
+
+template<KvTarget TARGET>
+cudaError_t launch_qkv(const QkvParams& p, cudaStream_t st)
+{
+    return p.tokens >= kTokensInFours ?
+               launch_kernel(qkv_bias_rope_transpose_kernel<TARGET, 4>, dim3((p.tokens + 3) / 4), dim3(kQkvThreads), 0, st, g_pdl != 0, p) :
+               launch_kernel(qkv_bias_rope_transpose_kernel<TARGET, 1>, dim3(p.tokens), dim3(kQkvThreads), 0, st, g_pdl != 0, p);
+}
 }  // namespace
 }  // namespace tmb
 
@@ -309,8 +341,8 @@ extern "C" int tm_add_fused_qkv_bias_transpose(void* q_buf, void* k_buf, void* v
     QkvParams p{(__half*)q_buf, (__half*)k_buf, (__half*)v_buf, (const __half*)QKV, (const __half*)qkv_bias, padding_offset,
                 history_length, input_length, batch_size, seq_len, head_num, kv_head_num, rotary_embedding_dim, rotary_embedding_base,
                 max_position_embeddings, use_dynamic_ntk, use_logn_attn};
-    const dim3 grid(token_num);
-    return status_of(launch_kernel(qkv_bias_rope_transpose_kernel<KvTarget::kBuffers>, grid, dim3(kQkvThreads), 0, (cudaStream_t)stream, g_pdl != 0, p));
+    p.tokens = token_num;
+    return status_of(launch_qkv<KvTarget::kBuffers>(p, (cudaStream_t)stream));
 }
 
 int tmb::prefill_write_qkv(void* q_buf, const void* qkv, const void* bias, const int* padding_offset, const int* history, const int* length,
@@ -325,8 +357,8 @@ int tmb::prefill_write_qkv(void* q_buf, const void* qkv, const void* bias, const
     p.batch = batch, p.seq_len = seq_len, p.H = heads, p.Hkv = kv_heads, p.rot_dim = kD, p.rope_base = rope_base, p.max_pos = max_seq_len;
     p.k_cache = k_cache, p.v_cache = v_cache, p.cache_offset = cache_offset, p.max_seq_len = max_seq_len;
     p.k_scale = kv_scale[0], p.k_zp = kv_scale[1], p.v_scale = kv_scale[2], p.v_zp = kv_scale[3];
-    return status_of(launch_kernel(int8 ? qkv_bias_rope_transpose_kernel<KvTarget::kCacheInt8> : qkv_bias_rope_transpose_kernel<KvTarget::kCache>,
-                                   dim3(tokens), dim3(kQkvThreads), 0, st, g_pdl != 0, p));
+    p.tokens = tokens;
+    return status_of(int8 ? launch_qkv<KvTarget::kCacheInt8>(p, st) : launch_qkv<KvTarget::kCache>(p, st));
 }
 
 extern "C" int tm_extend_kv_cache(void** k_dst, void** v_dst, size_t dst_offset, const void* k_src, const void* v_src,

@@ -1,5 +1,6 @@
 """GPU: the prefill driver writes keys and values straight to their cache rows; the same bits as the two public writers leave there one
-after the other, for ragged batches behind cached tokens, and nothing outside the new rows."""
+after the other, for ragged batches behind cached tokens, and nothing outside the new rows.  From 2048 tokens on a CTA takes four of
+them: the same bits again."""
 import numpy as np
 import pytest
 import torch
@@ -8,10 +9,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("int8", [True, False])
-@pytest.mark.parametrize("new,history", [([1], [0]), ([7, 0, 33], [5, 9, 0]), ([16, 17, 1, 24], [40, 0, 63, 8])])
-def test_rows_match_the_public_writers(int8, new, history):
+@pytest.mark.parametrize("new,history", [([1], [0]), ([7, 0, 33], [5, 9, 0]), ([16, 17, 1, 24], [40, 0, 63, 8]),
+                                         ([700, 811, 1, 538], [9, 0, 899, 100]), ([900, 900, 247, 1], [0, 0, 1, 3])])
+def test_rows_match_the_public_writers(int8, new, history, monkeypatch):
     from lmdeploy_b200 import lib as l, turbomind as tm
     from tests.test_gpu_llama import CFG, build
+    monkeypatch.setitem(CFG, "session_len", 64 if sum(new) < 2047 else 960)
     model, _, _ = build(int8, max_batch=4)
     B, S, H, G, hid = len(new), CFG["session_len"], CFG["head_num"], CFG["kv_head_num"], CFG["head_num"] * 128
     rng, dev = np.random.default_rng(sum(new)), "cuda"
@@ -48,3 +51,36 @@ def test_rows_match_the_public_writers(int8, new, history):
             rows[history[b]:history[b] + new[b]] = False
             assert torch.equal(got[b, 1:, :, rows], want[b, 1:, :, rows])
     model.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(5, 1), (8, 8)])
+@pytest.mark.parametrize("lengths,history", [([1024, 1024], [7, 0]), ([1021, 0, 3, 1025], [0, 5, 900, 31]), ([1300, 750, 1], [3000, 0, 64])])
+@pytest.mark.parametrize("bias,rot,ntk,logn", [(True, 128, 0, 0), (False, 64, 1, 1)])
+def test_four_tokens_a_block(heads, kv_heads, lengths, history, bias, rot, ntk, logn):
+    """One call for all sequences against one call for each, which are too short for it; rows behind a sequence's end stay."""
+    from lmdeploy_b200 import lib as l
+    S, T, n, dev = max(lengths), sum(lengths), (heads + 2 * kv_heads) * 128, "cuda"
+    g = torch.Generator(device=dev).manual_seed(T + heads)
+    y = torch.randn(T, n, device=dev, generator=g).half()
+    b = torch.randn(n, device=dev, generator=g).half() if bias else None
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    s = torch.cuda.current_stream().cuda_stream
+
+    def write(out, rows, lens, hist):
+        pad = ints([i * S - sum(lens[:i]) for i, k in enumerate(lens) for _ in range(k)])
+        le, hi = ints(lens), ints(hist)
+        l.check(l.lib.tm_add_fused_qkv_bias_transpose(*(o.data_ptr() for o in out), rows.data_ptr(), b.data_ptr() if bias else None, pad.data_ptr(),
+                                                      hi.data_ptr(), le.data_ptr(), len(lens), S, rows.shape[0], heads, kv_heads, 128, rot, 10000.0,
+                                                      1024, ntk, logn, s), "qkv")
+        torch.cuda.synchronize()
+
+    new = lambda: [torch.full((len(lengths), h, S, 128), 7.0, dtype=torch.float16, device=dev) for h in (heads, kv_heads, kv_heads)]
+    got, want = new(), new()
+    write(got, y, lengths, history)
+    at = 0
+    for i, k in enumerate(lengths):
+        if k:
+            write([o[i:i + 1] for o in want], y[at:at + k], [k], [history[i]])
+        at += k
+    for a, c in zip(got, want):
+        assert torch.equal(a, c)
