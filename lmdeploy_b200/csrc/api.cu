@@ -32,7 +32,7 @@ bool gemm_can_fuse_norm(const tm_handle* h, int m, int n, int k, bool producer)
     const auto fits = [&](const auto& pl) { return pl.workspace_floats * sizeof(float) <= h->scratch_bytes && pl.counter_ints <= h->counter_ints; };
     if (gemm_uses_tc(h, m, n, k)) {
         const GemmTcPlan pl = gemm_tc_plan(m, n, k, h->sm_count, true);
-        return fits(pl) && (!producer || gemm_tc_all_tiles_split(pl, k));
+        return fits(pl) && (!producer || (!pl.last_sums && gemm_tc_all_tiles_split(pl, k)));
     }
     const GemmSmallPlan pl = gemm_small_plan(m, n, k, h->sm_count, h->max_smem, h->gemv_cols);
     return fits(pl) && pl.t_chunks == 1 && (!producer || pl.cols_tiles > 0);
@@ -129,7 +129,7 @@ extern "C" int tm_gemm_s4_f16(tm_handle*  h,
             p.max_wait_cycles = h->gemm_wait_cycles;
             if (g_gemm_fusion) {
                 // the driver checked
-                if (per != n || workspace || (g_gemm_fusion->ssq_out && !gemm_tc_all_tiles_split(pl, k))) return TM_ERR_UNSUPPORTED;
+                if (per != n || workspace || (g_gemm_fusion->ssq_out && (pl.last_sums || !gemm_tc_all_tiles_split(pl, k)))) return TM_ERR_UNSUPPORTED;
                 p.norm = *g_gemm_fusion;
             }
             p.late_weight = !early;

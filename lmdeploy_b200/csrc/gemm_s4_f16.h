@@ -85,7 +85,7 @@ struct GemmTcParams {
     // filled in by gemm_tc_launch from the plan
     int units_per_cta, total_units, slots_per_chunk, n_col_tiles, token_tile, parts_per_tile;
     int       late_weight;      // 1: the kernel ahead may write the weight (a dependent launch waits before it reads any)
-    int       last_sums;        // 1: a split tile is reduced by the CTA that is done last, without a wait (no GemmNormFusion)
+    int       last_sums;        // 1: a split tile is reduced by the CTA that is done last, without a wait (GemmNormFusion: its consumer only)
     long long max_wait_cycles;  // bound of the wait for the partners of a split tile; 0 = the default
     GemmNormFusion norm;        // all null: a plain GEMM
 };

@@ -131,6 +131,7 @@ struct Bars {
     uint32_t tmem_base;
     int      flag;
     float    row_scale[128];  // 1 / rms per token (consumer of a folded norm)
+    unsigned long long ssq[128];  // sums of squares per token of this CTA's share (its producer)
 };
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
@@ -513,9 +514,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         constexpr int kMaxPending = 4;
         int           pend[kMaxPending] = {0, 0, 0, 0};
         int           n_pend = 0;
-        // producer side of a folded norm: per-token sums of squares of this CTA's share, in fixed point, kept in the (by then idle)
-        // activation ring until they go out with one atomic per token
-        unsigned long long* s_ssq = reinterpret_cast<unsigned long long*>(x_ring);
+        // producer side of a folded norm: per-token sums of squares of this CTA's share, in fixed point, until they go out with one
+        // atomic per token.  In a place of their own: they are cleared ahead of the barrier of the two teams, when the other team's
+        // products may still be reading the activation ring.
+        unsigned long long* s_ssq = bars->ssq;
         // Outputs of four adjacent features of a token from their sum
         auto finish = [&](int t, int col, float4 acc, uint2 res, uint2 gain, float inv) {
             if (p.norm.ssq_in) acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
