@@ -208,9 +208,10 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
         }
     };
     // The weights of the first ST - 1 units are requested before the kernel ahead of this one in the
-    // stream is known to be complete (nothing writes them).  Their activations follow after the wait as
+    // stream is known to be complete, unless it may write them.  Their activations follow after the wait as
     // plain loads and shared-memory stores, which the first barrier of the loop publishes: the first unit
     // then waits for its own 16 KB of weights only, not for the whole window of requests behind it.
+    if (p.late_weight) pdl_wait();
     const int x_k0 = i_k;
 #pragma unroll
     for (int sidx = 0; sidx < ST - 1; ++sidx) {
@@ -586,7 +587,7 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
         i_w += (size_t)(4 * warps) * slab_stride;  // this warp's next group: eight groups (of a strip's CTA) further down
         i_q += (size_t)warps * p.N * 4;
     };
-    // the packed weight is written by no kernel: its first copies start ahead of the wait for the kernel before
+    // unless the kernel before may write the packed weight, its first copies start ahead of the wait for it
     if (p.late_weight) pdl_wait();
     int issued = 0;
     for (; issued < ST && issued < n_groups; ++issued) issue_group(issued);

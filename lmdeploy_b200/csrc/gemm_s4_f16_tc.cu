@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         if (++w_g == G) w_g = 0, ++w_js;
     };
     if (warp == kWLoadWarp) {
-        // The packed weights are written by no kernel: the first copies start at once, ahead of the TMEM set-up (one stage: issuing
-        // them all takes longer than that) and of the wait for the kernel before this one.
+        // The first copies start at once, ahead of the TMEM set-up (one stage: issuing them all takes longer than that) and, unless the
+        // kernel before may write the packed weight, of the wait for it.
         if (elect_one()) {
             for (int s = 0; s < kWST; ++s) {
                 mbar_init(&bars->w_full[s], 1);

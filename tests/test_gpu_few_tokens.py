@@ -142,8 +142,8 @@ def test_tensor_core_tiles_at_their_edges(n, k, tokens, silu):
 
 @pytest.mark.parametrize("n,k,tokens", [(4096, 4096, 1), (4096, 11008, 8), (22016, 4096, 4), (12288, 4096, 40), (22016, 4096, 300)])
 def test_a_weight_written_by_the_kernel_ahead(n, k, tokens):
-    """Direct calls are dependent launches: the packed weight, its scales and the tokens that the kernel just ahead of the call writes
-    are the ones it multiplies."""
+    """The packed weight, its scales and the tokens that copies just ahead of a direct call write are the ones it multiplies (copies let
+    nothing start early; a kernel that does is in test_gpu_direct_calls.py)."""
     from lmdeploy_b200 import turbomind as tm
     from perf import cases
     sides = [cases._linear(cases._gen(s, n), n, k) for s in (1, 2)]
