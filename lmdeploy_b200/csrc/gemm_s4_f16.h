@@ -12,23 +12,83 @@ namespace tmb {
 
 // Residual add + RMSNorm folded into the GEMMs on either side in the decode step (decode driver only).
 // Producer side (o_proj, w2): whoever has the whole sum of an output adds the residual, stores it, writes
-// half((residual + y) * norm_weight) as the output and adds up every token's sum of squares in 2^-20 fixed point
-// (integer atomics: the order of the additions cannot change the result).
-// Consumer side (qkv, w13): the rows of the accumulator are scaled by rsqrt(ssq[t] * 2^-20 * inv_n + eps) before the
-// output is rounded, which completes the normalisation of its input.
+// half((residual + y) * norm_weight) as the output and adds up every token's sum of squares.
+// Consumer side (qkv, w13): the rows of the accumulator are scaled by 1 / rms before the output is rounded, which completes
+// the normalisation of its input.
+
+// A row's sum of squares.  Its parts (fp32 sums in a fixed order) are added as whole numbers, so that the order of the additions cannot
+// change the result: each to `fine`, in units of 2^(2 e - 24), where 2^e <= rms < 2^(e + 1) of the row ahead of this addition
+// (kLeastExponent at least); or, if it is 2^26 times 2^(2 e) or more, to `coarse`, in units of 2^-13.  Either way it keeps the bits that
+// count in an fp32 sum of the row.  Parts that are no numbers set the upper bit of `coarse`.
+struct RowSquares {
+    unsigned long long fine, coarse;  // of at most 2^12 parts (16384 values by four)
+    int                exponent;      // e
+    int                unused[3];     // 32 bytes: a sector
+};
 struct GemmNormFusion {
-    __half*                   residual    = nullptr;  // [T][N], producer
-    const __half*             norm_weight = nullptr;  // [N], producer
-    unsigned long long*       ssq_out     = nullptr;  // [T], producer
-    const unsigned long long* ssq_in      = nullptr;  // [T], consumer
-    float                     inv_n       = 0.f;      // 1 / (length of the normalised row), consumer
-    float                     eps         = 0.f;
+    __half*           residual    = nullptr;  // [T][N], producer
+    const __half*     norm_weight = nullptr;  // [N], producer
+    const RowSquares* ssq_before  = nullptr;  // [T] ahead of the addition, producer
+    RowSquares*       ssq_out     = nullptr;  // [T], producer
+    const RowSquares* ssq_in      = nullptr;  // [T], consumer
+    float             inv_n       = 0.f;      // 1 / (length of the normalised row)
+    float             eps         = 0.f;      // consumer
 };
 #ifdef __CUDACC__
-// consumer: 1 / rms of row t
-__device__ __forceinline__ float norm_row_scale(const GemmNormFusion& f, int t)
+constexpr int                kLeastExponent = -8, kMostExponent = 17;
+constexpr unsigned long long kNotFinite     = 1ull << 63;
+__device__ __forceinline__ float power_of_two(int e)  // in fp32's normal range
 {
-    return rsqrtf((float)__ldcg(f.ssq_in + t) * (1.f / 1048576.f) * f.inv_n + f.eps);
+    return __int_as_float((e + 127) << 23);
+}
+__device__ __forceinline__ RowSquares load_row_squares(const RowSquares* at)
+{
+    RowSquares       r{};
+    const ulonglong2 sums = __ldcg(reinterpret_cast<const ulonglong2*>(at));
+    r.fine = sums.x, r.coarse = sums.y, r.exponent = __ldcg(&at->exponent);
+    return r;
+}
+__device__ __forceinline__ float row_squares(const RowSquares& r)
+{
+    const float sum = __ull2float_rn(r.fine) * power_of_two(2 * r.exponent - 24);
+    if (r.coarse == 0ull) return sum;
+    return r.coarse >= kNotFinite ? __int_as_float(0x7fffffff) : sum + __ull2float_rn(r.coarse) * power_of_two(-13);
+}
+// floor(log2(rms)) from the mean square
+__device__ __forceinline__ int row_exponent(float mean_square)
+{
+    return min(max((((__float_as_int(mean_square) >> 23) & 0xff) - 127) >> 1, kLeastExponent), kMostExponent);
+}
+// consumer: 1 / rms of a row
+__device__ __forceinline__ float norm_row_scale(const GemmNormFusion& f, const RowSquares& r)
+{
+    return rsqrtf(row_squares(r) * f.inv_n + f.eps);
+}
+// producer: 2^-e
+__device__ __forceinline__ float norm_row_down(const GemmNormFusion& f, const RowSquares& before)
+{
+    return power_of_two(-row_exponent(row_squares(before) * f.inv_n));
+}
+__device__ __forceinline__ int exponent_of_down(float down)
+{
+    return 127 - (__float_as_int(down) >> 23);
+}
+// A part of a row's sum
+__device__ __forceinline__ void add_row_squares(RowSquares* at, float part, float down)
+{
+    const float units = part * (down * down * power_of_two(24));
+    if (units < power_of_two(50)) atomicAdd(&at->fine, __float2ull_rn(units));
+    else if (part < power_of_two(60)) atomicAdd(&at->coarse, __float2ull_rn(part * power_of_two(13)));
+    else atomicOr(&at->coarse, kNotFinite);
+}
+// The whole of it
+__device__ __forceinline__ RowSquares whole_row_squares(float sum, float inv_n)
+{
+    RowSquares r{};
+    r.exponent = row_exponent(sum * inv_n);
+    if (sum < power_of_two(60)) r.fine = __float2ull_rn(sum * power_of_two(24 - 2 * r.exponent));
+    else r.coarse = kNotFinite;
+    return r;
 }
 #endif
 

@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                             for (int i = 0; i < 4; ++i) {
                                 const int   n = col0 + (my_t0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8;
                                 const int   t = t0 + j * 8 + 2 * c + (i & 1);
-                                const float v = p.norm.ssq_in ? tot[w][a][j][i] * norm_row_scale(p.norm, min(t, p.T - 1)) : tot[w][a][j][i];
+                                const float v = p.norm.ssq_in ? tot[w][a][j][i] * norm_row_scale(p.norm, load_row_squares(p.norm.ssq_in + min(t, p.T - 1))) : tot[w][a][j][i];
                                 if (p.fused_silu) {
                                     // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair;
                                     // the partner column n^1 lives in lane^4
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                         }
                     }
                     if (p.norm.ssq_in) {
-                        const float inv = norm_row_scale(p.norm, t0 + t);
+                        const float inv = norm_row_scale(p.norm, load_row_squares(p.norm.ssq_in + t0 + t));
                         v.x *= inv, v.y *= inv, v.z *= inv, v.w *= inv;
                     }
                     const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     pdl_launch_dependents();
 
     // What this lane's outputs need beside their sums (value e = warp + 8 q of the strip's kVals) is on its way during the products:
-    // the row's 1 / rms (consumer of a folded norm), the residual and the norm weight (its producer).
+    // the row's factor (either side of a folded norm), the residual and the norm weight (its producer).
     constexpr int kVals = TILES * 8 * NT;
     struct Place {
         int n, t;
@@ -604,11 +604,14 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
         const int e = warp + q * kWarps, w = e / (8 * NT), a = e / (4 * NT) & 1, j = e / 4 % NT, i = e & 3;
         return Place{(tile0 + w) * kColsPerTile + a * 16 + r + (i >> 1) * 8, 8 * j + 2 * c + (i & 1)};
     };
-    float row_scale[kVals / kWarps], res[kVals / kWarps], gain[kVals / kWarps];
+    __shared__ float row_scale[8 * NT];
+    const bool       scales = (p.norm.ssq_in || p.norm.ssq_out) && rank == 0 && tid < p.T;  // (this warp has a group: the first one)
+    RowSquares       squares{};
+    if (scales) squares = load_row_squares((p.norm.ssq_in ? p.norm.ssq_in : p.norm.ssq_before) + tid);
+    float res[kVals / kWarps], gain[kVals / kWarps];
 #pragma unroll
     for (int q = 0; q < kVals / kWarps; ++q) {
         const Place at = place(q);
-        row_scale[q]   = p.norm.ssq_in ? norm_row_scale(p.norm, min(at.t, p.T - 1)) : 1.f;
         res[q] = gain[q] = 0.f;
         if (p.norm.ssq_out && rank == 0 && at.n < p.N && at.t < p.T) {
             res[q]  = __half2float(p.norm.residual[(size_t)at.t * p.N + at.n]);
@@ -648,6 +651,10 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
         // copies complete in the order they were committed: group `it` has landed once at most issued - it - 1 are pending
         cp_async_wait_pending(issued - it - 1);
         __syncwarp();  // every lane's copies of this group have landed, and every lane is done with the group before
+        if (scales && it == 0) {  // long there by now
+            row_scale[tid] = p.norm.ssq_in ? norm_row_scale(p.norm, squares) : norm_row_down(p.norm, squares);
+            if (p.norm.ssq_out && blockIdx.x == 0) p.norm.ssq_out[tid].exponent = exponent_of_down(row_scale[tid]);
+        }
         if (it >= 1 && issued < n_groups) {
             issue_group(slot == 0 ? ST - 1 : slot - 1);  // the slot of the group before: free now
             ++issued;
@@ -736,9 +743,8 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();  // the rings are free: they now hold the eight warps' partial sums, [warp][TILES x 8 values][lane]
     float* red = reinterpret_cast<float*>(smem_raw);
-    // sums of squares per token behind them (producer of a folded norm)
-    unsigned long long* s_ssq = reinterpret_cast<unsigned long long*>(red + kWarps * kVals * 32);
-    if (tid < 8 * NT) s_ssq[tid] = 0ull;
+    // sums of squares behind them, [value][column pair of the fragment] (producer of a folded norm)
+    float* s_ssq = red + kWarps * kVals * 32;
 #pragma unroll
     for (int w = 0; w < TILES; ++w)
 #pragma unroll
@@ -777,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     }
 #pragma unroll
     for (int q = 0; q < kVals / kWarps; ++q) {
-        const float v     = p.norm.ssq_in ? sums[q] * row_scale[q] : sums[q];
+        const float v     = p.norm.ssq_in ? sums[q] * row_scale[place(q).t] : sums[q];  // (of tokens that are not there: not stored)
         const int   n     = place(q).n, t = place(q).t;
         const bool  valid = n < p.N && t < p.T;
         if (p.norm.ssq_out) {
@@ -789,11 +795,10 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
                 p.norm.residual[(size_t)t * p.N + n] = hs;
                 p.C[(size_t)t * p.N + n]             = __float2half_rn(__half2float(hs) * gain[q]);
             }
-            // whole numbers: the same sum in any order.  The eight rows of a token first, then the warps, then the strips.
-            unsigned long long ss = valid ? (unsigned long long)__float2ll_rn(s * s * 1048576.f) : 0ull;
+            float ss = valid ? s * s : 0.f;  // the eight rows of a token here
 #pragma unroll
             for (int m = 4; m < 32; m *= 2) ss += __shfl_xor_sync(0xffffffffu, ss, m);
-            if (r == 0 && t < p.T) atomicAdd(s_ssq + t, ss);
+            if (r == 0) s_ssq[(warp + q * kWarps) * 4 + c] = ss;
         }
         else if (p.fused_silu) {
             // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pair; the partner column n ^ 1 lives in lane ^ 4
@@ -810,7 +815,13 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
     }
     if (p.norm.ssq_out) {
         __syncthreads();
-        if (tid < p.T) atomicAdd(p.norm.ssq_out + tid, s_ssq[tid]);
+        if (tid < p.T) {
+            // token tid's values: (tile, half, row pair) of its column pair
+            float ss = 0.f;
+#pragma unroll
+            for (int v = 0; v < TILES * 4; ++v) ss += s_ssq[((((v >> 1) * NT + tid / 8) << 2) + (v & 1) * 2 + (tid & 1)) * 4 + (tid & 7) / 2];
+            add_row_squares(p.norm.ssq_out + tid, ss, row_scale[tid]);
+        }
     }
 }
 

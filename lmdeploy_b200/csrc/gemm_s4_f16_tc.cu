@@ -130,9 +130,10 @@ struct Bars {
     uint64_t acc_full[kTeams], acc_empty[kTeams];  // per team
     uint32_t tmem_base;
     int      flag;
-    float    row_scale[128];  // 1 / rms per token (consumer of a folded norm)
-    unsigned long long ssq[128];  // sums of squares per token of this CTA's share (its producer)
+    float    row_scale[128];  // factor of a token (either side of a folded norm)
 };
+constexpr int kSquaresLd = 33;  // sums of squares of a token (producer of a folded norm): a share of a split tile has at most 32 quads of features
+
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
 {
@@ -514,13 +515,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         constexpr int kMaxPending = 4;
         int           pend[kMaxPending] = {0, 0, 0, 0};
         int           n_pend = 0;
-        // producer side of a folded norm: per-token sums of squares of this CTA's share, in fixed point, until they go out with one
-        // atomic per token.  In a place of their own: they are cleared ahead of the barrier of the two teams, when the other team's
-        // products may still be reading the activation ring.
-        unsigned long long* s_ssq = bars->ssq;
+        // producer side of a folded norm: sums of squares of this CTA's share, [token][quad of features], until a thread for each token adds
+        // them up.  In a place of their own: no ring may be written while the other team's products may be reading it.
+        float* s_ssq = reinterpret_cast<float*>(bars + 1);
         // Outputs of four adjacent features of a token from their sum
-        auto finish = [&](int t, int col, float4 acc, uint2 res, uint2 gain, float inv) {
-            if (p.norm.ssq_in) acc.x *= inv, acc.y *= inv, acc.z *= inv, acc.w *= inv;
+        auto finish = [&](int t, int quad, int col, float4 acc, uint2 res, uint2 gain, float scale) {
+            if (p.norm.ssq_in) acc.x *= scale, acc.y *= scale, acc.z *= scale, acc.w *= scale;
             const __half2 h0 = __floats2half2_rn(acc.x, acc.y), h1 = __floats2half2_rn(acc.z, acc.w);
             auto half2_of    = [](uint32_t v) { return __half22float2(reinterpret_cast<const __half2&>(v)); };
             auto word_of     = [](__half2 v) { return reinterpret_cast<const uint32_t&>(v); };
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 const float2 g0 = half2_of(gain.x), g1 = half2_of(gain.y);
                 *reinterpret_cast<uint2*>(p.C + at) =
                     make_uint2(word_of(__floats2half2_rn(a0.x * g0.x, a0.y * g0.y)), word_of(__floats2half2_rn(a1.x * g1.x, a1.y * g1.y)));
-                atomicAdd(s_ssq + t, (unsigned long long)__float2ll_rn(ss * 1048576.f));
+                s_ssq[t * kSquaresLd + quad] = ss;
             }
             else if (p.fused_silu) {
                 // kernels/gemm_s_f16/gemm_s4_f16.cu:31-43 on the fp16-rounded pairs (gate, up)
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 }
 #pragma unroll
                 for (int j = 0; j < kPieces; ++j) {
-                    if (i0 + j * kDqThreads < items) finish(tt[j], col0 + nn[j], acc[j], res[j], gain[j], p.norm.ssq_in ? bars->row_scale[tt[j]] : 1.f);
+                    if (i0 + j * kDqThreads < items) finish(tt[j], (nn[j] - f0) / 4, col0 + nn[j], acc[j], res[j], gain[j], p.norm.ssq_in ? bars->row_scale[tt[j]] : 1.f);
                 }
             }
         };
@@ -604,8 +604,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             int       c_first;
             const int n_split = tile_ctas(tjs, c_first);
             const int col0    = tjs * kSuperN;
-            if (p.norm.ssq_in && dtid < t_rows) bars->row_scale[dtid] = norm_row_scale(p.norm, t0 + dtid);
-            if (p.norm.ssq_out && dtid < t_rows) s_ssq[dtid] = 0ull;
             if (dtid == 0 && !p.last_sums) {
                 // Bounded wait for the other CTAs of the tile.  The plan splits tiles between CTAs only
                 // when the whole grid is one wave of at most one CTA per SM (gemm_tc_plan), so the
@@ -631,11 +629,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 through = atomicAdd(done + tjs, 1);
                 if (!tile_ok) __threadfence();
             }
+            const int j      = blockIdx.x - c_first;
+            const int n_cols = min(kSuperN, p.N - col0);  // N % 32 == 0
+            const int f0     = p.last_sums ? 0 : (n_cols * j / n_split) & ~3;
+            const int f1     = p.last_sums || j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
             if (tile_ok) {
-                const int    j      = blockIdx.x - c_first;
-                const int    n_cols = min(kSuperN, p.N - col0);  // N % 32 == 0
-                const int    f0     = p.last_sums ? 0 : (n_cols * j / n_split) & ~3;
-                const int    f1     = p.last_sums || j == n_split - 1 ? n_cols : ((n_cols * (j + 1) / n_split) & ~3);
                 const float* tile_slots = slots + (size_t)(c_first + tjs) * slot_floats;
                 if (f1 > f0) {
                     if (n_split <= 2 && !p.norm.ssq_out) sum_rows(Int<4>{}, Int<2>{}, Int<0>{}, tile_slots, n_split, f0, f1, col0);
@@ -644,7 +642,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 }
             }
             named_bar_sync(1, kDqThreads);  // everyone is done reading; the flag may be reused
-            if (p.norm.ssq_out && tile_ok && dtid < t_rows && s_ssq[dtid]) atomicAdd(p.norm.ssq_out + t0 + dtid, s_ssq[dtid]);
+            if (p.norm.ssq_out && tile_ok && dtid < t_rows && f1 > f0) {
+                float ss = 0.f;
+                for (int i0 = 0; i0 < (f1 - f0) / 4; i0 += 8) {
+                    float part[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) part[i] = i0 + i < (f1 - f0) / 4 ? s_ssq[dtid * kSquaresLd + i0 + i] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) ss += part[i];
+                }
+                add_row_squares(p.norm.ssq_out + t0 + dtid, ss, bars->row_scale[dtid]);
+            }
             if (dtid == 0 && p.last_sums) arrive[tjs] = 0;
             if (dtid == 0 && !p.last_sums && through == n_split - 1) {
                 // the last CTA through the wait resets both counts for the next launch; one that gave up counts too, so the counts
@@ -751,6 +759,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             if (js == u_begin / G) {
                 // What follows reads and writes scratch, tickets and the output, which the kernel before this one may still be using.
                 pdl_wait();
+                // the tokens' factors, under the last products; read behind a barrier of these threads (reduce_share)
+                if (const int t = kDqThreads - 1 - dtid; (p.norm.ssq_in || p.norm.ssq_out) && t < t_rows) {
+                    const RowSquares r = load_row_squares((p.norm.ssq_in ? p.norm.ssq_in : p.norm.ssq_before) + t0 + t);
+                    bars->row_scale[t] = p.norm.ssq_in ? norm_row_scale(p.norm, r) : norm_row_down(p.norm, r);
+                    if (p.norm.ssq_out && blockIdx.x == 0) p.norm.ssq_out[t0 + t].exponent = exponent_of_down(bars->row_scale[t]);
+                }
             }
             g = 0;
             ++js;
@@ -782,8 +796,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     }
                     else {
                         if (p.norm.ssq_in) {
+                            const float mine = norm_row_scale(p.norm, load_row_squares(p.norm.ssq_in + t0 + min(col + (lane & 15), t_rows - 1)));
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) v[i] *= norm_row_scale(p.norm, min(t0 + col + i, p.T - 1));
+                            for (int i = 0; i < 16; ++i) v[i] *= __shfl_sync(0xffffffffu, mine, i);
                         }
                         // Neighbouring lanes trade a token each, so that a lane holds two adjacent features of one token of every two: whole
                         // sectors, and (gate, up) side by side (22016 x 4096, 735 tokens: 129 us with a store of 2 bytes for every value, 114 so).
@@ -898,7 +913,8 @@ PFN_encodeTiled lookup_encode_tiled()
 
 size_t gemm_tc_smem_bytes(int token_tile)
 {
-    return 1024 + (size_t)(token_tile > 64 ? Shape<true>::kXST : Shape<false>::kXST) * 2 * token_tile * 128 + (size_t)kWST * kWStage + sizeof(Bars) + 64;
+    return 1024 + (size_t)(token_tile > 64 ? Shape<true>::kXST : Shape<false>::kXST) * 2 * token_tile * 128 + (size_t)kWST * kWStage + sizeof(Bars)
+           + (size_t)token_tile * kSquaresLd * sizeof(float) + 64;
 }
 
 GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)

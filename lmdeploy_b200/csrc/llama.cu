@@ -52,12 +52,12 @@ namespace {
 __global__ void prepare_step_kernel(const int* step, const int* start_step, const int* forced_ids, const int* picked,
                                     int* ids_in, unsigned char* inactive, int B, int max_steps, int vocab, const int* lengths,
                                     int* order, MmhaSeqDesc* desc, void* const* k_ptrs, void* const* v_ptrs, float2* rope_table,
-                                    float rope_base, int rot_dim, unsigned long long* ssq, int ssq_count)
+                                    float rope_base, int rot_dim, RowSquares* ssq, int ssq_count)
 {
     const int b    = blockIdx.x;
     const int mine = lengths[b];
     // the step's sums of squares (GemmNormFusion); here, as no operation that is not a kernel stands between dependent launches then
-    for (int i = b * blockDim.x + threadIdx.x; i < ssq_count; i += gridDim.x * blockDim.x) ssq[i] = 0ull;
+    for (int i = b * blockDim.x + threadIdx.x; i < ssq_count; i += gridDim.x * blockDim.x) ssq[i] = RowSquares{};
     // attention launch order: longest cached sequence first (rank by length, ties by index)
     __shared__ int s_rank;
     if (threadIdx.x == 0) {
@@ -173,7 +173,7 @@ int run_step(StepCtx& c)
     auto foldable = [&](const LlamaDenseWeight& w, bool producer) {
         return gemm_can_fuse_norm(m.h, (int)w.output_dims, B, (int)w.input_dims, producer);
     };
-    const bool fold = !tp_on && m.h->fold_norm && foldable(w0.qkv, false) && foldable(w0.output, true)
+    const bool fold = !tp_on && m.h->fold_norm && m.hidden <= 16384 && foldable(w0.qkv, false) && foldable(w0.output, true)
                       && foldable(w0.fused_gating_intermediate, false) && foldable(w0.ffn_output, true);
 
     prepare_step_kernel<<<B, 64, 0, s>>>(st.step, st.start_step, st.forced_ids, m.picked, m.ids_in, m.inactive, B, st.max_steps,
@@ -184,7 +184,13 @@ int run_step(StepCtx& c)
     if (!c.ok_cuda()) return c.rc;
 
     // LlamaDecoder.cc:198-206
-    if (!c.ok(tm_rmsnorm(m.hbuf, m.x, m.layers[0].self_attn_norm_weights, cfg.norm_eps, B, m.hidden, s))) return c.rc;
+    if (fold) {
+        const auto* w = (const __half*)m.layers[0].self_attn_norm_weights;
+        if (!c.ok(rmsnorm_launch(m.hbuf, m.x, w, cfg.norm_eps, B, m.hidden, s, g_pdl != 0, m.ssq) == cudaSuccess ? TM_OK : TM_ERR_CUDA)) return c.rc;
+    }
+    else if (!c.ok(tm_rmsnorm(m.hbuf, m.x, m.layers[0].self_attn_norm_weights, cfg.norm_eps, B, m.hidden, s))) {
+        return c.rc;
+    }
     ++c.launches;
 
     // Tensor parallel: the row-split GEMMs write their partial sums into a slot that the peers have mapped, and one
@@ -214,7 +220,8 @@ int run_step(StepCtx& c)
         ~FusionScope() { g_gemm_fusion = nullptr; }
     };
     auto ssq_of = [&](int idx) { return m.ssq + (size_t)idx * cfg.max_batch_size; };
-    // consumer: scale rows by the 1 / rms that the sums of squares `idx` give; producer: fold the add + norm-weight in
+    // Sums of squares of the rows that the norms of the step see: number 2 l ahead of layer l's attention, 2 l + 1 of its feed forward.
+    // Consumer: scale rows by what the sums `idx` give; producer: fold the add + norm weight in, and add up the sums `idx`.
     auto consumer = [&](int idx) {
         GemmNormFusion f;
         f.ssq_in = ssq_of(idx), f.inv_n = 1.f / (float)m.hidden, f.eps = cfg.norm_eps;
@@ -222,7 +229,7 @@ int run_step(StepCtx& c)
     };
     auto producer = [&](int idx, const void* norm_w) {
         GemmNormFusion f;
-        f.residual = m.x, f.norm_weight = (const __half*)norm_w, f.ssq_out = ssq_of(idx);
+        f.residual = m.x, f.norm_weight = (const __half*)norm_w, f.inv_n = 1.f / (float)m.hidden, f.ssq_before = ssq_of(idx - 1), f.ssq_out = ssq_of(idx);
         return f;
     };
 
@@ -231,7 +238,7 @@ int run_step(StepCtx& c)
         // ---- self attention (LlamaDecoderSelfAttentionLayer.cc:193-304)
         {
             NvtxRange r("qkv_gemm");
-            const GemmNormFusion f = consumer(2 * l - 1);
+            const GemmNormFusion f = consumer(2 * l);
             FusionScope          fs(fold && l > 0 ? &f : nullptr);
             if (!c.ok(linear.forward(m.qkv, m.hbuf, B, w.qkv, LlamaLinear::kGemm, s))) return c.rc;
         }
@@ -272,7 +279,7 @@ int run_step(StepCtx& c)
         }
         {
             NvtxRange r("o_gemm");
-            const GemmNormFusion f = producer(2 * l, w.ffn_norm_weights);
+            const GemmNormFusion f = producer(2 * l + 1, w.ffn_norm_weights);
             FusionScope          fs(fold ? &f : nullptr);
             if (!c.ok(linear.forward(part_o, m.ctx, B, w.output, LlamaLinear::kGemm, s))) return c.rc;
         }
@@ -284,11 +291,11 @@ int run_step(StepCtx& c)
         {
             NvtxRange r("ffn");
             {
-                const GemmNormFusion f = consumer(2 * l);
+                const GemmNormFusion f = consumer(2 * l + 1);
                 FusionScope          fs(fold ? &f : nullptr);
                 if (!c.ok(linear.forward(m.ffn, m.hbuf, B, w.fused_gating_intermediate, LlamaLinear::kFusedSiluFfn, s))) return c.rc;
             }
-            const GemmNormFusion f = producer(2 * l + 1, next_norm);
+            const GemmNormFusion f = producer(2 * l + 2, next_norm);
             FusionScope          fs(fold && !last ? &f : nullptr);
             if (!c.ok(linear.forward(part_f, m.ffn, B, w.ffn_output, LlamaLinear::kGemm, s))) return c.rc;
         }
@@ -395,7 +402,7 @@ extern "C" int tm_llama_create(tm_llama** out, tm_handle* h, tm_comm* comm, cons
     alloc((void**)&m->order, (size_t)B * sizeof(int));
     alloc((void**)&m->seq_desc, (size_t)B * sizeof(MmhaSeqDesc));
     alloc((void**)&m->rope_table, (size_t)B * 64 * sizeof(float2));
-    alloc((void**)&m->ssq, (size_t)2 * c.num_layer * B * sizeof(unsigned long long));
+    alloc((void**)&m->ssq, (size_t)2 * c.num_layer * B * sizeof(RowSquares));
     alloc(&m->cublas_ws, 32u << 20);
     if (e == cudaSuccess) e = cudaMemset(m->picked, 0, B * 4);
     bool ok = e == cudaSuccess;

@@ -54,7 +54,10 @@ MmhaPlan    mmha_plan(int B, int H, int Hkv, int max_len, int sm_count, int want
 cudaError_t mmha_launch(const MmhaPlan& plan, MmhaParams p, bool int8, cudaStream_t st, bool pdl = false);
 
 // RMSNorm kernels (norm.cu)
-cudaError_t rmsnorm_launch(__half* out, const __half* in, const __half* scale, float eps, int m, int n, cudaStream_t st, bool pdl = false);
+struct RowSquares;
+// `squares`, if any: the rows' sums of squares, for a norm folded into the GEMMs behind this one (gemm_s4_f16.h)
+cudaError_t rmsnorm_launch(__half* out, const __half* in, const __half* scale, float eps, int m, int n, cudaStream_t st, bool pdl = false,
+                           RowSquares* squares = nullptr);
 cudaError_t add_residual_rmsnorm_launch(
     __half* residual, __half* in_out, const __half* bias, const __half* scale, float eps, int m, int n, cudaStream_t st,
     bool pdl = false);

@@ -6,6 +6,7 @@
 // the residual stored as fp16, the sum of squares taken before that rounding, the
 // normalisation applied to the stored value.
 #include "common.cuh"
+#include "gemm_s4_f16.h"
 #include "mmha.h"
 
 namespace tmb {
@@ -31,7 +32,7 @@ __device__ __forceinline__ float block_sum(float v, float* red)
 // rows of 4096 / 8192: 98.8 / 182.7 us, 82.2 / 163.3 so, 6.5 TB/s; 735 rows of 4096: 6.8 and 6.1).
 template<bool RESIDUAL, int VEC>
 __global__ void __launch_bounds__(kNormThreads, VEC == 2 ? 8 : VEC == 4 ? 6 : 4)
-rmsnorm_kernel(__half* residual, __half* in_out, const __half* in, const __half* bias, const __half* scale, float eps, int n)
+rmsnorm_kernel(__half* residual, __half* in_out, const __half* in, const __half* bias, const __half* scale, float eps, int n, RowSquares* squares)
 {
     __shared__ float red[kNormThreads / 32];
     pdl_wait();  // the rows come from the kernel before this one
@@ -76,6 +77,7 @@ rmsnorm_kernel(__half* residual, __half* in_out, const __half* in, const __half*
     }
     const float total = block_sum(ss, red);
     const float inv   = rsqrtf(total / (float)n + eps);
+    if (!RESIDUAL && squares && threadIdx.x == 0) squares[blockIdx.x] = whole_row_squares(total, 1.f / (float)n);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) {
         const int v = threadIdx.x + i * kNormThreads;
@@ -98,17 +100,18 @@ rmsnorm_kernel(__half* residual, __half* in_out, const __half* in, const __half*
 
 }  // namespace
 
-cudaError_t rmsnorm_launch(__half* out, const __half* in, const __half* scale, float eps, int m, int n, cudaStream_t st, bool pdl)
+cudaError_t rmsnorm_launch(__half* out, const __half* in, const __half* scale, float eps, int m, int n, cudaStream_t st, bool pdl,
+                           RowSquares* squares)
 {
     const auto kernel = n <= 4096 ? rmsnorm_kernel<false, 2> : n <= 8192 ? rmsnorm_kernel<false, 4> : rmsnorm_kernel<false, 8>;
-    return launch_kernel(kernel, dim3(m), dim3(kNormThreads), 0, st, pdl, nullptr, out, in, nullptr, scale, eps, n);
+    return launch_kernel(kernel, dim3(m), dim3(kNormThreads), 0, st, pdl, nullptr, out, in, nullptr, scale, eps, n, squares);
 }
 
 cudaError_t add_residual_rmsnorm_launch(
     __half* residual, __half* in_out, const __half* bias, const __half* scale, float eps, int m, int n, cudaStream_t st, bool pdl)
 {
     const auto kernel = n <= 4096 ? rmsnorm_kernel<true, 2> : n <= 8192 ? rmsnorm_kernel<true, 4> : rmsnorm_kernel<true, 8>;
-    return launch_kernel(kernel, dim3(m), dim3(kNormThreads), 0, st, pdl, residual, in_out, nullptr, bias, scale, eps, n);
+    return launch_kernel(kernel, dim3(m), dim3(kNormThreads), 0, st, pdl, residual, in_out, nullptr, bias, scale, eps, n, nullptr);
 }
 
 }  // namespace tmb

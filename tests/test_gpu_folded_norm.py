@@ -40,3 +40,70 @@ def test_every_element_as_with_norm_kernels(size, batch):
     # activation that a product takes for zero in 64 of its inputs costs an output 4 % of its size.
     err, size_of = (got[0].double() - want.double()).abs(), want.double().abs()
     assert (err <= 2.0 ** -7 + size_of * 2.0 ** -8).all() and err.mean() <= 2.0 ** -10, (err.max().item(), err.mean().item())
+
+
+def _scaled(gen, n, k, factor, columns=slice(None)):
+    """A weight whose chosen columns are `factor` times as large, in the library's layout and as numbers"""
+    from perf import cases
+    state = gen.get_state()
+    w = cases._linear(gen, n, k)
+    gen.set_state(state)
+    q, z, s = cases._weight(gen, n, k)
+    s = s.clone()
+    s[:, columns] = (s[:, columns].float() * factor).half()
+    sz = w.scales_and_zeros
+    sz[:, columns, 1] = (sz[:, columns, 1].float() * factor).half()
+    assert torch.equal(sz[..., 1], s)
+    return w, ((q.view(-1, 128, n).half() - z[:, None].half()) * s[:, None]).view(k, n).double()
+
+
+class _Rows:
+    """Two layers of the 7B shape over one token per sequence and an empty cache (attention passes the values through), with a residual
+    stream of a given rms from the embedding on; the normed hidden rows in 64 bits."""
+
+    def __init__(self, batch, rms, seed):
+        from lmdeploy_b200 import llama
+        cfg = llama.LLAMA2_7B
+        hid, inter, layers, vocab = cfg.hidden, cfg.inter_size, 2, 1000
+        self.model = llama.LlamaModel(llama.LlamaConfig(cfg.head_num, cfg.kv_head_num, inter, layers, vocab, quant_policy=0), batch, 8, 0)
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        draw = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+        emb, head = (draw(vocab, hid) * rms).half(), (draw(vocab, hid) * 0.02).half()
+        norms = [(1 + 0.1 * draw(hid)).half() for _ in range(2 * layers + 1)]
+        values, halves = slice(2 * hid, 3 * hid), slice(1, None, 2)  # the value columns; the up columns of (gate, up) pairs
+        norm = lambda v, w: v / torch.sqrt((v * v).mean(-1, keepdim=True) + cfg.norm_eps) * w.double()  # noqa: E731
+        self.ids, self.stream, self.batch = torch.randint(0, vocab, (batch,), generator=g, device="cuda"), torch.cuda.Stream(), batch
+        x, per = emb[self.ids].double(), (rms / 1.6) ** 0.5  # what a half layer adds is as large as the rows
+        self.keep = []
+        for i in range(layers):
+            (wq, eq), (wo, eo) = _scaled(g, 3 * hid, hid, per, values), _scaled(g, hid, hid, per)
+            (wu, eu), (wd, ed) = _scaled(g, 2 * inter, hid, per, halves), _scaled(g, hid, inter, per)
+            self.model.set_layer(i, norms[2 * i], norms[2 * i + 1], wq, wo, wu, wd)
+            self.keep += [wq, wo, wu, wd]
+            x = x + (norm(x, norms[2 * i]) @ eq)[:, values] @ eo
+            y = norm(x, norms[2 * i + 1]) @ eu
+            x = x + (torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2]) @ ed
+        self.model.set_globals(emb, norms[-1], head)
+        self.keep += [emb, head] + norms
+        self.want = norm(x, norms[-1])
+
+    def error(self, fold):
+        """The largest error of a row, relative to it"""
+        self.model.handle.set_option("fold_norm", fold)
+        forced = self.ids.cpu().numpy()[None].astype(np.int32)
+        with torch.cuda.stream(self.stream):
+            st = self.model.new_state(self.batch, 1, forced_ids=forced, keep_hidden=True)
+            self.model.decode(st, 1, use_graph=False, stream=self.stream.cuda_stream)
+            self.model.check_status(self.stream.cuda_stream)
+        self.stream.synchronize()
+        return ((st.hidden.double() - self.want).norm(dim=1) / self.want.norm(dim=1)).max().item()
+
+
+@pytest.mark.parametrize("rms", [5e-4, 2e-3, 0.02, 1.0, 50.0])
+@pytest.mark.parametrize("batch", [1, 8, 24])
+def test_rows_of_any_size(batch, rms):
+    """Against 64 bits, no further off than with norm kernels of their own (the roundings are as many, in other places)."""
+    s = _Rows(batch, rms, batch)
+    folded, separate = s.error(1), s.error(0)
+    s.model.close()
+    assert folded <= 1.1 * separate + 2.0 ** -14, (folded, separate)
