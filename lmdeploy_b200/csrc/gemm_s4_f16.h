@@ -12,14 +12,17 @@ namespace tmb {
 
 // Residual add + RMSNorm folded into the GEMMs on either side in the decode step (decode driver only).
 // Producer side (o_proj, w2): whoever has the whole sum of an output adds the residual, stores it, writes
-// half((residual + y) * norm_weight) as the output and adds up every token's sum of squares.
-// Consumer side (qkv, w13): the rows of the accumulator are scaled by 1 / rms before the output is rounded, which completes
+// half((residual + y) * norm_weight * 2^-(e + 3)) as the output and adds up every token's sum of squares.
+// Consumer side (qkv, w13): the rows of the accumulator are scaled by 2^(e + 3) / rms before the output is rounded, which completes
 // the normalisation of its input.
+// 2^e <= rms < 2^(e + 1) of the row ahead of this addition (kLeastExponent at least), which both sides know.  What is stored has the
+// size of a normalised row, an eighth of it, whatever the size of the rows and weights: it falls among fp16's subnormal numbers no sooner
+// than what counts against the row's other values, and is finite as long as a value times its weight is below 2^19 * 2^e (a norm
+// kernel's output is always; here a row of zeros may not become 2048 in one addition, nor one of rms 1 500000).
 
 // A row's sum of squares.  Its parts (fp32 sums in a fixed order) are added as whole numbers, so that the order of the additions cannot
-// change the result: each to `fine`, in units of 2^(2 e - 24), where 2^e <= rms < 2^(e + 1) of the row ahead of this addition
-// (kLeastExponent at least); or, if it is 2^26 times 2^(2 e) or more, to `coarse`, in units of 2^-13.  Either way it keeps the bits that
-// count in an fp32 sum of the row.  Parts that are no numbers set the upper bit of `coarse`.
+// change the result: each to `fine`, in units of 2^(2 e - 24), or, if it is 2^26 times 2^(2 e) or more, to `coarse`, in units of 2^-13.
+// Either way it keeps the bits that count in an fp32 sum of the row.  Parts that are no numbers set the upper bit of `coarse`.
 struct RowSquares {
     unsigned long long fine, coarse;  // of at most 2^12 parts (16384 values by four)
     int                exponent;      // e
@@ -59,24 +62,23 @@ __device__ __forceinline__ int row_exponent(float mean_square)
 {
     return min(max((((__float_as_int(mean_square) >> 23) & 0xff) - 127) >> 1, kLeastExponent), kMostExponent);
 }
-// consumer: 1 / rms of a row
+// What a row is multiplied by: 2^(e + 3) / rms (consumer), 2^-(e + 3) (producer)
 __device__ __forceinline__ float norm_row_scale(const GemmNormFusion& f, const RowSquares& r)
 {
-    return rsqrtf(row_squares(r) * f.inv_n + f.eps);
+    return rsqrtf(row_squares(r) * f.inv_n + f.eps) * power_of_two(r.exponent + 3);
 }
-// producer: 2^-e
 __device__ __forceinline__ float norm_row_down(const GemmNormFusion& f, const RowSquares& before)
 {
-    return power_of_two(-row_exponent(row_squares(before) * f.inv_n));
+    return power_of_two(-3 - row_exponent(row_squares(before) * f.inv_n));
 }
 __device__ __forceinline__ int exponent_of_down(float down)
 {
-    return 127 - (__float_as_int(down) >> 23);
+    return 127 - 3 - (__float_as_int(down) >> 23);
 }
 // A part of a row's sum
 __device__ __forceinline__ void add_row_squares(RowSquares* at, float part, float down)
 {
-    const float units = part * (down * down * power_of_two(24));
+    const float units = part * (down * down * power_of_two(30));
     if (units < power_of_two(50)) atomicAdd(&at->fine, __float2ull_rn(units));
     else if (part < power_of_two(60)) atomicAdd(&at->coarse, __float2ull_rn(part * power_of_two(13)));
     else atomicOr(&at->coarse, kNotFinite);

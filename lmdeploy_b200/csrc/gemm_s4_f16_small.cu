@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(kThreads, TILES * NT == 1 ? 3 : 2) gemm_s4_f16
             const __half hs = __float2half_rn(s);
             if (valid) {
                 p.norm.residual[(size_t)t * p.N + n] = hs;
-                p.C[(size_t)t * p.N + n]             = __float2half_rn(__half2float(hs) * gain[q]);
+                p.C[(size_t)t * p.N + n]             = __float2half_rn(__half2float(hs) * (gain[q] * row_scale[t]));
             }
             float ss = valid ? s * s : 0.f;  // the eight rows of a token here
 #pragma unroll

@@ -535,7 +535,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 const size_t  at = (size_t)(t0 + t) * p.N + col;
                 *reinterpret_cast<uint2*>(p.norm.residual + at) = make_uint2(word_of(n0), word_of(n1));
                 const float2 a0 = __half22float2(n0), a1 = __half22float2(n1);
-                const float2 g0 = half2_of(gain.x), g1 = half2_of(gain.y);
+                float2       g0 = half2_of(gain.x), g1 = half2_of(gain.y);
+                g0.x *= scale, g0.y *= scale, g1.x *= scale, g1.y *= scale;  // a power of two
                 *reinterpret_cast<uint2*>(p.C + at) =
                     make_uint2(word_of(__floats2half2_rn(a0.x * g0.x, a0.y * g0.y)), word_of(__floats2half2_rn(a1.x * g1.x, a1.y * g1.y)));
                 s_ssq[t * kSquaresLd + quad] = ss;
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 }
 #pragma unroll
                 for (int j = 0; j < kPieces; ++j) {
-                    if (i0 + j * kDqThreads < items) finish(tt[j], (nn[j] - f0) / 4, col0 + nn[j], acc[j], res[j], gain[j], p.norm.ssq_in ? bars->row_scale[tt[j]] : 1.f);
+                    if (i0 + j * kDqThreads < items) finish(tt[j], (nn[j] - f0) / 4, col0 + nn[j], acc[j], res[j], gain[j], p.norm.ssq_in || p.norm.ssq_out ? bars->row_scale[tt[j]] : 1.f);
                 }
             }
         };

@@ -61,7 +61,7 @@ class _Rows:
     """Two layers of the 7B shape over one token per sequence and an empty cache (attention passes the values through), with a residual
     stream of a given rms from the embedding on; the normed hidden rows in 64 bits."""
 
-    def __init__(self, batch, rms, seed):
+    def __init__(self, batch, rms, seed, weight=1.0, jump=1.0):
         from lmdeploy_b200 import llama
         cfg = llama.LLAMA2_7B
         hid, inter, layers, vocab = cfg.hidden, cfg.inter_size, 2, 1000
@@ -69,15 +69,18 @@ class _Rows:
         g = torch.Generator(device="cuda").manual_seed(seed)
         draw = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
         emb, head = (draw(vocab, hid) * rms).half(), (draw(vocab, hid) * 0.02).half()
-        norms = [(1 + 0.1 * draw(hid)).half() for _ in range(2 * layers + 1)]
+        norms = [((1 + 0.1 * draw(hid)) * weight).half() for _ in range(2 * layers)] + [(1 + 0.1 * draw(hid)).half()]
         values, halves = slice(2 * hid, 3 * hid), slice(1, None, 2)  # the value columns; the up columns of (gate, up) pairs
         norm = lambda v, w: v / torch.sqrt((v * v).mean(-1, keepdim=True) + cfg.norm_eps) * w.double()  # noqa: E731
         self.ids, self.stream, self.batch = torch.randint(0, vocab, (batch,), generator=g, device="cuda"), torch.cuda.Stream(), batch
-        x, per = emb[self.ids].double(), (rms / 1.6) ** 0.5  # what a half layer adds is as large as the rows
+        x = emb[self.ids].double()
         self.keep = []
         for i in range(layers):
+            # what a half layer adds is as large as the rows, behind the first feed forward `jump` times as large
+            size = rms * jump if i else rms
+            per, per_ffn = (size / (1.6 * weight)) ** 0.5, (rms * jump / 1.6) ** 0.5 / weight
             (wq, eq), (wo, eo) = _scaled(g, 3 * hid, hid, per, values), _scaled(g, hid, hid, per)
-            (wu, eu), (wd, ed) = _scaled(g, 2 * inter, hid, per, halves), _scaled(g, hid, inter, per)
+            (wu, eu), (wd, ed) = _scaled(g, 2 * inter, hid, per_ffn, halves), _scaled(g, hid, inter, per_ffn)
             self.model.set_layer(i, norms[2 * i], norms[2 * i + 1], wq, wo, wu, wd)
             self.keep += [wq, wo, wu, wd]
             x = x + (norm(x, norms[2 * i]) @ eq)[:, values] @ eo
@@ -106,4 +109,14 @@ def test_rows_of_any_size(batch, rms):
     s = _Rows(batch, rms, batch)
     folded, separate = s.error(1), s.error(0)
     s.model.close()
-    assert folded <= 1.1 * separate + 2.0 ** -14, (folded, separate)
+    assert separate < 0.01 and folded <= 1.1 * separate + 2.0 ** -14, (folded, separate)
+
+
+@pytest.mark.parametrize("rms,weight,jump", [(600.0, 30.0, 1.0), (1500.0, 16.0, 1.0), (0.02, 1e-3, 1.0), (0.02, 1.0, 500.0), (1.0, 0.05, 200.0)])
+@pytest.mark.parametrize("batch", [1, 8, 24])
+def test_rows_and_weights_whose_product_leaves_the_range(batch, rms, weight, jump):
+    """A residual times a norm weight beyond 65504 or among subnormal numbers, and rows that grow by orders of magnitude at once."""
+    s = _Rows(batch, rms, batch, weight, jump)
+    folded, separate = s.error(1), s.error(0)
+    s.model.close()
+    assert separate < 0.01 and folded <= 1.1 * separate + 2.0 ** -14, (folded, separate)
