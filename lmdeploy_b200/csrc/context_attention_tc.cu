@@ -401,15 +401,15 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
         }
     }
     else {
-        // ============================================================ MMA issuer: one elected lane of the warp
-        const uint32_t idesc_qk = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-        const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(kD >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // B is MN-major
-        bool           ok       = true;
-        auto           issue_scores = [&](int t) {
-            const int buf = t & 1;
-            if (!mbar_wait_warp(&bars->k_full[buf], (t >> 1) & 1, p.max_wait_cycles)) return false;
-            tc_after();
-            if (elect_one()) {
+        // ============================================================ MMA issuer: one elected lane of the warp runs the whole loop, as a vote
+        // between its steps would stand in a chain that nothing hides where an SM has one CTA
+        if (elect_one()) {
+            const uint32_t idesc_qk = (1u << 4) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+            const uint32_t idesc_pv = (1u << 4) | (1u << 16) | ((uint32_t)(kD >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);  // B is MN-major
+            auto           issue_scores = [&](int t) {
+                const int buf = t & 1;
+                if (!mbar_wait(&bars->k_full[buf], (t >> 1) & 1, p.max_wait_cycles)) return false;
+                tc_after();
 #pragma unroll
                 for (int blk = 0; blk < 2; ++blk) {
                     const uint64_t dq = desc_kmajor(q_s + blk * kQBlock), dk = desc_kmajor(kv_s + buf * 2 * kTileBytes + blk * kTBlock);
@@ -417,30 +417,28 @@ __global__ void __launch_bounds__(kThreads, 2) context_attention_tc_kernel(CtxPa
                     for (int j = 0; j < 4; ++j) umma_ss(tmem + kColS + buf * kBN, dq + (uint64_t)(2 * j), dk + (uint64_t)(2 * j), idesc_qk, (blk | j) ? 1u : 0u);
                 }
                 umma_commit_to(&bars->s_full[buf]);
-            }
-            __syncwarp();
-            return true;
-        };
-        ok = issue_scores(0);
-        for (int t = 0; t < n_tiles && ok; ++t) {
-            // (the columns that tile t + 1's scores take held tile t - 1's probabilities, whose product was issued before)
-            ok = (t + 1 >= n_tiles || issue_scores(t + 1)) && mbar_wait_warp(&bars->p_full, t & 1, p.max_wait_cycles);
-            if (!ok) break;
-            tc_after();
-            const uint64_t dv = desc_mnmajor(kv_s + (t & 1) * 2 * kTileBytes + kTileBytes, kTBlock);
-            if (elect_one()) {
+                return true;
+            };
+            bool ok = issue_scores(0);
+            for (int t = 0; t < n_tiles && ok; ++t) {
+                // The columns that tile t + 1's scores take hold tile t - 1's probabilities: not before their product is complete (products
+                // of different shapes and accumulators are not promised to run in order)
+                if (t > 0 && t + 1 < n_tiles) ok = mbar_wait(&bars->pv_done, (t - 1) & 1, p.max_wait_cycles);
+                ok = ok && (t + 1 >= n_tiles || issue_scores(t + 1)) && mbar_wait(&bars->p_full, t & 1, p.max_wait_cycles);
+                if (!ok) break;
+                tc_after();
+                const uint64_t dv = desc_mnmajor(kv_s + (t & 1) * 2 * kTileBytes + kTileBytes, kTBlock);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) umma_ts(tmem + kColO, tmem + kColS + (t & 1) * kBN + 8 * j, dv + (uint64_t)(128 * j), idesc_pv, (t | j) ? 1u : 0u);
                 umma_commit_to(&bars->pv_done);
             }
-            __syncwarp();
-        }
-        if (!ok && (tid & 31) == 0) {
-            atomicOr(p.status, kStatusGemmPipeWait);
-            *(volatile int*)&bars->dead = 1;
+            if (!ok) {
+                atomicOr(p.status, kStatusGemmPipeWait);
+                *(volatile int*)&bars->dead = 1;
+            }
+            umma_commit_to(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
         }
         __syncwarp();
-        if (elect_one()) umma_commit_to(&bars->o_full);  // arrives when everything issued so far is complete (also on the give-up path)
     }
 
     tc_before();
