@@ -81,8 +81,9 @@ public:
     bool in_order() { return nested_ || !captured(); }
     bool begin(ScratchArea area);  // ahead of the first launch; false: a CUDA call failed
     // A direct call's kernels carry the attribute too, but wait for the kernel ahead before they read anything (late_weight): what
-    // they gain is its way out and their own launch (a plain launch of a 6 us kernel takes 8.2 us).  Not into a caller's capture.
-    bool dependent() { return h_->pdl != 0 && in_order(); }
+    // they gain is its way out and their own launch (a plain launch of a 6 us kernel takes 8.2 us).  Not into a caller's capture; inside
+    // a driver's call the driver says (g_pdl).
+    bool dependent() { return h_->pdl != 0 && !nested_ && !captured(); }
     bool hold();                   // all areas, for every call of this host thread on the handle until this object ends
 
 private:

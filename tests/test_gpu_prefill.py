@@ -391,3 +391,51 @@ def test_writers_never_leave_their_buffers():
     case["pad"] = np.asarray([0, 0, 100, -50], np.int32)          # tokens 2 and 3 point outside [1, 4]
     q, k, v = run_qkv(case, "ours", None)
     assert q[0, :, :2].any() and not q[0, :, 2:].any() and not k[0, :, 2:].any() and not v[0, :, 2:].any()
+
+
+def _programmatic_edges(graph):
+    """How many edges of a captured graph let a kernel start before the one ahead is complete, and how many there are"""
+    rt = C.CDLL("libcudart.so.12")
+    n = C.c_size_t(0)
+    args = [C.c_void_p(graph.raw_cuda_graph()), None, None, None, C.byref(n)]
+    assert rt.cudaGraphGetEdges_v2(*args) == 0
+    ends, data = [(C.c_void_p * n.value)() for _ in range(2)], (C.c_ubyte * (8 * n.value))()
+    args[1], args[2], args[3] = ends[0], ends[1], data
+    assert rt.cudaGraphGetEdges_v2(*args) == 0
+    return sum(data[8 * i + 2] == 1 for i in range(n.value)), n.value
+
+
+def test_a_prefill_that_the_caller_captures_is_plain_launches():
+    from lmdeploy_b200 import lib as l
+    from tests.test_gpu_llama import CFG, build
+    model, _, _ = build(False)
+    tokens = [[5, 6, 7, 8, 9, 10, 11], [20, 21]]
+    kept, real = [], l.lib.tm_llama_prefill
+
+    class Lib:  # the call's arguments, for a second one into a capture
+        def __getattr__(self, name):
+            return getattr(real_lib, name)
+
+        def tm_llama_prefill(self, m, state, stream):
+            kept.append((m, l.TmLlamaPrefillState.from_buffer_copy(state._obj)))
+            return real(m, state, stream)
+    real_lib, l.lib = l.lib, Lib()
+    try:
+        st = model.new_state(2, 1)
+        want = model.prefill(st, tokens, keep_hidden=True).clone()
+    finally:
+        l.lib = real_lib
+    m, c = kept[0]
+    ids, cu = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in (sum(tokens, []), [0, 7, 9]))
+    hist, ctx, hidden = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.tensor([7, 2], dtype=torch.int32, device="cuda"), torch.zeros_like(want)
+    c.input_ids, c.cu_seqlens, c.history_lengths, c.context_lengths, c.hidden_out = (t.data_ptr() for t in (ids, cu, hist, ctx, hidden))
+    graph, stream = torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        l.check(real(m, C.byref(c), stream.cuda_stream), "tm_llama_prefill")
+    assert _programmatic_edges(graph)[0] == 0 and _programmatic_edges(graph)[1] >= 7 * CFG["num_layer"]
+    graph.instantiate()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(hidden, want)
+    model.close()
