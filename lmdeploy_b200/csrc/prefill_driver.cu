@@ -71,8 +71,10 @@ extern "C" int tm_llama_prefill(tm_llama* m, const tm_llama_prefill_state* st, v
     cudaStream_t s   = (cudaStream_t)stream;
     ScratchUse   use(m->h, s);
     if (!use.hold()) return TM_ERR_CUDA;
-    // The gap ahead of a plain launch is 2 us, twelve times a layer (3 sequences, 735 tokens: 1750 us, 1632 as dependent launches);
-    // kernels of many waves gain nothing (8 x 2048 tokens: 53.3 and 53.9 ms).
+    // The gap ahead of a plain launch is 2 us, twelve times a layer: dependent launches gain where a layer is short, and up to 3000 tokens
+    // by more than runs differ.  Medians of four, us, plain / dependent: 7B, 2 layers, 256 tokens 504 / 472, 512 681 / 648, 1024 1022 / 977,
+    // 3072 2656 / 2606, 4096 3478 / 3480, 8192 6447 / 6461, 16384 12826 / 13189; 70B, 1 layer, 256 593 / 612, 1024 1774 / 1751, 8192
+    // 12602 / 12690.
     PdlScope     pdl_scope(T <= 4096 && use.dependent());
     int          prev = 0;
     cudaGetDevice(&prev);
