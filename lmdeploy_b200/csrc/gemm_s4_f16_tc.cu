@@ -614,18 +614,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 const long long t_begin = clock64();
                 for (;;) {
                     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(arrive + tjs) : "memory");
-                    if (seen >= n_split * kDqWarps || clock64() - t_begin > p.max_wait_cycles) break;
+                    if (seen >= n_split || clock64() - t_begin > p.max_wait_cycles) break;
                     __nanosleep(32);
                 }
-                if (seen < n_split * kDqWarps) atomicOr(p.status, kStatusGemmTmemWait);
-                bars->flag = seen >= n_split * kDqWarps;
+                if (seen < n_split) atomicOr(p.status, kStatusGemmTmemWait);
+                bars->flag = seen >= n_split;
             }
             named_bar_sync(1, kDqThreads);
             TC_TRACE(trow, 42, tjs);
             const bool tile_ok = p.last_sums || bars->flag != 0;  // read between the barriers: the next call may rewrite the flag
             int through = 0;
             if (dtid == 0 && !p.last_sums) {
-                // looked at behind the sums; a CTA that gave up has seen no full count that says that its own warps' have arrived
+                // looked at behind the sums; a CTA that gave up has seen no full count that says that its own has arrived
                 if (!tile_ok) __threadfence();
                 through = atomicAdd(done + tjs, 1);
                 if (!tile_ok) __threadfence();
@@ -834,12 +834,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             if (lane == 0 && !dead) mbar_arrive(&bars->acc_empty[m]);
             TC_TRACE(trow, 37, this_js);
             if (n_split > 1) {
-                // Publish the partial (its reduction waits until this CTA has no units left).  Each warp counts itself in: the warp's
-                // barrier orders its lanes' stores before the release of the one that counts.
-                if (!p.last_sums && lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrive + this_js) : "memory");
+                // Publish the partial (its reduction waits until this CTA has no units left): the barrier orders every thread's stores before
+                // the release of the one thread that then counts the CTA in.  (Each warp counting itself in: sixteen releases instead of one,
+                // 4096 x 4096 with 16 / 32 / 64 / 128 tokens 8.1 / 8.8 / 9.8 / 13.2 us, 7.8 / 8.2 / 9.2 / 12.4 so; 4096 x 11008 with 64
+                // 14.4 and 13.8.)
+                named_bar_sync(1, kDqThreads);
+                if (!p.last_sums && dtid == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrive + this_js) : "memory");
                 if (p.last_sums) {
-                    // the barrier orders every thread's stores before the fence of the one thread that then counts the CTA in
-                    named_bar_sync(1, kDqThreads);
                     if (dtid == 0) {
                         __threadfence();
                         const int before = atomicAdd(arrive + this_js, 1);
