@@ -14,11 +14,13 @@ thread_local const GemmNormFusion* g_gemm_fusion = nullptr;
 
 // The tcgen05 kernel, or the small-token ones?  Unless the caller drew the line: from 17 tokens on, and with 9 to 16 except for
 // products that the column-owner kernel does in one go of short rows, where the other's set-up and exchange weigh more than
-// its own re-reading of the activations (us, column owner / tcgen05: 4096 x 4096 with 12 tokens 9.0 / 9.9, 8192 x 1024 with
-// 16 tokens 6.2 / 8.4; 4096 x 11008 with 9 tokens 16.1 / 14.1, 8192 x 3584 with 16 13.8 / 11.6; stream-K for 57344 x 8192 with
-// 16 tokens 87 / 75).  There the weight is rounded to fp16((q - z) s), the format's own value, before the product, where the small-token
-// kernels keep whole numbers and a scale per group: against 64-bit sums of those values the error falls (11008 x 4096, 16 tokens,
-// 2.76e-4 / 2.07e-4).
+// its own re-reading of the activations.  In a row of dependent launches, us, column owner / tcgen05: 4096 x 4096 with 9 / 12 / 14 / 16
+// tokens 7.0 / 7.7 / 8.2 / 8.8 and 7.8 throughout, 8192 x 1024 4.1 / 4.6 / 4.8 / 5.1 and 6.6, 4096 x 11008 14.2 / 15.8 / 17.2 / 18.6 and
+// 11.7, 11008 x 4096 15.0 / 16.0 / 16.8 / 17.6 and 11.2; stream-K for 57344 x 8192 82 / 83 / 84 / 85 and 67.  Of the thirteen projections of
+// perf/cases.py the line takes the slower side for two: 8192 x 3584 with 10 to 14 tokens (10.3 and 9.2 with 12), 1280 x 8192 (6.5 / 7.0 /
+// 7.6 / 8.1 and 8.3).  The tcgen05 kernel rounds the weight to fp16((q - z) s), the format's own value, before the product, where the
+// small-token kernels keep whole numbers and a scale per group: against 64-bit sums of those values the error falls (11008 x 4096, 16
+// tokens, 2.76e-4 / 2.07e-4).
 static bool gemm_uses_tc(const tm_handle* h, int m, int n, int k)
 {
     if (h->gemm_tc_min_n >= 0) return n >= h->gemm_tc_min_n;

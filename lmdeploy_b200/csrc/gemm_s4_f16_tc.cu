@@ -970,8 +970,9 @@ GemmTcPlan gemm_tc_plan(int N, int T, int K, int sm_count, bool balance)
         pl.us = cut_us(pl.units_per_cta);
     }
     // Tiles that are cut only because it is faster are summed by the CTA that is done last: a product of that size never depended on
-    // its CTAs running together (4096 x 11008 with 1200 tokens 104.0 us, 105.0 with the wait; 57344 x 8192 with 32 tokens 79.9 / 81.8).
-    // With fewer tiles than SMs every CTA sums a share (4096 x 11008 with 16 / 64 tokens: 13.7 / 15.7 us, by the last one 15.0 / 25.2).
+    // its CTAs running together, and loses nothing by it (us, last one / each a share, two runs: 57344 x 8192 with 32 tokens 68, 71 / 74, 72,
+    // with 128 108, 110 / 110, 116; 8192 x 28672 with 300 tokens 150, 155 / 155, 152; 4096 x 11008 with 1200 130, 127 / 134, 126).
+    // With fewer tiles than SMs every CTA sums a share (4096 x 11008 with 16 / 64 tokens: 11.7 / 13.9 us, by the last one 12.8 / 22.9).
     pl.last_sums       = could && !whole;
     pl.slots_per_chunk = pl.ctas + pl.n_col_tiles;
     pl.smem_bytes      = gemm_tc_smem_bytes(pl.token_tile);
