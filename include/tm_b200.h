@@ -78,8 +78,9 @@ TM_API unsigned long long tm_launch_count(const tm_handle* h);
  * "gemv_cols" (the GEMM for few tokens: 0 = always the stream-K kernel, 1 = the column-owner kernel on 32-column strips where
  * all of them are resident at once, up to 16 tokens, 2 = on 64-column strips, up to 8 tokens),
  * "mmha_chunk" (cached tokens per KV split, 0 = automatic), "mmha_warps" (warps per attention CTA: 1, 2,
- * 4 or 0 = automatic), "pdl" (1 = programmatic dependent launch: the decode step, prefill of up to 4096 tokens, and
- * direct GEMM / MoE calls outside a capture, which wait for the kernel ahead before they read anything).
+ * 4 or 0 = automatic), "pdl" (1 = programmatic dependent launch: the decode step, prefill of up to 2048 tokens, the
+ * W4A16 products of a longer one, and direct GEMM / MoE calls; but for the decode step's, not into a capture of the caller's.  Direct
+ * calls and those products wait for the kernel ahead before they read anything).
  * Returns TM_ERR_INVALID_ARG for an unknown name or value. */
 TM_API int tm_set_option(tm_handle* h, const char* name, int value);
 

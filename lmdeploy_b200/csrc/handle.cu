@@ -12,7 +12,8 @@
 using namespace tmb;
 
 namespace tmb {
-thread_local int g_pdl = 0;
+thread_local int  g_pdl          = 0;
+thread_local bool g_pdl_products = false;
 
 namespace {
 thread_local const tm_handle* t_scratch_holder = nullptr;

@@ -64,9 +64,11 @@ struct KernelPreparation {
 // programmatic-dependent-launch attribute, and read weights before the kernel ahead is complete.  Direct callers may put any kernel
 // in front of ours: ScratchUse::dependent.
 extern thread_local int g_pdl;
+// ... and whether the W4A16 products alone, inside a driver's call, carry it (as direct calls: ScratchUse::dependent).
+extern thread_local bool g_pdl_products;
 struct PdlScope {
-    explicit PdlScope(int on) { g_pdl = on; }
-    ~PdlScope() { g_pdl = 0; }
+    explicit PdlScope(int on, bool products = false) { g_pdl = on, g_pdl_products = products; }
+    ~PdlScope() { g_pdl = 0, g_pdl_products = false; }
 };
 
 // Held by a call around the launches that use the handle's scratch and tickets.  Calls of one stream are in order by themselves; a
@@ -82,8 +84,8 @@ public:
     bool begin(ScratchArea area);  // ahead of the first launch; false: a CUDA call failed
     // A direct call's kernels carry the attribute too, but wait for the kernel ahead before they read anything (late_weight): what
     // they gain is its way out and their own launch (a plain launch of a 6 us kernel takes 8.2 us).  Not into a caller's capture; inside
-    // a driver's call the driver says (g_pdl).
-    bool dependent() { return h_->pdl != 0 && !nested_ && !captured(); }
+    // a driver's call the driver says.
+    bool dependent() { return h_->pdl != 0 && (nested_ ? g_pdl_products : !captured()); }
     bool hold();                   // all areas, for every call of this host thread on the handle until this object ends
 
 private:

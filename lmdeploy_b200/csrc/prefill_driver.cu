@@ -71,11 +71,12 @@ extern "C" int tm_llama_prefill(tm_llama* m, const tm_llama_prefill_state* st, v
     cudaStream_t s   = (cudaStream_t)stream;
     ScratchUse   use(m->h, s);
     if (!use.hold()) return TM_ERR_CUDA;
-    // The gap ahead of a plain launch is 2 us, twelve times a layer: dependent launches gain where a layer is short, and up to 3000 tokens
-    // by more than runs differ.  Medians of four, us, plain / dependent: 7B, 2 layers, 256 tokens 504 / 472, 512 681 / 648, 1024 1022 / 977,
-    // 3072 2656 / 2606, 4096 3478 / 3480, 8192 6447 / 6461, 16384 12826 / 13189; 70B, 1 layer, 256 593 / 612, 1024 1774 / 1751, 8192
-    // 12602 / 12690.
-    PdlScope     pdl_scope(T <= 4096 && use.dependent());
+    // The gap ahead of a plain launch is 2 us, twelve times a layer: short prefills gain by dependent launches.  In long ones only the
+    // W4A16 products do, whose set-up is long; the other kernels' early CTAs take slots from those still at work.  Means of four, us,
+    // plain / products / all: 7B, 4 layers, 256 tokens 860 / 819 / 794, 1024 1971 / 1944 / 1929, 3072 5207 / 5165 / 5272, 4096 6731 / 6713 / 6777,
+    // 6144 9648 / 9548 / 9800, 16384 (8 layers) 50708 / 50143 / 51477; 70B, 2 layers, 2048 6955 / 6953 / 6916, 8192 24900 / 24593 / 24816.
+    const bool   dependent = use.dependent();
+    PdlScope     pdl_scope(dependent && T <= 2048, dependent);
     int          prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(m->h->device);
