@@ -35,7 +35,10 @@ def _ptr(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 
 
-def _stream() -> int:
+def _stream(stream=None):
+    """The caller's stream, which has to be a whole number (ctypes alone would take the address of a bytes object for one), or the current one"""
+    if stream is not None:
+        return C.c_void_p(stream)
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
@@ -77,7 +80,7 @@ class GemmS4F16:
     def Run(self, C_out, A, B, Q, m, n, k, group_size, type, algo_id=-1, stream=None):
         """C[n, m] = B[n, k] . dequant(A, Q)^T  (m = output features, n = tokens)."""
         _need_cuda(C_out, A, B, Q)
-        st = _stream() if stream is None else stream
+        st = _stream(stream)
         s = _l.lib.tm_gemm_s4_f16(self.handle.ptr, _ptr(C_out), _ptr(A), _ptr(B), _ptr(Q), int(m), int(n), int(k),
                                   int(group_size), int(type), None, 0, st)
         _l.check(s, "GemmS4F16.Run")
@@ -197,19 +200,19 @@ def masked_multihead_attention(params: Masked_multihead_attention_params, stream
                                                                       int(p.use_logn_attn))
     c.rotary_embedding_base = p.rotary_embedding_base
     h = handle or _l.default_handle(p.out.device.index)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_mmha_decode(h.ptr, C.byref(c), st), "masked_multihead_attention")
 
 
 def invokeRootMeanSquareNorm(out, input, scale, eps, m, n, stream=None):
     _need_cuda(out, input, scale)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_rmsnorm(_ptr(out), _ptr(input), _ptr(scale), eps, m, n, st), "invokeRootMeanSquareNorm")
 
 
 def invokeFusedAddBiasResidualRMSNorm(residual, in_out, bias, scale, eps, batch_size, n_dims, stream=None):
     _need_cuda(residual, in_out, bias, scale)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_add_residual_rmsnorm(_ptr(residual), _ptr(in_out), _ptr(bias), _ptr(scale), eps, batch_size,
                                             n_dims, st), "invokeFusedAddBiasResidualRMSNorm")
 
@@ -232,7 +235,7 @@ def invokeAddFusedQKVBiasTranspose(q_buf, k_buf, v_buf, QKV, qkv_bias, padding_o
                                    rotary_embedding_dim, rotary_embedding_base, max_position_embeddings, use_dynamic_ntk,
                                    use_logn_attn, stream=None):
     _need_cuda(q_buf, k_buf, v_buf, QKV, qkv_bias, padding_offset, history_length, input_length)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_add_fused_qkv_bias_transpose(
         _ptr(q_buf), _ptr(k_buf), _ptr(v_buf), _ptr(QKV), _ptr(qkv_bias), _ptr(padding_offset), _ptr(history_length),
         _ptr(input_length), batch_size, seq_len, token_num, head_num, kv_head_num, size_per_head, rotary_embedding_dim,
@@ -244,7 +247,7 @@ def invokeExtendKVCache(k_dst, v_dst, dst_offset, k_src, v_src, local_batch_size
                         max_seq_len, size_per_head, local_head_num, stream=None, quant=0, kv_scale=None):
     """k_dst / v_dst: int64 device tensors holding one cache base pointer per sequence."""
     _need_cuda(k_dst, v_dst, k_src, v_src, query_length, history_length)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_extend_kv_cache(_ptr(k_dst), _ptr(v_dst), dst_offset, _ptr(k_src), _ptr(v_src), local_batch_size,
                                        _ptr(query_length), max_q_len, _ptr(history_length), max_seq_len, size_per_head,
                                        local_head_num, st, quant, _kv_scale(kv_scale)), "invokeExtendKVCache")
@@ -254,7 +257,7 @@ def invokeTransposeKVCache(key_cache_trans, val_cache_trans, key_cache, val_cach
                            max_kv_len, max_seq_len, size_per_head, head_num, head_n_rep, stream=None, quant=0,
                            kv_scale=None):
     _need_cuda(key_cache_trans, val_cache_trans, key_cache, val_cache, key_length)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_transpose_kv_cache(_ptr(key_cache_trans), _ptr(val_cache_trans), _ptr(key_cache), _ptr(val_cache),
                                           src_offset, batch_size, _ptr(key_length), max_kv_len, max_seq_len, size_per_head,
                                           head_num, head_n_rep, st, quant, _kv_scale(kv_scale)), "invokeTransposeKVCache")
@@ -275,5 +278,5 @@ def fusedMultiHeadAttention(attn_out, query, key_cache_ptrs, val_cache_ptrs, cac
     a.max_q_len, a.max_seq_len, a.quant_policy = max_q_len, max_seq_len, quant_policy
     if kv_scale is not None:
         a.kv_scale = _kv_scale(kv_scale)
-    st = _stream() if stream is None else stream
+    st = _stream(stream)
     _l.check(_l.lib.tm_context_attention(C.byref(a), st), "fusedMultiHeadAttention")
