@@ -30,31 +30,6 @@
 #include <algorithm>
 #include <mutex>
 
-#ifdef TM_B200_GEMM_TRACE
-// Developer build only (never defined by lmdeploy_b200/build.py): per-CTA time stamps of one launch.
-__device__ unsigned long long g_small_trace[640][4];  // start, first data, loop end, end (globaltimer ns)
-__device__ int                g_small_launch;
-extern "C" __attribute__((visibility("default"))) int tm_dev_gemv_trace(unsigned long long* out, int want_launch)
-{
-    cudaMemcpyFromSymbol(out, g_small_trace, sizeof(unsigned long long) * 640 * 4);
-    int z = -want_launch;   // the launch that reaches 0 is recorded
-    cudaMemcpyToSymbol(g_small_launch, &z, sizeof(z));
-    return 0;
-}
-__device__ __forceinline__ unsigned long long small_globaltimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-#define SMALL_TRACE(slot)                                                                                              \
-    do {                                                                                                                   \
-        if (trace_on && threadIdx.x == 0 && blockIdx.x < 640) g_small_trace[blockIdx.x][slot] = small_globaltimer();       \
-    } while (0)
-#else
-#define SMALL_TRACE(slot) do { } while (0)
-#endif
-
 namespace tmb {
 
 namespace {
@@ -134,10 +109,6 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
     const int lane = tid & 31;
     const int r    = lane >> 2;  // fragment row
     const int c    = lane & 3;   // fragment column pair
-#ifdef TM_B200_GEMM_TRACE
-    const bool trace_on = *(volatile int*)&g_small_launch == 0 && blockIdx.y == 0;
-    SMALL_TRACE(0);
-#endif
 
     // token chunk handled by this CTA row
     const int t0     = blockIdx.y * TP;
@@ -270,7 +241,6 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             cp_async_wait<ST - 2>();
-            if (it == 0 && u == 0) SMALL_TRACE(1);
             // every thread's copies for this unit have landed, and every warp is done with the unit before
             __syncthreads();
             if (to_issue > 0) issue_unit(s_fill, true);
@@ -356,7 +326,6 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                     tot[w][a][j][2] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[j][0], acc[w][a][j][2]), tot[w][a][j][2]);
                     tot[w][a][j][3] = fmaf(sh[w][a], fmaf(-zh[w][a], sx[j][1], acc[w][a][j][3]), tot[w][a][j][3]);
                 }
-        if (it + 2 >= n_units) SMALL_TRACE(2);
         const int  this_jt = jt;
         const int  tile0   = jt * kTilesPerUnit;
         const int  ntw     = min(kTilesPerUnit, n_tiles32 - tile0) - my_t0;  // tiles of this warp that exist
@@ -497,11 +466,6 @@ __global__ void __launch_bounds__(kThreads, ctas_per_sm_for(NT)) gemm_s4_f16_sma
                     for (int i = 0; i < 4; ++i) tot[w][a][j][i] = 0.f;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-#ifdef TM_B200_GEMM_TRACE
-    SMALL_TRACE(3);
-    __syncthreads();
-    if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) atomicAdd(&g_small_launch, 1);
-#endif
 }
 
 // ---- column-owner variant for up to 16 tokens -------------------------------------------------------------------

@@ -34,57 +34,6 @@
 #include <array>
 #include <cuda.h>  // CUtensorMap (types only: the encoder is looked up through the runtime)
 
-#ifdef TM_B200_GEMM_TRACE
-// Developer build only (never defined by lmdeploy_b200/build.py): time stamps of selected warps of selected CTAs.
-__device__ long long g_tc_trace[8][2048];
-__device__ int       g_tc_trace_n[8];
-__device__ unsigned long long g_tc_span[512][2];  // per launch: first CTA start, last CTA end (globaltimer ns)
-__device__ int                g_tc_launch;
-__device__ unsigned long long g_tc_cta[160][4];   // launch 5: per CTA start, end (ns), smid, units
-extern "C" __attribute__((visibility("default"))) int tm_dev_gemm_ctas(unsigned long long* out)
-{
-    cudaMemcpyFromSymbol(out, g_tc_cta, sizeof(unsigned long long) * 640);
-    return 0;
-}
-extern "C" __attribute__((visibility("default"))) int tm_dev_gemm_spans(unsigned long long* out, int reset)
-{
-    cudaMemcpyFromSymbol(out, g_tc_span, sizeof(unsigned long long) * 1024);
-    if (reset) {
-        static unsigned long long init[1024];
-        for (int i = 0; i < 512; ++i) { init[2 * i] = ~0ull; init[2 * i + 1] = 0ull; }
-        cudaMemcpyToSymbol(g_tc_span, init, sizeof(init));
-        int z = 0;
-        cudaMemcpyToSymbol(g_tc_launch, &z, sizeof(z));
-    }
-    return 0;
-}
-__device__ __forceinline__ unsigned long long tc_globaltimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-extern "C" __attribute__((visibility("default"))) int tm_dev_gemm_trace(long long* out, int* counts)
-{
-    cudaMemcpyFromSymbol(out, g_tc_trace, sizeof(long long) * 8 * 2048);
-    cudaMemcpyFromSymbol(counts, g_tc_trace_n, sizeof(int) * 8);
-    int zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    cudaMemcpyToSymbol(g_tc_trace_n, zero, sizeof(zero));
-    return 0;
-}
-#define TC_TRACE(row, tag, unit)                                                                                       \
-    do {                                                                                                                   \
-        if ((row) >= 0 && (threadIdx.x & 31) == 0 && trace_i < 2046) {                                                     \
-            g_tc_trace[row][trace_i]     = ((long long)(tag) << 32) | (unsigned)(unit);                                    \
-            g_tc_trace[row][trace_i + 1] = clock64();                                                                      \
-            trace_i += 2;                                                                                                  \
-            g_tc_trace_n[row] = trace_i;                                                                                   \
-        }                                                                                                                  \
-    } while (0)
-#else
-#define TC_TRACE(row, tag, unit) do { } while (0)
-#endif
-
 namespace tmb {
 namespace {
 
@@ -133,7 +82,6 @@ struct Bars {
     float    row_scale[128];  // factor of a token (either side of a folded norm)
 };
 constexpr int kSquaresLd = 33;  // sums of squares of a token (producer of a folded norm): a share of a split tile has at most 32 quads of features
-
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
 {
@@ -294,17 +242,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     const int tid  = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-#ifdef TM_B200_GEMM_TRACE
-    int trow = -1, trace_i = 0;
-    if (blockIdx.x == 0 && blockIdx.y == 0) trow = warp == 0 ? 0 : warp == 1 ? 1 : warp == kDqWarp0 ? 2 : warp == kDqWarp0 + 8 ? 3 : -1;
-    if (blockIdx.x == 64 && blockIdx.y == 0) trow = warp == kDqWarp0 ? 4 : warp == 1 ? 5 : warp == kDqWarp0 + 5 ? 6 : -1;
-    if (blockIdx.x == gridDim.x - 1 && blockIdx.y == 0) trow = warp == kDqWarp0 ? 7 : trow;
-    TC_TRACE(trow, 1, 0);
-    const int launch_idx = *(volatile int*)&g_tc_launch;
-    const long long clk_begin = clock64();
-    const unsigned long long gt_begin = tc_globaltimer();
-    if (tid == 0 && launch_idx < 512) atomicMin(&g_tc_span[launch_idx][0], gt_begin);
-#endif
 
     const int t0     = blockIdx.y * 128;
     const int t_rows = min(TT, p.T - t0);
@@ -326,7 +263,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         c_first = (tile * G) / upc;
         return ((tile + 1) * G - 1) / upc - c_first + 1;
     };
-    const int n_tiles32 = p.N / 32;
 
     const int  dw = warp - kDqWarp0;  // 0..15 for the expanding warps
     // A unit's packed weight, four slabs of eight adjacent tiles, and its row of {zero, scale}: a box each (zeros beyond N).  Copies of
@@ -382,7 +318,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem   = bars->tmem_base;
-    TC_TRACE(trow, 2, 0);
     const uint32_t a_base = tmem + kTeams * accS;  // first expanded-weight stage
 
     if (warp == 0) {
@@ -397,7 +332,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
         if (elect_one()) {
             int g = u_begin % G, it = 0, st = 0;
             for (uint32_t ph = 1; it < n_units; ++it) {  // (a fresh barrier counts as having completed the phase before)
-                TC_TRACE(trow, 10, it);
                 if (!mbar_wait(&bars->x_empty[st], ph)) {
                     atomicOr(p.status, kStatusGemmPipeWait);
                     break;
@@ -464,7 +398,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     ok = ok && mbar_wait(&bars->a_full[m][sa], pa);
                     if (!ok) break;
                     tc_fence_after();
-                    TC_TRACE(trow, 20, it);
                     const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols;
                     umma_f16_ts_x4(d_tmem, a_tmem, lo + part * kb_step, d_hi, idesc, part == 0 && first ? 1u : 0u);
                     if (S::kParts == 1) umma_f16_ts_x4(d_tmem, a_tmem + 32, lo + kb_step, d_hi, idesc, 0u);
@@ -476,7 +409,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                     break;
                 }
                 umma_commit(&bars->x_empty[sx]);
-                TC_TRACE(trow, 21, it);
                 first = last;
                 if (last) {
                     umma_commit(&bars->acc_full[m]);
@@ -621,7 +553,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 bars->flag = seen >= n_split;
             }
             named_bar_sync(1, kDqThreads);
-            TC_TRACE(trow, 42, tjs);
             const bool tile_ok = p.last_sums || bars->flag != 0;  // read between the barriers: the next call may rewrite the flag
             int through = 0;
             if (dtid == 0 && !p.last_sums) {
@@ -681,7 +612,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             const int this_js = js;
             const int seg_end = it + min(G - g, n_units - it);
             for (; u < seg_end; u += 2) {
-                TC_TRACE(trow, 30, u);
                 warp_wait(w_full + sw * 8, pw, dead, p.status, kStatusGemmPipeWait);
                 const uint32_t wa = my_w + sw * kWStage, qa = my_q + sw * kWStage;
                 const uint32_t qv[4]     = {shared_load4<0>(qa), shared_load4<32>(qa), shared_load4<64>(qa), shared_load4<96>(qa)};
@@ -731,7 +661,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                         // once: a fresh barrier counts as having completed the phase before)
                         warp_wait(a_empty + sa * 8, pa ^ 1u, dead, p.status, kStatusGemmPipeWait);
                         tc_fence_after();
-                        TC_TRACE(trow, 32, u);
                     }
                     // rows q*32 + a*16 .. +15 (TMEM lanes), k = 64 half .. +63 (32 columns)
                     const uint32_t a_tmem = a_base + (m * kAST + sa) * kACols + a_lane + (begins ? 0u : 32u);
@@ -743,7 +672,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) arrive_at(a_full + sa * 8);
-                        TC_TRACE(trow, 33, u);
                         if (half == 0) {
                             ++sa;  // the unit's second stage; kAST is even then
                         }
@@ -774,10 +702,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             int       c_first;
             const int n_split = tile_ctas(this_js, c_first);
             const int col0    = this_js * kSuperN;
-            TC_TRACE(trow, 34, this_js);
             warp_wait(smem_u32(&bars->acc_full[m]), seg_idx & 1, dead, p.status, kStatusGemmTmemWait);
             tc_fence_after();
-            TC_TRACE(trow, 35, this_js);
             const int n_glob = col0 + n_row;
             const uint32_t my_acc = tmem + m * accS + ((uint32_t)(q * 32) << 16);
             if (!dead) {
@@ -832,7 +758,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
             tc_fence_before();
             __syncwarp();
             if (lane == 0 && !dead) mbar_arrive(&bars->acc_empty[m]);
-            TC_TRACE(trow, 37, this_js);
             if (n_split > 1) {
                 // Publish the partial (its reduction waits until this CTA has no units left): the barrier orders every thread's stores before
                 // the release of the one thread that then counts the CTA in.  (Each warp counting itself in: sixteen releases instead of one,
@@ -857,12 +782,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
                 }
                 pend[n_pend++] = this_js;
             }
-            TC_TRACE(trow, 38, this_js);
         }
-        TC_TRACE(trow, 40, 0);
         for (int i = 0; i < n_pend; ++i) {
             reduce_share(pend[i]);
-            TC_TRACE(trow, 41, i);
         }
     }
 
@@ -871,28 +793,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_s4_f16_tc_kernel(GemmTcParam
     if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kTmemCols) : "memory");
     }
-#ifdef TM_B200_GEMM_TRACE
-    if (tid == 0 && launch_idx < 512) {
-        atomicMax(&g_tc_span[launch_idx][1], tc_globaltimer());
-        if (launch_idx == 5 && blockIdx.x < 160 && blockIdx.y == 0) {
-            unsigned smid;
-            asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-            g_tc_cta[blockIdx.x][0] = gt_begin;
-            g_tc_cta[blockIdx.x][1] = tc_globaltimer();
-            g_tc_cta[blockIdx.x][2] = smid;
-            g_tc_cta[blockIdx.x][3] = (unsigned long long)n_units;
-        }
-        if (blockIdx.x == 0 && blockIdx.y == 0) {
-            if (launch_idx + 256 < 512) {   // CTA 0's own duration in SM cycles and in ns, stored 256 rows further down
-                g_tc_span[launch_idx + 256][0] = (unsigned long long)(clock64() - clk_begin);
-                g_tc_span[launch_idx + 256][1] = tc_globaltimer() - gt_begin;
-            }
-            // the last thing CTA 0 does; every CTA of the launch has long read the index
-            __threadfence();
-            atomicAdd(&g_tc_launch, 1);
-        }
-    }
-#endif
 }
 
 using PFN_encodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

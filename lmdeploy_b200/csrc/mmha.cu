@@ -23,31 +23,6 @@
 #include <algorithm>
 #include <cfloat>
 
-#ifdef TM_B200_GEMM_TRACE
-// Developer build only (never defined by lmdeploy_b200/build.py): per-CTA time stamps of one launch.
-__device__ unsigned long long g_mmha_trace[4096][12];
-__device__ int                g_mmha_launch;
-extern "C" __attribute__((visibility("default"))) int tm_dev_mmha_trace(unsigned long long* out, int want_launch)
-{
-    cudaMemcpyFromSymbol(out, g_mmha_trace, sizeof(unsigned long long) * 4096 * 12);
-    int z = -want_launch;
-    cudaMemcpyToSymbol(g_mmha_launch, &z, sizeof(z));
-    return 0;
-}
-__device__ __forceinline__ unsigned long long mmha_globaltimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-#define MMHA_TRACE(slot)                                                                                               \
-    do {                                                                                                                   \
-        if (trace_on && threadIdx.x == 0) g_mmha_trace[trace_id][slot] = mmha_globaltimer();                               \
-    } while (0)
-#else
-#define MMHA_TRACE(slot) do { } while (0)
-#endif
-
 namespace tmb {
 namespace {
 
@@ -217,11 +192,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
     const int lane = tid & 31;
     const int g    = lane >> 2;
     const int c    = lane & 3;
-#ifdef TM_B200_GEMM_TRACE
-    const int  trace_id = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    const bool trace_on = *(volatile int*)&g_mmha_launch == 0 && trace_id < 4096;
-    MMHA_TRACE(0);
-#endif
 
     // `order`, `finished` and `lengths` are written by kernels earlier in the stream, but never by the
     // kernel directly ahead of this one (a GEMM), whose own wait has already covered them.  A CTA
@@ -317,8 +287,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
         cp_async_commit();
     }
 
-    MMHA_TRACE(1);   // first copies issued
-
     // ---------------------------------------------------------------- q (+k, v of the new token)
     // The rotation coefficients depend on the position only: they are taken from the table the decode driver fills
     // once per step (positions do not depend on layer or head), or worked out here, before the wait for the kernel
@@ -363,7 +331,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
             }
         }
     }
-    MMHA_TRACE(8);   // coefficients done
 
     // The cache rows requested above were written by earlier steps; q, k, v of the new token come
     // from the kernel before this one.
@@ -417,9 +384,7 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
             }
         }
     }
-    MMHA_TRACE(9);   // q, k, v staged by this thread
     __syncthreads();
-    MMHA_TRACE(10);
 
     // per-head sum of q (for a non-zero K zero point) and the new token's own score
     for (int h = warp; h < kHeadsPerCta; h += kWarps) {
@@ -447,7 +412,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
         }
     }
 
-    MMHA_TRACE(11);  // sums done
     __syncthreads();
 
     // ---------------------------------------------------------------- Q fragments, softmax state
@@ -483,11 +447,9 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
     }
 
     // ---------------------------------------------------------------- main loop over this warp's blocks
-    MMHA_TRACE(2);   // prologue done
     for (int blk = 0; blk < my_blocks; ++blk) {
         cp_async_wait<NSTAGE - 1>();   // block blk has landed; the NSTAGE - 1 blocks after it may still be on their way
         __syncwarp();
-        if (blk == 0) MMHA_TRACE(3);   // first block landed
         const int            stage = blk % NSTAGE;
         const unsigned char* ks    = my_ring + stage * 2 * TILEB;
         const unsigned char* vs    = ks + TILEB;
@@ -644,9 +606,7 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
         cp_async_commit();
     }
     cp_async_wait<0>();
-    MMHA_TRACE(4);   // warp 0 done with its blocks
     __syncthreads();
-    MMHA_TRACE(5);   // all warps done
 
     // ---------------------------------------------------------------- merge the warps (ring is free now)
     // part[w]: m[8] | l[8] | o[8 heads][128]   (fp32, real units)
@@ -756,15 +716,6 @@ __global__ void __launch_bounds__(W * 32, (INT8 ? 16 : 12) / W) mmha_decode_kern
             }
         }
     }
-#ifdef TM_B200_GEMM_TRACE
-    MMHA_TRACE(6);
-    if (trace_on && tid == 0) {
-        unsigned smid;
-        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-        g_mmha_trace[trace_id][7] = ((unsigned long long)smid << 32) | (unsigned)tlength;
-    }
-    if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) atomicAdd(&g_mmha_launch, 1);
-#endif
     if (n_split == 1) {
         return;
     }
