@@ -20,7 +20,7 @@
 // What bounds it.  With few tokens the bytes of a unit take 0.4 us, its expansion 0.5-0.55 (65 % of the issue slots; 375 warp
 // instructions per warp and unit, of which 208 unpack and scale).  Copies by the expanding warps (cp.async, 64-bit addresses) and
 // issuers that voted between the steps of a unit cost 82 more instructions and left the issuing lane, a chain of 1100 cycles a unit,
-// as the bound.  57344 x 8192, 21 / 64 tokens: 74 / 84 -> 59 / 75 us in a row of dependent launches (4.1 TB/s).
+// as the bound.  57344 x 8192, 16 / 64 tokens: 85 / 93 -> 67 / 76 us in a row of dependent launches over weights beyond the L2 (3.7 TB/s).
 // Partial tiles of CTAs that share a column tile meet in scratch memory; every CTA of the tile then
 // sums its own share of the feature rows in a fixed order.  Every wait is bounded.
 //

@@ -438,7 +438,8 @@ int window_attention_step(tm_handle* h, const WindowAttention& a, const MixerCal
     // Two CTAs fit an SM: no more splits than have a slot at once (16 sequences x 8 kv heads, 2177 keys, us with 1 / 2 / 3 / 4
     // splits: 47 / 49 / 59 / 55), and of these the number that leaves the busiest warp the fewest blocks for what a split
     // costs in the merge (one sequence with 1 / 2 / 4 / 8 / 16 / 32 splits: 43 / 33 / 27 / 25 / 25 / 29; a block takes a warp
-    // 0.62 us, the merge 2 and 0.12 a split; 200 keys: 16 unsplit, 18 with two or four).
+    // 0.62 us, the merge 2 and 0.12 a split; 200 keys: 16 unsplit, 18 with two or four).  The 0.62 is of an idle GPU, where it decides; with
+    // every SM at work the memory's rate bounds a block (16 sequences: 18 blocks a warp take 36 us), and `most` is what counts.
     const long long most = std::min<long long>(kMaxSplits, std::max(1ll, 2ll * h->sm_count / items));
     long long splits = 1;
     double    best   = 1e30;

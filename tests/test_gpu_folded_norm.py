@@ -90,8 +90,7 @@ class _Rows:
         self.keep += [emb, head] + norms
         self.want = norm(x, norms[-1])
 
-    def error(self, fold):
-        """The largest error of a row, relative to it"""
+    def hidden(self, fold):
         self.model.handle.set_option("fold_norm", fold)
         forced = self.ids.cpu().numpy()[None].astype(np.int32)
         with torch.cuda.stream(self.stream):
@@ -99,7 +98,11 @@ class _Rows:
             self.model.decode(st, 1, use_graph=False, stream=self.stream.cuda_stream)
             self.model.check_status(self.stream.cuda_stream)
         self.stream.synchronize()
-        return ((st.hidden.double() - self.want).norm(dim=1) / self.want.norm(dim=1)).max().item()
+        return st.hidden.clone()
+
+    def error(self, fold):
+        """The largest error of a row, relative to it"""
+        return ((self.hidden(fold).double() - self.want).norm(dim=1) / self.want.norm(dim=1)).max().item()
 
 
 @pytest.mark.parametrize("rms", [5e-4, 2e-3, 0.02, 1.0, 50.0])
@@ -120,3 +123,20 @@ def test_rows_and_weights_whose_product_leaves_the_range(batch, rms, weight, jum
     folded, separate = s.error(1), s.error(0)
     s.model.close()
     assert separate < 0.01 and folded <= 1.1 * separate + 2.0 ** -14, (folded, separate)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("batch", [2, 20])
+def test_a_row_that_is_not_finite_stays_alone(batch, value):
+    """An embedding with such a value makes its own row NaN and leaves the others' bits as they were."""
+    s = _Rows(batch, 1.0, batch)
+    emb = s.keep[-7]
+    assert emb.shape == (1000, 4096)
+    clean = s.hidden(1)
+    bad = s.ids == s.ids[0]
+    emb[s.ids[0], 5] = value
+    torch.cuda.synchronize()
+    spoilt, separate = s.hidden(1), s.hidden(0)
+    s.model.close()
+    assert spoilt[bad].isnan().all() and separate[bad].isnan().all()
+    assert torch.equal(spoilt[~bad], clean[~bad])
